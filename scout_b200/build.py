@@ -132,7 +132,7 @@ def build_reference(force: bool = False) -> None:
     """Compiles the reference's binaries from its own sources (checker only)."""
     script = os.path.join(ORACLE, "build_ref.sh")
     ref = reference_dir()
-    if not (os.path.exists(script) and os.path.isdir(ref)):
+    if not (os.path.exists(script) and os.path.isdir(os.path.join(ref, "src"))):
         return
     env = dict(os.environ, SCOUT_REFERENCE_DIR=ref, FORCE="1" if force else "0")
     r = subprocess.run(["bash", script], env=env, capture_output=True, text=True)
