@@ -77,8 +77,8 @@ typedef struct scout_sched {
     int64_t search_bound;     /* CC local-search bound (vertices); 0 = reference rule */
     int64_t search_limit;     /* CC: a class with more deletions left to search than this is
                                  recomputed instead (0 = 32; < 0 = always search)        */
-    int32_t blocks_per_sm;    /* persistent repair kernels: resident blocks per SM (1..4;
-                                 0 = as many as fit, at most 4)                          */
+    int32_t blocks_per_sm;    /* persistent repair kernels: 256-thread quarters of the one
+                                 block per SM (1..4; 0 = all four)                       */
     int32_t chunk_log2;       /* BFS queue item = 2^chunk_log2 row entries (8..13; 0 = 8,
                                  the best measured on a B200)                            */
     int32_t prefetched;       /* 1: this call's edits (same count, no ops) are the batch given

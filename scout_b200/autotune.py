@@ -2,8 +2,8 @@
 
 Knobs (all exact: they change speed, never results; every configuration's final solution is
 checksummed and the sweep fails if two differ):
-  blocks_per_sm     resident blocks per SM of the persistent repair kernels (1, 2, 4): more
-                    blocks hide latency, fewer make each grid barrier cheaper
+  blocks_per_sm     256-thread quarters of the persistent repair kernels' one block per SM
+                    (1, 2, 4): more threads hide latency, fewer synchronise faster
   chunk_log2        BFS queue item = 2^chunk_log2 row entries (8 .. 13): smaller items spread a
                     hub's row over more warps, larger ones cost fewer queue entries
   lanes_per_vertex  BFS: most lanes sharing one queue item when a round has fewer items than

@@ -53,12 +53,12 @@ int pin_grow(scout_ctx* c, void** p, int64_t* cap, int64_t need) {
     return SCOUT_OK;
 }
 
+// One block per SM.
 int coop_launch(scout_ctx* c, const void* fn, int threads, void** args, size_t smem) {
     int per_sm = 0;
     SCOUT_CU(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem));
     if (per_sm < 1) return c->fail(SCOUT_E_CUDA, "persistent kernel does not fit on an SM");
-    per_sm = std::min(per_sm, c->tune_blocks_per_sm > 0 ? c->tune_blocks_per_sm : 4);
-    dim3 grid((unsigned)(per_sm * c->sm_count)), block((unsigned)threads);
+    dim3 grid((unsigned)c->sm_count), block((unsigned)threads);
     // the grid barrier's arrival counter starts every launch at zero (its error flag persists
     // until the batch's counters are read)
     SCOUT_CU(c, cudaMemsetAsync(&c->d_bar->count, 0, sizeof(unsigned int), c->s_main));
@@ -319,7 +319,7 @@ static void fill_stats(scout_ctx* c, scout_batch_stats* st, int64_t launch0) {
 }
 
 // Common prologue of a batch: validation, counters, classification + merge of the edits.
-// Tuning knobs of a call: persistent-kernel blocks per SM (1..4, 0 = as many as fit) and the
+// Tuning knobs of a call: 256-thread quarters of a persistent block (1..4, 0 = four) and the
 // BFS queue item size (2^8 .. 2^13 row entries, 0 = 2^8).
 static int apply_tuning(scout_ctx* c, const scout_sched& sd) {
     if (sd.blocks_per_sm < 0 || sd.blocks_per_sm > 4) return c->fail(SCOUT_E_INVALID, "blocks_per_sm must be 0..4");

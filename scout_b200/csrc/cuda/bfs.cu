@@ -26,9 +26,7 @@
 
 namespace scout {
 
-// At least four blocks per SM: the register budget this grants (64 per thread) holds the
-// kernel without spills (the unconstrained build spilled to local memory at 40 registers).
-__global__ void __launch_bounds__(BFS_THREADS, 4) k_bfs(BfsParams p) { bfs_body(p); }
+__global__ void __launch_bounds__(REPAIR_THREADS, 1) k_bfs(BfsParams p) { bfs_body(p); }
 
 
 // The kernel's parameters for the context's current batch (buffers ensured first).
@@ -70,7 +68,7 @@ static int bfs_launch(scout_ctx* c, int mode, const int* mode_dev, scout_batch_s
     BfsParams p;
     SCOUT_RC(bfs_params(c, mode, mode_dev, &p));
     void* args[] = {&p};
-    return coop_launch(c, (const void*)k_bfs, BFS_THREADS, args, 0);
+    return coop_launch(c, (const void*)k_bfs, repair_threads(c), args, 0);
 }
 
 int bfs_repair(scout_ctx* c, int mode, const int* mode_dev, scout_batch_stats* st) {

@@ -7,7 +7,6 @@
 
 namespace scout {
 
-constexpr int BFS_THREADS = 256;
 constexpr int PSCAN = 4;   // row entries per lane and step in the seed scan
 
 struct BfsParams {
@@ -428,8 +427,6 @@ static __device__ bool full_bfs(const BfsParams& p, int mode, long long& bytes, 
     return true;
 }
 
-// At least four blocks per SM: the register budget this grants (64 per thread) holds the
-// kernel without spills (the unconstrained build spilled to local memory at 40 registers).
 __device__ __forceinline__ void bfs_body(const BfsParams& p) {
     const int W = gwarp_count();
     const int wid = gwarp_id();

@@ -27,7 +27,7 @@
 
 namespace scout {
 
-__global__ void __launch_bounds__(CC_THREADS) k_cc(CcParams p) { cc_body(p); }
+__global__ void __launch_bounds__(REPAIR_THREADS, 1) k_cc(CcParams p) { cc_body(p); }
 
 
 __global__ void k_cc_init(int32_t* __restrict__ uf, int32_t* __restrict__ cnt, int32_t* __restrict__ newmin,
@@ -108,7 +108,7 @@ static int cc_launch(scout_ctx* c, const scout_sched* sched, int variant, const 
         attr_done.fetch_or(bit);
     }
     void* args[] = {&p};
-    return coop_launch(c, (const void*)k_cc, CC_THREADS, args, CC_SMEM);
+    return coop_launch(c, (const void*)k_cc, repair_threads(c), args, CC_SMEM);
 }
 
 int cc_repair(scout_ctx* c, const scout_sched* sched, int variant, const int* mode_dev, scout_batch_stats* st) {

@@ -7,7 +7,6 @@
 
 namespace scout {
 
-constexpr int CC_THREADS = 256;
 constexpr int CC_HCAP = 8192;     // shared hash-set slots per side
 constexpr int CC_FCAP = 4096;     // frontier capacity
 constexpr int CC_MAX_BOUND = 4000;
@@ -117,15 +116,15 @@ static __device__ int cc_search(const CcParams& p, int32_t u, int32_t v, int32_t
         if (rv.len < ru.len) { Row tmp = ru; ru = rv; rv = tmp; }
         const int32_t* a = p.g.pool + ru.start;
         const int32_t* b = p.g.pool + rv.start;
-        for (int i = t; i < ru.len && !ld_volatile(&s_met); i += CC_THREADS) {
+        for (int i = t; i < ru.len && !ld_volatile(&s_met); i += (int)blockDim.x) {
             long long k = lower_bound_i32(b, rv.len, a[i]);
             if (k < rv.len && b[k] == a[i]) s_met = 1;
         }
-        bytes += 4LL * ((ru.len + CC_THREADS - 1 - t) / CC_THREADS) * 8;
+        bytes += 4LL * ((ru.len + (int)blockDim.x - 1 - t) / (int)blockDim.x) * 8;
     }
     __syncthreads();
     if (s_met) return 0;
-    for (int i = t; i < 2 * CC_HCAP; i += CC_THREADS) sm[i] = -1;
+    for (int i = t; i < 2 * CC_HCAP; i += (int)blockDim.x) sm[i] = -1;
     __syncthreads();
     __shared__ long long s_vol[2], s_nvol;
     if (t == 0) {
@@ -151,7 +150,7 @@ static __device__ int cc_search(const CcParams& p, int32_t u, int32_t v, int32_t
         if (t == 0) { s_nn = 0; s_nvol = 0; }
         __syncthreads();
         // warp per frontier vertex, lanes over its row
-        for (int i = t / WARP; i < fn; i += CC_THREADS / WARP) {
+        for (int i = t / WARP; i < fn; i += (int)blockDim.x / WARP) {
             int32_t x = fr[sd][i];
             Row r = p.g.row[x];
             const int32_t* rw = p.g.pool + r.start;
@@ -185,7 +184,7 @@ static __device__ int cc_search(const CcParams& p, int32_t u, int32_t v, int32_t
         if (s_met) return 0;
         if (s_over) return 2;
         const int nn = s_nn;
-        for (int i = t; i < nn; i += CC_THREADS) fr[sd][i] = nf[i];
+        for (int i = t; i < nn; i += (int)blockDim.x) fr[sd][i] = nf[i];
         __syncthreads();
         if (t == 0) { s_fn[sd] = nn; s_vol[sd] = s_nvol; }
         __syncthreads();
@@ -196,7 +195,7 @@ static __device__ int cc_search(const CcParams& p, int32_t u, int32_t v, int32_t
     __shared__ long long s_off;
     if (t == 0) { s_size = 0; s_min = INT32_MAX; }
     __syncthreads();
-    for (int i = t; i < CC_HCAP; i += CC_THREADS) {
+    for (int i = t; i < CC_HCAP; i += (int)blockDim.x) {
         int32_t x = hs[ex][i];
         if (x >= 0) { atomicAdd(&s_size, 1); atomicMin(&s_min, x); }
     }
@@ -221,7 +220,7 @@ static __device__ int cc_search(const CcParams& p, int32_t u, int32_t v, int32_t
         __shared__ int s_w;
         if (t == 0) s_w = 0;
         __syncthreads();
-        for (int i = t; i < CC_HCAP; i += CC_THREADS) {
+        for (int i = t; i < CC_HCAP; i += (int)blockDim.x) {
             int32_t x = hs[ex][i];
             if (x >= 0) p.side[s_off + atomicAdd(&s_w, 1)] = x;
         }
@@ -486,10 +485,10 @@ __device__ __forceinline__ void cc_body(const CcParams& p) {
             __shared__ int32_t s_key[2048];
             __shared__ int s_cnt[2048];
             __shared__ unsigned long long s_best;
-            for (int i = threadIdx.x; i < 2048; i += CC_THREADS) { s_key[i] = -1; s_cnt[i] = 0; }
+            for (int i = threadIdx.x; i < 2048; i += (int)blockDim.x) { s_key[i] = -1; s_cnt[i] = 0; }
             if (threadIdx.x == 0) s_best = 0;
             __syncthreads();
-            for (int i = threadIdx.x; i < 4096; i += CC_THREADS) {
+            for (int i = threadIdx.x; i < 4096; i += (int)blockDim.x) {
                 int64_t v = (int64_t)(((unsigned long long)i * 2654435761ull) % (unsigned long long)n);
                 int32_t r = ld_volatile(p.vp + v);
                 if (r < 0) continue;
@@ -501,7 +500,7 @@ __device__ __forceinline__ void cc_body(const CcParams& p) {
                 }
             }
             __syncthreads();
-            for (int i = threadIdx.x; i < 2048; i += CC_THREADS)
+            for (int i = threadIdx.x; i < 2048; i += (int)blockDim.x)
                 if (s_cnt[i] > 0)
                     atomicMax(&s_best, ((unsigned long long)s_cnt[i] << 32) | (uint32_t)s_key[i]);
             __syncthreads();
@@ -548,7 +547,7 @@ __device__ __forceinline__ void cc_body(const CcParams& p) {
             const int32_t v = p.side[i];
             Row r = p.g.row[v];
             const int32_t* rw = p.g.pool + r.start;
-            for (long long k = AF_FIRST + threadIdx.x; k < r.len; k += CC_THREADS) {
+            for (long long k = AF_FIRST + threadIdx.x; k < r.len; k += blockDim.x) {
                 int32_t w = rw[k];
                 if (ld_volatile(p.vp + w) < 0) atomicExch(&p.ctr->pad, 1);
                 else uf_union(p.vp, v, w);

@@ -17,7 +17,7 @@
 
 namespace scout {
 
-__global__ void __launch_bounds__(COL_THREADS) k_coloring(ColParams p) { coloring_body(p); }
+__global__ void __launch_bounds__(REPAIR_THREADS, 1) k_coloring(ColParams p) { coloring_body(p); }
 
 
 __global__ void k_fill_marker(int32_t* __restrict__ m, int64_t n) {
@@ -65,7 +65,7 @@ int coloring_repair(scout_ctx* c, scout_batch_stats* st) {
     ColParams p;
     SCOUT_RC(coloring_params(c, &p));
     void* args[] = {&p};
-    return coop_launch(c, (const void*)k_coloring, COL_THREADS, args, 0);
+    return coop_launch(c, (const void*)k_coloring, repair_threads(c), args, 0);
 }
 
 }  // namespace scout

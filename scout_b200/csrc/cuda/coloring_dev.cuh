@@ -7,7 +7,6 @@
 
 namespace scout {
 
-constexpr int COL_THREADS = 256;
 constexpr int COL_WIN = 1024;            // colours per bitmap window
 constexpr int COL_WORDS = COL_WIN / 32;
 constexpr int COL_BIG = 4096;            // rows longer than this are processed by a whole block
@@ -66,8 +65,8 @@ static __device__ int smallest_free(const ColParams& p, int32_t x, int tid, int 
 }
 
 __device__ __forceinline__ void coloring_body(const ColParams& p) {
-    __shared__ unsigned s_bm[COL_THREADS / WARP][COL_WORDS];
-    __shared__ int s_res[COL_THREADS / WARP];
+    __shared__ unsigned s_bm[REPAIR_THREADS / WARP][COL_WORDS];
+    __shared__ int s_res[REPAIR_THREADS / WARP];
     __shared__ unsigned s_bbm[COL_WORDS];
     __shared__ int s_bres;
     __shared__ int s_flag;
@@ -118,7 +117,7 @@ __device__ __forceinline__ void coloring_body(const ColParams& p) {
         for (int i = blockIdx.x; i < cnt; i += gridDim.x) {   // longer rows: one block
             int32_t x = p.list[cur][i];
             if (p.g.row[x].len <= COL_BIG) continue;
-            int c = smallest_free(p, x, threadIdx.x, COL_THREADS, s_bbm, BlockSync(), &s_bres, bytes);
+            int c = smallest_free(p, x, threadIdx.x, (int)blockDim.x, s_bbm, BlockSync(), &s_bres, bytes);
             if (threadIdx.x == 0) { p.prop[i] = c; p.marker[x] = c; }
             __syncthreads();
         }
@@ -152,11 +151,11 @@ __device__ __forceinline__ void coloring_body(const ColParams& p) {
             int c = p.prop[i];
             if (threadIdx.x == 0) s_flag = 0;
             __syncthreads();
-            for (long long k = threadIdx.x; k < r.len; k += COL_THREADS) {
+            for (long long k = threadIdx.x; k < r.len; k += blockDim.x) {
                 int32_t w = rw[k];
                 if (w < x && ld_volatile(p.marker + w) == c) s_flag = 1;
             }
-            bytes += 8LL * ((r.len + COL_THREADS - 1 - threadIdx.x) / COL_THREADS);
+            bytes += 8LL * ((r.len + (int)blockDim.x - 1 - (int)threadIdx.x) / (int)blockDim.x);
             __syncthreads();
             if (threadIdx.x == 0 && s_flag) p.list[nxt][atomicAdd(&p.ctr->list_count[nxt], 1)] = x;
             __syncthreads();

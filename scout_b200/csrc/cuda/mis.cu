@@ -15,7 +15,7 @@
 
 namespace scout {
 
-__global__ void __launch_bounds__(MIS_THREADS) k_mis(MisParams p) { mis_body(p); }
+__global__ void __launch_bounds__(REPAIR_THREADS, 1) k_mis(MisParams p) { mis_body(p); }
 
 
 // The kernel's parameters for the context's current batch (buffers ensured first).
@@ -44,7 +44,7 @@ int mis_repair(scout_ctx* c, scout_batch_stats* st) {
     MisParams p;
     SCOUT_RC(mis_params(c, &p));
     void* args[] = {&p};
-    return coop_launch(c, (const void*)k_mis, MIS_THREADS, args, 0);
+    return coop_launch(c, (const void*)k_mis, repair_threads(c), args, 0);
 }
 
 }  // namespace scout

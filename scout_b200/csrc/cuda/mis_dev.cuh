@@ -7,8 +7,6 @@
 
 namespace scout {
 
-constexpr int MIS_THREADS = 256;
-
 struct MisParams {
     DGraph g;
     int32_t* mis;

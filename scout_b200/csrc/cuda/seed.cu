@@ -18,7 +18,7 @@
 
 namespace scout {
 
-constexpr int SEED_THREADS = 256;
+constexpr int SEED_THREADS = 1024;
 constexpr int32_t UNDECIDED = -1;
 
 struct SeedParams {
@@ -35,7 +35,7 @@ __device__ __forceinline__ int lower_prefix(const int32_t* r, int len, int32_t v
     return (int)lower_bound_i32(r, len, v);
 }
 
-__global__ void __launch_bounds__(SEED_THREADS) k_seed_greedy(SeedParams p) {
+__global__ void __launch_bounds__(SEED_THREADS, 1) k_seed_greedy(SeedParams p) {
     const int64_t n = p.g.n;
     const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     const int64_t T = (int64_t)gridDim.x * blockDim.x;

@@ -8,7 +8,7 @@
 // MIS store's, each over its own store and work queues, with its own counters and its own
 // bounded grid barrier (zeroed before the launch). Every block takes part in every repair, so
 // each repair sees the same grid as when launched alone; the kernel's register count is the
-// largest of the four bodies', within the four-blocks-per-SM budget all four already meet.
+// largest of the four bodies', within the 64 per thread a 1,024-thread block allows.
 #include "ctx.cuh"
 #include "bfs_dev.cuh"
 #include "cc_dev.cuh"
@@ -21,11 +21,6 @@
 
 namespace scout {
 
-constexpr int UNION_THREADS = 256;
-static_assert(BFS_THREADS == UNION_THREADS && CC_THREADS == UNION_THREADS && COL_THREADS == UNION_THREADS &&
-                  MIS_THREADS == UNION_THREADS,
-              "the fused repair runs every body with the same block size");
-
 struct UnionRound {
     int has_bfs, has_cc, has_col, has_mis;
     BfsParams bfs;
@@ -34,7 +29,7 @@ struct UnionRound {
     MisParams mis;
 };
 
-__global__ void __launch_bounds__(UNION_THREADS, 4) k_union_round(UnionRound u) {
+__global__ void __launch_bounds__(REPAIR_THREADS, 1) k_union_round(UnionRound u) {
     if (u.has_bfs) bfs_body(u.bfs);
     if (u.has_cc) cc_body(u.cc);
     if (u.has_col) coloring_body(u.col);
@@ -78,14 +73,14 @@ int union_launch(scout_ctx* const* cs, const int* problems, const scout_sched* s
             attr_done.fetch_or(bit);
         }
     }
+    const int threads = repair_threads(c0);
     int per_sm = 0;
-    SCOUT_CU(c0, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_union_round, UNION_THREADS, smem));
+    SCOUT_CU(c0, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_union_round, threads, smem));
     if (per_sm < 1) return c0->fail(SCOUT_E_CUDA, "fused repair kernel does not fit on an SM");
-    per_sm = std::min(per_sm, c0->tune_blocks_per_sm > 0 ? c0->tune_blocks_per_sm : 4);
     void* args[] = {&u};
     SCOUT_CU(c0, cudaEventRecord(c0->ev_t[4], c0->s_main));
-    SCOUT_CU(c0, cudaLaunchCooperativeKernel((const void*)k_union_round, dim3((unsigned)(per_sm * c0->sm_count)),
-                                             dim3(UNION_THREADS), args, smem, c0->s_main));
+    SCOUT_CU(c0, cudaLaunchCooperativeKernel((const void*)k_union_round, dim3((unsigned)c0->sm_count),
+                                             dim3((unsigned)threads), args, smem, c0->s_main));
     SCOUT_CU(c0, cudaEventRecord(c0->ev_t[5], c0->s_main));
     c0->nlaunch += 1;
     SCOUT_CU(c0, cudaEventRecord(c0->ev_union, c0->s_main));
