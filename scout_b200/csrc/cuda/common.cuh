@@ -22,6 +22,14 @@ struct __align__(16) Row {
     int cap;           // reserved elements at start (>= len)
 };
 
+// One affected row of a batch's merge: its old version, where the new one goes (the same place
+// for a row compacted where it lies), and its half-edits [b, d) insertions, [d, e) deletions.
+struct __align__(16) MergeRow {
+    long long start, dst;
+    int len;
+    int b, d, e;
+};
+
 // Device-resident graph handle passed by value to kernels.
 struct DGraph {
     const Row* row;

@@ -19,7 +19,8 @@ struct DevCounters {
     int n_half;         // applied half-edits (2 per applied edit)
     int n_aff;          // vertices whose row changed
     int n_small, n_large;     // rows of the short-row merge / long rows compacted in place
-    int n_slices, n_pad;      // merge slices
+    int n_slices, n_long;     // merge slices / rows they belong to
+    int plan_ticket, merge_ticket;   // tiles of the plan, items of the merge handed out so far
     long long new_elems;      // elements written to the pool this batch (HBM part when split)
     long long new_elems_host; // tiered store, split batch: elements written to the host pool
     long long nnz_delta;      // inserted minus deleted entries
@@ -48,8 +49,7 @@ struct DevCounters {
     int sched_del;            // deletion half-edits
     int decision;             // repair variant the kernels run (read on the device)
     int sort_err;             // 1: a sort look-back wait timed out, 2: a sort position out of range,
-                              // 3: a bulk copy into shared memory (row merge) did not complete,
-                              // 4: a scan look-back wait timed out
+                              // 4: a look-back wait of a scan or of the merge plan timed out
     int sched_flags;          // 1 features computed, 2 model applied
     float feat[24];
     float pred[4];
@@ -132,8 +132,7 @@ struct scout_ctx {
     int32_t* stamp_b = nullptr;
     int32_t* stamp_c = nullptr;
     int32_t* stamp_d = nullptr;
-    int32_t* aux_v = nullptr;     // per-vertex int scratch (marker / uf parent)
-    int32_t* aux_w = nullptr;
+    int32_t* aux_v = nullptr;     // per-vertex int scratch (label canonicalisation)
     uint32_t epoch = 0;
 
     // ---- per-batch workspace: one allocation, carved per batch size (grow-only) ----
@@ -146,15 +145,12 @@ struct scout_ctx {
     unsigned long long* d_keys = nullptr;       // half-edit keys (2m)
     unsigned long long* d_keys_alt = nullptr;   // radix ping-pong (2m)
     unsigned long long* d_hkeys = nullptr;      // sorted half-edits of the current batch
-    long long* d_mdp = nullptr;     // matched-deletion prefix, aligned with keys (2m)
+    long long* d_mdp = nullptr;     // matched deletions before every half-edit (2m int32; room for 2m int64)
     int32_t* d_aff = nullptr;       // affected vertex ids (2m)
-    int64_t* d_aff_seg = nullptr;   // [3 * 2m]: segment begin, first deletion, end
-    int64_t* d_aff_len = nullptr;   // new length, then exclusive offsets (2m + 1)
-    int64_t* d_aff_len2 = nullptr;  // tiered split batches: lengths / offsets of the host rows (2m + 1)
-    int32_t* d_aff_small = nullptr; // affected rows merged by the short-row merge (2m)
-    int32_t* d_aff_long = nullptr;  // long affected rows compacted in place (2m)
-    int64_t* d_small_off = nullptr; // short-row lengths, then their exclusive scan (2m + 1)
-    scout::Row* d_old_row = nullptr;   // descriptors of the affected rows before the batch (2m)
+    int32_t* d_seg_b = nullptr;     // their segments' begins in the half-edits (2m + 1)
+    int32_t* d_seg_d = nullptr;     // their segments' first deletions (2m)
+    int32_t* d_longs = nullptr;     // long affected rows compacted in place (2m)
+    scout::MergeRow* d_mrow = nullptr;   // merge records: short rows from the front, others from the back (2m)
     int64_t* d_slices = nullptr;  int64_t cap_slices = 0;   // merge items (row << 32 | slice)
     int64_t* d_coff = nullptr;      // compaction offsets (n + 1)
     int key_bits = 0;
@@ -258,6 +254,7 @@ int sort_keys(scout_ctx* c, unsigned long long* keys, unsigned long long* alt, i
 // scan.cu: exclusive scan of int64 values in place; *total receives the sum (device ptr or null)
 int scan_i64(scout_ctx* c, int64_t* data, int64_t n, int64_t* d_total);
 int sort_reserve(scout_ctx* c, int64_t nkeys);
+unsigned next_stamp();   // sort.cu: look-back stamps, unique across the process
 // graph.cu: every buffer a batch of up to m edits can grow, allocated now
 int graph_reserve_batch(scout_ctx* c, int64_t m);
 // problem scratch allocated on first use, or ahead of time by scout_reserve

@@ -15,18 +15,17 @@
 //                     (HybridGraph::isAdjacent, FlashGraph.h:356-366); emits two half-edit
 //                     keys (u, op, v) and (v, op, u) per applied edit
 //   sort_keys         groups half-edits by vertex; inserts before deletes; neighbours sorted
-//   k_seg_heads/tails affected-vertex list and its key segments
-//   k_row_alloc       old descriptor, new space (old length + insertions; none for a short
-//                     row that only loses entries), short-row list, slices of long rows
-//   scan_i64          new rows' offsets in the pool
-//   k_plan_match      per deletion: the old entry it cancels (multiset rule); matched flags
-//   scan_i64          matched deletions before every half-edit
-//   k_plan_place      per insertion: its final slot in the new row; per matched deletion: the
-//                     old entry's tombstone (sign bit); per row: the new descriptor
-//   k_merge_small     survivors of short rows, balanced groups of ~UNIT entries per warp
-//   k_merge_slices    survivors of longer rows, one warp per slice of SLICE entries, so a hub
-//                     row is spread over many warps
-//   k_merge_long_inplace  rows longer than a slice that only lose entries, a block per row
+//   k_plan            one pass over the sorted half-edits: one search of each in its old row (an
+//                     insertion's position, the old entry a deletion cancels by the multiset
+//                     rule), the affected rows and their segments, and the running count of
+//                     matched deletions (decoupled look-back)
+//   k_row_plan        per affected row: its new space (old length + insertions; none for a row
+//                     that only loses entries and is short), its new descriptor, its record in
+//                     the list of short rows or of slices of longer ones
+//   k_merge           the new rows: survivors and insertions of short rows (a few rows per warp)
+//                     and of slices of SLICE old entries (a warp each, so a hub row is spread
+//                     over many warps), positions taken from the sorted edit events
+//   k_merge_long_inplace  tiered store: rows longer than IN_PLACE_LEN that only lose entries
 #include "ctx.cuh"
 
 #include <algorithm>
@@ -34,18 +33,20 @@
 
 namespace scout {
 
-constexpr int SLICE = 4096;          // old-row entries streamed by one warp in the slice merge
-constexpr int SMALL_LEN = 128;       // rows up to this length go to the short-row merge
+constexpr int SLICE = 2048;          // old-row entries merged by one warp at a time
+constexpr int SMALL_LEN = 128;       // rows up to this length (and 32 half-edits) are short
+constexpr int IN_PLACE_LEN = 4096;   // longest deletion-only row compacted in place by one warp
 
 // A row whose half-edits are all deletions is rewritten in place: its survivors only move
-// towards the row start, it keeps its start and capacity, and it takes no pool space (short
-// rows in the short-row merge, rows of one slice by their warp in the slice merge). A longer
-// one is compacted in place by one block (k_merge_long_inplace: its slices would overlap) only
-// when `long_in_place` is set, in the tiered store, whose HBM room is scarce; in the all-HBM
-// store it is rewritten at the pool tail by the slice merge, spread over many warps.
+// towards the row start, it keeps its start and capacity, and it takes no pool space (one warp
+// merges the whole row). A longer one is compacted in place by one block (k_merge_long_inplace:
+// its slices would overlap) only when `long_in_place` is set, in the tiered store, whose HBM
+// room is scarce; in the all-HBM store it is rewritten at the pool tail, spread over many warps.
 __host__ __device__ __forceinline__ bool in_place_row(long long insertions, int old_len, bool long_in_place) {
-    return insertions == 0 && (old_len <= SLICE || long_in_place);
+    return insertions == 0 && (old_len <= IN_PLACE_LEN || long_in_place);
 }
+
+__device__ __forceinline__ bool in_hbm(const Row& r, long long cap) { return r.start >= 0 && r.start < cap; }
 
 // ---------------------------------------------------------------------------------------
 // Staging
@@ -163,350 +164,656 @@ __device__ __forceinline__ int32_t key_u(unsigned long long k, int B) { return (
 __device__ __forceinline__ int32_t key_v(unsigned long long k, int B) { return (int32_t)(k & ((1ull << B) - 1)); }
 __device__ __forceinline__ int key_op(unsigned long long k, int B) { return (int)((k >> B) & 1ull); }
 
-// Heads of vertex segments get an affected index; slot[u] remembers it for the tails.
-__global__ void k_seg_heads(const unsigned long long* __restrict__ keys, int B, DevCounters* __restrict__ ctr,
-                            int32_t* __restrict__ aff, int64_t* __restrict__ seg, int32_t* __restrict__ slot) {
-    const int64_t nh = ctr->n_half;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nh; i += (int64_t)gridDim.x * blockDim.x) {
-        int32_t u = key_u(keys[i], B);
-        bool head = i == 0 || key_u(keys[i - 1], B) != u;
-        int a = warp_append(head, &ctr->n_aff);
-        if (head) {
-            aff[a] = u;
-            seg[3 * (int64_t)a] = i;
-            slot[u] = a;
+constexpr int PLAN_THREADS = 256;
+constexpr int PLAN_WARPS = PLAN_THREADS / WARP;
+constexpr int PLAN_STEPS = 4;                          // half-edits per thread, their searches interleaved
+constexpr int PLAN_TILE = PLAN_THREADS * PLAN_STEPS;
+constexpr uint64_t PLAN_WAIT_LIMIT_NS = 1000000000ull;   // 1 s
+constexpr unsigned long long PLAN_TAG = 0x5Aull << 56;
+
+// One pass over the sorted half-edits. Each is searched once in its old row:
+//   insertion y   position = number of old entries <= y; it is placed before that entry
+//   deletion d    multiset rule: the r-th copy of d among a row's deletions cancels the r-th copy
+//                 of d in the old row (DeltaOverlay::removeEdge forgets one added copy or
+//                 tombstones the base edge, FlashGraph.h:236-243); position = the cancelled
+//                 entry, or the end of d's copies when none is left (not matched)
+// epos[k] = position << 1 | matched, non-decreasing along a row's insertions and along its
+// deletions; E[k] = matched deletions before half-edit k (E[n_half] the total); the affected
+// rows in id order with their segments (seg_b[a], seg_b[a + 1]) and first deletions seg_d[a].
+// The running counts of heads and matched deletions go from tile to tile by a decoupled
+// look-back (state: three words per tile, as in the single-pass scan).
+//
+// What bounds it: dependent reads of the binary searches (a thread keeps PLAN_STEPS searches
+// in flight, and neighbouring threads search the same rows). 10^6 edits at scale 22: 123 us; the
+// launches it replaces (segment heads and tails, two searches of every half-edit, a scan and its
+// clears) took 300 us, and on small batches most of their time was the seven launches.
+__global__ void __launch_bounds__(PLAN_THREADS) k_plan(const Row* __restrict__ row, const int32_t* __restrict__ pool,
+                                                       const unsigned long long* __restrict__ keys, int B,
+                                                       DevCounters* __restrict__ ctr, int32_t* __restrict__ aff,
+                                                       int32_t* __restrict__ seg_b, int32_t* __restrict__ seg_d,
+                                                       uint32_t* __restrict__ epos, int32_t* __restrict__ E,
+                                                       unsigned long long* __restrict__ st, unsigned stamp) {
+    __shared__ int s_tile;
+    __shared__ unsigned long long s_cnt[PLAN_WARPS];
+    __shared__ unsigned long long s_prefix;
+    const int nh = ctr->n_half;
+    const int w = threadIdx.x / WARP;
+    const unsigned l = lane_id();
+    if (threadIdx.x == 0) s_tile = atomicAdd(&ctr->plan_ticket, 1);
+    __syncthreads();
+    const int tile = s_tile;
+    const int k0 = tile * PLAN_TILE + w * (PLAN_STEPS * WARP) + (int)l;
+    if (tile * (long long)PLAN_TILE >= nh) return;   // whole block; no tile after it has work either
+    unsigned long long key[PLAN_STEPS];
+    const int32_t* O[PLAN_STEPS];
+    int lo[PLAN_STEPS], hi[PLAN_STEPS], len[PLAN_STEPS];
+#pragma unroll
+    for (int s = 0; s < PLAN_STEPS; s++) {
+        const int k = k0 + s * WARP;
+        key[s] = k < nh ? keys[k] : ~0ull;
+    }
+#pragma unroll
+    for (int s = 0; s < PLAN_STEPS; s++) {
+        lo[s] = hi[s] = len[s] = 0;
+        O[s] = pool;
+        if (k0 + s * WARP < nh) {
+            const Row r = row[key_u(key[s], B)];
+            O[s] = pool + r.start;
+            len[s] = hi[s] = r.len;
         }
     }
-}
-
-__global__ void k_seg_tails(const unsigned long long* __restrict__ keys, int B, const DevCounters* __restrict__ ctr,
-                            int64_t* __restrict__ seg, const int32_t* __restrict__ slot) {
-    const int64_t nh = ctr->n_half;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nh; i += (int64_t)gridDim.x * blockDim.x) {
-        int32_t u = key_u(keys[i], B);
-        bool tail = i == nh - 1 || key_u(keys[i + 1], B) != u;
-        if (tail) seg[3 * (int64_t)slot[u] + 2] = i + 1;
-        int op = key_op(keys[i], B);
-        bool first_del = op == 1 && (i == 0 || key_u(keys[i - 1], B) != u || key_op(keys[i - 1], B) == 0);
-        bool no_del_tail = tail && op == 0;
-        if (first_del) seg[3 * (int64_t)slot[u] + 1] = i;
-        else if (no_del_tail) seg[3 * (int64_t)slot[u] + 1] = i + 1;
+    // lower bounds, one step of every search per turn
+    while (true) {
+        bool more = false;
+        int32_t x[PLAN_STEPS];
+#pragma unroll
+        for (int s = 0; s < PLAN_STEPS; s++)
+            if (lo[s] < hi[s]) x[s] = O[s][(lo[s] + hi[s]) >> 1];
+#pragma unroll
+        for (int s = 0; s < PLAN_STEPS; s++)
+            if (lo[s] < hi[s]) {
+                const int mid = (lo[s] + hi[s]) >> 1;
+                if (x[s] < key_v(key[s], B)) lo[s] = mid + 1; else hi[s] = mid;
+                more |= lo[s] < hi[s];
+            }
+        if (!more) break;
+    }
+    unsigned hm[PLAN_STEPS], mm[PLAN_STEPS];
+#pragma unroll
+    for (int s = 0; s < PLAN_STEPS; s++) {
+        const int k = k0 + s * WARP;
+        bool matched = false, head = false;
+        if (k < nh) {
+            const unsigned long long kk = key[s];
+            const int32_t y = key_v(kk, B);
+            const unsigned long long pk = k > 0 ? keys[k - 1] : ~kk;
+            head = k == 0 || key_u(pk, B) != key_u(kk, B);
+            int at = lo[s];
+            const bool here = at < len[s] && O[s][at] == y;
+            if (key_op(kk, B) == 0) {
+                if (here) at += (int)upper_bound_i32(O[s] + at, len[s] - at, y);
+            } else {
+                int rank = 0;   // copies of this deletion before it
+                if (pk == kk) {
+                    int j = k - 1;
+                    while (j > 0 && keys[j - 1] == kk) j--;
+                    rank = k - j;
+                }
+                matched = here && at + rank < len[s] && O[s][at + rank] == y;
+                if (matched) at += rank;
+                else if (here) at += (int)upper_bound_i32(O[s] + at, len[s] - at, y);
+            }
+            epos[k] = ((uint32_t)at << 1) | (matched ? 1u : 0u);
+        }
+        hm[s] = __ballot_sync(0xffffffffu, head);
+        mm[s] = __ballot_sync(0xffffffffu, matched);
+    }
+    // heads << 32 | matched deletions: per warp, then before this tile
+    if (l == 0) {
+        unsigned long long c = 0;
+#pragma unroll
+        for (int s = 0; s < PLAN_STEPS; s++) c += ((unsigned long long)__popc(hm[s]) << 32) | (unsigned)__popc(mm[s]);
+        s_cnt[w] = c;
+    }
+    __syncthreads();
+    if (w == 0) {   // publish, look back 32 tiles per step, publish the prefix
+        unsigned long long tot = 0;
+        for (int j = 0; j < PLAN_WARPS; j++) tot += s_cnt[j];
+        const unsigned long long want = PLAN_TAG | ((unsigned long long)stamp << 2);
+        unsigned long long* me = st + 3 * (int64_t)tile;
+        unsigned long long prefix = 0;
+        if (tile > 0) {
+            if (l == 0) {
+                me[1] = tot;
+                __threadfence();
+                *(volatile unsigned long long*)me = want | 1ull;
+            }
+            const uint64_t t0 = globaltimer_ns();
+            for (int end = tile - 1;; end -= WARP) {
+                const int j = end - (int)l;           // lane 0 looks at the nearest tile
+                unsigned long long sw = want | 2ull;  // tiles before the first: a prefix of 0
+                bool ok = true;
+                if (j >= 0) {
+                    const unsigned long long* pj = st + 3 * (int64_t)j;
+                    sw = ld_volatile(pj);
+                    for (unsigned it = 1; (sw & ~3ull) != want || (sw & 3ull) == 0; it++) {
+                        if ((it & 63) == 0 && globaltimer_ns() - t0 > PLAN_WAIT_LIMIT_NS) { ok = false; break; }
+                        sw = ld_volatile(pj);
+                    }
+                }
+                if (!__all_sync(0xffffffffu, ok)) {
+                    if (l == 0) atomicCAS(&ctr->sort_err, 0, 4);
+                    break;
+                }
+                __threadfence();
+                const bool pre = (sw & 3ull) == 2;
+                unsigned long long v = 0;
+                if (j >= 0) v = ld_volatile(st + 3 * (int64_t)j + (pre ? 2 : 1));
+                const unsigned pm = __ballot_sync(0xffffffffu, pre);
+                const int f = pm ? __ffs(pm) - 1 : WARP;   // nearest tile with an inclusive prefix
+                if ((int)l > f) v = 0;
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                prefix += v;
+                if (pm) break;
+            }
+        }
+        if (l == 0) {
+            me[2] = prefix + tot;
+            __threadfence();
+            *(volatile unsigned long long*)me = want | 2ull;
+            s_prefix = prefix;
+        }
+    }
+    __syncthreads();
+    unsigned long long base = s_prefix;
+    for (int j = 0; j < w; j++) base += s_cnt[j];
+    int heads = (int)(base >> 32), match = (int)(base & 0xffffffffu);
+    const unsigned lt = (1u << l) - 1;
+#pragma unroll
+    for (int s = 0; s < PLAN_STEPS; s++) {
+        const int k = k0 + s * WARP;
+        if (k < nh) {
+            const unsigned long long kk = key[s];
+            const int32_t u = key_u(kk, B);
+            const bool head = (hm[s] >> l) & 1u;
+            const int a = heads + __popc(hm[s] & lt) + (head ? 1 : 0) - 1;
+            const int e = match + __popc(mm[s] & lt);
+            E[k] = e;
+            if (head) {
+                aff[a] = u;
+                seg_b[a] = k;
+            }
+            const int op = key_op(kk, B);
+            if (op == 1) {
+                if (head || key_op(keys[k - 1], B) == 0) seg_d[a] = k;
+            } else if (k == nh - 1 || key_u(keys[k + 1], B) != u) {
+                seg_d[a] = k + 1;
+            }
+            if (k == nh - 1) {
+                E[nh] = e + (int)((mm[s] >> l) & 1u);
+                seg_b[a + 1] = nh;
+                ctr->n_aff = a + 1;
+            }
+        }
+        heads += __popc(hm[s]);
+        match += __popc(mm[s]);
     }
 }
 
-// Deletion keys are read as neighbour ids through this view.
-struct KeySpan {
-    const unsigned long long* k;
-    int B;
-    __device__ __forceinline__ int32_t operator[](long long i) const { return key_v(k[i], B); }
+// Per affected row: the space of its new version (old length + insertions: slots of matched
+// deletions stay unused until the next compaction), its new descriptor and its merge record.
+// Space and list slots are taken by one set of atomics per block (the order of rows in the pool
+// does not matter).
+constexpr int ROW_THREADS = 256;
+
+struct RowPlan {
+    Row* row;
+    DevCounters* ctr;
+    const int32_t* aff;
+    const int32_t* seg_b;
+    const int32_t* seg_d;
+    const int32_t* E;
+    MergeRow* mrow;        // short rows from the front, the others from the back
+    int64_t mcap;
+    int64_t* slices;       // (record << 32 | slice)
+    int64_t slice_cap;
+    int32_t* longs;        // records of long rows compacted in place
+    bool long_in_place;
+    bool split;            // rows whose old version is not in HBM go to the second destination
+    long long hbm_cap;     // in HBM: 0 <= start < hbm_cap
+    long long base_hbm, base_host;
 };
-template <typename S>
-__device__ __forceinline__ long long lb_span(S s, long long n, int32_t x) {
-    long long lo = 0, hi = n;
-    while (lo < hi) { long long mid = (lo + hi) >> 1; if (s[mid] < x) lo = mid + 1; else hi = mid; }
-    return lo;
-}
-template <typename S>
-__device__ __forceinline__ long long ub_span(S s, long long n, int32_t x) {
-    long long lo = 0, hi = n;
-    while (lo < hi) { long long mid = (lo + hi) >> 1; if (s[mid] <= x) lo = mid + 1; else hi = mid; }
-    return lo;
-}
 
-__device__ __forceinline__ long long warp_lower_bound(const int64_t* a, long long n, long long x) {
-    // first i in [0, n) with a[i] >= x (n if none), 32 probes per step (all lanes call)
-    long long lo = 0, hi = n;
-    while (hi - lo > WARP) {
-        const long long step = (hi - lo + WARP - 1) / WARP;
-        const long long pos = lo + (long long)lane_id() * step;
-        const bool less = pos < hi && a[pos] < x;
-        const int c = __popc(__ballot_sync(0xffffffffu, less));   // probes below x form a prefix
-        const long long nlo = c == 0 ? lo : lo + (long long)(c - 1) * step + 1;
-        const long long nhi = c == 0 ? lo : min(hi, lo + (long long)c * step);
-        lo = nlo;
-        hi = max(nlo, nhi);
-        if (c == 0) break;
+__device__ __forceinline__ long long block_scan_rows(long long x, long long* total) {
+    __shared__ long long ws[ROW_THREADS / WARP];
+    const long long inc = warp_incl_scan(x);
+    const int w = threadIdx.x / WARP;
+    __syncthreads();   // the previous scan's sums are read
+    if (lane_id() == WARP - 1) ws[w] = inc;
+    __syncthreads();
+    long long before = 0, tot = 0;
+#pragma unroll
+    for (int j = 0; j < ROW_THREADS / WARP; j++) {
+        before += j < w ? ws[j] : 0;
+        tot += ws[j];
     }
-    const long long pos = lo + lane_id();
-    const bool less = pos < hi && a[pos] < x;
-    return lo + __popc(__ballot_sync(0xffffffffu, less));
+    *total = tot;
+    return before + inc - x;
 }
 
-// Per affected row: its descriptor before the batch and the space of its new row (old length
-// + insertions: slots of matched deletions stay unused until the next compaction). Rows up
-// to SMALL_LEN entries go to the short-row merge, longer ones are cut into merge slices
-// (rows past one slice that only lose entries go to the in-place block merge instead).
-__global__ void k_row_alloc(const Row* __restrict__ row, DevCounters* __restrict__ ctr, const int32_t* __restrict__ aff,
-                            const int64_t* __restrict__ seg, Row* __restrict__ old_row, int64_t* __restrict__ alloc,
-                            int32_t* __restrict__ small, int64_t* __restrict__ small_len, int64_t* __restrict__ slices,
-                            int64_t slice_cap, int32_t* __restrict__ longs, bool long_in_place) {
-    const int A = ctr->n_aff;
-    const int T = gridDim.x * blockDim.x;
-    for (int b = (int)(blockIdx.x * blockDim.x + threadIdx.x) - (int)lane_id(); b < A; b += T) {
-        const int a = b + (int)lane_id();
-        const bool ok = a < A;
-        int ns = 0;
-        bool sm = false, lip = false;
-        if (ok) {
-            const long long b0 = seg[3 * (int64_t)a], sp = seg[3 * (int64_t)a + 1];
-            const Row r = row[aff[a]];
-            old_row[a] = r;
-            const bool ip = in_place_row(sp - b0, r.len, long_in_place);
-            alloc[a] = ip ? 0 : (long long)r.len + (sp - b0);
-            sm = r.len <= SMALL_LEN;
-            lip = ip && r.len > SLICE;   // longer than a slice, compacted in place: one block
-            ns = sm || lip ? 0 : (r.len + SLICE - 1) / SLICE;
-        }
-        const int lat = warp_append(lip, &ctr->n_large);
-        if (lip) longs[lat] = a;
-        const int at = warp_append(ok && sm, &ctr->n_small);
-        if (ok && sm) {
-            small[at] = a;
-            small_len[at] = old_row[a].len;   // the merge balances its groups by old length
-        }
-        const int inc = warp_incl_scan_i(ns);
-        int base = 0;
-        if (lane_id() == WARP - 1 && inc) base = atomicAdd(&ctr->n_slices, inc);
-        base = __shfl_sync(0xffffffffu, base, WARP - 1);
-        const long long s0 = (long long)base + inc - ns;
-        if (s0 + ns > slice_cap) { if (ns) atomicExch(&ctr->overflow, 1); continue; }
-        for (int s = 0; s < ns; s++) slices[s0 + s] = ((long long)a << 32) | s;
-    }
-}
-
-// Searches of an old row whose cancelled entries may already carry the tombstone bit (the
-// sign bit, so the masked values stay sorted while the row is being marked).
-__device__ __forceinline__ int32_t unmark(int32_t x) { return x & 0x7fffffff; }
-__device__ __forceinline__ long long ub_masked(const int32_t* a, long long n, int32_t x) {
-    long long lo = 0, hi = n;
-    while (lo < hi) { long long mid = (lo + hi) >> 1; if (unmark(a[mid]) <= x) lo = mid + 1; else hi = mid; }
-    return lo;
-}
-
-// Plan, step 1: one thread per half-edit. Multiset rule: the r-th copy of d among a row's
-// deletions cancels the r-th copy of d in the old row (DeltaOverlay::removeEdge forgets one
-// added copy or tombstones the base edge, FlashGraph.h:236-243). A deletion records dpos =
-// (at << 1) | matched, with at the cancelled entry, or the end of d's copies when none is
-// left, so dpos is non-decreasing along a row's sorted deletions; flag = matched (0 for
-// insertions and for the unused tail up to H) feeds one exclusive scan over all half-edits.
-__global__ void k_plan_match(const int32_t* __restrict__ pool, const unsigned long long* __restrict__ keys, int B,
-                             const DevCounters* __restrict__ ctr, const int32_t* __restrict__ slot,
-                             const int64_t* __restrict__ seg, const Row* __restrict__ old_row,
-                             long long* __restrict__ dpos, long long* __restrict__ flag, long long H) {
-    const long long nh = ctr->n_half;
-    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < H; k += (long long)gridDim.x * blockDim.x) {
-        const unsigned long long key = k < nh ? keys[k] : 0ull;
-        long long f = 0;
-        if (k < nh && key_op(key, B) == 1) {
-            const int a = slot[key_u(key, B)];
-            const long long sp = seg[3 * (int64_t)a + 1], e0 = seg[3 * (int64_t)a + 2];
-            const int32_t d = key_v(key, B);
-            long long rank = 0;
-            if (k > sp && key_v(keys[k - 1], B) == d) rank = k - (sp + lb_span(KeySpan{keys + sp, B}, e0 - sp, d));
-            const Row r = old_row[a];
-            const int32_t* O = pool + r.start;
-            const long long lo = lower_bound_i32(O, r.len, d);
-            const bool matched = lo + rank < r.len && O[lo + rank] == d;
-            const long long at = matched ? lo + rank : lo + upper_bound_i32(O + lo, r.len - lo, d);
-            dpos[k] = (at << 1) | (matched ? 1 : 0);
-            f = matched ? 1 : 0;
-        }
-        flag[k] = f;
-    }
-}
-
-// Plan, step 2 (after the scan: E[k] = matched deletions before half-edit k): one thread per
-// half-edit. An insertion y (j-th of its row) lands at j + #old <= y - #cancelled <= y of the
-// new row and is written there; a matched deletion tombstones its old entry; the first
-// half-edit of a row writes the row's new descriptor.
-__global__ void k_plan_place(int32_t* __restrict__ pool, Row* __restrict__ row, const unsigned long long* __restrict__ keys,
-                             int B, DevCounters* __restrict__ ctr, const int32_t* __restrict__ slot,
-                             const int64_t* __restrict__ seg, const Row* __restrict__ old_row,
-                             const int64_t* __restrict__ off, long long tail, const long long* __restrict__ dpos,
-                             const long long* __restrict__ E, bool long_in_place) {
-    const long long nh = ctr->n_half;
-    long long nnz_delta = 0, bytes = 0;
-    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < nh; k += (long long)gridDim.x * blockDim.x) {
-        const unsigned long long key = keys[k];
-        const int32_t u = key_u(key, B);
-        const int a = slot[u];
-        const long long b0 = seg[3 * (int64_t)a], sp = seg[3 * (int64_t)a + 1], e0 = seg[3 * (int64_t)a + 2];
-        const Row r = old_row[a];
-        int32_t* O = pool + r.start;
-        if (k < sp) {
-            const int32_t y = key_v(key, B);
-            const long long ubo = ub_masked(O, r.len, y);
-            const long long ubd = ub_span(KeySpan{keys + sp, B}, e0 - sp, y);
-            const long long del = E[sp + ubd] - E[sp];
-            pool[tail + off[a] + (k - b0) + ubo - del] = y;
-        } else {
-            const long long dp = dpos[k];
-            if (dp & 1) O[dp >> 1] = key_v(key, B) | (int32_t)0x80000000;
-        }
-        if (k == b0) {
-            const long long p = sp - b0, q = e0 - sp;
-            const long long nl = (long long)r.len + p - (E[e0] - E[sp]);
-            row[u] = in_place_row(p, r.len, long_in_place) ? Row{r.start, (int)nl, r.cap}
-                                            : Row{tail + off[a], (int)nl, (int)(r.len + p)};
-            nnz_delta += nl - r.len;
-            bytes += 4 * (r.len + nl) + 8 * (p + q) + 16;
-        }
+// Tiered store: the growth of each destination, before anything is placed.
+__global__ void __launch_bounds__(ROW_THREADS) k_row_sizes(RowPlan p) {
+    const int A = p.ctr->n_aff;
+    long long nh = 0, nc = 0;
+    for (int a = blockIdx.x * ROW_THREADS + threadIdx.x; a < A; a += gridDim.x * ROW_THREADS) {
+        const Row r = p.row[p.aff[a]];
+        const int ins = p.seg_d[a] - p.seg_b[a];
+        if (in_place_row(ins, r.len, p.long_in_place)) continue;
+        if (p.split && !in_hbm(r, p.hbm_cap)) nc += (long long)r.len + ins;
+        else nh += (long long)r.len + ins;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-        nnz_delta += __shfl_xor_sync(__activemask(), nnz_delta, o);
-        bytes += __shfl_xor_sync(__activemask(), bytes, o);
+        nh += __shfl_xor_sync(0xffffffffu, nh, o);
+        nc += __shfl_xor_sync(0xffffffffu, nc, o);
+    }
+    if (lane_id() == 0 && nh) atomicAdd((unsigned long long*)&p.ctr->new_elems, (unsigned long long)nh);
+    if (lane_id() == 0 && nc) atomicAdd((unsigned long long*)&p.ctr->new_elems_host, (unsigned long long)nc);
+}
+
+__global__ void __launch_bounds__(ROW_THREADS) k_row_plan(RowPlan p) {
+    __shared__ long long s_base[6];
+    const int A = p.ctr->n_aff;
+    long long nnz_delta = 0, bytes = 0;
+    for (int a0 = blockIdx.x * ROW_THREADS; a0 < A; a0 += gridDim.x * ROW_THREADS) {
+        const int a = a0 + threadIdx.x;
+        const bool ok = a < A;
+        Row r{0, 0, 0};
+        int32_t u = 0;
+        int b = 0, d = 0, e = 0, nl = 0, ns = 0;
+        bool ip = false, cold = false, sm = false, lip = false;
+        if (ok) {
+            u = p.aff[a];
+            r = p.row[u];
+            b = p.seg_b[a];
+            d = p.seg_d[a];
+            e = p.seg_b[a + 1];
+            nl = r.len + (d - b) - (p.E[e] - p.E[d]);
+            ip = in_place_row(d - b, r.len, p.long_in_place);
+            cold = p.split && !in_hbm(r, p.hbm_cap);
+            lip = ip && r.len > IN_PLACE_LEN;
+            sm = r.len <= SMALL_LEN && e - b <= WARP;
+            ns = sm || lip ? 0 : ip ? 1 : max(1, (r.len + SLICE - 1) / SLICE);
+            nnz_delta += nl - r.len;
+            bytes += 4LL * ((long long)r.len + nl) + 8LL * (e - b) + 16;
+        }
+        const long long need = ok && !ip ? (long long)r.len + (d - b) : 0;
+        long long th, tc = 0, tn, oh, oc = 0;
+        oh = block_scan_rows(cold ? 0 : need, &th);
+        if (p.split) oc = block_scan_rows(cold ? need : 0, &tc);
+        // counts packed: slices 34 bits, short rows, other rows, long rows in place 10 bits each
+        const long long on = block_scan_rows((long long)ns | ((long long)(ok && sm) << 34) | ((long long)(ok && !sm) << 44) |
+                                                 ((long long)lip << 54), &tn);
+        if (threadIdx.x == 0) {
+            if (th) s_base[0] = (long long)atomicAdd((unsigned long long*)&p.ctr->new_elems, (unsigned long long)th);
+            if (tc) s_base[1] = (long long)atomicAdd((unsigned long long*)&p.ctr->new_elems_host, (unsigned long long)tc);
+            s_base[2] = atomicAdd(&p.ctr->n_slices, (int)(tn & ((1ll << 34) - 1)));
+            s_base[3] = atomicAdd(&p.ctr->n_small, (int)(tn >> 34) & 1023);
+            s_base[4] = atomicAdd(&p.ctr->n_long, (int)(tn >> 44) & 1023);
+            s_base[5] = atomicAdd(&p.ctr->n_large, (int)(tn >> 54) & 1023);
+        }
+        __syncthreads();
+        if (ok) {
+            long long dst = r.start;
+            if (!ip) dst = cold ? p.base_host + s_base[1] + oc : p.base_hbm + s_base[0] + oh;
+            const long long at = sm ? s_base[3] + ((on >> 34) & 1023) : p.mcap - 1 - (s_base[4] + ((on >> 44) & 1023));
+            p.mrow[at] = MergeRow{r.start, dst, r.len, b, d, e};
+            p.row[u] = ip ? Row{r.start, nl, r.cap} : Row{dst, nl, r.len + (d - b)};
+            if (lip) p.longs[s_base[5] + ((on >> 54) & 1023)] = (int32_t)at;
+            const long long s0 = s_base[2] + (on & ((1ll << 34) - 1));
+            if (s0 + ns > p.slice_cap) { if (ns) atomicExch(&p.ctr->overflow, 1); }
+            else for (int s = 0; s < ns; s++) p.slices[s0 + s] = (at << 32) | s;
+        }
+        __syncthreads();   // the bases are read before the next rows overwrite them
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        nnz_delta += __shfl_xor_sync(0xffffffffu, nnz_delta, o);
+        bytes += __shfl_xor_sync(0xffffffffu, bytes, o);
     }
     if (lane_id() == 0 && (nnz_delta || bytes)) {
-        atomicAdd((unsigned long long*)&ctr->nnz_delta, (unsigned long long)nnz_delta);
-        atomicAdd((unsigned long long*)&ctr->update_bytes, (unsigned long long)bytes);
+        atomicAdd((unsigned long long*)&p.ctr->nnz_delta, (unsigned long long)nnz_delta);
+        atomicAdd((unsigned long long*)&p.ctr->update_bytes, (unsigned long long)bytes);
     }
 }
 
-// Short rows, balanced: the short rows' old lengths are scanned (soff) and cut into groups of
-// about UNIT entries (a row belongs to the group its first entry falls in), one warp per
-// group. The warp takes the group's rows 32 at a time, one row per lane, and streams their
-// entries 32 at a time, every lane finding its row by a search over the lanes' prefix sums.
-// A surviving entry x lands at (survivors of its row before it) + (#insertions of its row
-// < x); the insertion values of the 32 rows are staged in shared memory when they fit, and
-// per-row survivor counts carry across chunks in shared memory.
+// ---- the merge -------------------------------------------------------------------------------
+// A row's new version is its old one with every entry moved by a count: old entry e that is not
+// cancelled lands at e + (insertions at positions <= e) - (matched deletions before e), and
+// insertion j of position i at i + j - (matched deletions before i). Between two events of the
+// row's sorted edit list the shift is constant, so the merge compares no values: a warp enters
+// the events of 1,024 old entries into bitmaps, a lane per event, and copies the entries 32 at a
+// time, each finding its shift by counting bits.
+//
+// What bounds it: for long rows HBM traffic (old rows read, new rows written) at 32 warps per SM
+// with up to 16 loads in flight per lane; for short ones the instructions per row. 10^6
+// preferential edits at scale 22 (0.92 GB of rows): 360 us, 10^4 edits there (0.25 GB): 64 us;
+// 680 and 122 us for the three kernels before it and the scan they waited on, which searched
+// the insertions for every surviving entry.
 constexpr int MERGE_THREADS = 256;
-constexpr int UNIT = 1024;
-constexpr int ICAP = 512;
+constexpr int MERGE_WARPS = MERGE_THREADS / WARP;
+constexpr int MERGE_U = 8;                 // 32-entry groups of a slice in flight
+constexpr int MERGE_ROWS = 4;              // short rows in flight per warp
 
-__global__ void __launch_bounds__(MERGE_THREADS) k_merge_small(
-        int32_t* __restrict__ pool, const unsigned long long* __restrict__ keys, int B,
-        const DevCounters* __restrict__ ctr, const int64_t* __restrict__ seg, const Row* __restrict__ old_row,
-        const int64_t* __restrict__ off, long long tail, const int32_t* __restrict__ small,
-        const int64_t* __restrict__ soff) {
-    __shared__ int s_cnt[MERGE_THREADS / WARP][WARP];
-    __shared__ int32_t s_ins[MERGE_THREADS / WARP][ICAP];
-    const int w = threadIdx.x / WARP;
-    const unsigned lane = lane_id();
-    const int ns = ctr->n_small;
-    const long long total = soff[ns];
-    const long long G = (total + UNIT - 1) / UNIT;
-    for (long long g = gwarp_id(); g < G; g += gwarp_count()) {
-        const long long i0 = warp_lower_bound(soff, ns, g * UNIT);
-        const long long i1 = warp_lower_bound(soff, ns, (g + 1) * UNIT);
-        for (long long rb = i0; rb < i1; rb += WARP) {
-            const long long i = rb + lane;
-            long long st = 0, ob = 0, ib = 0;
-            int len = 0, p = 0;
-            if (i < i1) {
-                const int a = small[i];
-                const Row r = old_row[a];
-                st = r.start;
-                len = r.len;
-                ib = seg[3 * (int64_t)a];
-                p = (int)(seg[3 * (int64_t)a + 1] - ib);
-                ob = in_place_row(p, len, false) ? st : tail + off[a];   // short: the flag is moot
-            }
-            s_cnt[w][lane] = 0;
-            const int pin = warp_incl_scan_i(p);
-            const int ptot = __shfl_sync(0xffffffffu, pin, WARP - 1);
-            const int pex = pin - p;
-            const bool staged = ptot <= ICAP;
-            if (staged)
-                for (int t = 0; t < p; t++) s_ins[w][pex + t] = key_v(keys[ib + t], B);
-            __syncwarp();
-            const int incl = warp_incl_scan_i(len);
-            const int tot = __shfl_sync(0xffffffffu, incl, WARP - 1);
-            const int excl = incl - len;
-            constexpr int U = 4;   // chunks per step: their loads are issued before any store
-            for (int e00 = 0; e00 < tot; e00 += U * WARP) {
-                int jj[U];
-                int32_t xx[U];
-#pragma unroll
-                for (int u = 0; u < U; u++) {
-                    const int e = e00 + u * WARP + (int)lane;
-                    int lo = 0, hi = WARP - 1;
-#pragma unroll
-                    for (int it = 0; it < 5; it++) {
-                        const int mid = (lo + hi + 1) >> 1;
-                        if (__shfl_sync(0xffffffffu, excl, mid) <= e) lo = mid; else hi = mid - 1;
-                    }
-                    jj[u] = lo;
-                    const int ej = __shfl_sync(0xffffffffu, excl, lo);
-                    const long long sj = __shfl_sync(0xffffffffu, st, lo);
-                    xx[u] = e < tot ? pool[sj + (e - ej)] : -1;
-                }
-                // rows rewritten in place: every load of this step precedes every store (a
-                // survivor's store lands at or before its load, and before any later load)
-                __syncwarp();
-#pragma unroll
-                for (int u = 0; u < U; u++) {
-                    const int e0 = e00 + u * WARP;
-                    if (e0 >= tot) break;   // uniform
-                    const int j = jj[u];
-                    const int32_t x = xx[u];
-                    const int e = e0 + (int)lane;
-                    const int ej = __shfl_sync(0xffffffffu, excl, j);
-                    const int lj = __shfl_sync(0xffffffffu, len, j);
-                    const long long oj = __shfl_sync(0xffffffffu, ob, j);
-                    const long long ij = __shfl_sync(0xffffffffu, ib, j);
-                    const int pj = __shfl_sync(0xffffffffu, p, j);
-                    const int xj = __shfl_sync(0xffffffffu, pex, j);
-                    const bool in = e < tot;
-                    const bool surv = x >= 0;
-                    const unsigned m = __ballot_sync(0xffffffffu, surv);
-                    const int fl = max(ej - e0, 0);                    // first lane of row j in this chunk
-                    const int ll = min(ej + lj - e0, WARP) - 1;        // last lane of row j in this chunk
-                    const unsigned below = (1u << lane) - 1;
-                    const unsigned from_fl = ~((1u << fl) - 1);
-                    if (surv) {
-                        int lbI = 0;
-                        if (pj > 0) {
-                            if (staged) {
-                                int a = 0, b = pj;
-                                while (a < b) { int mid = (a + b) >> 1; if (s_ins[w][xj + mid] < x) a = mid + 1; else b = mid; }
-                                lbI = a;
-                            } else {
-                                lbI = (int)lb_span(KeySpan{keys + ij, B}, pj, x);
-                            }
-                        }
-                        pool[oj + s_cnt[w][j] + __popc(m & below & from_fl) + lbI] = x;
-                    }
-                    __syncwarp();
-                    if (in && (int)lane == ll) {
-                        const unsigned upto = ll >= WARP - 1 ? 0xffffffffu : ((1u << (ll + 1)) - 1);
-                        s_cnt[w][j] += __popc(m & upto & from_fl);
-                    }
-                    __syncwarp();
-                }
-            }
+// The events of MERGE_CHUNK old entries of a row, in shared memory (one per warp).
+constexpr int MERGE_CHUNK = 32 * WARP;
+// Word w of a chunk's 32: x a bit per cancelled entry, y a bit per entry that insertions go
+// before, z insertions before the word (bit 30: several go before one entry), w cancelled
+// entries before the word.
+typedef uint4 ChunkEvents[WARP];
+
+// First half-edit in [b, e) whose position is >= x (positions ascending), 32 probes per step;
+// every lane calls it and gets the same answer.
+__device__ __forceinline__ int warp_lb_event(const uint32_t* epos, int b, int e, int x) {
+    int lo = b, hi = e;
+    while (hi - lo > WARP) {
+        const int step = (hi - lo + WARP - 1) / WARP;
+        const int at = lo + (int)lane_id() * step;
+        const int c = __popc(__ballot_sync(0xffffffffu, at < hi && (int)(epos[at] >> 1) < x));   // probes below x
+        if (c == 0) { hi = lo; break; }
+        const int nlo = lo + (c - 1) * step + 1;
+        hi = min(hi, lo + c * step);
+        lo = nlo;
+    }
+    const int at = lo + (int)lane_id();
+    return lo + __popc(__ballot_sync(0xffffffffu, at < hi && (int)(epos[at] >> 1) < x));
+}
+
+// The events in [c0, c1) of the row (half-edits from *ii and *id on) are entered, a lane each:
+// insertions written to their places, the words left for the entries. Both cursors move past
+// the chunk. Returns the chunk's cancelled entries.
+static __device__ __forceinline__ int chunk_events(int32_t* __restrict__ N, const unsigned long long* __restrict__ keys,
+                                                   int B, const uint32_t* __restrict__ epos, const MergeRow& r, int c0,
+                                                   int c1, int* ii, int* id, bool any_ins, bool any_del, int gone,
+                                                   ChunkEvents& ev) {
+    const int l = (int)lane_id();
+    __syncwarp();   // the previous chunk's words are read
+    ev[l] = make_uint4(0u, 0u, 0u, 0u);
+    __syncwarp();
+    int dtot = 0;
+    if (any_del) {
+        for (int k = *id;; k += WARP) {
+            const uint32_t e = k + l < r.e ? epos[k + l] : ~0u;
+            const int pos = (int)(e >> 1);
+            const bool in = pos < c1;
+            if (in && (e & 1u)) atomicOr(&ev[(pos - c0) >> 5].x, 1u << ((pos - c0) & 31));
+            const unsigned m = __ballot_sync(0xffffffffu, in);
+            if (m != 0xffffffffu) { *id = k + __popc(m); break; }
         }
+        __syncwarp();
+        const int mine = __popc(ev[l].x);
+        const int inc = warp_incl_scan_i(mine);
+        dtot = __shfl_sync(0xffffffffu, inc, WARP - 1);
+        ev[l].w = (unsigned)(inc - mine);
+        __syncwarp();
+    }
+    if (any_ins) {
+        for (int k = *ii;; k += WARP) {
+            const int pos = k + l < r.d ? (int)(epos[k + l] >> 1) : INT32_MAX;
+            const bool in = pos < c1;
+            if (in) {
+                const int w = (pos - c0) >> 5;
+                const unsigned bit = 1u << ((pos - c0) & 31);
+                atomicOr(&ev[w].y, bit);
+                atomicAdd(&ev[w].z, 1u);
+                N[pos + (k + l - r.b) - gone - (int)ev[w].w - __popc(ev[w].x & (bit - 1))] = key_v(keys[k + l], B);
+            }
+            const unsigned m = __ballot_sync(0xffffffffu, in);
+            if (m != 0xffffffffu) { *ii = k + __popc(m); break; }
+        }
+        __syncwarp();
+        const int cnt = (int)ev[l].z;
+        const int inc = warp_incl_scan_i(cnt);
+        ev[l].z = (unsigned)(inc - cnt) | (__popc(ev[l].y) != cnt ? 1u << 30 : 0u);
+        __syncwarp();
+    }
+    return dtot;
+}
+
+// Old entries [s0, s1) of one row, by one warp.
+static __device__ __forceinline__ void merge_slice(int32_t* __restrict__ pool, const unsigned long long* __restrict__ keys,
+                                                   int B, const uint32_t* __restrict__ epos, const int32_t* __restrict__ E,
+                                                   const MergeRow& r, int s0, int s1, ChunkEvents& ev) {
+    constexpr int STEP = MERGE_U * WARP;
+    const int l = (int)lane_id();
+    const unsigned lt = (1u << l) - 1, le = lt | (1u << l);
+    const int32_t* O = pool + r.start + l;   // this lane's entry of a group at 0
+    int32_t* N = pool + r.dst;
+    int32_t x[MERGE_U];
+#pragma unroll
+    for (int u = 0; u < MERGE_U; u++) x[u] = s0 + u * WARP + l < s1 ? O[s0 + u * WARP] : 0;
+    int id = r.d, ii = r.b;   // events not below the chunk
+    if (s0 > 0) {
+        ii = warp_lb_event(epos, r.b, r.d, s0);
+        id = warp_lb_event(epos, r.d, r.e, s0);
+    }
+    int gone = id > r.d ? E[id] - E[r.d] : 0;   // matched deletions before the chunk
+    for (int c0 = s0; c0 < s1; c0 += MERGE_CHUNK) {
+        const int c1 = min(c0 + MERGE_CHUNK, s1);
+        const int shift = (ii - r.b) - gone;
+        const int ni = ii < r.d ? (int)(epos[ii] >> 1) : INT32_MAX, nd = id < r.e ? (int)(epos[id] >> 1) : INT32_MAX;
+        const int ib = ii;
+        const bool quiet = ni >= c1 && nd >= c1;   // no event among the chunk's entries
+        if (!quiet) gone += chunk_events(N, keys, B, epos, r, c0, c1, &ii, &id, ni < c1, nd < c1, gone, ev);
+        for (int b0 = c0; b0 < c1; b0 += STEP) {
+            int32_t nx[MERGE_U];
+            if (b0 + 2 * STEP <= s1) {
+#pragma unroll
+                for (int u = 0; u < MERGE_U; u++) nx[u] = O[b0 + STEP + u * WARP];
+            } else {
+#pragma unroll
+                for (int u = 0; u < MERGE_U; u++) nx[u] = b0 + STEP + u * WARP + l < s1 ? O[b0 + STEP + u * WARP] : 0;
+            }
+            __syncwarp();   // a row compacted where it lies: these loads precede the stores below
+            int32_t* M = N + b0 + shift + l;
+            if (quiet && b0 + STEP <= c1) {
+#pragma unroll
+                for (int u = 0; u < MERGE_U; u++) M[u * WARP] = x[u];
+            } else if (quiet) {
+#pragma unroll
+                for (int u = 0; u < MERGE_U; u++)
+                    if (b0 + u * WARP + l < c1) M[u * WARP] = x[u];
+            } else {
+#pragma unroll
+                for (int u = 0; u < MERGE_U; u++) {
+                    const uint4 w = ev[(b0 - c0) / WARP + u];
+                    int to = (int)(w.z & ~(1u << 30)) - (int)w.w - __popc(w.x & lt);
+                    if (w.z >> 30) {   // uniform: several insertions before one entry, counted one by one
+                        for (int k = ib + (int)(w.z & ~(1u << 30)); k < r.d; k++) {
+                            const int pos = (int)(epos[k] >> 1);
+                            if (pos >= b0 + (u + 1) * WARP) break;
+                            to += pos <= b0 + u * WARP + l;
+                        }
+                    } else {
+                        to += __popc(w.y & le);
+                    }
+                    if (b0 + u * WARP + l < c1 && !((w.x >> l) & 1u)) M[u * WARP + to] = x[u];
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < MERGE_U; u++) x[u] = nx[u];
+        }
+    }
+    if (s1 == r.len)   // insertions past the last entry
+        for (int k = ii + l; k < r.d; k += WARP) N[r.len + (k - r.b) - gone] = key_v(keys[k], B);
+}
+
+// Short rows (at most SMALL_LEN entries and 32 half-edits): all events of a row fit one warp.
+static __device__ __forceinline__ void merge_short(int32_t* __restrict__ pool, const unsigned long long* __restrict__ keys,
+                                                   int B, const uint32_t* __restrict__ epos,
+                                                   const MergeRow* __restrict__ mrow, int i0, int cnt) {
+    const int l = (int)lane_id();
+    const unsigned lt = (1u << l) - 1, le = lt | (1u << l);
+    MergeRow r{0, 0, 0, 0, 0, 0};
+    if (l < cnt) r = mrow[i0 + l];
+    for (int j0 = 0; j0 < cnt; j0 += MERGE_ROWS) {
+        long long st[MERGE_ROWS], ds[MERGE_ROWS];
+        int len[MERGE_ROWS], pos[MERGE_ROWS], ne[MERGE_ROWS];
+        int32_t x0[MERGE_ROWS], x1[MERGE_ROWS], y[MERGE_ROWS];
+        bool ins[MERGE_ROWS], del[MERGE_ROWS];
+#pragma unroll
+        for (int u = 0; u < MERGE_ROWS; u++) {   // the loads of MERGE_ROWS rows
+            const int j = (j0 + u) & (WARP - 1);
+            const bool have = j0 + u < cnt;
+            st[u] = __shfl_sync(0xffffffffu, r.start, j);
+            ds[u] = __shfl_sync(0xffffffffu, r.dst, j);
+            len[u] = __shfl_sync(0xffffffffu, r.len, j);
+            const int b = __shfl_sync(0xffffffffu, r.b, j);
+            int p = __shfl_sync(0xffffffffu, r.d, j) - b;
+            ne[u] = __shfl_sync(0xffffffffu, r.e, j) - b;
+            if (!have) { len[u] = 0; p = 0; ne[u] = 0; }
+            const uint32_t e = l < ne[u] ? epos[b + l] : 0u;
+            pos[u] = (int)(e >> 1);
+            del[u] = (e & 1u) != 0;   // matched deletions only
+            ins[u] = l < p;
+            y[u] = l < p ? key_v(keys[b + l], B) : 0;
+            x0[u] = l < len[u] ? pool[st[u] + l] : 0;
+            x1[u] = WARP + l < len[u] ? pool[st[u] + WARP + l] : 0;
+        }
+        __syncwarp();   // rows compacted where they lie: these loads precede the stores
+#pragma unroll
+        for (int u = 0; u < MERGE_ROWS; u++) {
+            int32_t* N = pool + ds[u];
+            const int32_t* O = pool + st[u];
+            int32_t x = x0[u], xn = x1[u];
+            if (ne[u] <= 1) {   // one half-edit (most rows) or none left here
+                const int at = __shfl_sync(0xffffffffu, pos[u], 0);
+                const bool in = __shfl_sync(0xffffffffu, (int)ins[u], 0) != 0;
+                const bool cut = __shfl_sync(0xffffffffu, (int)del[u], 0) != 0;
+                for (int e = l; e - l < len[u]; e += WARP) {
+                    const int32_t xnn = e + 2 * WARP < len[u] ? O[e + 2 * WARP] : 0;
+                    __syncwarp();
+                    const int to = e + (in && e >= at) - (cut && e > at);
+                    if (e < len[u] && !(cut && e == at)) N[to] = x;
+                    x = xn;
+                    xn = xnn;
+                }
+                if (l == 0 && in) N[at] = y[u];
+                continue;
+            }
+            int shift = 0, gone = 0;   // insertions minus cancelled entries, and cancelled entries, before the group
+            for (int e0 = 0; e0 < len[u]; e0 += WARP) {
+                int32_t xnn = 0;
+                if (e0 + 2 * WARP < len[u]) xnn = e0 + 2 * WARP + l < len[u] ? O[e0 + 2 * WARP + l] : 0;
+                const int at = pos[u] - e0;
+                const bool here = (unsigned)at < WARP;
+                const unsigned bit = 1u << (at & 31);
+                const unsigned dm = __reduce_or_sync(0xffffffffu, del[u] && here ? bit : 0u);
+                const bool in = ins[u] && here && pos[u] < len[u];
+                const unsigned mi = __ballot_sync(0xffffffffu, in);
+                int to = e0 + l + shift - __popc(dm & lt);
+                if (mi) {
+                    const unsigned im = __reduce_or_sync(0xffffffffu, in ? bit : 0u);
+                    if (__popc(im) == __popc(mi)) {
+                        to += __popc(im & le);
+                    } else {
+                        for (unsigned q = mi; q; q &= q - 1)
+                            to += __shfl_sync(0xffffffffu, at, __ffs(q) - 1) <= l;
+                    }
+                    if (in) N[pos[u] + l - gone - __popc(dm & (bit - 1))] = y[u];
+                }
+                __syncwarp();
+                if (e0 + l < len[u] && !((dm >> l) & 1u)) N[to] = x;
+                shift += __popc(mi) - __popc(dm);
+                gone += __popc(dm);
+                x = xn;
+                xn = xnn;
+            }
+            if (ins[u] && pos[u] == len[u]) N[pos[u] + l - gone] = y[u];   // past the last entry
+        }
+    }
+}
+
+__global__ void __launch_bounds__(MERGE_THREADS, 4) k_merge(
+        int32_t* __restrict__ pool, const unsigned long long* __restrict__ keys, int B, DevCounters* __restrict__ ctr,
+        const uint32_t* __restrict__ epos, const int32_t* __restrict__ E, const MergeRow* __restrict__ mrow, int64_t mcap,
+        const int64_t* __restrict__ slices, int64_t slice_cap) {
+    __shared__ ChunkEvents s_ev[MERGE_WARPS];
+    if (ctr->overflow) return;   // the slice list did not fit (the host reports it)
+    const int nsl = (int)min((int64_t)ctr->n_slices, slice_cap);
+    const int nsm = ctr->n_small;
+    // rows of a warp's turn: up to 32, fewer while that leaves warps without any
+    const int per = min(WARP, max(MERGE_ROWS, (nsm + gwarp_count() - 1) / gwarp_count()));
+    const int items = nsl + (nsm + per - 1) / per;
+    int it = gwarp_id();   // the first item of every warp; the rest are handed out
+    while (it < items) {
+        int nx = 0;
+        if (lane_id() == 0) nx = gwarp_count() + atomicAdd(&ctr->merge_ticket, 1);
+        if (it < nsl) {
+            const int64_t item = slices[it];
+            const MergeRow r = mrow[item >> 32];
+            const int s = (int)(item & 0xffffffffLL);
+            const bool whole = r.dst == r.start;   // compacted where it lies: one warp, front to back
+            const int s0 = whole ? 0 : s * SLICE;
+            merge_slice(pool, keys, B, epos, E, r, s0, whole ? r.len : min(r.len, s0 + SLICE), s_ev[threadIdx.x / WARP]);
+        } else {
+            const int i0 = (it - nsl) * per;
+            merge_short(pool, keys, B, epos, mrow, i0, min(per, nsm - i0));
+        }
+        it = __shfl_sync(0xffffffffu, nx, 0);
     }
 }
 
 // Long rows that only lose entries, compacted in place: one block per row streams it front to
-// back in chunks of LIP_CHUNK entries; every entry of a chunk is loaded before any survivor
-// of that chunk is stored, and a survivor's new position (survivors before it in the row)
-// never exceeds its old one, so no store lands on an entry still to be read.
+// back in chunks of LIP_CHUNK entries, marking the chunk's cancelled entries from the row's
+// sorted events; every entry of a chunk is loaded before any survivor of that chunk is stored,
+// and a survivor's new position (survivors before it in the row) never exceeds its old one, so
+// no store lands on an entry still to be read.
 constexpr int LIP_THREADS = 256;
 constexpr int LIP_U = 4;
 constexpr int LIP_CHUNK = LIP_THREADS * LIP_U;
 
 __global__ void __launch_bounds__(LIP_THREADS) k_merge_long_inplace(int32_t* __restrict__ pool,
                                                                     const DevCounters* __restrict__ ctr,
+                                                                    const uint32_t* __restrict__ epos,
                                                                     const int32_t* __restrict__ longs,
-                                                                    const Row* __restrict__ old_row) {
+                                                                    const MergeRow* __restrict__ mrow) {
     __shared__ int s_warp[LIP_U][LIP_THREADS / WARP];
+    __shared__ unsigned s_gone[LIP_CHUNK / WARP];
+    __shared__ int s_next;
     const int t = threadIdx.x, w = t / WARP;
     const unsigned lt = (1u << lane_id()) - 1;
     const int nl = ctr->n_large;
     for (int li = blockIdx.x; li < nl; li += gridDim.x) {
-        const Row r = old_row[longs[li]];
+        const MergeRow r = mrow[longs[li]];
         int32_t* O = pool + r.start;
         long long run = 0;
-        for (long long b = 0; b < r.len; b += LIP_CHUNK) {
+        int k = r.d;   // first event not below the chunk
+        for (int b = 0; b < r.len; b += LIP_CHUNK) {
+            const int lim = b > INT32_MAX - LIP_CHUNK ? INT32_MAX : b + LIP_CHUNK;
+            if (t < LIP_CHUNK / WARP) s_gone[t] = 0;
+            if (t == 0) s_next = r.e;
+            __syncthreads();
+            for (bool more = true; more;) {
+                const int i = k + t;
+                const uint32_t e = i < r.e ? epos[i] : 0u;
+                const bool in = i < r.e && (int)(e >> 1) < lim;
+                if (in && (e & 1u)) atomicOr(&s_gone[((e >> 1) - b) >> 5], 1u << (((e >> 1) - b) & 31));
+                if (i < r.e && !in) atomicMin(&s_next, i);
+                more = __syncthreads_and(in) != 0;
+                if (more) k += LIP_THREADS;
+            }
+            k = s_next;
             int32_t x[LIP_U];
             unsigned m[LIP_U];
 #pragma unroll
             for (int u = 0; u < LIP_U; u++) {
-                const long long i = b + u * LIP_THREADS + t;
-                x[u] = i < r.len ? O[i] : -1;
-                m[u] = __ballot_sync(0xffffffffu, x[u] >= 0);
+                const int rel = u * LIP_THREADS + t;
+                const long long i = (long long)b + rel;
+                const bool keep = i < r.len && !((s_gone[rel >> 5] >> (rel & 31)) & 1u);
+                x[u] = keep ? O[i] : -1;
+                m[u] = __ballot_sync(0xffffffffu, keep);
                 if (lane_id() == 0) s_warp[u][w] = __popc(m[u]);
             }
             __syncthreads();   // every load of the chunk is done; the warp counts are visible
@@ -515,9 +822,9 @@ __global__ void __launch_bounds__(LIP_THREADS) k_merge_long_inplace(int32_t* __r
             for (int u = 0; u < LIP_U; u++) {
                 int before = 0, total = 0;
 #pragma unroll
-                for (int k = 0; k < LIP_THREADS / WARP; k++) {
-                    const int cnt = s_warp[u][k];
-                    before += k < w ? cnt : 0;
+                for (int q = 0; q < LIP_THREADS / WARP; q++) {
+                    const int cnt = s_warp[u][q];
+                    before += q < w ? cnt : 0;
                     total += cnt;
                 }
                 if (x[u] >= 0) O[base + before + __popc(m[u] & lt)] = x[u];
@@ -525,265 +832,6 @@ __global__ void __launch_bounds__(LIP_THREADS) k_merge_long_inplace(int32_t* __r
             }
             run = base;
             __syncthreads();   // the counts are read before the next chunk overwrites them
-        }
-    }
-}
-
-// Rows past SMALL_LEN: one warp per slice of SLICE old-row entries (most rows a batch touches
-// in a scale-free graph are its hubs, so this merge carries most of the bytes, with a few
-// instructions per entry: a ballot, a population count, and a search of the insertions only
-// where they fall inside a chunk's value range). The survivors before the slice are
-// its start minus the matched deletions before it (one search in the non-decreasing dpos);
-// survivor x lands at (#survivors before it) + (#insertions < x), the insertion count
-// searched only inside the range spanned by the chunk's values.
-//
-// A slice of an HBM row is staged in shared memory by the bulk-copy engine: each warp owns two
-// MS_CH-entry buffers and their mbarriers; lane 0 issues cp.async.bulk (non-multicast) of the
-// 16-byte-aligned cover of the next chunk while the warp merges the current one from shared
-// memory, so the old row is read in MS_CH * 4-byte transfers with no load instruction per
-// entry. Every wait on an mbarrier is bounded: past the limit the warp flags sort_err = 3,
-// waits (bounded again) for its copies in flight and leaves. Rows in host memory (tiered
-// store) and slices whose aligned cover would pass the pool's end are read with direct loads.
-constexpr int MS_WARPS = 8;
-constexpr int MS_THREADS = MS_WARPS * WARP;
-constexpr int MS_CH = 512;                 // entries per staged chunk
-constexpr int MS_BUF = MS_CH + 8;          // buffer: chunk + 16-byte alignment slack on both ends
-constexpr int MS_ISTAGE = 448;             // insertion keys of a slice (or one merge step) staged per warp (48 KB static limit)
-constexpr long long MBAR_SPIN_LIMIT = 1ll << 24;
-
-__device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint64_t* bar) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(bar)) : "memory");
-}
-__device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-// lane 0: one arrival that expects `bytes`, then the bulk copy global -> shared completing on bar
-__device__ __forceinline__ void bulk_g2s(int32_t* dst, const int32_t* src, unsigned bytes, uint64_t* bar) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes) : "memory");
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"(smem_addr(dst)), "l"(src), "r"(bytes), "r"(smem_addr(bar))
-                 : "memory");
-}
-__device__ __forceinline__ bool mbar_test(uint64_t* bar, unsigned parity) {
-    unsigned ok;
-    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-                 : "=r"(ok)
-                 : "r"(smem_addr(bar)), "r"(parity)
-                 : "memory");
-    return ok != 0;
-}
-// all lanes: bounded wait for the given phase of bar; false when the limit was reached
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity) {
-    for (long long it = 0; it < MBAR_SPIN_LIMIT; it++) {
-        if (mbar_test(bar, parity)) return true;
-        if (it > 64) __nanosleep(128);
-    }
-    return false;
-}
-
-// First index i in [0, n] with I[i] >= x (I ascending), 32 probes per step (every lane calls
-// it and gets the same answer): a search of a few thousand keys is three dependent loads.
-__device__ __forceinline__ long long warp_lb_key(const KeySpan& I, long long n, int32_t x) {
-    long long lo = 0, hi = n;
-    while (hi - lo > WARP) {
-        const long long step = (hi - lo + WARP - 1) / WARP;
-        const long long pos = lo + (long long)lane_id() * step;
-        const int c = __popc(__ballot_sync(0xffffffffu, pos < hi && I[pos] < x));   // probes below x
-        if (c == 0) { hi = lo; break; }
-        const long long nlo = lo + (long long)(c - 1) * step + 1;
-        hi = min(hi, lo + (long long)c * step);
-        lo = nlo;
-    }
-    const long long pos = lo + lane_id();
-    return lo + __popc(__ballot_sync(0xffffffffu, pos < hi && I[pos] < x));
-}
-
-// First index i in [from, p] with I[i] >= t (I ascending), the warp reading 32 keys per step
-// forward from `from`; every lane calls it and gets the same answer.
-__device__ __forceinline__ long long ins_advance(const KeySpan& I, long long p, long long from, int32_t t) {
-    for (long long i = from; i < p; i += WARP) {
-        const long long j = i + lane_id();
-        const unsigned m = __ballot_sync(0xffffffffu, j < p && I[j] < t);   // a prefix of the lanes
-        const int k = __popc(m);
-        if (k < WARP) return i + k;
-    }
-    return p;
-}
-
-// Merges old-row entries [b, e) (absolute pool indices) read through `get`, updating the running
-// survivor count; every lane calls it. Survivor x lands at run + (survivors before it in its
-// step) + (insertions < x). With pre >= 0 the slice's whole insertion range I[i0, i0 + pre)
-// is already in s_ins and each survivor searches it there. Otherwise the insertions below the
-// step's smallest value are `cur`, which only moves forward along the row (the old entries are
-// ascending): each step advances it to its value range [xmin, xmax) with coalesced reads of
-// the insertion keys, stages the keys of that range in s_ins when they fit, and searches them.
-template <typename Get>
-__device__ __forceinline__ void merge_span(long long b, long long e, Get get, int32_t* out, long long& run,
-                                           const KeySpan& I, long long p, long long& cur, int32_t* s_ins,
-                                           int pre, long long i0, unsigned lt) {
-    constexpr int U = 4;
-    for (long long base = b; base < e; base += U * WARP) {
-        int32_t x[U];
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-            const long long i = base + u * WARP + lane_id();
-            x[u] = i < e ? get(i) : -1;
-        }
-        if (pre >= 0) {
-#pragma unroll
-            for (int u = 0; u < U; u++) {
-                const bool surv = x[u] >= 0;
-                const unsigned m = __ballot_sync(0xffffffffu, surv);
-                if (surv) {
-                    int lo = 0, hi = pre;
-                    while (lo < hi) { const int mid = (lo + hi) >> 1; if (s_ins[mid] < x[u]) lo = mid + 1; else hi = mid; }
-                    out[run + __popc(m & lt) + i0 + lo] = x[u];
-                }
-                run += __popc(m);
-            }
-            continue;
-        }
-        long long cl = cur, nin = 0;
-        if (cur < p) {
-            int xmin = INT32_MAX, xmax = -1;
-#pragma unroll
-            for (int u = 0; u < U; u++)
-                if (x[u] >= 0) { xmin = min(xmin, x[u]); xmax = max(xmax, x[u]); }
-            xmin = __reduce_min_sync(0xffffffffu, xmin);
-            xmax = __reduce_max_sync(0xffffffffu, xmax);
-            if (xmax >= 0) {
-                cl = ins_advance(I, p, cur, xmin);
-                const long long ch = ins_advance(I, p, cl, xmax);
-                nin = ch - cl;
-                cur = ch;
-                if (nin > 0 && nin <= MS_ISTAGE) {
-                    for (long long j = lane_id(); j < nin; j += WARP) s_ins[j] = I[cl + j];
-                    __syncwarp();
-                }
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-            const bool surv = x[u] >= 0;
-            const unsigned m = __ballot_sync(0xffffffffu, surv);
-            if (surv) {
-                long long lbI = cl;
-                if (nin > 0) {
-                    if (nin <= MS_ISTAGE) {
-                        int lo = 0, hi = (int)nin;
-                        while (lo < hi) { const int mid = (lo + hi) >> 1; if (s_ins[mid] < x[u]) lo = mid + 1; else hi = mid; }
-                        lbI += lo;
-                    } else {
-                        lbI += lb_span(KeySpan{I.k + cl, I.B}, nin, x[u]);
-                    }
-                }
-                out[run + __popc(m & lt) + lbI] = x[u];
-            }
-            run += __popc(m);
-        }
-        __syncwarp();   // s_ins is read before the next step stages another range
-    }
-}
-
-__global__ void __launch_bounds__(MS_THREADS) k_merge_slices(
-        int32_t* __restrict__ pool, long long pool_cap, const unsigned long long* __restrict__ keys, int B,
-        DevCounters* __restrict__ ctr, const int64_t* __restrict__ seg, const Row* __restrict__ old_row,
-        const int64_t* __restrict__ off, long long tail, const long long* __restrict__ E,
-        const long long* __restrict__ dpos, const int64_t* __restrict__ slices, int64_t slice_cap,
-        bool long_in_place) {
-    __shared__ __align__(16) int32_t s_buf[MS_WARPS][2][MS_BUF];
-    __shared__ __align__(8) uint64_t s_bar[MS_WARPS][2];
-    __shared__ int32_t s_ins[MS_WARPS][MS_ISTAGE];
-    const int w = threadIdx.x / WARP;
-    const unsigned lt = (1u << lane_id()) - 1;
-    if (lane_id() == 0) {
-        mbar_init(&s_bar[w][0]);
-        mbar_init(&s_bar[w][1]);
-        fence_proxy_async_smem();   // the initialised barriers are visible to the bulk-copy engine
-    }
-    __syncwarp();
-    unsigned phase[2] = {0u, 0u};
-    const long long nsl = min((long long)ctr->n_slices, (long long)slice_cap);
-    for (long long it = gwarp_id(); it < nsl; it += gwarp_count()) {
-        const long long item = slices[it];
-        const int a = (int)(item >> 32), s = (int)(item & 0xffffffffLL);
-        const Row r = old_row[a];
-        const long long b0 = seg[3 * (int64_t)a], sp = seg[3 * (int64_t)a + 1], e0 = seg[3 * (int64_t)a + 2];
-        const long long p = sp - b0, q = e0 - sp;
-        const long long s0 = (long long)s * SLICE, s1 = min((long long)r.len, s0 + SLICE);
-        if (s0 >= s1) continue;
-        long long md = 0;
-        if (q > 0 && s0 > 0 && lane_id() == 0) {
-            long long lo = 0, hi = q;
-            while (lo < hi) { long long mid = (lo + hi) >> 1; if ((dpos[sp + mid] >> 1) < s0) lo = mid + 1; else hi = mid; }
-            md = E[sp + lo] - E[sp];
-        }
-        long long run = s0 - __shfl_sync(0xffffffffu, md, 0);
-        // a row compacted in place is one slice here: every survivor lands at or before its old
-        // position, which its warp has already read
-        int32_t* out = pool + (in_place_row(p, r.len, long_in_place) ? r.start : tail + off[a]);
-        const KeySpan I{keys + b0, B};
-        const long long abs0 = r.start + s0, abs1 = r.start + s1;   // pool indices of the slice
-        // The insertions that can land among this slice's entries: I[i0, i1), i0 those below its
-        // first value, i1 those below its last (tombstones keep the value under the sign bit).
-        // When they fit they are staged in shared memory once for the whole slice.
-        long long i0 = 0, i1 = p;
-        if (p > 0) {
-            if (s0 > 0) i0 = warp_lb_key(I, p, unmark(pool[abs0]));
-            if (s1 < r.len) i1 = warp_lb_key(I, p, unmark(pool[abs1 - 1]));
-        }
-        const int pre = i1 - i0 <= MS_ISTAGE ? (int)(i1 - i0) : -1;
-        if (pre > 0) {
-            int32_t* si = s_ins[w];
-            for (int j0 = 0; j0 < pre; j0 += 4 * WARP) {
-                int32_t v[4];
-#pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    const int j = j0 + u * WARP + (int)lane_id();
-                    v[u] = j < pre ? I[i0 + j] : 0;
-                }
-#pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    const int j = j0 + u * WARP + (int)lane_id();
-                    if (j < pre) si[j] = v[u];
-                }
-            }
-            __syncwarp();
-        }
-        long long cur = i0;
-        const bool staged = r.start >= 0 && ((abs1 + 3) & ~3LL) <= pool_cap;
-        if (!staged) {
-            merge_span(abs0, abs1, [&](long long i) { return pool[i]; }, out, run, I, p, cur, s_ins[w], pre, i0, lt);
-            __syncwarp();   // s_ins is read before the next slice stages its insertions
-            continue;
-        }
-        const int nch = (int)((s1 - s0 + MS_CH - 1) / MS_CH);
-        auto issue = [&](int k) {   // lane 0
-            const long long lo = abs0 + (long long)k * MS_CH, hi = min(abs1, lo + MS_CH);
-            const long long a0 = lo & ~3LL, a1 = (hi + 3) & ~3LL;
-            bulk_g2s(s_buf[w][k & 1], pool + a0, (unsigned)((a1 - a0) * 4), &s_bar[w][k & 1]);
-        };
-        if (lane_id() == 0) {
-            issue(0);
-            if (nch > 1) issue(1);
-        }
-        for (int k = 0; k < nch; k++) {
-            const int bsel = k & 1;
-            if (!mbar_wait(&s_bar[w][bsel], phase[bsel])) {
-                // give up: flag it, let the copies in flight land (bounded), leave
-                if (lane_id() == 0) atomicCAS(&ctr->sort_err, 0, 3);
-                mbar_wait(&s_bar[w][bsel], phase[bsel]);
-                if (k + 1 < nch) mbar_wait(&s_bar[w][bsel ^ 1], phase[bsel ^ 1]);
-                return;
-            }
-            phase[bsel] ^= 1u;
-            const long long lo = abs0 + (long long)k * MS_CH, hi = min(abs1, lo + MS_CH);
-            const int32_t* sb = s_buf[w][bsel] - (lo & ~3LL);   // indexed by absolute pool index
-            merge_span(lo, hi, [&](long long i) { return sb[i]; }, out, run, I, p, cur, s_ins[w], pre, i0, lt);
-            __syncwarp();   // every lane is done with this buffer before it is refilled
-            if (k + 2 < nch && lane_id() == 0) {
-                fence_proxy_async_smem();   // the warp's reads of the buffer precede the copy's writes
-                issue(k + 2);
-            }
         }
     }
 }
@@ -884,7 +932,6 @@ __global__ void k_rows_compacted(Row* __restrict__ row, const int64_t* __restric
 }
 
 // ---- tiered store ---------------------------------------------------------------------------
-__device__ __forceinline__ bool in_hbm(const Row& r, long long cap) { return r.start >= 0 && r.start < cap; }
 __device__ __forceinline__ int len_bin(int len) { return 31 - __clz(len + 1); }
 
 __global__ void k_row_lens_hbm(const Row* __restrict__ row, int64_t n, long long cap, int64_t* __restrict__ out) {
@@ -923,28 +970,6 @@ __global__ void k_rows_evicted(Row* __restrict__ row, const int64_t* __restrict_
     }
 }
 
-// Split batches: the allocation of an affected row goes to the host lengths when its old
-// version lives in the host pool (lenH keeps the HBM rows' allocations).
-__global__ void k_split_alloc(const Row* __restrict__ old_row, const DevCounters* __restrict__ ctr, long long cap,
-                              int64_t* __restrict__ lenH, int64_t* __restrict__ lenC) {
-    const int A = ctr->n_aff;
-    for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < A; a += gridDim.x * blockDim.x) {
-        if (!in_hbm(old_row[a], cap)) {
-            lenC[a] = lenH[a];
-            lenH[a] = 0;
-        }
-    }
-}
-
-// Absolute destinations (element offsets from the HBM pool) of a split batch's rows.
-__global__ void k_abs_off(const Row* __restrict__ old_row, const DevCounters* __restrict__ ctr, long long cap,
-                          int64_t* __restrict__ offH, const int64_t* __restrict__ offC, long long hbm_base,
-                          long long host_base) {
-    const int A = ctr->n_aff;
-    for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < A; a += gridDim.x * blockDim.x)
-        offH[a] = in_hbm(old_row[a], cap) ? hbm_base + offH[a] : host_base + offC[a];
-}
-
 // After the HBM rows were copied to the new pool: HBM rows point at their copies, host rows
 // keep their address (their offset is re-based on the new pool).
 __global__ void k_rows_compacted_tiered(Row* __restrict__ row, const int64_t* __restrict__ off, int32_t n,
@@ -975,8 +1000,7 @@ int ws_ensure(scout_ctx* c, int64_t m) {
     size_t sz[] = {
         (size_t)M * sizeof(scout_edge), (size_t)M, (size_t)M,
         (size_t)H * 8, (size_t)H * 8, (size_t)(H + 1) * 8,
-        (size_t)H * 4, (size_t)3 * H * 8, (size_t)(H + 1) * 8, (size_t)H * 4, (size_t)(H + 1) * 8, (size_t)H * sizeof(Row),
-        (size_t)(H + 1) * 8, (size_t)H * 4};
+        (size_t)H * 4, (size_t)(H + 1) * 4, (size_t)H * 4, (size_t)H * 4, (size_t)H * sizeof(MergeRow)};
     size_t total = 0;
     for (size_t s : sz) total += align256(s);
     if (c->ws) dev_free(c, c->ws, (size_t)c->ws_bytes);
@@ -994,13 +1018,10 @@ int ws_ensure(scout_ctx* c, int64_t m) {
     c->d_keys_alt = (unsigned long long*)take(sz[4]);
     c->d_mdp = (long long*)take(sz[5]);
     c->d_aff = (int32_t*)take(sz[6]);
-    c->d_aff_seg = (int64_t*)take(sz[7]);
-    c->d_aff_len = (int64_t*)take(sz[8]);
-    c->d_aff_small = (int32_t*)take(sz[9]);
-    c->d_small_off = (int64_t*)take(sz[10]);
-    c->d_old_row = (Row*)take(sz[11]);
-    c->d_aff_len2 = (int64_t*)take(sz[12]);
-    c->d_aff_long = (int32_t*)take(sz[13]);
+    c->d_seg_b = (int32_t*)take(sz[7]);
+    c->d_seg_d = (int32_t*)take(sz[8]);
+    c->d_longs = (int32_t*)take(sz[9]);
+    c->d_mrow = (MergeRow*)take(sz[10]);
     c->d_hkeys = c->d_keys;
     return SCOUT_OK;
 }
@@ -1050,8 +1071,7 @@ int counters_fetch(scout_ctx* c) {
         return c->fail(SCOUT_E_STATE, "the component labels do not describe the components of the graph "
                                       "(an edge joins two labels); upload a consistent labelling");
     if (c->h_ctr->sort_err == 1) return c->fail(SCOUT_E_TIMEOUT, "a sort look-back wait timed out");
-    if (c->h_ctr->sort_err == 3) return c->fail(SCOUT_E_TIMEOUT, "a bulk copy of a row slice into shared memory did not complete");
-    if (c->h_ctr->sort_err == 4) return c->fail(SCOUT_E_TIMEOUT, "a scan look-back wait timed out");
+    if (c->h_ctr->sort_err == 4) return c->fail(SCOUT_E_TIMEOUT, "a scan or merge-plan look-back wait timed out");
     if (c->h_ctr->sort_err) return c->fail(SCOUT_E_STATE, "the sort computed a position out of range");
     if (c->h_bar->err != 0 || c->h_ctr->overflow)
         return c->fail(SCOUT_E_CAPACITY, "a device work list overflowed its capacity");
@@ -1061,7 +1081,7 @@ int counters_fetch(scout_ctx* c) {
 int graph_ensure_scratch(scout_ctx* c) {
     if (c->stamp_a) return SCOUT_OK;
     size_t bytes = (size_t)c->n * sizeof(int32_t);
-    int32_t** arrs[] = {&c->stamp_a, &c->stamp_b, &c->stamp_c, &c->stamp_d, &c->aux_v, &c->aux_w};
+    int32_t** arrs[] = {&c->stamp_a, &c->stamp_b, &c->stamp_c, &c->stamp_d, &c->aux_v};
     for (auto a : arrs) {
         SCOUT_RC(dev_alloc(c, (void**)a, bytes, "per-vertex scratch"));
         SCOUT_CU(c, cudaMemsetAsync(*a, 0, bytes, c->s_main));
@@ -1332,53 +1352,52 @@ int graph_update(scout_ctx* c, const scout_edge* edits, const uint8_t* ops, int6
     c->d_hkeys = sorted;
     const int64_t H = 2 * m;
     const int64_t Amax = std::min<int64_t>(H, n);
-    int nbh = blocks_for(H, 256);
-    k_seg_heads<<<nbh, 256, 0, c->s_main>>>(sorted, B, c->d_ctr, c->d_aff, c->d_aff_seg, c->aux_w);
-    k_seg_tails<<<nbh, 256, 0, c->s_main>>>(sorted, B, c->d_ctr, c->d_aff_seg, c->aux_w);
-    SCOUT_LAUNCH(c, "segments");
-    c->nlaunch += 2;
     // merge slices: the long rows' ceil(len / SLICE) sum to at most nnz / SLICE + Amax
     SCOUT_RC(dev_grow(c, &c->d_slices, &c->cap_slices, c->nnz / SLICE + Amax + 1024, "merge slices"));
-    // split: tiered store, rows whose old version lives in HBM are rewritten into HBM and host
-    // rows into the host pool (two scans); otherwise one scan for one destination
-    auto row_alloc = [&](bool again, bool split) -> int {
-        SCOUT_CU(c, cudaMemsetAsync(c->d_aff_len, 0, (size_t)(Amax + 1) * 8, c->s_main));
-        SCOUT_CU(c, cudaMemsetAsync(c->d_small_off, 0, (size_t)(Amax + 1) * 8, c->s_main));
-        if (again) SCOUT_CU(c, cudaMemsetAsync(&c->d_ctr->n_small, 0, 4 * sizeof(int), c->s_main));   // n_small .. n_pad
-        k_row_alloc<<<blocks_for(Amax, 256), 256, 0, c->s_main>>>(c->row, c->d_ctr, c->d_aff, c->d_aff_seg,
-                                                                  c->d_old_row, c->d_aff_len, c->d_aff_small,
-                                                                  c->d_small_off, c->d_slices, c->cap_slices,
-                                                                  c->d_aff_long, c->tiered);
-        SCOUT_LAUNCH(c, "k_row_alloc");
-        c->nlaunch += 1;
-        if (split) {
-            SCOUT_CU(c, cudaMemsetAsync(c->d_aff_len2, 0, (size_t)(Amax + 1) * 8, c->s_main));
-            k_split_alloc<<<blocks_for(Amax, 256), 256, 0, c->s_main>>>(c->d_old_row, c->d_ctr, (long long)c->pool_cap,
-                                                                        c->d_aff_len, c->d_aff_len2);
-            SCOUT_LAUNCH(c, "k_split_alloc");
-            c->nlaunch += 1;
-            SCOUT_RC(scan_i64(c, c->d_aff_len2, Amax + 1, (int64_t*)&c->d_ctr->new_elems_host));
-        } else if (again) {
-            SCOUT_CU(c, cudaMemsetAsync(&c->d_ctr->new_elems_host, 0, 8, c->s_main));
-        }
-        // Exclusive scan over Amax + 1 entries (the tail entries are zero): the new row of
-        // affected row a starts at tail + off[a]; the total is this batch's pool growth.
-        return scan_i64(c, c->d_aff_len, Amax + 1, (int64_t*)&c->d_ctr->new_elems);
-    };
+    uint32_t* epos = (uint32_t*)(sorted == c->d_keys ? c->d_keys_alt : c->d_keys);   // the free ping-pong half
+    int32_t* E = (int32_t*)c->d_mdp;
+    const int64_t tiles = (H + PLAN_TILE - 1) / PLAN_TILE;
+    SCOUT_RC(dev_grow(c, &c->d_scan_tmp, &c->cap_scan, std::max<int64_t>(64, 1 + 3 * tiles), "scan look-back"));
+    k_plan<<<(unsigned)tiles, PLAN_THREADS, 0, c->s_main>>>(c->row, c->pool, sorted, B, c->d_ctr, c->d_aff, c->d_seg_b,
+                                                            c->d_seg_d, epos, E,
+                                                            (unsigned long long*)c->d_scan_tmp + 1, next_stamp());
+    SCOUT_LAUNCH(c, "k_plan");
+    c->nlaunch += 1;
+    RowPlan rp;
+    rp.row = c->row;
+    rp.ctr = c->d_ctr;
+    rp.aff = c->d_aff;
+    rp.seg_b = c->d_seg_b;
+    rp.seg_d = c->d_seg_d;
+    rp.E = E;
+    rp.mrow = c->d_mrow;
+    rp.mcap = 2 * c->ws_m;
+    rp.slices = c->d_slices;
+    rp.slice_cap = c->cap_slices;
+    rp.longs = c->d_longs;
+    rp.long_in_place = c->tiered;
+    rp.hbm_cap = c->pool_cap;
+    rp.split = c->tiered;   // rows whose old version lives in HBM are rewritten into HBM, host rows into the host pool
+    rp.base_hbm = c->tail;
+    rp.base_host = 0;
     c->batch_dest = c->tiered ? 2 : 0;
-    SCOUT_RC(row_alloc(false, c->tiered));
-    long long dest = c->tail;   // element offset from the HBM pool where the new rows start
+    const int nbr = blocks_for(Amax, ROW_THREADS, 8 * c->sm_count);
     if (c->tiered) {
         // the exact growth, before anything is written. HBM part too large: compact (evicting
         // short rows to the host pool); larger than three quarters of the HBM pool: the whole
         // batch goes to the host pool. Host pool full: compacted in place on the host.
         long long grow[2] = {0, 0};   // HBM, host
-        auto read_grow = [&]() -> int {
+        auto read_grow = [&](bool again) -> int {
+            if (again) SCOUT_CU(c, cudaMemsetAsync(&c->d_ctr->new_elems, 0, 16, c->s_main));
+            rp.hbm_cap = c->pool_cap;
+            k_row_sizes<<<nbr, ROW_THREADS, 0, c->s_main>>>(rp);
+            SCOUT_LAUNCH(c, "k_row_sizes");
+            c->nlaunch += 1;
             SCOUT_CU(c, cudaMemcpyAsync(grow, &c->d_ctr->new_elems, 16, cudaMemcpyDeviceToHost, c->s_main));
             SCOUT_CU(c, cudaStreamSynchronize(c->s_main));
             return SCOUT_OK;
         };
-        SCOUT_RC(read_grow());
+        SCOUT_RC(read_grow(false));
         // a hinted next batch is gathered into the free HBM above this merge: keep room for about
         // its endpoint rows at the average degree (two per edit), at most a quarter of the pool.
         // More room means evicting more rows to the host pool on every compaction, which costs
@@ -1399,58 +1418,34 @@ int graph_update(scout_ctx* c, const scout_edge* edits, const uint8_t* ops, int6
                 c->batch_dest = 1;
                 c->host_batches++;
             }
-            SCOUT_RC(row_alloc(true, c->batch_dest == 2));
-            SCOUT_RC(read_grow());
+            rp.split = c->batch_dest == 2;
+            SCOUT_RC(read_grow(true));
         }
         const long long host_need = c->batch_dest == 1 ? grow[0] : grow[1];
         if (c->host_tail + host_need > c->host_cap) {
             SCOUT_RC(host_compact(c));
             if (c->host_tail + host_need > c->host_cap)
                 return c->fail(SCOUT_E_CAPACITY, "tiered store: the host pool cannot take this batch's rows");
-            SCOUT_RC(row_alloc(true, c->batch_dest == 2));
         }
         c->merge_tail = c->tail + (c->batch_dest == 1 ? 0 : grow[0]);
         const long long host_base = elem_delta(c->host_pool, c->pool) + c->host_tail;
-        if (c->batch_dest == 1) {
-            dest = host_base;
-        } else {
-            k_abs_off<<<blocks_for(Amax, 256), 256, 0, c->s_main>>>(c->d_old_row, c->d_ctr, (long long)c->pool_cap,
-                                                                    c->d_aff_len, c->d_aff_len2, (long long)c->tail,
-                                                                    host_base);
-            SCOUT_LAUNCH(c, "k_abs_off");
-            c->nlaunch += 1;
-            dest = 0;   // the offsets are absolute
-        }
+        SCOUT_CU(c, cudaMemsetAsync(&c->d_ctr->new_elems, 0, 16, c->s_main));   // counted again by the allocation
+        rp.hbm_cap = c->pool_cap;
+        rp.base_hbm = c->batch_dest == 1 ? host_base : c->tail;
+        rp.base_host = host_base;
     }
-    long long* dpos = (long long*)(sorted == c->d_keys ? c->d_keys_alt : c->d_keys);   // the free ping-pong half
-    long long* E = c->d_mdp;   // matched flags, then their exclusive scan (H + 1 entries)
-    k_plan_match<<<blocks_for(H, 256), 256, 0, c->s_main>>>(c->pool, sorted, B, c->d_ctr, c->aux_w, c->d_aff_seg,
-                                                            c->d_old_row, dpos, E, (long long)H);
-    SCOUT_LAUNCH(c, "k_plan_match");
-    SCOUT_CU(c, cudaMemsetAsync(E + H, 0, sizeof(long long), c->s_main));
-    SCOUT_RC(scan_i64(c, (int64_t*)E, H + 1, nullptr));
-    k_plan_place<<<blocks_for(H, 256), 256, 0, c->s_main>>>(c->pool, c->row, sorted, B, c->d_ctr, c->aux_w,
-                                                            c->d_aff_seg, c->d_old_row, c->d_aff_len,
-                                                            dest, dpos, E, c->tiered);
-    SCOUT_LAUNCH(c, "k_plan_place");
-    SCOUT_RC(scan_i64(c, c->d_small_off, Amax + 1, nullptr));
-    // the row merges loop over their work lists: a grid of at most four blocks per SM
-    const int64_t groups = std::min<int64_t>(c->nnz, Amax * (int64_t)SMALL_LEN) / UNIT + 1;
-    const int res4 = 4 * c->sm_count;
-    k_merge_small<<<std::min(blocks_for(groups * WARP, MERGE_THREADS), res4), MERGE_THREADS, 0, c->s_main>>>(
-        c->pool, sorted, B, c->d_ctr, c->d_aff_seg, c->d_old_row, c->d_aff_len, dest, c->d_aff_small,
-        c->d_small_off);
-    k_merge_long_inplace<<<(unsigned)std::min<int64_t>(std::max<int64_t>(1, Amax), 8 * (int64_t)c->sm_count),
-                           LIP_THREADS, 0, c->s_main>>>(c->pool, c->d_ctr, c->d_aff_long, c->d_old_row);
-    k_merge_slices<<<std::min(blocks_for(std::min<int64_t>(c->cap_slices, c->nnz / SLICE + Amax + 1024) * WARP,
-                                         MS_THREADS),
-                              res4),
-                     MS_THREADS,
-                     0, c->s_main>>>(c->pool, (long long)c->pool_cap, sorted, B, c->d_ctr, c->d_aff_seg,
-                                     c->d_old_row, c->d_aff_len, dest, E, dpos, c->d_slices, c->cap_slices,
-                                     c->tiered);
-    SCOUT_LAUNCH(c, "merge");
-    c->nlaunch += 6;
+    k_row_plan<<<nbr, ROW_THREADS, 0, c->s_main>>>(rp);
+    SCOUT_LAUNCH(c, "k_row_plan");
+    k_merge<<<(unsigned)std::min<int64_t>(4 * c->sm_count, (Amax + c->nnz / SLICE) / MERGE_WARPS + 1), MERGE_THREADS, 0,
+              c->s_main>>>(c->pool, sorted, B, c->d_ctr, epos, E, c->d_mrow, 2 * c->ws_m, c->d_slices, c->cap_slices);
+    SCOUT_LAUNCH(c, "k_merge");
+    c->nlaunch += 2;
+    if (c->tiered) {
+        k_merge_long_inplace<<<(unsigned)std::min<int64_t>(std::max<int64_t>(1, Amax), 8 * (int64_t)c->sm_count),
+                               LIP_THREADS, 0, c->s_main>>>(c->pool, c->d_ctr, epos, c->d_longs, c->d_mrow);
+        SCOUT_LAUNCH(c, "k_merge_long_inplace");
+        c->nlaunch += 1;
+    }
     return SCOUT_OK;
 }
 

@@ -244,6 +244,7 @@ __global__ void k_sort_small(unsigned long long* __restrict__ keys, int n, int b
 constexpr int SCAN_THREADS = 256;
 constexpr int SCAN_ITEMS = 8;
 constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
+constexpr int LOOKBACK_TILE = 1024;   // the smallest tile whose look-back uses the scan's state (the merge plan's)
 
 __device__ __forceinline__ long long block_excl_scan(long long x, long long* total) {
     __shared__ long long ws[SCAN_THREADS / WARP];
@@ -352,7 +353,6 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_lb(T* __restrict__ a, int
     }
 }
 
-static unsigned next_stamp();
 
 template <typename T>
 static int scan_any(scout_ctx* c, T* data, int64_t n, int64_t* d_total) {
@@ -375,7 +375,7 @@ int scan_i64(scout_ctx* c, int64_t* data, int64_t n, int64_t* d_total) { return 
 // Sizes the radix histogram and the scan partials for sorts of up to nkeys keys and scans
 // of up to nkeys entries, so later calls allocate nothing.
 // Look-back stamps are unique across the process (contexts share freed device memory).
-static unsigned next_stamp() {
+unsigned next_stamp() {
     static std::atomic<unsigned> counter{0};
     unsigned s = 0;
     while (s == 0) s = (counter.fetch_add(1) + 1) & ((1u << 30) - 1);
@@ -389,7 +389,7 @@ int sort_reserve(scout_ctx* c, int64_t nkeys) {
     if (c->d_sort_hist != before)   // fresh memory: no stale look-back entry may match a stamp
         SCOUT_CU(c, cudaMemsetAsync(c->d_sort_hist, 0, (size_t)c->cap_hist * 4, c->s_main));
     const int64_t scan_n = nkeys + 1;
-    SCOUT_RC(dev_grow(c, &c->d_scan_tmp, &c->cap_scan, std::max<int64_t>(64, 1 + 3 * ((scan_n + SCAN_TILE - 1) / SCAN_TILE)),
+    SCOUT_RC(dev_grow(c, &c->d_scan_tmp, &c->cap_scan, std::max<int64_t>(64, 1 + 3 * ((scan_n + LOOKBACK_TILE - 1) / LOOKBACK_TILE)),
                       "scan look-back"));
     return SCOUT_OK;
 }
