@@ -66,6 +66,18 @@ __device__ __forceinline__ int warp_incl_scan_i(int x) {
     return x;
 }
 
+// The lanes whose low 8 bits of d equal this lane's, by eight ballots.
+__device__ __forceinline__ unsigned match_digit(unsigned d) {
+    unsigned peers = 0xffffffffu;
+#pragma unroll
+    for (int b = 0; b < 8; b++) {
+        const bool one = (d >> b) & 1u;
+        const unsigned m = __ballot_sync(0xffffffffu, one);
+        peers &= one ? m : ~m;
+    }
+    return peers;
+}
+
 // Warp-aggregated append: every lane with `pred` gets a distinct slot of `q` through one
 // atomicAdd per warp. Returns the slot (or -1); slots beyond cap are not written and the
 // caller sees the overflow in the counter.
@@ -105,6 +117,27 @@ __device__ __forceinline__ bool dg_adjacent(const DGraph& g, int32_t u, int32_t 
     const int32_t* a = g.pool + ru.start;
     long long k = lower_bound_i32(a, ru.len, v);
     return k < ru.len && a[k] == v;
+}
+
+// The same with three probes per step: half the dependent reads, for calls that are bound by their
+// latency alone.
+__device__ __forceinline__ bool dg_adjacent_wide(const DGraph& g, int32_t u, int32_t v) {
+    Row ru = g.row[u], rv = g.row[v];
+    if (rv.len < ru.len) { Row t = ru; ru = rv; rv = t; int32_t s = u; u = v; v = s; }
+    const int32_t* a = g.pool + ru.start;
+    int lo = 0, hi = ru.len;
+    bool hit = false;
+    while (lo < hi) {
+        const int n = hi - lo, mid = lo + (n >> 1), q1 = lo + (n >> 2), q3 = mid + (n >> 2);
+        const int32_t x1 = a[q1], x2 = a[mid], x3 = a[q3];
+        hit = x1 == v || x2 == v || x3 == v;
+        if (hit) break;
+        if (x1 > v) hi = q1;
+        else if (x2 > v) { lo = q1 + 1; hi = mid; }
+        else if (x3 > v) { lo = mid + 1; hi = q3; }
+        else lo = q3 + 1;
+    }
+    return hit;
 }
 
 // ---------------------------------------------------------------------------------------

@@ -152,6 +152,7 @@ struct scout_ctx {
     int32_t* d_longs = nullptr;     // long affected rows compacted in place (2m)
     scout::MergeRow* d_mrow = nullptr;   // merge records: short rows from the front, others from the back (2m)
     int64_t* d_slices = nullptr;  int64_t cap_slices = 0;   // merge items (row << 32 | slice)
+    void* d_update = nullptr;       // scratch of the one-launch update
     int64_t* d_coff = nullptr;      // compaction offsets (n + 1)
     int key_bits = 0;
 

@@ -123,22 +123,25 @@ __device__ __forceinline__ unsigned long long pack_key(uint32_t u, uint32_t op, 
     return ((unsigned long long)u << (B + 1)) | ((unsigned long long)op << B) | v;
 }
 
+// One edit's classification: bit 0 valid, bit 1 insertion, bit 2 applied. WIDE as in plan_search.
+template <bool WIDE>
+__device__ __forceinline__ int classify_edit(const DGraph& g, int32_t u, int32_t v, int op) {
+    if (!(u >= 0 && u < g.n && v >= 0 && v < g.n && u != v)) return 0;
+    const bool adj = WIDE ? dg_adjacent_wide(g, u, v) : dg_adjacent(g, u, v);
+    bool ins = op == SCOUT_OP_INSERT, applied = op == SCOUT_OP_INSERT ? !adj : adj;
+    if (op != SCOUT_OP_INSERT && op != SCOUT_OP_DELETE) { ins = !adj; applied = true; }
+    return 1 | (ins ? 2 : 0) | (applied ? 4 : 0);
+}
+
 __global__ void k_classify(DGraph g, const scout_edge* __restrict__ e, const uint8_t* __restrict__ ops, int64_t m,
                            int B, unsigned long long* __restrict__ keys, uint8_t* __restrict__ eflag,
                            DevCounters* __restrict__ ctr, int emit) {
     const unsigned long long SENT = (B + B + 1) >= 64 ? ~0ull : ((1ull << (B + B + 1)) - 1);
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x) {
-        int32_t u = e[i].u, v = e[i].v;
-        bool valid = u >= 0 && u < g.n && v >= 0 && v < g.n && u != v;
-        bool ins = false, applied = false;
-        if (valid) {
-            bool adj = dg_adjacent(g, u, v);
-            int op = ops ? ops[i] : SCOUT_OP_TOGGLE;
-            if (op == SCOUT_OP_INSERT) { ins = true; applied = !adj; }
-            else if (op == SCOUT_OP_DELETE) { ins = false; applied = adj; }
-            else { ins = !adj; applied = true; }
-        }
-        eflag[i] = (uint8_t)((valid ? 1 : 0) | (ins ? 2 : 0) | (applied ? 4 : 0));
+        const int32_t u = e[i].u, v = e[i].v;
+        const int f = classify_edit<false>(g, u, v, ops ? ops[i] : SCOUT_OP_TOGGLE);
+        const bool valid = f & 1, ins = f & 2, applied = f & 4;
+        eflag[i] = (uint8_t)f;
         unsigned mi = __ballot_sync(__activemask(), valid && ins);
         unsigned md = __ballot_sync(__activemask(), valid && !ins);
         unsigned ma = __ballot_sync(__activemask(), valid && applied);
@@ -187,6 +190,134 @@ constexpr unsigned long long PLAN_TAG = 0x5Aull << 56;
 // in flight, and neighbouring threads search the same rows). 10^6 edits at scale 22: 123 us; the
 // launches it replaces (segment heads and tails, two searches of every half-edit, a scan and its
 // clears) took 300 us, and on small batches most of their time was the seven launches.
+//
+// plan_search: the searches of a thread's half-edits k0 + STRIDE s (`at(k)` reads sorted half-edit
+// k), their positions, and the warps' head and match ballots. Warps converge on return.
+// WIDE: three probes per step (a quarter of the range is left) where the chain of dependent
+// reads is all there is, on batches too small to fill the memory system; one probe (half) else.
+template <int STEPS, int STRIDE, bool WIDE, typename At>
+__device__ __forceinline__ void plan_search(const Row* __restrict__ row, const int32_t* __restrict__ pool,
+                                            const unsigned long long (&key)[STEPS], int B, int nh, int k0, At at,
+                                            uint32_t* __restrict__ epos, unsigned (&hm)[STEPS], unsigned (&mm)[STEPS]) {
+    const int32_t* O[STEPS];
+    int lo[STEPS], hi[STEPS], len[STEPS];
+#pragma unroll
+    for (int s = 0; s < STEPS; s++) {
+        lo[s] = hi[s] = len[s] = 0;
+        O[s] = pool;
+        if (k0 + s * STRIDE < nh) {
+            const Row r = row[key_u(key[s], B)];
+            O[s] = pool + r.start;
+            len[s] = hi[s] = r.len;
+        }
+    }
+    // lower bounds, one step of every search per turn
+    while (true) {
+        bool more = false;
+        int32_t x[STEPS], x1[STEPS], x3[STEPS];
+#pragma unroll
+        for (int s = 0; s < STEPS; s++)
+            if (lo[s] < hi[s]) {
+                const int n = hi[s] - lo[s];
+                x[s] = O[s][lo[s] + (n >> 1)];
+                if (WIDE) {
+                    x1[s] = O[s][lo[s] + (n >> 2)];
+                    x3[s] = O[s][lo[s] + (n >> 1) + (n >> 2)];
+                }
+            }
+#pragma unroll
+        for (int s = 0; s < STEPS; s++)
+            if (lo[s] < hi[s]) {
+                const int32_t y = key_v(key[s], B);
+                const int n = hi[s] - lo[s], mid = lo[s] + (n >> 1), q1 = lo[s] + (n >> 2), q3 = mid + (n >> 2);
+                if (x[s] < y) lo[s] = mid + 1; else hi[s] = mid;
+                if (WIDE) {   // q1 <= mid <= q3 < the old hi
+                    if (x1[s] >= y) hi[s] = min(hi[s], q1); else lo[s] = max(lo[s], q1 + 1);
+                    if (x3[s] < y) lo[s] = max(lo[s], q3 + 1); else hi[s] = min(hi[s], q3);
+                }
+                more |= lo[s] < hi[s];
+            }
+        if (!more) break;
+    }
+#pragma unroll
+    for (int s = 0; s < STEPS; s++) {
+        const int k = k0 + s * STRIDE;
+        bool matched = false, head = false;
+        if (k < nh) {
+            const unsigned long long kk = key[s];
+            const int32_t y = key_v(kk, B);
+            const unsigned long long pk = k > 0 ? at(k - 1) : ~kk;
+            head = k == 0 || key_u(pk, B) != key_u(kk, B);
+            int pos = lo[s];
+            const bool here = pos < len[s] && O[s][pos] == y;
+            if (key_op(kk, B) == 0) {
+                if (here) pos += (int)upper_bound_i32(O[s] + pos, len[s] - pos, y);
+            } else {
+                int rank = 0;   // copies of this deletion before it
+                if (pk == kk) {
+                    int j = k - 1;
+                    while (j > 0 && at(j - 1) == kk) j--;
+                    rank = k - j;
+                }
+                matched = here && pos + rank < len[s] && O[s][pos + rank] == y;
+                if (matched) pos += rank;
+                else if (here) pos += (int)upper_bound_i32(O[s] + pos, len[s] - pos, y);
+            }
+            epos[k] = ((uint32_t)pos << 1) | (matched ? 1u : 0u);
+        }
+        hm[s] = __ballot_sync(0xffffffffu, head);
+        mm[s] = __ballot_sync(0xffffffffu, matched);
+    }
+}
+
+// plan_finish: the segments and running counts, given the heads << 32 | matches before the warp.
+template <int STEPS, typename At>
+__device__ __forceinline__ void plan_finish(const unsigned long long (&key)[STEPS], int B, int nh, int k0, At at,
+                                            const unsigned (&hm)[STEPS], const unsigned (&mm)[STEPS],
+                                            unsigned long long base, DevCounters* __restrict__ ctr,
+                                            int32_t* __restrict__ aff, int32_t* __restrict__ seg_b,
+                                            int32_t* __restrict__ seg_d, int32_t* __restrict__ E) {
+    const unsigned l = lane_id(), lt = (1u << l) - 1;
+    int heads = (int)(base >> 32), match = (int)(base & 0xffffffffu);
+#pragma unroll
+    for (int s = 0; s < STEPS; s++) {
+        const int k = k0 + s * WARP;
+        if (k < nh) {
+            const unsigned long long kk = key[s];
+            const int32_t u = key_u(kk, B);
+            const bool head = (hm[s] >> l) & 1u;
+            const int a = heads + __popc(hm[s] & lt) + (head ? 1 : 0) - 1;
+            const int e = match + __popc(mm[s] & lt);
+            E[k] = e;
+            if (head) {
+                aff[a] = u;
+                seg_b[a] = k;
+            }
+            const int op = key_op(kk, B);
+            if (op == 1) {
+                if (head || key_op(at(k - 1), B) == 0) seg_d[a] = k;
+            } else if (k == nh - 1 || key_u(at(k + 1), B) != u) {
+                seg_d[a] = k + 1;
+            }
+            if (k == nh - 1) {
+                E[nh] = e + (int)((mm[s] >> l) & 1u);
+                seg_b[a + 1] = nh;
+                ctr->n_aff = a + 1;
+            }
+        }
+        heads += __popc(hm[s]);
+        match += __popc(mm[s]);
+    }
+}
+
+template <int STEPS>
+__device__ __forceinline__ unsigned long long plan_count(const unsigned (&hm)[STEPS], const unsigned (&mm)[STEPS]) {
+    unsigned long long c = 0;
+#pragma unroll
+    for (int s = 0; s < STEPS; s++) c += ((unsigned long long)__popc(hm[s]) << 32) | (unsigned)__popc(mm[s]);
+    return c;
+}
+
 __global__ void __launch_bounds__(PLAN_THREADS) k_plan(const Row* __restrict__ row, const int32_t* __restrict__ pool,
                                                        const unsigned long long* __restrict__ keys, int B,
                                                        DevCounters* __restrict__ ctr, int32_t* __restrict__ aff,
@@ -202,79 +333,18 @@ __global__ void __launch_bounds__(PLAN_THREADS) k_plan(const Row* __restrict__ r
     if (threadIdx.x == 0) s_tile = atomicAdd(&ctr->plan_ticket, 1);
     __syncthreads();
     const int tile = s_tile;
-    const int k0 = tile * PLAN_TILE + w * (PLAN_STEPS * WARP) + (int)l;
     if (tile * (long long)PLAN_TILE >= nh) return;   // whole block; no tile after it has work either
+    const int k0 = tile * PLAN_TILE + w * (PLAN_STEPS * WARP) + (int)l;
+    auto at = [&](int k) { return keys[k]; };
     unsigned long long key[PLAN_STEPS];
-    const int32_t* O[PLAN_STEPS];
-    int lo[PLAN_STEPS], hi[PLAN_STEPS], len[PLAN_STEPS];
 #pragma unroll
     for (int s = 0; s < PLAN_STEPS; s++) {
         const int k = k0 + s * WARP;
         key[s] = k < nh ? keys[k] : ~0ull;
     }
-#pragma unroll
-    for (int s = 0; s < PLAN_STEPS; s++) {
-        lo[s] = hi[s] = len[s] = 0;
-        O[s] = pool;
-        if (k0 + s * WARP < nh) {
-            const Row r = row[key_u(key[s], B)];
-            O[s] = pool + r.start;
-            len[s] = hi[s] = r.len;
-        }
-    }
-    // lower bounds, one step of every search per turn
-    while (true) {
-        bool more = false;
-        int32_t x[PLAN_STEPS];
-#pragma unroll
-        for (int s = 0; s < PLAN_STEPS; s++)
-            if (lo[s] < hi[s]) x[s] = O[s][(lo[s] + hi[s]) >> 1];
-#pragma unroll
-        for (int s = 0; s < PLAN_STEPS; s++)
-            if (lo[s] < hi[s]) {
-                const int mid = (lo[s] + hi[s]) >> 1;
-                if (x[s] < key_v(key[s], B)) lo[s] = mid + 1; else hi[s] = mid;
-                more |= lo[s] < hi[s];
-            }
-        if (!more) break;
-    }
     unsigned hm[PLAN_STEPS], mm[PLAN_STEPS];
-#pragma unroll
-    for (int s = 0; s < PLAN_STEPS; s++) {
-        const int k = k0 + s * WARP;
-        bool matched = false, head = false;
-        if (k < nh) {
-            const unsigned long long kk = key[s];
-            const int32_t y = key_v(kk, B);
-            const unsigned long long pk = k > 0 ? keys[k - 1] : ~kk;
-            head = k == 0 || key_u(pk, B) != key_u(kk, B);
-            int at = lo[s];
-            const bool here = at < len[s] && O[s][at] == y;
-            if (key_op(kk, B) == 0) {
-                if (here) at += (int)upper_bound_i32(O[s] + at, len[s] - at, y);
-            } else {
-                int rank = 0;   // copies of this deletion before it
-                if (pk == kk) {
-                    int j = k - 1;
-                    while (j > 0 && keys[j - 1] == kk) j--;
-                    rank = k - j;
-                }
-                matched = here && at + rank < len[s] && O[s][at + rank] == y;
-                if (matched) at += rank;
-                else if (here) at += (int)upper_bound_i32(O[s] + at, len[s] - at, y);
-            }
-            epos[k] = ((uint32_t)at << 1) | (matched ? 1u : 0u);
-        }
-        hm[s] = __ballot_sync(0xffffffffu, head);
-        mm[s] = __ballot_sync(0xffffffffu, matched);
-    }
-    // heads << 32 | matched deletions: per warp, then before this tile
-    if (l == 0) {
-        unsigned long long c = 0;
-#pragma unroll
-        for (int s = 0; s < PLAN_STEPS; s++) c += ((unsigned long long)__popc(hm[s]) << 32) | (unsigned)__popc(mm[s]);
-        s_cnt[w] = c;
-    }
+    plan_search<PLAN_STEPS, WARP, false>(row, pool, key, B, nh, k0, at, epos, hm, mm);
+    if (l == 0) s_cnt[w] = plan_count<PLAN_STEPS>(hm, mm);
     __syncthreads();
     if (w == 0) {   // publish, look back 32 tiles per step, publish the prefix
         unsigned long long tot = 0;
@@ -328,37 +398,7 @@ __global__ void __launch_bounds__(PLAN_THREADS) k_plan(const Row* __restrict__ r
     __syncthreads();
     unsigned long long base = s_prefix;
     for (int j = 0; j < w; j++) base += s_cnt[j];
-    int heads = (int)(base >> 32), match = (int)(base & 0xffffffffu);
-    const unsigned lt = (1u << l) - 1;
-#pragma unroll
-    for (int s = 0; s < PLAN_STEPS; s++) {
-        const int k = k0 + s * WARP;
-        if (k < nh) {
-            const unsigned long long kk = key[s];
-            const int32_t u = key_u(kk, B);
-            const bool head = (hm[s] >> l) & 1u;
-            const int a = heads + __popc(hm[s] & lt) + (head ? 1 : 0) - 1;
-            const int e = match + __popc(mm[s] & lt);
-            E[k] = e;
-            if (head) {
-                aff[a] = u;
-                seg_b[a] = k;
-            }
-            const int op = key_op(kk, B);
-            if (op == 1) {
-                if (head || key_op(keys[k - 1], B) == 0) seg_d[a] = k;
-            } else if (k == nh - 1 || key_u(keys[k + 1], B) != u) {
-                seg_d[a] = k + 1;
-            }
-            if (k == nh - 1) {
-                E[nh] = e + (int)((mm[s] >> l) & 1u);
-                seg_b[a + 1] = nh;
-                ctr->n_aff = a + 1;
-            }
-        }
-        heads += __popc(hm[s]);
-        match += __popc(mm[s]);
-    }
+    plan_finish<PLAN_STEPS>(key, B, nh, k0, at, hm, mm, base, ctr, aff, seg_b, seg_d, E);
 }
 
 // Per affected row: the space of its new version (old length + insertions: slots of matched
@@ -385,21 +425,24 @@ struct RowPlan {
     long long base_hbm, base_host;
 };
 
-__device__ __forceinline__ long long block_scan_rows(long long x, long long* total) {
-    __shared__ long long ws[ROW_THREADS / WARP];
-    const long long inc = warp_incl_scan(x);
-    const int w = threadIdx.x / WARP;
-    __syncthreads();   // the previous scan's sums are read
-    if (lane_id() == WARP - 1) ws[w] = inc;
+// Exclusive scans of two values over the block (at most 32 warps) at once, and their totals.
+__device__ __forceinline__ void block_scan2(long long& x, long long& y, long long* tx, long long* ty) {
+    __shared__ long long ws[2][WARP + 1];
+    const int w = threadIdx.x / WARP, l = (int)lane_id();
+    const long long ix = warp_incl_scan(x), iy = warp_incl_scan(y);
+    if (l == WARP - 1) { ws[0][w] = ix; ws[1][w] = iy; }
     __syncthreads();
-    long long before = 0, tot = 0;
-#pragma unroll
-    for (int j = 0; j < ROW_THREADS / WARP; j++) {
-        before += j < w ? ws[j] : 0;
-        tot += ws[j];
+    if (w < 2) {
+        const long long v = l < (int)(blockDim.x / WARP) ? ws[w][l] : 0;
+        const long long iv = warp_incl_scan(v);
+        ws[w][l] = iv - v;
+        if (l == WARP - 1) ws[w][WARP] = iv;
     }
-    *total = tot;
-    return before + inc - x;
+    __syncthreads();
+    x = ws[0][w] + ix - x;
+    y = ws[1][w] + iy - y;
+    *tx = ws[0][WARP];
+    *ty = ws[1][WARP];
 }
 
 // Tiered store: the growth of each destination, before anything is placed.
@@ -422,12 +465,16 @@ __global__ void __launch_bounds__(ROW_THREADS) k_row_sizes(RowPlan p) {
     if (lane_id() == 0 && nc) atomicAdd((unsigned long long*)&p.ctr->new_elems_host, (unsigned long long)nc);
 }
 
-__global__ void __launch_bounds__(ROW_THREADS) k_row_plan(RowPlan p) {
+// BLOCK: rows are taken a block's threads at a time, with one set of atomics on the counters;
+// else 32 at a time by a warp, with no barrier (few rows, nothing to save on atomics).
+template <bool BLOCK>
+__device__ __forceinline__ void row_plan(const RowPlan& p, int A, int group, int groups) {
+    const int ROWS = BLOCK ? (int)blockDim.x : WARP;
     __shared__ long long s_base[6];
-    const int A = p.ctr->n_aff;
+    const int t = BLOCK ? (int)threadIdx.x : (int)lane_id();
     long long nnz_delta = 0, bytes = 0;
-    for (int a0 = blockIdx.x * ROW_THREADS; a0 < A; a0 += gridDim.x * ROW_THREADS) {
-        const int a = a0 + threadIdx.x;
+    for (int a0 = group * ROWS; a0 < A; a0 += groups * ROWS) {
+        const int a = a0 + t;
         const bool ok = a < A;
         Row r{0, 0, 0};
         int32_t u = 0;
@@ -435,10 +482,10 @@ __global__ void __launch_bounds__(ROW_THREADS) k_row_plan(RowPlan p) {
         bool ip = false, cold = false, sm = false, lip = false;
         if (ok) {
             u = p.aff[a];
-            r = p.row[u];
             b = p.seg_b[a];
             d = p.seg_d[a];
             e = p.seg_b[a + 1];
+            r = p.row[u];
             nl = r.len + (d - b) - (p.E[e] - p.E[d]);
             ip = in_place_row(d - b, r.len, p.long_in_place);
             cold = p.split && !in_hbm(r, p.hbm_cap);
@@ -449,33 +496,58 @@ __global__ void __launch_bounds__(ROW_THREADS) k_row_plan(RowPlan p) {
             bytes += 4LL * ((long long)r.len + nl) + 8LL * (e - b) + 16;
         }
         const long long need = ok && !ip ? (long long)r.len + (d - b) : 0;
-        long long th, tc = 0, tn, oh, oc = 0;
-        oh = block_scan_rows(cold ? 0 : need, &th);
-        if (p.split) oc = block_scan_rows(cold ? need : 0, &tc);
-        // counts packed: slices 34 bits, short rows, other rows, long rows in place 10 bits each
-        const long long on = block_scan_rows((long long)ns | ((long long)(ok && sm) << 34) | ((long long)(ok && !sm) << 44) |
-                                                 ((long long)lip << 54), &tn);
-        if (threadIdx.x == 0) {
-            if (th) s_base[0] = (long long)atomicAdd((unsigned long long*)&p.ctr->new_elems, (unsigned long long)th);
-            if (tc) s_base[1] = (long long)atomicAdd((unsigned long long*)&p.ctr->new_elems_host, (unsigned long long)tc);
-            s_base[2] = atomicAdd(&p.ctr->n_slices, (int)(tn & ((1ll << 34) - 1)));
-            s_base[3] = atomicAdd(&p.ctr->n_small, (int)(tn >> 34) & 1023);
-            s_base[4] = atomicAdd(&p.ctr->n_long, (int)(tn >> 44) & 1023);
-            s_base[5] = atomicAdd(&p.ctr->n_large, (int)(tn >> 54) & 1023);
+        // counts packed: slices 30 bits, short rows, other rows, long rows in place 11 bits each
+        long long th, tc = 0, tn, t0, oh = cold ? 0 : need, oc = 0;
+        long long on = (long long)ns | ((long long)(ok && sm) << 30) | ((long long)(ok && !sm) << 41) | ((long long)lip << 52);
+        auto scan2 = [](long long& x, long long& y, long long* tx, long long* ty) {
+            if (BLOCK) {
+                block_scan2(x, y, tx, ty);
+            } else {
+                const long long ix = warp_incl_scan(x), iy = warp_incl_scan(y);
+                x = ix - x;
+                y = iy - y;
+                *tx = __shfl_sync(0xffffffffu, ix, WARP - 1);
+                *ty = __shfl_sync(0xffffffffu, iy, WARP - 1);
+            }
+        };
+        scan2(oh, on, &th, &tn);
+        if (p.split) {
+            long long zero = 0;
+            oc = cold ? need : 0;
+            if (BLOCK) __syncthreads();   // the first scan's sums are read
+            scan2(oc, zero, &tc, &t0);
         }
-        __syncthreads();
+        // one thread per counter: the atomics' latencies overlap
+        long long base = 0;
+        if (t < 2) {
+            const long long x = t ? tc : th;
+            if (x)
+                base = (long long)atomicAdd((unsigned long long*)(t ? &p.ctr->new_elems_host : &p.ctr->new_elems),
+                                            (unsigned long long)x);
+        } else if (t < 6) {
+            int* to = t == 2 ? &p.ctr->n_slices : t == 3 ? &p.ctr->n_small : t == 4 ? &p.ctr->n_long : &p.ctr->n_large;
+            const int x = t == 2 ? (int)(tn & ((1ll << 30) - 1)) : (int)(tn >> (30 + 11 * (t - 3))) & 2047;
+            if (x) base = atomicAdd(to, x);
+        }
+        long long bs[6];
+        if (BLOCK) {
+            if (t < 6) s_base[t] = base;
+            __syncthreads();
+        }
+#pragma unroll
+        for (int j = 0; j < 6; j++) bs[j] = BLOCK ? s_base[j] : __shfl_sync(0xffffffffu, base, j);
         if (ok) {
             long long dst = r.start;
-            if (!ip) dst = cold ? p.base_host + s_base[1] + oc : p.base_hbm + s_base[0] + oh;
-            const long long at = sm ? s_base[3] + ((on >> 34) & 1023) : p.mcap - 1 - (s_base[4] + ((on >> 44) & 1023));
+            if (!ip) dst = cold ? p.base_host + bs[1] + oc : p.base_hbm + bs[0] + oh;
+            const long long at = sm ? bs[3] + ((on >> 30) & 2047) : p.mcap - 1 - (bs[4] + ((on >> 41) & 2047));
             p.mrow[at] = MergeRow{r.start, dst, r.len, b, d, e};
             p.row[u] = ip ? Row{r.start, nl, r.cap} : Row{dst, nl, r.len + (d - b)};
-            if (lip) p.longs[s_base[5] + ((on >> 54) & 1023)] = (int32_t)at;
-            const long long s0 = s_base[2] + (on & ((1ll << 34) - 1));
+            if (lip) p.longs[bs[5] + ((on >> 52) & 2047)] = (int32_t)at;
+            const long long s0 = bs[2] + (on & ((1ll << 30) - 1));
             if (s0 + ns > p.slice_cap) { if (ns) atomicExch(&p.ctr->overflow, 1); }
             else for (int s = 0; s < ns; s++) p.slices[s0 + s] = (at << 32) | s;
         }
-        __syncthreads();   // the bases are read before the next rows overwrite them
+        if (BLOCK) __syncthreads();   // the bases and sums are read before the next rows overwrite them
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -486,6 +558,10 @@ __global__ void __launch_bounds__(ROW_THREADS) k_row_plan(RowPlan p) {
         atomicAdd((unsigned long long*)&p.ctr->nnz_delta, (unsigned long long)nnz_delta);
         atomicAdd((unsigned long long*)&p.ctr->update_bytes, (unsigned long long)bytes);
     }
+}
+
+__global__ void __launch_bounds__(ROW_THREADS) k_row_plan(RowPlan p) {
+    row_plan<true>(p, p.ctr->n_aff, (int)blockIdx.x, (int)gridDim.x);
 }
 
 // ---- the merge -------------------------------------------------------------------------------
@@ -735,18 +811,19 @@ static __device__ __forceinline__ void merge_short(int32_t* __restrict__ pool, c
     }
 }
 
-__global__ void __launch_bounds__(MERGE_THREADS, 4) k_merge(
-        int32_t* __restrict__ pool, const unsigned long long* __restrict__ keys, int B, DevCounters* __restrict__ ctr,
-        const uint32_t* __restrict__ epos, const int32_t* __restrict__ E, const MergeRow* __restrict__ mrow, int64_t mcap,
-        const int64_t* __restrict__ slices, int64_t slice_cap) {
-    __shared__ ChunkEvents s_ev[MERGE_WARPS];
-    if (ctr->overflow) return;   // the slice list did not fit (the host reports it)
-    const int nsl = (int)min((int64_t)ctr->n_slices, slice_cap);
-    const int nsm = ctr->n_small;
+// The batch's rows, by every warp of the grid; `ev`: the warp's chunk events.
+static __device__ __forceinline__ void merge_rows(int32_t* __restrict__ pool, const unsigned long long* __restrict__ keys,
+                                                  int B, DevCounters* __restrict__ ctr, const uint32_t* __restrict__ epos,
+                                                  const int32_t* __restrict__ E, const MergeRow* __restrict__ mrow,
+                                                  const int64_t* __restrict__ slices, int64_t slice_cap, ChunkEvents& ev) {
+    if (ld_volatile(&ctr->overflow)) return;   // the slice list did not fit (the host reports it)
+    const int nsl = (int)min((int64_t)ld_volatile(&ctr->n_slices), slice_cap);
+    const int nsm = ld_volatile(&ctr->n_small);
     // rows of a warp's turn: up to 32, fewer while that leaves warps without any
     const int per = min(WARP, max(MERGE_ROWS, (nsm + gwarp_count() - 1) / gwarp_count()));
     const int items = nsl + (nsm + per - 1) / per;
-    int it = gwarp_id();   // the first item of every warp; the rest are handed out
+    // the first item of every warp, neighbouring ones on different SMs; the rest are handed out
+    int it = (int)(threadIdx.x / WARP * gridDim.x + blockIdx.x);
     while (it < items) {
         int nx = 0;
         if (lane_id() == 0) nx = gwarp_count() + atomicAdd(&ctr->merge_ticket, 1);
@@ -756,13 +833,240 @@ __global__ void __launch_bounds__(MERGE_THREADS, 4) k_merge(
             const int s = (int)(item & 0xffffffffLL);
             const bool whole = r.dst == r.start;   // compacted where it lies: one warp, front to back
             const int s0 = whole ? 0 : s * SLICE;
-            merge_slice(pool, keys, B, epos, E, r, s0, whole ? r.len : min(r.len, s0 + SLICE), s_ev[threadIdx.x / WARP]);
+            merge_slice(pool, keys, B, epos, E, r, s0, whole ? r.len : min(r.len, s0 + SLICE), ev);
         } else {
             const int i0 = (it - nsl) * per;
             merge_short(pool, keys, B, epos, mrow, i0, min(per, nsm - i0));
         }
         it = __shfl_sync(0xffffffffu, nx, 0);
     }
+}
+
+__global__ void __launch_bounds__(MERGE_THREADS, 4) k_merge(
+        int32_t* __restrict__ pool, const unsigned long long* __restrict__ keys, int B, DevCounters* __restrict__ ctr,
+        const uint32_t* __restrict__ epos, const int32_t* __restrict__ E, const MergeRow* __restrict__ mrow,
+        const int64_t* __restrict__ slices, int64_t slice_cap) {
+    __shared__ ChunkEvents s_ev[MERGE_WARPS];
+    merge_rows(pool, keys, B, ctr, epos, E, mrow, slices, slice_cap, s_ev[threadIdx.x / WARP]);
+}
+
+// ---- up to UPDATE_MAX edits: the whole update in one launch ------------------------------------
+// A cooperative kernel, one block per SM, of the phases that larger batches launch one by one,
+// with the bounded grid barrier between them: classification; the sort; the plan, a stretch of
+// consecutive half-edits per block, its running counts added up from the blocks before; the
+// rows' plan; the merge. The sort is one of two:
+//   up to UPDATE_PAIRS half-edits   every key's place is the number of smaller keys: a warp per
+//                                   key against all of them in shared memory
+//   more                            sample sort: UPDATE_SPLIT keys at regular places are ranked
+//                                   that way; they split the keys into buckets (about n / 2,048
+//                                   keys each), whose keys are ranked among themselves
+//
+// What bounds it: the latency of two searches in rows, the barriers (6 to 9 of them) and the
+// merge's traffic. Up to UPDATE_MAX edits it is faster than the launches it replaces (each about
+// 4 us on the host, and the radix sort's passes wait on one another): whole call with them and
+// so: 1,000 edits on 65,536 vertices 203 -> 180 us, 10,000 at scale 22 409 -> 363, 100,003 on
+// 1.5 M vertices 466 -> 438. Beyond it a thread would hold more than two keys and the buckets'
+// quadratic ranking overtakes the radix passes.
+constexpr int UPDATE_THREADS = 1024;
+constexpr int UPDATE_WARPS = UPDATE_THREADS / WARP;
+constexpr int64_t UPDATE_MAX = 131072;
+constexpr int UPDATE_PAIRS = 4096;
+constexpr int UPDATE_SPLIT = 2048;
+constexpr int UPDATE_ROWS = 16384;   // more affected rows are planned by blocks, fewer by warps
+// device scratch: splitters, bucket counts, the blocks' plan counts
+constexpr int64_t UPDATE_SCRATCH = UPDATE_SPLIT * 8 + (UPDATE_SPLIT + 64) * 4 + 1024 * 8;
+
+struct UpdateParams {
+    DGraph g;
+    int32_t* pool;
+    const scout_edge* e;
+    const uint8_t* ops;
+    int m, B;
+    unsigned long long* raw;    // half-edits as classified (2m)
+    unsigned long long* tmp;    // half-edits by bucket (may share E's memory, written later)
+    unsigned long long* keys;   // sorted
+    uint8_t* eflag;
+    uint32_t* epos;             // may share `raw`'s memory: written after the sort
+    unsigned long long* split;  // UPDATE_SPLIT
+    int* bucket;                // UPDATE_SPLIT + 1 counts
+    unsigned long long* cnt;    // heads << 32 | matches per block
+    int rows;                   // 0: stop after the plan (tiered store: the host decides where rows go)
+    RowPlan rp;                 // its aff, seg_b, seg_d and E are written here
+    int32_t *aff, *seg_b, *seg_d, *E;
+    GridBar* bar;
+};
+
+// First index of the ascending a[0, n) whose value is above x (n <= 2^12).
+template <typename T>
+__device__ __forceinline__ int first_above(const T* a, int n, T x) {
+    int lo = 0, hi = n;
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (a[mid] <= x) lo = mid + 1; else hi = mid;
+    }
+    return lo;
+}
+
+// The half-edits p.raw[0, n) in ascending order into p.keys, all blocks; `smem`: 32 KB. Returns
+// false when a barrier failed. Ends before a barrier: the caller's next one publishes the order.
+static __device__ bool update_sort(const UpdateParams& p, int n, unsigned long long SENT, unsigned char* smem) {
+    const int t = threadIdx.x, w = t / WARP, l = (int)lane_id();
+    const int G = (int)gridDim.x, wid = w * G + (int)blockIdx.x, W = G * UPDATE_WARPS;
+    const int tid = (int)blockIdx.x * UPDATE_THREADS + t, T = G * UPDATE_THREADS;
+    unsigned long long* k = (unsigned long long*)smem;
+    if (n <= UPDATE_PAIRS) {
+        for (int i = t; i < n; i += UPDATE_THREADS) k[i] = ld_volatile(p.raw + i);
+        __syncthreads();
+        for (int j = wid; j < n; j += W) {
+            const unsigned long long x = k[j];
+            if (x == SENT) continue;   // past the half-edits; no one reads it
+            int c = 0;
+            for (int i = l; i < n; i += WARP) c += k[i] < x || (k[i] == x && i < j);
+            c = __reduce_add_sync(0xffffffffu, c);
+            if (l == 0) p.keys[c] = x;
+        }
+        return true;
+    }
+    // the sample, ranked like that
+    for (int i = t; i < UPDATE_SPLIT; i += UPDATE_THREADS) k[i] = ld_volatile(p.raw + (long long)i * n / UPDATE_SPLIT);
+    __syncthreads();
+    for (int j = wid; j < UPDATE_SPLIT; j += W) {
+        const unsigned long long x = k[j];
+        int c = 0;
+        for (int i = l; i < UPDATE_SPLIT; i += WARP) c += k[i] < x || (k[i] == x && i < j);
+        c = __reduce_add_sync(0xffffffffu, c);
+        if (l == 0) p.split[c] = x;
+    }
+    if (!grid_sync(p.bar, 65)) return false;
+    // every key's bucket and its place there (in the order the atomics came)
+    for (int i = t; i < UPDATE_SPLIT; i += UPDATE_THREADS) k[i] = ld_volatile(p.split + i);
+    __syncthreads();
+    unsigned long long key[2] = {SENT, SENT};   // n <= 2 T
+    int b[2] = {0, 0}, at[2] = {0, 0};
+#pragma unroll
+    for (int s = 0; s < 2; s++) {
+        const int i = tid + s * T;
+        if (i < n) key[s] = ld_volatile(p.raw + i);
+        if (key[s] != SENT) {
+            b[s] = first_above(k, UPDATE_SPLIT, key[s]);
+            at[s] = atomicAdd(p.bucket + b[s], 1);
+        }
+    }
+    if (!grid_sync(p.bar, 66)) return false;
+    int* off = (int*)smem;   // the buckets' first places, and the end
+    {
+        static_assert(UPDATE_SPLIT == 2 * UPDATE_THREADS, "two buckets per thread and the last one");
+        const int c0 = ld_volatile(p.bucket + 2 * t), c1 = ld_volatile(p.bucket + 2 * t + 1);
+        long long x = c0 + c1, y = 0, tx, ty;
+        block_scan2(x, y, &tx, &ty);   // its barriers are past the splitters' last reader
+        off[2 * t] = (int)x;
+        off[2 * t + 1] = (int)x + c0;
+        if (t == 0) {
+            off[UPDATE_SPLIT] = (int)tx;
+            off[UPDATE_SPLIT + 1] = (int)tx + ld_volatile(p.bucket + UPDATE_SPLIT);
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int s = 0; s < 2; s++)
+        if (key[s] != SENT) p.tmp[off[b[s]] + at[s]] = key[s];
+    if (!grid_sync(p.bar, 67)) return false;
+    const int total = off[UPDATE_SPLIT + 1];
+    for (int i = tid; i < total; i += T) {
+        const unsigned long long x = ld_volatile(p.tmp + i);
+        const int q = first_above(off, UPDATE_SPLIT + 2, i) - 1;   // the bucket of place i
+        const int q0 = off[q], q1 = off[q + 1];
+        int c = 0;
+        for (int j = q0; j < q1; j++) {
+            const unsigned long long y = p.tmp[j];
+            c += y < x || (y == x && j < i);
+        }
+        p.keys[q0 + c] = x;
+    }
+    return true;
+}
+
+__global__ void __launch_bounds__(UPDATE_THREADS, 1) k_update(UpdateParams p) {
+    __shared__ __align__(16) unsigned char s_mem[UPDATE_PAIRS * 8];   // the sort's, later the warps' chunk events
+    static_assert(sizeof(s_mem) >= UPDATE_WARPS * sizeof(ChunkEvents) && sizeof(s_mem) >= UPDATE_SPLIT * 8, "fits");
+    const int t = threadIdx.x, w = t / WARP, l = (int)lane_id();
+    const int G = (int)gridDim.x, T = G * UPDATE_THREADS;
+    const int B = p.B;
+    DevCounters* ctr = p.rp.ctr;
+    // classification; neighbouring edits on different SMs
+    const unsigned long long SENT = (B + B + 1) >= 64 ? ~0ull : ((1ull << (B + B + 1)) - 1);
+    if (blockIdx.x == 0)
+        for (int i = t; i <= UPDATE_SPLIT; i += UPDATE_THREADS) p.bucket[i] = 0;
+    for (int i0 = t * G; i0 - l * G < p.m; i0 += T) {   // uniform per warp
+        const int i = i0 + (int)blockIdx.x;
+        int f = 0;
+        if (i < p.m) {
+            const int32_t u = p.e[i].u, v = p.e[i].v;
+            f = classify_edit<true>(p.g, u, v, p.ops ? p.ops[i] : SCOUT_OP_TOGGLE);
+            p.eflag[i] = (uint8_t)f;
+            const bool half = (f & 5) == 5;
+            const uint32_t op = f & 2 ? 0u : 1u;
+            p.raw[2 * i] = half ? pack_key((uint32_t)u, op, (uint32_t)v, B) : SENT;
+            p.raw[2 * i + 1] = half ? pack_key((uint32_t)v, op, (uint32_t)u, B) : SENT;
+        }
+        const unsigned mi = __ballot_sync(0xffffffffu, (f & 3) == 3), md = __ballot_sync(0xffffffffu, (f & 3) == 1);
+        const unsigned ma = __ballot_sync(0xffffffffu, (f & 5) == 5);
+        if (l == 0) {
+            if (mi) atomicAdd(&ctr->n_ins, __popc(mi));
+            if (md) atomicAdd(&ctr->n_del, __popc(md));
+            if (ma) atomicAdd(&ctr->n_half, 2 * __popc(ma));
+        }
+    }
+    if (!grid_sync(p.bar, 60)) return;
+    if (!update_sort(p, 2 * p.m, SENT, s_mem)) return;
+    if (!grid_sync(p.bar, 61)) return;
+    // the plan: per block a stretch of whole 32-groups, at most 2,048 half-edits
+    const int nh = ld_volatile(&ctr->n_half);
+    const int groups = (nh + WARP - 1) / WARP;
+    const int stretch = (groups + G - 1) / G * WARP;
+    const int first = (int)blockIdx.x * stretch, end = min(nh, first + stretch);
+    const int k0 = first + t;
+    auto at = [&](int k) { return ld_volatile(p.keys + k); };
+    unsigned long long key[2];
+#pragma unroll
+    for (int s = 0; s < 2; s++) key[s] = k0 + s * UPDATE_THREADS < end ? at(k0 + s * UPDATE_THREADS) : ~0ull;
+    unsigned hm[2], mm[2];
+    plan_search<2, UPDATE_THREADS, true>(p.g.row, p.g.pool, key, B, end, k0, at, p.epos, hm, mm);
+    // counts of the warp's two groups: the first groups of all warps come before the second ones
+    long long c0 = 0, c1 = 0, t0, t1;
+    if (l == 0) {
+        c0 = ((long long)__popc(hm[0]) << 32) | __popc(mm[0]);
+        c1 = ((long long)__popc(hm[1]) << 32) | __popc(mm[1]);
+    }
+    block_scan2(c0, c1, &t0, &t1);
+    if (t == 0) p.cnt[blockIdx.x] = (unsigned long long)(t0 + t1);
+    if (!grid_sync(p.bar, 62)) return;
+    long long all = 0, before = 0;
+    for (int j = l; j < G; j += WARP) {
+        const long long c = (long long)ld_volatile(p.cnt + j);
+        all += c;
+        before += j < (int)blockIdx.x ? c : 0;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        all += __shfl_xor_sync(0xffffffffu, all, o);
+        before += __shfl_xor_sync(0xffffffffu, before, o);
+    }
+#pragma unroll
+    for (int s = 0; s < 2; s++) {   // lane 0's exclusive counts are those before the group
+        const long long base = before + (s ? t0 : 0) + __shfl_sync(0xffffffffu, s ? c1 : c0, 0);
+        const unsigned long long kk[1] = {key[s]};
+        const unsigned h1[1] = {hm[s]}, m1[1] = {mm[s]};
+        const int k = k0 + s * UPDATE_THREADS;
+        plan_finish<1>(kk, B, k < end ? nh : 0, k, at, h1, m1, (unsigned long long)base, ctr, p.aff, p.seg_b, p.seg_d, p.E);
+    }
+    if (!p.rows) return;
+    if (!grid_sync(p.bar, 63)) return;
+    const int A = (int)(all >> 32);
+    if (A > UPDATE_ROWS) row_plan<true>(p.rp, A, (int)blockIdx.x, G);
+    else row_plan<false>(p.rp, A, w * G + (int)blockIdx.x, G * UPDATE_WARPS);
+    if (!grid_sync(p.bar, 64)) return;
+    merge_rows(p.pool, p.keys, B, ctr, p.epos, p.E, p.rp.mrow, p.rp.slices, p.rp.slice_cap, ((ChunkEvents*)s_mem)[w]);
 }
 
 // Long rows that only lose entries, compacted in place: one block per row streams it front to
@@ -1026,9 +1330,15 @@ int ws_ensure(scout_ctx* c, int64_t m) {
     return SCOUT_OK;
 }
 
+static int update_ensure(scout_ctx* c) {   // scratch of the one-launch update
+    if (c->d_update) return SCOUT_OK;
+    return dev_alloc(c, &c->d_update, (size_t)UPDATE_SCRATCH, "update scratch");
+}
+
 int graph_reserve_batch(scout_ctx* c, int64_t m) {
     SCOUT_RC(lists_ensure(c));
     SCOUT_RC(ws_ensure(c, m));
+    SCOUT_RC(update_ensure(c));
     const int64_t Amax = std::min<int64_t>(2 * m, c->n);
     SCOUT_RC(dev_grow(c, &c->d_slices, &c->cap_slices, c->pool_cap / SLICE + Amax + 1024, "merge slices"));
     SCOUT_RC(sort_reserve(c, std::max<int64_t>(2 * c->ws_m, c->n + 1)));
@@ -1343,26 +1653,11 @@ int graph_update(scout_ctx* c, const scout_edge* edits, const uint8_t* ops, int6
     SCOUT_RC(upload_edits(c, edits, ops, m, &d_src));
     SCOUT_CU(c, cudaEventRecord(c->ev_t[3], c->s_main));
     DGraph g = dgraph(c);
-    k_classify<<<blocks_for(m, 256), 256, 0, c->s_main>>>(g, d_src, ops ? c->d_ops : nullptr, m, B, c->d_keys,
-                                                         c->d_eflag, c->d_ctr, 1);
-    SCOUT_LAUNCH(c, "k_classify");
-    c->nlaunch += 1;
-    unsigned long long* sorted = nullptr;
-    SCOUT_RC(sort_keys(c, c->d_keys, c->d_keys_alt, 2 * m, 2 * B + 1, &sorted));
-    c->d_hkeys = sorted;
     const int64_t H = 2 * m;
     const int64_t Amax = std::min<int64_t>(H, n);
     // merge slices: the long rows' ceil(len / SLICE) sum to at most nnz / SLICE + Amax
     SCOUT_RC(dev_grow(c, &c->d_slices, &c->cap_slices, c->nnz / SLICE + Amax + 1024, "merge slices"));
-    uint32_t* epos = (uint32_t*)(sorted == c->d_keys ? c->d_keys_alt : c->d_keys);   // the free ping-pong half
     int32_t* E = (int32_t*)c->d_mdp;
-    const int64_t tiles = (H + PLAN_TILE - 1) / PLAN_TILE;
-    SCOUT_RC(dev_grow(c, &c->d_scan_tmp, &c->cap_scan, std::max<int64_t>(64, 1 + 3 * tiles), "scan look-back"));
-    k_plan<<<(unsigned)tiles, PLAN_THREADS, 0, c->s_main>>>(c->row, c->pool, sorted, B, c->d_ctr, c->d_aff, c->d_seg_b,
-                                                            c->d_seg_d, epos, E,
-                                                            (unsigned long long*)c->d_scan_tmp + 1, next_stamp());
-    SCOUT_LAUNCH(c, "k_plan");
-    c->nlaunch += 1;
     RowPlan rp;
     rp.row = c->row;
     rp.ctr = c->d_ctr;
@@ -1381,6 +1676,51 @@ int graph_update(scout_ctx* c, const scout_edge* edits, const uint8_t* ops, int6
     rp.base_hbm = c->tail;
     rp.base_host = 0;
     c->batch_dest = c->tiered ? 2 : 0;
+    unsigned long long* sorted = c->d_keys;
+    uint32_t* epos = (uint32_t*)c->d_keys_alt;
+    const bool one = m <= UPDATE_MAX && H <= 2 * (int64_t)c->sm_count * UPDATE_THREADS;
+    if (one) {
+        SCOUT_RC(update_ensure(c));
+        UpdateParams up;
+        up.g = g;
+        up.pool = c->pool;
+        up.e = d_src;
+        up.ops = ops ? c->d_ops : nullptr;
+        up.m = (int)m;
+        up.B = B;
+        up.raw = c->d_keys_alt;
+        up.tmp = (unsigned long long*)c->d_mdp;
+        up.keys = sorted;
+        up.eflag = c->d_eflag;
+        up.epos = epos;
+        up.split = (unsigned long long*)c->d_update;
+        up.cnt = up.split + UPDATE_SPLIT;
+        up.bucket = (int*)(up.cnt + 1024);
+        up.rows = c->tiered ? 0 : 1;
+        up.rp = rp;
+        up.aff = c->d_aff;
+        up.seg_b = c->d_seg_b;
+        up.seg_d = c->d_seg_d;
+        up.E = E;
+        up.bar = c->d_bar;
+        void* args[] = {&up};
+        SCOUT_RC(coop_launch(c, (const void*)k_update, UPDATE_THREADS, args, 0));
+    } else {
+        k_classify<<<blocks_for(m, 256), 256, 0, c->s_main>>>(g, d_src, ops ? c->d_ops : nullptr, m, B, c->d_keys,
+                                                             c->d_eflag, c->d_ctr, 1);
+        SCOUT_LAUNCH(c, "k_classify");
+        c->nlaunch += 1;
+        SCOUT_RC(sort_keys(c, c->d_keys, c->d_keys_alt, 2 * m, 2 * B + 1, &sorted));
+        epos = (uint32_t*)(sorted == c->d_keys ? c->d_keys_alt : c->d_keys);   // the free ping-pong half
+        const int64_t tiles = (H + PLAN_TILE - 1) / PLAN_TILE;
+        SCOUT_RC(dev_grow(c, &c->d_scan_tmp, &c->cap_scan, std::max<int64_t>(64, 1 + 3 * tiles), "scan look-back"));
+        k_plan<<<(unsigned)tiles, PLAN_THREADS, 0, c->s_main>>>(c->row, c->pool, sorted, B, c->d_ctr, c->d_aff, c->d_seg_b,
+                                                                c->d_seg_d, epos, E,
+                                                                (unsigned long long*)c->d_scan_tmp + 1, next_stamp());
+        SCOUT_LAUNCH(c, "k_plan");
+        c->nlaunch += 1;
+    }
+    c->d_hkeys = sorted;
     const int nbr = blocks_for(Amax, ROW_THREADS, 8 * c->sm_count);
     if (c->tiered) {
         // the exact growth, before anything is written. HBM part too large: compact (evicting
@@ -1434,12 +1774,14 @@ int graph_update(scout_ctx* c, const scout_edge* edits, const uint8_t* ops, int6
         rp.base_hbm = c->batch_dest == 1 ? host_base : c->tail;
         rp.base_host = host_base;
     }
-    k_row_plan<<<nbr, ROW_THREADS, 0, c->s_main>>>(rp);
-    SCOUT_LAUNCH(c, "k_row_plan");
-    k_merge<<<(unsigned)std::min<int64_t>(4 * c->sm_count, (Amax + c->nnz / SLICE) / MERGE_WARPS + 1), MERGE_THREADS, 0,
-              c->s_main>>>(c->pool, sorted, B, c->d_ctr, epos, E, c->d_mrow, 2 * c->ws_m, c->d_slices, c->cap_slices);
-    SCOUT_LAUNCH(c, "k_merge");
-    c->nlaunch += 2;
+    if (!one || c->tiered) {
+        k_row_plan<<<nbr, ROW_THREADS, 0, c->s_main>>>(rp);
+        SCOUT_LAUNCH(c, "k_row_plan");
+        k_merge<<<(unsigned)std::min<int64_t>(4 * c->sm_count, (Amax + c->nnz / SLICE) / MERGE_WARPS + 1), MERGE_THREADS, 0,
+                  c->s_main>>>(c->pool, sorted, B, c->d_ctr, epos, E, c->d_mrow, c->d_slices, c->cap_slices);
+        SCOUT_LAUNCH(c, "k_merge");
+        c->nlaunch += 2;
+    }
     if (c->tiered) {
         k_merge_long_inplace<<<(unsigned)std::min<int64_t>(std::max<int64_t>(1, Amax), 8 * (int64_t)c->sm_count),
                                LIP_THREADS, 0, c->s_main>>>(c->pool, c->d_ctr, epos, c->d_longs, c->d_mrow);

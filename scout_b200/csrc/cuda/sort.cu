@@ -1,14 +1,17 @@
 // sort.cu -- stable LSD radix sort of 64-bit keys and an exclusive int64 scan.
 //
-// The batch merge groups half-edits by (vertex, op, neighbour) with one sort. Small sorts run
-// in one CTA entirely in shared memory (one launch). Larger ones follow the one-sweep scheme
+// The batch merge groups half-edits by (vertex, op, neighbour) with one sort (batches small
+// enough for the one-launch update sort inside it, graph.cu). It follows the one-sweep scheme
 // (Adinets and Merrill, "Onesweep: a faster least significant digit radix sort for GPUs",
 // 2022): one kernel histograms every 8-bit digit of every pass at once and turns the
 // histograms into global digit offsets; then each pass is ONE kernel whose blocks take tiles in
 // order from an atomic counter, rank their keys stably (each warp ranks its own contiguous 512
-// keys with __match_any_sync), publish their digit counts and obtain the counts of all earlier
+// keys, matching digits by ballots), publish their digit counts and obtain the counts of all earlier
 // tiles by a decoupled look-back, and write the tile out through shared memory so that runs of
-// equal digits land contiguously. 1 + passes launches instead of five per pass.
+// equal digits land contiguously. 1 + passes launches instead of five per pass. 2 M keys at scale
+// 22: 205 us; 249 with one earlier tile read per step of the look-back, digits matched by
+// __match_any_sync (its time grows with the distinct digits in a warp) and the histograms'
+// prefixes summed by one thread.
 #include "ctx.cuh"
 
 #include <algorithm>
@@ -17,10 +20,6 @@
 namespace scout {
 
 constexpr int SORT_RADIX = 256;
-// 2 * 10240 keys * 8 B + 33 * 256 * 4 B of tables = 197,632 B of dynamic shared memory,
-// under the 220 KB opt-in requested below.
-constexpr int SMALL_SORT_MAX = 10240;
-constexpr int SMALL_SORT_THREADS = 1024;
 
 // ---- one-sweep radix sort -------------------------------------------------------------------
 constexpr int OS_THREADS = 256;
@@ -30,6 +29,7 @@ constexpr int OS_TILE = OS_THREADS * OS_STEPS;      // 4096 keys per tile
 constexpr int OS_STEPS_SMALL = 4;                   // mid-size sorts: 1024-key tiles fill more SMs
 constexpr int OS_TILE_SMALL = OS_THREADS * OS_STEPS_SMALL;
 constexpr int OS_MAX_PASSES = 8;
+constexpr int OS_LOOK = 8;                          // earlier tiles' counts read at once
 // control block in the sort buffer (32-bit words): [pass][256] histograms, then global digit
 // offsets; the done counter; the per-pass tile counters; the look-back entries (64-bit) follow
 constexpr int OS_DONE = OS_MAX_PASSES * SORT_RADIX;
@@ -59,17 +59,20 @@ __global__ void __launch_bounds__(OS_THREADS) k_os_hist(const unsigned long long
     __syncthreads();
     if (!last) return;
     __threadfence();
-    for (int p = 0; p < passes; p++) {   // thread d: exclusive prefix of digit d in pass p
-        __shared__ unsigned int col[SORT_RADIX];
-        col[threadIdx.x] = ld_volatile(&ctl[p * SORT_RADIX + threadIdx.x]);
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            unsigned run = 0;
-            for (int d = 0; d < SORT_RADIX; d++) { const unsigned c = col[d]; col[d] = run; run += c; }
+    // exclusive prefix of every pass's digits, a warp per pass: eight digits per lane
+    for (int p = threadIdx.x / WARP; p < passes; p += OS_WARPS) {
+        unsigned c[8], sum = 0;
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            c[j] = ld_volatile(&ctl[p * SORT_RADIX + 8 * (int)lane_id() + j]);
+            sum += c[j];
         }
-        __syncthreads();
-        ctl[p * SORT_RADIX + threadIdx.x] = col[threadIdx.x];
-        __syncthreads();
+        unsigned run = (unsigned)warp_incl_scan_i((int)sum) - sum;
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            ctl[p * SORT_RADIX + 8 * (int)lane_id() + j] = run;
+            run += c[j];
+        }
     }
     if (threadIdx.x < OS_MAX_PASSES) ctl[OS_TILECTR + threadIdx.x] = 0;
     if (threadIdx.x == 0) ctl[OS_DONE] = 0;
@@ -106,8 +109,9 @@ __global__ void __launch_bounds__(OS_THREADS) k_os_pass(const unsigned long long
         const int64_t i = wbase + s * WARP + l;
         const bool valid = i < n;
         key[s] = valid ? src[i] : ~0ull;
-        const unsigned d = valid ? (unsigned)(key[s] >> shift) & 255u : 256u;
-        const unsigned peers = __match_any_sync(0xffffffffu, d);
+        const unsigned d = (unsigned)(key[s] >> shift) & 255u;
+        const unsigned vm = __ballot_sync(0xffffffffu, valid);
+        const unsigned peers = match_digit(d) & (valid ? vm : ~vm);
         const int leader = __ffs(peers) - 1;
         unsigned c = 0;
         if (valid && l == leader) c = wh[w][d];
@@ -131,19 +135,32 @@ __global__ void __launch_bounds__(OS_THREADS) k_os_pass(const unsigned long long
         gbase[t] = ctl[pass * SORT_RADIX + t];
     } else {
         atomicExch(mine, tag | OS_AGG | tot[t]);
+        // the counts of earlier tiles, OS_LOOK of them in flight: the tiles run at the same time, so
+        // most have only their own count published and the walk is a chain of loads
         unsigned long long excl = 0;
         int j = tile - 1;
         const uint64_t start = globaltimer_ns();
         while (j >= 0) {
-            const unsigned long long v = ld_volatile(lb + (int64_t)j * SORT_RADIX + t);
-            if ((v >> 34) == (unsigned long long)stamp && (v & (3ull << 32))) {
-                excl += v & 0xffffffffull;
-                if (v & OS_INC) break;
-                j--;
-                continue;
+            unsigned long long v[OS_LOOK];
+#pragma unroll
+            for (int u = 0; u < OS_LOOK; u++)
+                v[u] = j - u >= 0 ? ld_volatile(lb + (int64_t)(j - u) * SORT_RADIX + t) : tag | OS_INC;
+            bool stop = false, waits = false;
+#pragma unroll
+            for (int u = 0; u < OS_LOOK; u++) {
+                const bool ready = (v[u] >> 34) == (unsigned long long)stamp && (v[u] & (3ull << 32));
+                if (!stop && !waits) {
+                    if (ready) {
+                        excl += v[u] & 0xffffffffull;
+                        j--;
+                        stop = (v[u] & OS_INC) != 0;
+                    } else {
+                        waits = true;
+                    }
+                }
             }
-            if (globaltimer_ns() - start > OS_WAIT_LIMIT_NS) { atomicExch(err, 1); break; }
-            __nanosleep(32);
+            if (stop) break;
+            if (waits && globaltimer_ns() - start > OS_WAIT_LIMIT_NS) { atomicExch(err, 1); break; }
         }
         atomicExch(mine, tag | OS_INC | (excl + tot[t]));
         gbase[t] = (long long)ctl[pass * SORT_RADIX + t] + (long long)excl;
@@ -182,60 +199,6 @@ __global__ void __launch_bounds__(OS_THREADS) k_os_pass(const unsigned long long
         if (pos >= 0 && pos < n) dst[pos] = k;
         else atomicExch(err, 2);
     }
-}
-
-// Whole sort of n <= SMALL_SORT_MAX keys in one CTA (dynamic shared memory: 2 * n keys).
-__global__ void k_sort_small(unsigned long long* __restrict__ keys, int n, int bits) {
-    // Dynamic shared layout: a[n], b[n] (ping-pong keys), then a [NW + 1][256] table of
-    // per-warp digit offsets with the chunk totals in its last row.
-    extern __shared__ unsigned long long sm[];
-    constexpr int NW = SMALL_SORT_THREADS / WARP;
-    __shared__ unsigned int cnt[SORT_RADIX];
-    unsigned long long* a = sm;
-    unsigned long long* b = sm + n;
-    unsigned int* wtab = (unsigned int*)(sm + 2 * (size_t)n);
-    const int t = threadIdx.x, w = t / WARP, l = t % WARP;
-    for (int i = t; i < n; i += blockDim.x) a[i] = keys[i];
-    __syncthreads();
-    for (int shift = 0; shift < bits; shift += 8) {
-        if (t < SORT_RADIX) cnt[t] = 0;
-        __syncthreads();
-        for (int i = t; i < n; i += blockDim.x) atomicAdd(&cnt[(unsigned)(a[i] >> shift) & 255u], 1u);
-        __syncthreads();
-        if (t == 0) {
-            unsigned run = 0;
-            for (int d = 0; d < SORT_RADIX; d++) { unsigned c = cnt[d]; cnt[d] = run; run += c; }
-        }
-        __syncthreads();
-        for (int c0 = 0; c0 < n; c0 += blockDim.x) {
-            int i = c0 + t;
-            bool valid = i < n;
-            unsigned long long key = valid ? a[i] : 0ull;
-            unsigned d = valid ? (unsigned)(key >> shift) & 255u : 256u;
-            for (int j = t; j < NW * SORT_RADIX; j += blockDim.x) wtab[j] = 0;
-            __syncthreads();
-            unsigned peers = __match_any_sync(0xffffffffu, d);
-            unsigned rank = __popc(peers & ((1u << l) - 1));
-            if (valid && rank == 0) wtab[w * SORT_RADIX + d] = __popc(peers);
-            __syncthreads();
-            if (t < SORT_RADIX) {
-                unsigned run = 0;
-                for (int j = 0; j < NW; j++) {
-                    unsigned c = wtab[j * SORT_RADIX + t];
-                    wtab[j * SORT_RADIX + t] = run;
-                    run += c;
-                }
-                wtab[NW * SORT_RADIX + t] = run;   // chunk total of digit t
-            }
-            __syncthreads();
-            if (valid) b[cnt[d] + wtab[w * SORT_RADIX + d] + rank] = key;
-            __syncthreads();
-            if (t < SORT_RADIX) cnt[t] += wtab[NW * SORT_RADIX + t];
-            __syncthreads();
-        }
-        unsigned long long* s = a; a = b; b = s;
-    }
-    for (int i = t; i < n; i += blockDim.x) keys[i] = a[i];
 }
 
 // ---------------------------------------------------------------------------------------
@@ -398,20 +361,6 @@ int sort_keys(scout_ctx* c, unsigned long long* keys, unsigned long long* alt, i
               unsigned long long** sorted_out) {
     *sorted_out = keys;
     if (n <= 1) return SCOUT_OK;
-    if (n <= SMALL_SORT_MAX) {
-        constexpr int NW = SMALL_SORT_THREADS / WARP;
-        size_t smem = 2 * (size_t)n * sizeof(unsigned long long) + (size_t)(NW + 1) * SORT_RADIX * sizeof(unsigned);
-        static std::atomic<unsigned long long> attr_done{0};   // per-device setting, once per device
-        const unsigned long long bit = 1ull << (c->device & 63);
-        if (!(attr_done.load() & bit)) {
-            SCOUT_CU(c, cudaFuncSetAttribute(k_sort_small, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-            attr_done.fetch_or(bit);
-        }
-        k_sort_small<<<1, SMALL_SORT_THREADS, smem, c->s_main>>>(keys, (int)n, bits);
-        SCOUT_LAUNCH(c, "k_sort_small");
-        c->nlaunch += 1;
-        return SCOUT_OK;
-    }
     const int passes = (bits + 7) / 8;
     if (passes > OS_MAX_PASSES) return c->fail(SCOUT_E_INVALID, "sort keys wider than 64 bits");
     // large tiles once they give every SM two of them, else small tiles

@@ -83,10 +83,12 @@ def test_rows_at_the_edges(kind, tiered):
             assert ctx.info()["nnz"] == og.csr()[0][-1], f"batch {k + 1}: live entries"
 
 
-@pytest.mark.parametrize("m", [1, 511, 512, 513, 1024, 5120, 5121])
-def test_half_edit_tiles(rmat16, m):
-    """Batch sizes around the plan's tile (1,024 half-edits) and the one-block sort (10,240);
-    pairs repeated inside the batch are classified once each against the same state."""
+@pytest.mark.parametrize("m", [1, 16, 511, 512, 513, 2047, 2048, 2049, 5121, 75776, 131071, 131072, 131073])
+def test_update_sizes(rmat16, m):
+    """Batch sizes around the update's pair-ranked sort (4,096 half-edits), one half-edit per
+    thread (148 x 1,024), the one-launch update's limit (131,072 edits) and the separate
+    launches beyond it; pairs repeated inside the batch are classified once each against the
+    same state, some of them many times."""
     off, adj = rmat16[1]
     rng = np.random.default_rng(m)
     e = rng.integers(0, len(off) - 1, (m, 2)).astype(np.int32)
@@ -95,6 +97,8 @@ def test_half_edit_tiles(rmat16, m):
     e[: m // 4, 0] = at
     e[: m // 4, 1] = adj[off[at]]                       # existing edges
     e[m - m // 8:] = e[: m // 8]                        # repeated pairs
+    e[m // 2: m // 2 + m // 16] = e[0]                  # one pair over and over
+    e[m // 3] = (-1, 5)                                 # an invalid edit
     og = orc.Graph(off, adj)
     with sb.Context(0) as ctx:
         ctx.load_csr(off, adj)
