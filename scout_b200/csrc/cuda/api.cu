@@ -53,18 +53,24 @@ int pin_grow(scout_ctx* c, void** p, int64_t* cap, int64_t need) {
     return SCOUT_OK;
 }
 
-// One block per SM.
-int coop_launch(scout_ctx* c, const void* fn, int threads, void** args, size_t smem) {
-    int per_sm = 0;
-    SCOUT_CU(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem));
-    if (per_sm < 1) return c->fail(SCOUT_E_CUDA, "persistent kernel does not fit on an SM");
-    dim3 grid((unsigned)c->sm_count), block((unsigned)threads);
-    // the grid barrier's arrival counter starts every launch at zero (its error flag persists
-    // until the batch's counters are read)
-    SCOUT_CU(c, cudaMemsetAsync(&c->d_bar->count, 0, sizeof(unsigned int), c->s_main));
-    SCOUT_CU(c, cudaLaunchCooperativeKernel(fn, grid, block, args, smem, c->s_main));
+// One block per SM (the launch itself is refused when that does not fit).
+int coop_launch_own(scout_ctx* c, const void* fn, int threads, void** args, size_t smem) {
+    SCOUT_CU(c, cudaLaunchCooperativeKernel(fn, dim3((unsigned)c->sm_count), dim3((unsigned)threads), args, smem, c->s_main));
     c->nlaunch += 1;
     return SCOUT_OK;
+}
+
+// The barrier's arrival counter starts every launch at zero; the batch's start zeroed it for the
+// first one (its error flag persists until the batch's counters are read).
+int bar_clear(scout_ctx* c, cudaStream_t s) {
+    if (c->bar_used) SCOUT_CU(c, cudaMemsetAsync(&c->d_bar->count, 0, sizeof(unsigned int), s));
+    c->bar_used = true;
+    return SCOUT_OK;
+}
+
+int coop_launch(scout_ctx* c, const void* fn, int threads, void** args, size_t smem) {
+    SCOUT_RC(bar_clear(c, c->s_main));
+    return coop_launch_own(c, fn, threads, args, smem);
 }
 
 static void release(scout_ctx* c) {
@@ -76,10 +82,10 @@ static void release(scout_ctx* c) {
     if (c->host_pool) { cudaFreeHost(c->host_pool); c->host_pool = nullptr; }
     void* devs[] = {c->row, c->pool, c->spare, c->level, c->color, c->label, c->mis, c->stamp_a, c->stamp_b, c->stamp_c, c->stamp_d,
                     c->aux_v, c->ws, c->d_qbuf[0], c->d_qbuf[1], c->d_qbuf[2], c->d_list[0], c->d_list[1],
-                    c->d_commit, c->d_sort_hist, c->d_scan_tmp, c->d_slices, c->d_update, c->d_coff, c->d_misc, c->d_cc, c->bfs_lv, c->d_sources, c->d_ctr, c->d_bar, c->d_flags, c->d_stage_ids[0],
+                    c->d_commit, c->d_sort_hist, c->d_scan_tmp, c->d_slices, c->d_update, c->d_coff, c->d_misc, c->d_cc, c->bfs_lv, c->d_sources, c->d_batch, c->d_flags, c->d_stage_ids[0],
                     c->d_stage_ids[1], c->d_stage_off[0], c->d_stage_off[1]};
     for (void* p : devs) if (p) cudaFree(p);
-    void* hosts[] = {c->h_ctr, c->h_bar, c->h_pin_edits, c->h_pin_commit, c->h_slab[0], c->h_slab[1],
+    void* hosts[] = {c->h_batch, c->h_pin_edits, c->h_pin_commit, c->h_slab[0], c->h_slab[1],
                      c->h_slab_off[0], c->h_slab_off[1], c->h_slab_ids[0], c->h_slab_ids[1]};
     for (void* p : hosts) if (p) cudaFreeHost(p);
     for (int i = 0; i < 8; i++) if (c->ev_t[i]) cudaEventDestroy(c->ev_t[i]);
@@ -188,18 +194,17 @@ int scout_ctx_create(int device, uint64_t budget, scout_ctx** out) {
     ok = ok && cudaEventCreate(&c->ev_gather0) == cudaSuccess && cudaEventCreate(&c->ev_gather1) == cudaSuccess;
     ok = ok && cudaEventCreateWithFlags(&c->ev_pf, cudaEventDisableTiming) == cudaSuccess;
     ok = ok && cudaEventCreateWithFlags(&c->ev_union, cudaEventDisableTiming) == cudaSuccess;
-    ok = ok && cudaMallocHost((void**)&c->h_ctr, sizeof(DevCounters)) == cudaSuccess &&
-         cudaMallocHost((void**)&c->h_bar, sizeof(GridBar)) == cudaSuccess;
+    ok = ok && cudaMallocHost((void**)&c->h_batch, sizeof(DevBatch)) == cudaSuccess;
     if (!ok) { cudaError_t le = cudaGetLastError(); release(c); return cuda_fail(nullptr, le, "context streams"); }
-    int rc = dev_alloc(c, (void**)&c->d_ctr, sizeof(DevCounters), "counters");
-    if (rc == SCOUT_OK) rc = dev_alloc(c, (void**)&c->d_bar, sizeof(GridBar), "grid barrier");
+    int rc = dev_alloc(c, (void**)&c->d_batch, sizeof(DevBatch), "counters");
     if (rc == SCOUT_OK) rc = dev_alloc(c, (void**)&c->d_flags, 64, "error flags");
     if (rc != SCOUT_OK) { std::string m = c->err; release(c); return host_fail(rc, m); }
-    cudaMemset(c->d_ctr, 0, sizeof(DevCounters));
-    cudaMemset(c->d_bar, 0, sizeof(GridBar));
+    cudaMemset(c->d_batch, 0, sizeof(DevBatch));
+    c->d_ctr = &c->d_batch->ctr;
+    c->d_bar = &c->d_batch->bar[1];
+    c->h_ctr = &c->h_batch->ctr;
     cudaMemset(c->d_flags, 0, 64);
-    std::memset(c->h_ctr, 0, sizeof(DevCounters));   // scout_sched_last before any repair reads it
-    std::memset(c->h_bar, 0, sizeof(GridBar));
+    std::memset(c->h_batch, 0, sizeof(DevBatch));   // scout_sched_last before any repair reads it
     *out = c;
     return SCOUT_OK;
 }
@@ -224,6 +229,7 @@ int scout_state_upload(scout_ctx* c, int problem, const int32_t* sol, int64_t n)
             if (sol[v] < 0 || sol[v] >= n) return c->fail(SCOUT_E_INVALID, "component labels must lie in [0, n)");
     cudaSetDevice(c->device);
     if (!*slot) SCOUT_RC(dev_alloc(c, (void**)slot, (size_t)n * 4, "solution state"));
+    c->pairs_ready = false;   // a commit reads the entries' values as they are now
     SCOUT_CU(c, cudaMemcpyAsync(*slot, sol, (size_t)n * 4, cudaMemcpyHostToDevice, c->s_main));
     if (problem == SCOUT_CC) {   // min-vertex-id labels
         SCOUT_RC(graph_ensure_scratch(c));
@@ -305,7 +311,7 @@ static void fill_stats(scout_ctx* c, scout_batch_stats* st, int64_t launch0) {
     st->del_effective = c->last_problem == SCOUT_CC ? h.splits : h.del_eff;
     st->hbm_bytes = h.hbm_bytes;
     st->update_bytes = h.update_bytes;
-    st->d2h_bytes += sizeof(DevCounters);
+    st->d2h_bytes += sizeof(DevBatch);
     st->ms_compact = ev_ms(c->ev_t[6], c->ev_t[7]);
     st->ms_h2d = ev_ms(c->ev_t[7], c->ev_t[3]);
     st->ms_update = ev_ms(c->ev_t[3], c->ev_t[1]);
@@ -365,11 +371,14 @@ int commit_gather(scout_ctx* c, int problem, const int32_t** pairs, int64_t* cou
     int32_t** slot = state_slot(c, problem);
     if (!slot || !*slot) return c->fail(SCOUT_E_STATE, "nothing to commit for this problem");
     if (problem != c->last_problem) return c->fail(SCOUT_E_STATE, "the last repair was for another problem");
-    cudaSetDevice(c->device);
     const int64_t cnt = c->last_changed;
     *pairs = nullptr;
     *count = 0;
-    if (cnt > 0) {
+    if (cnt > 0 && c->pairs_ready) {   // few entries: they came with the batch's counters
+        *pairs = c->h_batch->pairs;
+        *count = cnt;
+    } else if (cnt > 0) {
+        cudaSetDevice(c->device);
         SCOUT_RC(pin_grow(c, &c->h_pin_commit, &c->cap_pin_commit, cnt * 8));
         k_commit_gather<<<blocks_for(cnt, 256), 256, 0, c->s_main>>>(c->d_list[0], c->d_ctr, *slot, c->d_commit);
         SCOUT_LAUNCH(c, "k_commit_gather");
@@ -521,6 +530,7 @@ int scout_repair_probe(scout_ctx* c, int problem, const scout_edge* edits, const
                                         c->s_main));
             SCOUT_CU(c, cudaMemcpyAsync(state, pre, (size_t)n * 4, cudaMemcpyDeviceToDevice, c->s_main));
             SCOUT_CU(c, cudaMemsetAsync(c->d_bar, 0, sizeof(GridBar), c->s_main));
+            c->bar_used = false;
             c->epoch++;
         }
         SCOUT_CU(c, cudaEventRecord(c->ev_t[4], c->s_main));

@@ -51,6 +51,7 @@ int bfs_params(scout_ctx* c, int mode, const int* mode_dev, BfsParams* out) {
     p.qtag0 = c->qtag;
     p.ctr = c->d_ctr;
     p.bar = c->d_bar;
+    p.pairs = c->d_batch->pairs;
     p.mode = mode;
     p.mode_dev = mode_dev;
     p.lv_new = c->bfs_lv;

@@ -7,6 +7,8 @@
 
 namespace scout {
 
+constexpr int BFS_Q_SEED = 5;    // queue of the rows that seed invalidated vertices (buffer 2)
+constexpr int BFS_Q_RELAX = 6;   // first of the relax rounds' three queues (buffers 0, 1, 2)
 constexpr int PSCAN = 4;   // row entries per lane and step in the seed scan
 
 struct BfsParams {
@@ -34,6 +36,7 @@ struct BfsParams {
     int chunk, chunk_log2;    // row entries per queue item (a power of two, 256 .. 8192)
     const int32_t* sources;   // when nsrc > 0: every listed vertex is a level-0 root (a union of
     int nsrc;                 // disjoint graphs, one source each); else `source` alone
+    int32_t* pairs;           // commit_pairs
     int max_share;            // most warps that share one queue item (lanes_per_vertex / 32)
 };
 
@@ -70,7 +73,7 @@ __device__ __forceinline__ void push_vertex(const BfsParams& p, bool pred, int32
     long long start = (long long)base + incl - nit;
     for (int k = 0; k < nit; k++) {
         long long pos = start + k;
-        if (pos < p.qcap) p.q[qi][pos] = ((unsigned long long)k << 32) | (uint32_t)y;
+        if (pos < p.qcap) p.q[qi % 3][pos] = ((unsigned long long)k << 32) | (uint32_t)y;
         else atomicExch(&p.ctr->overflow, 1);
     }
 }
@@ -97,7 +100,7 @@ __device__ __forceinline__ void push_vertex2(const BfsParams& p, bool pa, int32_
         const long long pos = start + k;
         const int32_t v = k < na ? ya : yb;
         const int kk = k < na ? k : k - na;
-        if (pos < p.qcap) p.q[qi][pos] = ((unsigned long long)kk << 32) | (uint32_t)v;
+        if (pos < p.qcap) p.q[qi % 3][pos] = ((unsigned long long)kk << 32) | (uint32_t)v;
         else atomicExch(&p.ctr->overflow, 1);
     }
 }
@@ -150,7 +153,7 @@ static __device__ void relax_round(const BfsParams& p, int cur, int nxt, uint32_
         const int g = warps_per_item(cnt, W, p.chunk, p.max_share);
         for (long long wv = gwarp_id(); wv < (long long)cnt * g; wv += W) {
             const int item = (int)(wv / g), part = (int)(wv % g);
-            const unsigned long long it = p.q[cur][item];
+            const unsigned long long it = p.q[cur % 3][item];
             const int32_t v = (int32_t)(it & 0xffffffffu);
             const int chunk = (int)(it >> 32);
             const Row r = p.g.row[v];
@@ -166,7 +169,7 @@ static __device__ void relax_round(const BfsParams& p, int cur, int nxt, uint32_
     for (long long gbase = (long long)gwarp_id() * per; gbase < cnt; gbase += (long long)W * per) {
         long long idx = gbase + lane_id();
         bool valid = (int)lane_id() < per && idx < cnt;
-        unsigned long long item = valid ? p.q[cur][idx] : 0ull;
+        unsigned long long item = valid ? p.q[cur % 3][idx] : 0ull;
         int32_t v = (int32_t)(item & 0xffffffffu);
         int chunk = (int)(item >> 32);
         long long s = 0;
@@ -234,7 +237,7 @@ __device__ __forceinline__ void push_new(const BfsParams& p, bool pred, int32_t 
     long long start = (long long)base + incl - nit;
     for (int k = 0; k < nit; k++) {
         long long pos = start + k;
-        if (pos < p.qcap) p.q[qi][pos] = ((unsigned long long)k << 32) | (uint32_t)y;
+        if (pos < p.qcap) p.q[qi % 3][pos] = ((unsigned long long)k << 32) | (uint32_t)y;
         else atomicExch(&p.ctr->overflow, 1);
     }
 }
@@ -263,7 +266,7 @@ static __device__ void td_step(const BfsParams& p, int32_t* lv, int cur, int nxt
         const int g = warps_per_item(cnt, W, p.chunk, p.max_share);
         for (long long wv = gwarp_id(); wv < (long long)cnt * g; wv += W) {
             const int item = (int)(wv / g), part = (int)(wv % g);
-            const unsigned long long it = p.q[cur][item];
+            const unsigned long long it = p.q[cur % 3][item];
             const int32_t v = (int32_t)(it & 0xffffffffu);
             const int chunk = (int)(it >> 32);
             const Row r = p.g.row[v];
@@ -278,7 +281,7 @@ static __device__ void td_step(const BfsParams& p, int32_t* lv, int cur, int nxt
     for (long long gbase = (long long)gwarp_id() * per; gbase < cnt; gbase += (long long)W * per) {
         long long idx = gbase + lane_id();
         bool valid = (int)lane_id() < per && idx < cnt;
-        unsigned long long item = valid ? p.q[cur][idx] : 0ull;
+        unsigned long long item = valid ? p.q[cur % 3][idx] : 0ull;
         int32_t v = (int32_t)(item & 0xffffffffu);
         int chunk = (int)(item >> 32);
         long long s = 0;
@@ -437,6 +440,7 @@ __device__ __forceinline__ void bfs_body(const BfsParams& p) {
     int rounds = 0;
     uint32_t tag = p.qtag0;
     int cur = 0;
+    if (update_failed(p.bar)) return;
     phase_mark(&p.ctr->phase_ns[0]);
 
     const int mode = p.mode_dev ? *p.mode_dev : p.mode;
@@ -498,7 +502,7 @@ __device__ __forceinline__ void bfs_body(const BfsParams& p) {
             // current one is checked. None of them changes during this pass: levels are fixed in
             // this phase, and a single-chunk candidate is queued once per round and invalidated
             // only by its own warp (a long one's mark is set after the barrier below).
-            unsigned long long it_n = wid < cnt ? p.q[cur][wid] : 0ull;
+            unsigned long long it_n = wid < cnt ? p.q[cur % 3][wid] : 0ull;
             Row r_n{0, 0, 0};
             int lc_n = 0, si_n = 0;
             if (wid < cnt) {
@@ -507,7 +511,7 @@ __device__ __forceinline__ void bfs_body(const BfsParams& p) {
                 lc_n = ld_level(p.level + cn);
                 si_n = ld_volatile(p.st_inval + cn);
             }
-            unsigned long long it_nn = wid + W < cnt ? p.q[cur][wid + W] : 0ull;
+            unsigned long long it_nn = wid + W < cnt ? p.q[cur % 3][wid + W] : 0ull;
             for (int i = wid; i < cnt; i += W) {
                 const unsigned long long item = it_n;
                 const Row r = r_n;
@@ -520,7 +524,7 @@ __device__ __forceinline__ void bfs_body(const BfsParams& p) {
                     lc_n = ld_level(p.level + cn);
                     si_n = ld_volatile(p.st_inval + cn);
                 }
-                it_nn = (long long)i + 2 * W < cnt ? p.q[cur][i + 2 * W] : 0ull;
+                it_nn = (long long)i + 2 * W < cnt ? p.q[cur % 3][i + 2 * W] : 0ull;
                 const int32_t c = (int32_t)(item & 0xffffffffu);
                 const int chunk = (int)(item >> 32);
                 const bool big = r.len > p.chunk;
@@ -578,7 +582,7 @@ __device__ __forceinline__ void bfs_body(const BfsParams& p) {
                     bool nt = false;
                     int32_t c = 0;
                     if (i < cnt) {
-                        const unsigned long long item = p.q[cur][i];
+                        const unsigned long long item = p.q[cur % 3][i];
                         c = (int32_t)(item & 0xffffffffu);
                         if ((item >> 32) == 0 && p.g.row[c].len > p.chunk && ld_volatile(p.found + c) != (int32_t)tag)
                             nt = atomicExch(&p.st_inval[c], p.epoch) != p.epoch;
@@ -589,7 +593,7 @@ __device__ __forceinline__ void bfs_body(const BfsParams& p) {
                 if (!grid_sync(p.bar, 8)) return;
                 if (leader) p.ctr->list_count[2] = 0;
                 for (int i = wid; i < cnt; i += W) {
-                    const unsigned long long item = p.q[cur][i];
+                    const unsigned long long item = p.q[cur % 3][i];
                     const int32_t c = (int32_t)(item & 0xffffffffu);
                     const Row r = p.g.row[c];
                     if (r.len <= p.chunk || ld_volatile(p.found + c) == (int32_t)tag ||
@@ -620,9 +624,10 @@ __device__ __forceinline__ void bfs_body(const BfsParams& p) {
         // ---- B: reset and seed --------------------------------------------------------------
         // Every invalidated vertex restarts at +inf and queues its row's chunks in q[2]; each
         // chunk then offers (min level of its valid neighbours) + 1. Inserted edges seed their
-        // endpoints. Both push into q[0], where the relax rounds start.
-        if (leader) { p.ctr->q_count[0] = 0; p.ctr->q_count[1] = 0; p.ctr->q_count[2] = 0; }
-        if (!grid_sync(p.bar, 4)) return;
+        // endpoints. Both push into the relax rounds' first queue. The queues of this phase and of
+        // the relax rounds have counters of their own (zero since the batch began), so that no
+        // barrier clears the invalidation's; without an invalidated vertex the reset and its
+        // barrier fall away.
         const int ninv = ld_volatile(&p.ctr->list_count[0]);
         tag++;
         for (int64_t b = tid - (tid & (WARP - 1)); b < ninv; b += T) {
@@ -636,14 +641,14 @@ __device__ __forceinline__ void bfs_body(const BfsParams& p) {
             }
             int ti = warp_append(nt, &p.ctr->changed);
             if (nt) p.touched[ti] = c;
-            push_vertex(p, ok, c, 2, tag, true, false);
+            push_vertex(p, ok, c, BFS_Q_SEED, tag, true, false);
         }
-        if (!grid_sync(p.bar, 5)) return;
+        if (ninv > 0 && !grid_sync(p.bar, 5)) return;
         tag++;
         // boundary seeds: warp per chunk of an invalidated vertex's row
-        const int nseed = qcount(p, 2);
+        const int nseed = ninv > 0 ? qcount(p, BFS_Q_SEED) : 0;
         for (int i = wid; i < nseed; i += W) {
-            const unsigned long long item = p.q[2][i];
+            const unsigned long long item = p.q[BFS_Q_SEED % 3][i];
             const int32_t c = (int32_t)(item & 0xffffffffu);
             const Row r = p.g.row[c];
             const long long c0 = ((long long)(item >> 32) << p.chunk_log2);
@@ -674,7 +679,7 @@ __device__ __forceinline__ void bfs_body(const BfsParams& p) {
                 unsigned old = atomicMin((unsigned*)(p.level + c), cand);
                 dec = old > cand;
             }
-            push_vertex(p, dec, c, 0, tag, true, false);
+            push_vertex(p, dec, c, BFS_Q_RELAX, tag, true, false);
         }
         // insertion seeds: thread per half-edit
         for (int64_t b = tid - (tid & (WARP - 1)); b < nh; b += T) {
@@ -697,17 +702,17 @@ __device__ __forceinline__ void bfs_body(const BfsParams& p) {
             }
             const unsigned md = __ballot_sync(0xffffffffu, dec);   // insertions that lowered a level
             if (lane_id() == 0 && md) atomicAdd(&p.ctr->ins_eff, __popc(md));
-            push_vertex(p, dec, y, 0, tag, true, true);
+            push_vertex(p, dec, y, BFS_Q_RELAX, tag, true, true);
         }
         if (!grid_sync(p.bar, 6)) return;
-        cur = 0;
+        cur = BFS_Q_RELAX;
     }
     phase_mark(&p.ctr->phase_ns[2]);
     // ---- C: relax rounds -------------------------------------------------------------------
     while (true) {
         const int cnt = qcount(p, cur);
         if (cnt == 0) break;
-        const int nxt = (cur + 1) % 3, zer = (cur + 2) % 3;
+        const int nxt = BFS_Q_RELAX + (cur + 1) % 3, zer = BFS_Q_RELAX + (cur + 2) % 3;
         if (leader) p.ctr->q_count[zer] = 0;
         tag++;
         relax_round(p, cur, nxt, tag, bytes);
@@ -716,6 +721,7 @@ __device__ __forceinline__ void bfs_body(const BfsParams& p) {
         cur = nxt;
     }
     phase_mark(&p.ctr->phase_ns[3]);
+    commit_pairs(p.touched, p.level, p.ctr, p.pairs);
     // ---- counters ----------------------------------------------------------------------------
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) bytes += __shfl_xor_sync(0xffffffffu, bytes, o);

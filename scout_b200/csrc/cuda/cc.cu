@@ -94,6 +94,7 @@ int cc_params(scout_ctx* c, const scout_sched* sched, int variant, const int* mo
     p.mode_dev = mode_dev;
     p.ctr = c->d_ctr;
     p.bar = c->d_bar;
+    p.pairs = c->d_batch->pairs;
     return SCOUT_OK;
 }
 

@@ -41,6 +41,7 @@ struct CcParams {
     int bound;
     int variant;        // 0 incremental, 1 recompute every class, 2 recompute every class a
                         // deletion that no common neighbour settles touches (search limit 0)
+    int32_t* pairs;       // commit_pairs
     const int* mode_dev;  // when set, the variant is read here (decided on the device by the scheduler)
     DevCounters* ctr;
     GridBar* bar;
@@ -242,6 +243,7 @@ __device__ __forceinline__ void cc_body(const CcParams& p) {
     const int full = variant == 1;
     const int limit = variant == 2 ? 0 : p.search_limit;
 
+    if (update_failed(p.bar)) return;
     phase_mark(&p.ctr->phase_ns[0]);
     if (!full) {
         // ---- P0: unions of inserted edges ---------------------------------------------------
@@ -568,6 +570,8 @@ __device__ __forceinline__ void cc_body(const CcParams& p) {
     if (tid == 0) bytes += 16LL * n;
 done:
     phase_mark(&p.ctr->phase_ns[4]);
+    if (!grid_sync(p.bar, 48)) return;
+    commit_pairs(p.touched, p.label, p.ctr, p.pairs);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) bytes += __shfl_xor_sync(0xffffffffu, bytes, o);
     if (lane_id() == 0) atomicAdd((unsigned long long*)&p.ctr->hbm_bytes, (unsigned long long)bytes);

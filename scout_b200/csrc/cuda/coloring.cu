@@ -57,6 +57,7 @@ int coloring_params(scout_ctx* c, ColParams* out) {
     p.epoch = (int32_t)c->epoch;
     p.ctr = c->d_ctr;
     p.bar = c->d_bar;
+    p.pairs = c->d_batch->pairs;
     return SCOUT_OK;
 }
 

@@ -24,6 +24,7 @@ struct ColParams {
     int32_t* st_round;   // dedupe of the initial marking (epoch)
     int32_t* st_touch;
     int32_t epoch;
+    int32_t* pairs;      // commit_pairs
     DevCounters* ctr;
     GridBar* bar;
 };
@@ -77,6 +78,7 @@ __device__ __forceinline__ void coloring_body(const ColParams& p) {
     long long bytes = 0;
     int rounds = 0;
 
+    if (update_failed(p.bar)) return;
     // ---- marking: higher endpoint of every same-colour inserted edge (pre-batch colours) ----
     const int nh = ld_volatile(&p.ctr->n_half);
     for (int64_t b = tid - (tid & (WARP - 1)); b < nh; b += T) {
@@ -180,6 +182,7 @@ __device__ __forceinline__ void coloring_body(const ColParams& p) {
         if (!grid_sync(p.bar, 13)) return;
         cur = nxt;
     }
+    commit_pairs(p.touched, p.color, p.ctr, p.pairs);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) bytes += __shfl_xor_sync(0xffffffffu, bytes, o);
     if (lane_id() == 0) atomicAdd((unsigned long long*)&p.ctr->hbm_bytes, (unsigned long long)bytes);

@@ -202,6 +202,10 @@ __device__ __forceinline__ bool grid_sync(GridBar* b, int tag = 0) {
     return s_ok != 0;
 }
 
+// A batch has two barriers side by side: the update kernel's, then the repair kernel's. The
+// repair (given its own) does not start on a store whose update gave up.
+__device__ __forceinline__ bool update_failed(const GridBar* repair_bar) { return ld_volatile(&(repair_bar - 1)->err) != 0; }
+
 __device__ __forceinline__ void grid_fail(GridBar* b, int code) { atomicCAS(&b->err, 0, code); }
 
 // Phase timestamp written by one thread right after a grid barrier (profiling aid).

@@ -26,7 +26,7 @@ struct DevCounters {
     long long nnz_delta;      // inserted minus deleted entries
     long long update_bytes;   // algorithmic bytes of the row merge
     // repair
-    int q_count[4];           // rotating queue counters
+    int q_count[12];          // queue counters (BFS: three rotating ones per phase, queue i lies in buffer i % 3)
     int list_count[4];        // auxiliary list counters
     int rounds;
     int changed;
@@ -51,8 +51,19 @@ struct DevCounters {
     int sort_err;             // 1: a sort look-back wait timed out, 2: a sort position out of range,
                               // 4: a look-back wait of a scan or of the merge plan timed out
     int sched_flags;          // 1 features computed, 2 model applied
+    int pairs_ok;             // the repair left its changed entries in DevBatch::pairs (when they fit)
     float feat[24];
     float pred[4];
+};
+
+// What a batch zeroes at its start and copies back at its end, in one piece: the counters, the
+// barriers of the update and of the repair, and the changed entries when they are few (then
+// the commit needs no launch and no copy of its own; not zeroed).
+constexpr int COMMIT_PAIRS = 1024;
+struct DevBatch {
+    DevCounters ctr;
+    scout::GridBar bar[2];
+    int32_t pairs[2 * COMMIT_PAIRS];   // (id, value)
 };
 
 struct scout_ctx {
@@ -174,10 +185,13 @@ struct scout_ctx {
     int32_t* probe_buf = nullptr;   // probe: pre-repair state, first variant's result, mismatch counter
     DevCounters* d_ctr_snap = nullptr;
 
-    DevCounters* d_ctr = nullptr;
-    DevCounters* h_ctr = nullptr;   // pinned
-    scout::GridBar* d_bar = nullptr;
-    scout::GridBar* h_bar = nullptr; // pinned
+    DevBatch* d_batch = nullptr;
+    DevBatch* h_batch = nullptr;     // pinned
+    DevCounters* d_ctr = nullptr;    // d_batch's and h_batch's counters
+    DevCounters* h_ctr = nullptr;
+    scout::GridBar* d_bar = nullptr; // the repair's barrier (d_batch->bar[1])
+    bool bar_used = false;           // a kernel has used it since the batch began
+    bool pairs_ready = false;        // h_batch->pairs holds the last repair's changed entries
     int* d_flags = nullptr;          // staging / seal error flags (int[16])
 
     // ---- pinned staging ----
@@ -241,6 +255,18 @@ int host_fail(int code, const std::string& msg);   // thread-local message for c
         if (rc_ != SCOUT_OK) return rc_;     \
     } while (0)
 
+// End of a repair, after a grid barrier that follows the last change: the changed entries, when
+// they are few, beside the counters that the host copies next.
+__device__ __forceinline__ void commit_pairs(const int32_t* touched, const int32_t* val, DevCounters* ctr, int32_t* pairs) {
+    const int n = ld_volatile(&ctr->changed);
+    if (n <= COMMIT_PAIRS)
+        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+            const int32_t v = ld_volatile(touched + i);
+            ((int2*)pairs)[i] = make_int2(v, ld_volatile(val + v));
+        }
+    if (blockIdx.x == 0 && threadIdx.x == 0) ctr->pairs_ok = 1;
+}
+
 inline DGraph dgraph(const scout_ctx* c) { return DGraph{c->row, c->pool, (int32_t)c->n}; }
 inline int blocks_for(int64_t items, int threads, int cap = 148 * 32) {
     int64_t b = (items + threads - 1) / threads;
@@ -298,8 +324,11 @@ constexpr int REPAIR_THREADS = 1024;
 inline int repair_threads(const scout_ctx* c) {
     return c->tune_blocks_per_sm > 0 ? 256 * c->tune_blocks_per_sm : REPAIR_THREADS;
 }
-// persistent launch helper
+// persistent launch helpers: a launch that waits on d_bar (cleared when it was used before), one
+// on a barrier of its own
 int coop_launch(scout_ctx* c, const void* fn, int threads, void** args, size_t smem);
+int coop_launch_own(scout_ctx* c, const void* fn, int threads, void** args, size_t smem);
+int bar_clear(scout_ctx* c, cudaStream_t s);
 // gather.cu: the hinted next batch's edits to the device and (tiered store) its cold rows into
 // free HBM from `base` on a copy stream, after the current merge is queued; gather_finish waits
 // for the gather (main stream and host) and moves the tail.

@@ -29,6 +29,7 @@
 #include "ctx.cuh"
 
 #include <algorithm>
+#include <cstddef>
 #include <cstring>
 
 namespace scout {
@@ -816,9 +817,9 @@ static __device__ __forceinline__ void merge_rows(int32_t* __restrict__ pool, co
                                                   int B, DevCounters* __restrict__ ctr, const uint32_t* __restrict__ epos,
                                                   const int32_t* __restrict__ E, const MergeRow* __restrict__ mrow,
                                                   const int64_t* __restrict__ slices, int64_t slice_cap, ChunkEvents& ev) {
-    if (ld_volatile(&ctr->overflow)) return;   // the slice list did not fit (the host reports it)
-    const int nsl = (int)min((int64_t)ld_volatile(&ctr->n_slices), slice_cap);
-    const int nsm = ld_volatile(&ctr->n_small);
+    const int over = ld_volatile(&ctr->overflow), sl = ld_volatile(&ctr->n_slices), nsm = ld_volatile(&ctr->n_small);
+    if (over) return;   // the slice list did not fit (the host reports it)
+    const int nsl = (int)min((int64_t)sl, slice_cap);
     // rows of a warp's turn: up to 32, fewer while that leaves warps without any
     const int per = min(WARP, max(MERGE_ROWS, (nsm + gwarp_count() - 1) / gwarp_count()));
     const int items = nsl + (nsm + per - 1) / per;
@@ -857,9 +858,9 @@ __global__ void __launch_bounds__(MERGE_THREADS, 4) k_merge(
 // rows' plan; the merge. The sort is one of two:
 //   up to UPDATE_PAIRS half-edits   every key's place is the number of smaller keys: a warp per
 //                                   key against all of them in shared memory
-//   more                            sample sort: UPDATE_SPLIT keys at regular places are ranked
-//                                   that way; they split the keys into buckets (about n / 2,048
-//                                   keys each), whose keys are ranked among themselves
+//   more                            sample sort: 2,048 or 4,096 keys at regular places are ranked
+//                                   that way; they split the keys into buckets (10 to 64 keys on
+//                                   average), whose keys are ranked among themselves
 //
 // What bounds it: the latency of two searches in rows, the barriers (6 to 9 of them) and the
 // merge's traffic. Up to UPDATE_MAX edits it is faster than the launches it replaces (each about
@@ -871,7 +872,8 @@ constexpr int UPDATE_THREADS = 1024;
 constexpr int UPDATE_WARPS = UPDATE_THREADS / WARP;
 constexpr int64_t UPDATE_MAX = 131072;
 constexpr int UPDATE_PAIRS = 4096;
-constexpr int UPDATE_SPLIT = 2048;
+constexpr int UPDATE_SPLIT = 4096;   // splitters; half of them up to UPDATE_FEW half-edits
+constexpr int UPDATE_FEW = 65536;
 constexpr int UPDATE_ROWS = 16384;   // more affected rows are planned by blocks, fewer by warps
 // device scratch: splitters, bucket counts, the blocks' plan counts
 constexpr int64_t UPDATE_SCRATCH = UPDATE_SPLIT * 8 + (UPDATE_SPLIT + 64) * 4 + 1024 * 8;
@@ -896,7 +898,7 @@ struct UpdateParams {
     GridBar* bar;
 };
 
-// First index of the ascending a[0, n) whose value is above x (n <= 2^12).
+// First index of the ascending a[0, n) whose value is above x (n <= 2^13).
 template <typename T>
 __device__ __forceinline__ int first_above(const T* a, int n, T x) {
     int lo = 0, hi = n;
@@ -927,19 +929,20 @@ static __device__ bool update_sort(const UpdateParams& p, int n, unsigned long l
         }
         return true;
     }
+    const int S = n <= UPDATE_FEW ? UPDATE_SPLIT / 2 : UPDATE_SPLIT;   // 2,048 or 4,096
     // the sample, ranked like that
-    for (int i = t; i < UPDATE_SPLIT; i += UPDATE_THREADS) k[i] = ld_volatile(p.raw + (long long)i * n / UPDATE_SPLIT);
+    for (int i = t; i < S; i += UPDATE_THREADS) k[i] = ld_volatile(p.raw + (long long)i * n / S);
     __syncthreads();
-    for (int j = wid; j < UPDATE_SPLIT; j += W) {
+    for (int j = wid; j < S; j += W) {
         const unsigned long long x = k[j];
         int c = 0;
-        for (int i = l; i < UPDATE_SPLIT; i += WARP) c += k[i] < x || (k[i] == x && i < j);
+        for (int i = l; i < S; i += WARP) c += k[i] < x || (k[i] == x && i < j);
         c = __reduce_add_sync(0xffffffffu, c);
         if (l == 0) p.split[c] = x;
     }
     if (!grid_sync(p.bar, 65)) return false;
     // every key's bucket and its place there (in the order the atomics came)
-    for (int i = t; i < UPDATE_SPLIT; i += UPDATE_THREADS) k[i] = ld_volatile(p.split + i);
+    for (int i = t; i < S; i += UPDATE_THREADS) k[i] = ld_volatile(p.split + i);
     __syncthreads();
     unsigned long long key[2] = {SENT, SENT};   // n <= 2 T
     int b[2] = {0, 0}, at[2] = {0, 0};
@@ -948,22 +951,30 @@ static __device__ bool update_sort(const UpdateParams& p, int n, unsigned long l
         const int i = tid + s * T;
         if (i < n) key[s] = ld_volatile(p.raw + i);
         if (key[s] != SENT) {
-            b[s] = first_above(k, UPDATE_SPLIT, key[s]);
+            b[s] = first_above(k, S, key[s]);
             at[s] = atomicAdd(p.bucket + b[s], 1);
         }
     }
     if (!grid_sync(p.bar, 66)) return false;
     int* off = (int*)smem;   // the buckets' first places, and the end
     {
-        static_assert(UPDATE_SPLIT == 2 * UPDATE_THREADS, "two buckets per thread and the last one");
-        const int c0 = ld_volatile(p.bucket + 2 * t), c1 = ld_volatile(p.bucket + 2 * t + 1);
-        long long x = c0 + c1, y = 0, tx, ty;
+        const int per = S / UPDATE_THREADS;   // 2 or 4 buckets per thread, and the last one
+        int c[4];
+        long long x = 0, y = 0, tx, ty;
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            c[q] = q < per ? ld_volatile(p.bucket + per * t + q) : 0;
+            x += c[q];
+        }
         block_scan2(x, y, &tx, &ty);   // its barriers are past the splitters' last reader
-        off[2 * t] = (int)x;
-        off[2 * t + 1] = (int)x + c0;
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            if (q < per) off[per * t + q] = (int)x;
+            x += c[q];
+        }
         if (t == 0) {
-            off[UPDATE_SPLIT] = (int)tx;
-            off[UPDATE_SPLIT + 1] = (int)tx + ld_volatile(p.bucket + UPDATE_SPLIT);
+            off[S] = (int)tx;
+            off[S + 1] = (int)tx + ld_volatile(p.bucket + S);
         }
         __syncthreads();
     }
@@ -971,10 +982,10 @@ static __device__ bool update_sort(const UpdateParams& p, int n, unsigned long l
     for (int s = 0; s < 2; s++)
         if (key[s] != SENT) p.tmp[off[b[s]] + at[s]] = key[s];
     if (!grid_sync(p.bar, 67)) return false;
-    const int total = off[UPDATE_SPLIT + 1];
+    const int total = off[S + 1];
     for (int i = tid; i < total; i += T) {
         const unsigned long long x = ld_volatile(p.tmp + i);
-        const int q = first_above(off, UPDATE_SPLIT + 2, i) - 1;   // the bucket of place i
+        const int q = first_above(off, S + 2, i) - 1;   // the bucket of place i
         const int q0 = off[q], q1 = off[q + 1];
         int c = 0;
         for (int j = q0; j < q1; j++) {
@@ -1041,17 +1052,20 @@ __global__ void __launch_bounds__(UPDATE_THREADS, 1) k_update(UpdateParams p) {
     block_scan2(c0, c1, &t0, &t1);
     if (t == 0) p.cnt[blockIdx.x] = (unsigned long long)(t0 + t1);
     if (!grid_sync(p.bar, 62)) return;
-    long long all = 0, before = 0;
-    for (int j = l; j < G; j += WARP) {
-        const long long c = (long long)ld_volatile(p.cnt + j);
-        all += c;
-        before += j < (int)blockIdx.x ? c : 0;
+    __shared__ long long s_all, s_before;
+    if (w == 0) {
+        long long all = 0, before = 0;
+        for (int j = l; j < G; j += WARP) {
+            const long long c = (long long)ld_volatile(p.cnt + j);
+            all += c;
+            before += j < (int)blockIdx.x ? c : 0;
+        }
+        all = warp_incl_scan(all);
+        before = warp_incl_scan(before);
+        if (l == WARP - 1) { s_all = all; s_before = before; }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        all += __shfl_xor_sync(0xffffffffu, all, o);
-        before += __shfl_xor_sync(0xffffffffu, before, o);
-    }
+    __syncthreads();
+    const long long all = s_all, before = s_before;
 #pragma unroll
     for (int s = 0; s < 2; s++) {   // lane 0's exclusive counts are those before the group
         const long long base = before + (s ? t0 : 0) + __shfl_sync(0xffffffffu, s ? c1 : c0, 0);
@@ -1366,25 +1380,27 @@ int lists_ensure(scout_ctx* c) {
 
 int batch_begin(scout_ctx* c) {
     SCOUT_RC(gather_finish(c, nullptr, nullptr, nullptr));   // no graph work while a gather runs
-    SCOUT_CU(c, cudaMemsetAsync(c->d_ctr, 0, sizeof(DevCounters), c->s_main));
-    SCOUT_CU(c, cudaMemsetAsync(c->d_bar, 0, sizeof(GridBar), c->s_main));
+    SCOUT_CU(c, cudaMemsetAsync(c->d_batch, 0, offsetof(DevBatch, pairs), c->s_main));
+    c->bar_used = false;
+    c->pairs_ready = false;
     return SCOUT_OK;
 }
 
 int counters_fetch(scout_ctx* c) {
-    SCOUT_CU(c, cudaMemcpyAsync(c->h_ctr, c->d_ctr, sizeof(DevCounters), cudaMemcpyDeviceToHost, c->s_main));
-    SCOUT_CU(c, cudaMemcpyAsync(c->h_bar, c->d_bar, sizeof(GridBar), cudaMemcpyDeviceToHost, c->s_main));
+    SCOUT_CU(c, cudaMemcpyAsync(c->h_batch, c->d_batch, sizeof(DevBatch), cudaMemcpyDeviceToHost, c->s_main));
     SCOUT_CU(c, cudaStreamSynchronize(c->s_main));
-    if (c->h_bar->err == 1)
-        return c->fail(SCOUT_E_TIMEOUT, "a device grid barrier timed out (tag " + std::to_string(c->h_bar->where) + ")");
+    for (const GridBar& b : c->h_batch->bar)
+        if (b.err == 1)
+            return c->fail(SCOUT_E_TIMEOUT, "a device grid barrier timed out (tag " + std::to_string(b.where) + ")");
     if (c->h_ctr->pad)
         return c->fail(SCOUT_E_STATE, "the component labels do not describe the components of the graph "
                                       "(an edge joins two labels); upload a consistent labelling");
     if (c->h_ctr->sort_err == 1) return c->fail(SCOUT_E_TIMEOUT, "a sort look-back wait timed out");
     if (c->h_ctr->sort_err == 4) return c->fail(SCOUT_E_TIMEOUT, "a scan or merge-plan look-back wait timed out");
     if (c->h_ctr->sort_err) return c->fail(SCOUT_E_STATE, "the sort computed a position out of range");
-    if (c->h_bar->err != 0 || c->h_ctr->overflow)
+    if (c->h_batch->bar[0].err != 0 || c->h_batch->bar[1].err != 0 || c->h_ctr->overflow)
         return c->fail(SCOUT_E_CAPACITY, "a device work list overflowed its capacity");
+    c->pairs_ready = c->h_ctr->pairs_ok && c->h_ctr->changed <= COMMIT_PAIRS;
     return SCOUT_OK;
 }
 
@@ -1702,9 +1718,9 @@ int graph_update(scout_ctx* c, const scout_edge* edits, const uint8_t* ops, int6
         up.seg_b = c->d_seg_b;
         up.seg_d = c->d_seg_d;
         up.E = E;
-        up.bar = c->d_bar;
+        up.bar = &c->d_batch->bar[0];
         void* args[] = {&up};
-        SCOUT_RC(coop_launch(c, (const void*)k_update, UPDATE_THREADS, args, 0));
+        SCOUT_RC(coop_launch_own(c, (const void*)k_update, UPDATE_THREADS, args, 0));
     } else {
         k_classify<<<blocks_for(m, 256), 256, 0, c->s_main>>>(g, d_src, ops ? c->d_ops : nullptr, m, B, c->d_keys,
                                                              c->d_eflag, c->d_ctr, 1);

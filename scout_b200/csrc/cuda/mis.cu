@@ -36,6 +36,7 @@ int mis_params(scout_ctx* c, MisParams* out) {
     p.epoch = (int32_t)c->epoch;
     p.ctr = c->d_ctr;
     p.bar = c->d_bar;
+    p.pairs = c->d_batch->pairs;
     return SCOUT_OK;
 }
 

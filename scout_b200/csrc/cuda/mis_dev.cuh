@@ -19,6 +19,7 @@ struct MisParams {
     int32_t* st_done;      // == epoch: decided this batch
     int32_t* st_touch;
     int32_t epoch;
+    int32_t* pairs;        // commit_pairs
     DevCounters* ctr;
     GridBar* bar;
 };
@@ -47,6 +48,7 @@ __device__ __forceinline__ void mis_body(const MisParams& p) {
     long long bytes = 0;
     int rounds = 0;
 
+    if (update_failed(p.bar)) return;
     // ---- 1: conflicts of inserted edges, evaluated on the pre-batch set ----------------
     for (int64_t b = tid - (tid & (WARP - 1)); b < nh; b += T) {
         int64_t k = b + lane_id();
@@ -158,6 +160,7 @@ __device__ __forceinline__ void mis_body(const MisParams& p) {
         if (!grid_sync(p.bar, 24)) return;
         cur = nxt;
     }
+    commit_pairs(p.touched, p.mis, p.ctr, p.pairs);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) bytes += __shfl_xor_sync(0xffffffffu, bytes, o);
     if (lane_id() == 0) atomicAdd((unsigned long long*)&p.ctr->hbm_bytes, (unsigned long long)bytes);

@@ -64,7 +64,7 @@ int union_launch(scout_ctx* const* cs, const int* problems, const scout_sched* s
         SCOUT_CU(c0, cudaStreamWaitEvent(c0->s_main, cs[i]->ev_union, 0));
     }
     for (int i = 0; i < ne; i++)   // every repair's grid barrier starts at zero
-        SCOUT_CU(c0, cudaMemsetAsync(&cs[i]->d_bar->count, 0, sizeof(unsigned int), c0->s_main));
+        SCOUT_RC(bar_clear(cs[i], c0->s_main));
     if (smem) {   // the dynamic shared-memory opt-in: once per device
         static std::atomic<unsigned long long> attr_done{0};
         const unsigned long long bit = 1ull << (c0->device & 63);
