@@ -96,3 +96,55 @@ def test_prefetched_gather_stays_exact(rmat16, problem, hbm_frac):
         o2, a2 = ref.graph()
         assert np.array_equal(o1, o2) and np.array_equal(a1, a2)
         assert gathered > 0
+
+
+@pytest.mark.parametrize("lens", ["short", "mixed", "one_long"])
+def test_host_pool_compaction(lens):
+    """Batches that rewrite host rows until the host pool is compacted several times: rows of equal
+    short length, of 0 to 700 entries, and one that fills most of the graph. The adjacency equals
+    an all-HBM store's after every batch."""
+    rng = np.random.default_rng(3)
+    n = 30000
+    rows = [set() for _ in range(n)]
+    if lens == "one_long":
+        hub = set(int(v) for v in rng.choice(np.arange(1, n), size=25000, replace=False))
+        rows[0] = hub
+        for v in hub:
+            rows[v].add(0)
+    else:
+        k = 8 if lens == "short" else 700
+        for u in rng.choice(n, size=n if lens == "short" else 900, replace=False).tolist():
+            for v in rng.integers(0, n, rng.integers(0, k) + 1).tolist():
+                if u != v:
+                    rows[u].add(v)
+                    rows[v].add(u)
+    off = np.concatenate([[0], np.cumsum([len(r) for r in rows])]).astype(np.int64)
+    adj = np.concatenate([np.array(sorted(r), dtype=np.int32) for r in rows])
+    level = sb.HostCsr.from_arrays(off, adj).init_state("bfs", 0)
+    with sb.Context(0) as t, sb.Context(0) as ref:
+        t.load_tiered(off, adj, hbm_entries=4096)
+        ref.load_csr(off, adj)
+        for c in (t, ref):
+            c.upload("bfs", level)
+        cap = t.tier_info()["host_cap"]
+        used, compactions = t.tier_info()["host_used"], 0
+        for k in range(120):
+            e = rng.integers(0, n, (1500, 2)).astype(np.int32)   # insertions grow the rows they rewrite
+            e[:, 0] = rng.integers(0, 400, 1500)
+            for c in (t, ref):
+                c.repair("bfs", e)
+            now = t.tier_info()["host_used"]
+            assert now <= cap
+            if now < used:
+                compactions += 1
+                o1, a1 = t.graph()
+                o2, a2 = ref.graph()
+                assert np.array_equal(o1, o2) and np.array_equal(a1, a2), f"batch {k + 1}"
+            used = now
+            if compactions == 3:
+                break
+        assert np.array_equal(t.download("bfs"), ref.download("bfs"))
+        o1, a1 = t.graph()
+        o2, a2 = ref.graph()
+        assert np.array_equal(o1, o2) and np.array_equal(a1, a2)
+        assert compactions > 0, "the host pool was never compacted"
