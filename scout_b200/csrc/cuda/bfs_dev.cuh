@@ -7,8 +7,10 @@
 
 namespace scout {
 
+constexpr int BFS_Q_REST = 9;    // invalidation: the other chunks of long candidates (buffers 0, 1, 2)
 constexpr int BFS_Q_SEED = 5;    // queue of the rows that seed invalidated vertices (buffer 2)
 constexpr int BFS_Q_RELAX = 6;   // first of the relax rounds' three queues (buffers 0, 1, 2)
+constexpr int CHECK_ITEMS = 8;   // candidates a warp checks at a time (invalidation)
 constexpr int PSCAN = 4;   // row entries per lane and step in the seed scan
 
 struct BfsParams {
@@ -41,6 +43,9 @@ struct BfsParams {
 };
 
 __device__ __forceinline__ int32_t ld_level(const int32_t* p) { return ld_volatile(p); }
+// A level that no one writes before the next grid barrier: read through L1 (rows repeat the same
+// hubs), where a volatile read always goes to L2.
+__device__ __forceinline__ int32_t ld_fixed(const int32_t* p) { return *p; }
 
 // Warp-cooperative push (all 32 lanes call): lanes with `pred` push vertex y into queue qn
 // once per round (tag), split into chunk-sized items; first touches of the batch are
@@ -78,17 +83,14 @@ __device__ __forceinline__ void push_vertex(const BfsParams& p, bool pred, int32
     }
 }
 
-// push_vertex (chunked, no touch list) of two vertices per lane at once: the dedupe atomics and
-// row-length loads of both are in flight together, and one atomicAdd reserves both's items.
+// push_vertex (one item per vertex, no touch list) of two vertices per lane at once: the dedupe
+// atomics of both are in flight together, and one atomicAdd reserves both's items.
 __device__ __forceinline__ void push_vertex2(const BfsParams& p, bool pa, int32_t ya, bool pb, int32_t yb, int qi,
                                              uint32_t tag) {
     bool fa = false, fb = false;
     if (pa) fa = atomicExch(&p.st_q[ya], tag) != tag;
     if (pb) fb = atomicExch(&p.st_q[yb], tag) != tag;   // ya == yb: only the first push counts
-    int na = 0, nb = 0;
-    if (fa) na = max(1, (p.g.row[ya].len + p.chunk - 1) >> p.chunk_log2);
-    if (fb) nb = max(1, (p.g.row[yb].len + p.chunk - 1) >> p.chunk_log2);
-    const int nit = na + nb;
+    const int na = fa, nit = (int)fa + (int)fb;
     const int incl = warp_incl_scan_i(nit);
     const int tot = __shfl_sync(0xffffffffu, incl, WARP - 1);
     if (tot == 0) return;
@@ -96,13 +98,62 @@ __device__ __forceinline__ void push_vertex2(const BfsParams& p, bool pa, int32_
     if (lane_id() == WARP - 1) base = atomicAdd(&p.ctr->q_count[qi], tot);
     base = __shfl_sync(0xffffffffu, base, WARP - 1);
     const long long start = (long long)base + incl - nit;
-    for (int k = 0; k < nit; k++) {
-        const long long pos = start + k;
-        const int32_t v = k < na ? ya : yb;
-        const int kk = k < na ? k : k - na;
-        if (pos < p.qcap) p.q[qi % 3][pos] = ((unsigned long long)kk << 32) | (uint32_t)v;
+    if (start + nit > p.qcap) { if (nit) atomicExch(&p.ctr->overflow, 1); return; }
+    if (fa) p.q[qi % 3][start] = (uint32_t)ya;
+    if (fb) p.q[qi % 3][start + na] = (uint32_t)yb;
+}
+
+// Every chunk but the first of row y (`chunks` of them in all) into queue qi; one warp, all lanes.
+__device__ __forceinline__ void push_rest(const BfsParams& p, int32_t y, int chunks, int qi) {
+    int base = 0;
+    if (lane_id() == 0) base = atomicAdd(&p.ctr->q_count[qi], chunks - 1);
+    base = __shfl_sync(0xffffffffu, base, 0);
+    for (int k = 1 + (int)lane_id(); k < chunks; k += WARP) {
+        const long long pos = (long long)base + k - 1;
+        if (pos < p.qcap) p.q[qi % 3][pos] = ((unsigned long long)k << 32) | (uint32_t)y;
         else atomicExch(&p.ctr->overflow, 1);
     }
+}
+
+// Has one of the entries rw[0, n) a valid parent level (lc - 1)? The warp, 256 entries at a time: a
+// chunk is two dependent reads, not sixteen.
+static __device__ __forceinline__ bool parent_among(const BfsParams& p, const int32_t* rw, int n, int lc, long long& bytes) {
+    constexpr int U = 8;
+    for (int b0 = 0; b0 < n; b0 += U * WARP) {
+        int32_t w[U];
+        int lw[U];
+        bool ok = false;
+#pragma unroll
+        for (int u = 0; u < U; u++) w[u] = b0 + u * WARP + (int)lane_id() < n ? rw[b0 + u * WARP + (int)lane_id()] : -1;
+#pragma unroll
+        for (int u = 0; u < U; u++) lw[u] = w[u] >= 0 ? ld_fixed(p.level + w[u]) : -2;
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            if (lw[u] == lc - 1 && w[u] >= 0) ok = ok || ld_volatile(p.st_inval + w[u]) != p.epoch;
+            if (w[u] >= 0) bytes += 8;
+        }
+        if (__any_sync(0xffffffffu, ok)) return true;
+    }
+    return false;
+}
+
+// The children (level lc + 1) among rw[0, n) of an invalidated vertex are queued for a check.
+static __device__ __forceinline__ void push_children(const BfsParams& p, const int32_t* rw, int n, int lc, int qi,
+                                                     uint32_t tag, long long& bytes) {
+    constexpr int U = 4;
+    for (int b0 = 0; b0 < n; b0 += U * WARP) {
+        int32_t w[U];
+        int lw[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) w[u] = b0 + u * WARP + (int)lane_id() < n ? rw[b0 + u * WARP + (int)lane_id()] : -1;
+#pragma unroll
+        for (int u = 0; u < U; u++) lw[u] = w[u] >= 0 ? ld_fixed(p.level + w[u]) : -2;
+        for (int u = 0; u < U; u++) {
+            const bool ch = w[u] >= 0 && lw[u] == lc + 1 && ld_volatile(p.st_inval + w[u]) != p.epoch;
+            if (__any_sync(0xffffffffu, ch)) push_vertex(p, ch, w[u], qi, tag, false, false);
+        }
+    }
+    if (lane_id() == 0) bytes += 8LL * max(n, 0);
 }
 
 __device__ __forceinline__ int qcount(const BfsParams& p, int qi) {
@@ -363,7 +414,7 @@ static __device__ void bu_step(const BfsParams& p, int32_t* lv, int nxt, int d, 
 static __device__ bool full_bfs(const BfsParams& p, int mode, long long& bytes, int& rounds) {
     int32_t* lv = p.lv_new;
     const int64_t n = p.g.n;
-    const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t tid = gthread_id();
     const int64_t T = (int64_t)gridDim.x * blockDim.x;
     const bool leader = blockIdx.x == 0 && threadIdx.x == 0;
     for (int64_t v = tid; v < n; v += T) lv[v] = -1;
@@ -433,7 +484,7 @@ static __device__ bool full_bfs(const BfsParams& p, int mode, long long& bytes, 
 __device__ __forceinline__ void bfs_body(const BfsParams& p) {
     const int W = gwarp_count();
     const int wid = gwarp_id();
-    const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t tid = gthread_id();
     const int64_t T = (int64_t)gridDim.x * blockDim.x;
     const bool leader = blockIdx.x == 0 && threadIdx.x == 0;
     long long bytes = 0;
@@ -459,11 +510,14 @@ __device__ __forceinline__ void bfs_body(const BfsParams& p) {
     }
     {
         // ---- A: invalidation -------------------------------------------------------------
-        // Candidates are queued as chunk-sized items of their rows. A single-chunk candidate
-        // is settled by one warp (parent check, invalidation, children pushed). A longer one
-        // is checked chunk by chunk (any chunk with a valid parent marks found = tag); after
-        // a barrier its first item decides, and after another every chunk of an invalidated
-        // candidate pushes its children, so a hub's row is spread over many warps.
+        // A candidate is queued once; a warp looks for a valid parent in its row's first chunk, where
+        // nearly every candidate has one. A candidate of a single chunk is settled there (children
+        // pushed if it has none). The other chunks of a longer one are queued only if the first
+        // holds no parent: after a barrier they are checked side by side (any chunk with one marks
+        // found = tag), after another the candidate is decided, and after a third every chunk
+        // of an invalidated candidate pushes its children, so a hub's row is spread over many
+        // warps. (With every chunk queued at once, a 10^6-edit batch at scale 22 checked 422,000
+        // items in the first rounds, most of them of rows whose first chunk settles them.)
         const int nh = ld_volatile(&p.ctr->n_half);
         tag++;
         // two half-edits per thread and step (k and k + T): their loads overlap, and both
@@ -480,7 +534,7 @@ __device__ __forceinline__ void bfs_body(const BfsParams& p) {
                     const int32_t x = (int32_t)(key >> (p.B + 1));
                     y[h] = (int32_t)(key & ((1ull << p.B) - 1));
                     if (op == 1) {
-                        const int lx = ld_level(p.level + x), ly = ld_level(p.level + y[h]);
+                        const int lx = ld_fixed(p.level + x), ly = ld_fixed(p.level + y[h]);
                         cand[h] = lx >= 0 && ly == lx + 1;
                     }
                 }
@@ -495,125 +549,178 @@ __device__ __forceinline__ void bfs_body(const BfsParams& p) {
             const int cnt = qcount(p, cur);
             if (cnt == 0) break;
             const int nxt = (cur + 1) % 3, zer = (cur + 2) % 3;
-            if (leader) p.ctr->q_count[zer] = 0;
-            tag++;
-            // Software pipeline over the warp's candidates: the queue item two candidates ahead,
-            // and the row, level and invalidation mark of the next one, are loaded while the
-            // current one is checked. None of them changes during this pass: levels are fixed in
-            // this phase, and a single-chunk candidate is queued once per round and invalidated
-            // only by its own warp (a long one's mark is set after the barrier below).
-            unsigned long long it_n = wid < cnt ? p.q[cur % 3][wid] : 0ull;
-            Row r_n{0, 0, 0};
-            int lc_n = 0, si_n = 0;
-            if (wid < cnt) {
-                const int32_t cn = (int32_t)(it_n & 0xffffffffu);
-                r_n = p.g.row[cn];
-                lc_n = ld_level(p.level + cn);
-                si_n = ld_volatile(p.st_inval + cn);
+            const int rest = BFS_Q_REST + zer;   // its items lie in the buffer that is free this round
+            if (leader) {
+                p.ctr->q_count[zer] = 0;
+                p.ctr->q_count[BFS_Q_REST + (zer + 1) % 3] = 0;   // the next round's
+                p.ctr->tick[nxt] = 0;
             }
-            unsigned long long it_nn = wid + W < cnt ? p.q[cur % 3][wid + W] : 0ull;
-            for (int i = wid; i < cnt; i += W) {
-                const unsigned long long item = it_n;
-                const Row r = r_n;
-                const int lc = lc_n;
-                const int si = si_n;
-                it_n = it_nn;
-                if (i + W < cnt) {   // the next candidate's item arrived during this one's wait
-                    const int32_t cn = (int32_t)(it_n & 0xffffffffu);
-                    r_n = p.g.row[cn];
-                    lc_n = ld_level(p.level + cn);
-                    si_n = ld_volatile(p.st_inval + cn);
+            tag++;
+            // A warp takes up to CHECK_ITEMS candidates at a time (fewer while that leaves warps
+            // without any): a lane each holds their vertex, row, level and invalidation mark,
+            // loaded while the previous candidates are checked; their first entries, and those
+            // entries' levels, are in flight together. None of what is loaded ahead changes
+            // during this pass: levels are fixed in this phase, and a candidate is queued once
+            // per round and invalidated only by its own warp (a long one after the barriers
+            // below). What bounds it: the random reads of levels (32 bytes of L2 traffic each). The
+            // invalidation of a 10^6-edit batch at scale 22 (174,000 candidates in the first round)
+            // took 315 us with a warp per candidate, 32 entries at a time and every chunk of
+            // long rows queued; 275 us without the latter; 215 us with eight entries first.
+            const int per = min(CHECK_ITEMS, max(1, (cnt + W - 1) / W));
+            const int l = (int)lane_id();
+            // (the queue holds vertices alone here: chunk 0; -1 marks a lane without one)
+            auto load_item = [&](long long i) { return l < per && i + l < cnt ? (int32_t)p.q[cur % 3][i + l] : -1; };
+            struct Cand { Row r; int lc, si; };
+            auto load_cand = [&](int32_t c) {
+                Cand d{Row{0, 0, 0}, 0, 0};
+                if (c >= 0) {
+                    d.r = p.g.row[c];
+                    d.lc = ld_fixed(p.level + c);
+                    d.si = ld_volatile(p.st_inval + c);
                 }
-                it_nn = (long long)i + 2 * W < cnt ? p.q[cur % 3][i + 2 * W] : 0ull;
-                const int32_t c = (int32_t)(item & 0xffffffffu);
-                const int chunk = (int)(item >> 32);
-                const bool big = r.len > p.chunk;
-                if (c == p.source || lc <= 0 || si == p.epoch) {
-                    if (big && lane_id() == 0) p.found[c] = (int32_t)tag;   // nothing to decide
-                    continue;
-                }
-                const long long c0 = ((long long)chunk << p.chunk_log2);
-                const int clen = (int)min((long long)p.chunk, (long long)r.len - c0);
-                const int32_t* rw = p.g.pool + r.start + c0;
-                bool found = false;
-                // 32 entries per step: most candidates keep a parent early in the row, and wider
-                // steps (measured with four entries per lane) only add random level reads
-                for (int b0 = 0; b0 < clen && !found; b0 += WARP) {
-                    const int k = b0 + (int)lane_id();
-                    bool ok = false;
-                    if (k < clen) {
-                        const int32_t w = rw[k];
-                        ok = ld_level(p.level + w) == lc - 1 && ld_volatile(p.st_inval + w) != p.epoch;
-                        bytes += 8;
+                return d;
+            };
+            // the first two turns of every warp are fixed, the rest handed out (rows take unequal time)
+            long long i = (long long)wid * per, i_n = i + (long long)W * per;
+            int32_t it_n = load_item(i);
+            Cand cd_n = load_cand(it_n);
+            int32_t it_nn = load_item(i_n);
+            while (i < cnt) {
+                int tk = 0;
+                if (l == 0) tk = atomicAdd(&p.ctr->tick[cur], 1);
+                const int32_t it_c = it_n;
+                const Cand cd = cd_n;
+                it_n = it_nn;   // arrived during the previous candidates' waits
+                cd_n = load_cand(it_n);
+                const bool live = it_c >= 0 && it_c != p.source && cd.lc > 0 && cd.si != p.epoch;
+                const int clen = live ? min(p.chunk, cd.r.len) : 0;
+                // the first eight entries of every candidate, eight lanes each: nearly all have a
+                // parent there, and the random reads of levels are what this pass costs
+                unsigned none = __ballot_sync(0xffffffffu, live);   // without a parent so far
+                {
+                    int32_t w[CHECK_ITEMS / 4];
+                    int lw[CHECK_ITEMS / 4];
+#pragma unroll
+                    for (int h = 0; h < CHECK_ITEMS / 4; h++) {
+                        const int u = 4 * h + (l >> 3);
+                        const long long st = __shfl_sync(0xffffffffu, cd.r.start, u);
+                        const int len = __shfl_sync(0xffffffffu, clen, u);
+                        w[h] = (l & 7) < len ? p.g.pool[st + (l & 7)] : -1;
                     }
-                    found = __any_sync(0xffffffffu, ok);
+#pragma unroll
+                    for (int h = 0; h < CHECK_ITEMS / 4; h++) lw[h] = w[h] >= 0 ? ld_fixed(p.level + w[h]) : -2;
+#pragma unroll
+                    for (int h = 0; h < CHECK_ITEMS / 4; h++) {
+                        const int lc = __shfl_sync(0xffffffffu, cd.lc, 4 * h + (l >> 3));
+                        const bool at = w[h] >= 0 && lw[h] == lc - 1;
+                        const unsigned m = __ballot_sync(0xffffffffu, at), group = 0xffu << (l & 24);
+                        // the first of a candidate's parents is checked (another, below, if it is invalid)
+                        const bool ok = at && !(m & group & ((1u << l) - 1)) && ld_volatile(p.st_inval + w[h]) != p.epoch;
+                        const unsigned f = __ballot_sync(0xffffffffu, ok);
+#pragma unroll
+                        for (int g = 0; g < 4; g++)
+                            if (f & (0xffu << (8 * g))) none &= ~(1u << (4 * h + g));
+                        if (w[h] >= 0) bytes += 8;
+                    }
                 }
-                if (big) {
+                // the others 32 entries per step, until each has a valid parent or no entries left
+                unsigned open = none;
+                auto load_entries = [&](int u, int b0) {   // (0 entries where there is no candidate)
+                    const long long st = __shfl_sync(0xffffffffu, cd.r.start, u);
+                    const int len = __shfl_sync(0xffffffffu, clen, u);
+                    return ((open >> u) & 1u) && b0 + l < len ? p.g.pool[st + b0 + l] : -1;
+                };
+                int32_t w[CHECK_ITEMS];
+#pragma unroll
+                for (int u = 0; u < CHECK_ITEMS; u++) w[u] = load_entries(u, 0);
+                for (int b0 = 0; open; b0 += WARP) {
+                    int32_t nx[CHECK_ITEMS];   // the next step's, loaded while these are checked
+                    int lw[CHECK_ITEMS];
+#pragma unroll
+                    for (int u = 0; u < CHECK_ITEMS; u++) {
+                        lw[u] = w[u] >= 0 ? ld_fixed(p.level + w[u]) : -2;
+                        nx[u] = load_entries(u, b0 + WARP);
+                    }
+                    unsigned hit = 0;
+#pragma unroll
+                    for (int u = 0; u < CHECK_ITEMS; u++) {
+                        const int lc = __shfl_sync(0xffffffffu, cd.lc, u);
+                        const bool ok = w[u] >= 0 && lw[u] == lc - 1 && ld_volatile(p.st_inval + w[u]) != p.epoch;
+                        if (w[u] >= 0) bytes += 8;
+                        if (__any_sync(0xffffffffu, ok)) hit |= 1u << u;
+                    }
+                    none &= ~hit;
+                    open = none & __ballot_sync(0xffffffffu, b0 + WARP < clen);
+#pragma unroll
+                    for (int u = 0; u < CHECK_ITEMS; u++) w[u] = (open >> u) & 1u ? nx[u] : -1;
+                }
+                const long long i_nn = ((long long)2 * W + __shfl_sync(0xffffffffu, tk, 0)) * per;
+                it_nn = load_item(i_nn);
+                i = i_n;
+                i_n = i_nn;
+                for (; none; none &= none - 1) {
+                    const int u = __ffs(none) - 1;
+                    const int32_t c = __shfl_sync(0xffffffffu, it_c, u);
+                    Row r;
+                    r.start = __shfl_sync(0xffffffffu, cd.r.start, u);
+                    r.len = __shfl_sync(0xffffffffu, cd.r.len, u);
+                    const int lc = __shfl_sync(0xffffffffu, cd.lc, u);
+                    if (r.len > p.chunk) {
+                        push_rest(p, c, (r.len + p.chunk - 1) >> p.chunk_log2, rest);
+                        continue;
+                    }
                     if (lane_id() == 0) {
-                        if (found) p.found[c] = (int32_t)tag;
-                        if (chunk == 0) p.ctr->list_count[2] = 1;   // a long candidate this round
+                        p.st_inval[c] = p.epoch;
+                        int at = atomicAdd(&p.ctr->list_count[0], 1);
+                        p.inval[at] = c;
                     }
-                    continue;
+                    __syncwarp();
+                    push_children(p, p.g.pool + r.start, r.len, lc, nxt, tag, bytes);
+                    if (lane_id() == 0) bytes += 24;
                 }
-                if (found) continue;
-                if (lane_id() == 0) {
-                    p.st_inval[c] = p.epoch;
-                    int at = atomicAdd(&p.ctr->list_count[0], 1);
-                    p.inval[at] = c;
-                }
-                __syncwarp();
-                for (int b0 = 0; b0 < clen; b0 += WARP) {
-                    int k = b0 + (int)lane_id();
-                    bool ch = false;
-                    int32_t w = 0;
-                    if (k < clen) {
-                        w = rw[k];
-                        ch = ld_level(p.level + w) == lc + 1 && ld_volatile(p.st_inval + w) != p.epoch;
-                    }
-                    push_vertex(p, ch, w, nxt, tag, true, false);
-                }
-                if (lane_id() == 0) bytes += 8LL * clen + 24;
             }
             if (!grid_sync(p.bar, 3)) return;
-            if (ld_volatile(&p.ctr->list_count[2])) {
-                // long candidates: decide on the first item, then push children from every chunk
-                for (int64_t b = tid - (tid & (WARP - 1)); b < cnt; b += T) {
+            const int nrest = qcount(p, rest);
+            if (nrest) {
+                // long candidates without a parent in their first chunk: the others
+                for (int i = wid; i < nrest; i += W) {
+                    const unsigned long long item = p.q[rest % 3][i];
+                    const int32_t c = (int32_t)(item & 0xffffffffu);
+                    const Row r = p.g.row[c];
+                    const int lc = ld_fixed(p.level + c);
+                    const long long c0 = ((long long)(item >> 32) << p.chunk_log2);
+                    const int clen = (int)min((long long)p.chunk, (long long)r.len - c0);
+                    const int32_t* rw = p.g.pool + r.start + c0;
+                    if (ld_volatile(p.found + c) == (int32_t)tag) continue;   // another chunk has one
+                    if (parent_among(p, rw, clen, lc, bytes) && l == 0) p.found[c] = (int32_t)tag;
+                }
+                if (!grid_sync(p.bar, 10)) return;
+                // decide on a candidate's first item here (chunk 1)
+                for (int64_t b = tid - (tid & (WARP - 1)); b < nrest; b += T) {
                     const int64_t i = b + lane_id();
                     bool nt = false;
                     int32_t c = 0;
-                    if (i < cnt) {
-                        const unsigned long long item = p.q[cur % 3][i];
+                    if (i < nrest) {
+                        const unsigned long long item = p.q[rest % 3][i];
                         c = (int32_t)(item & 0xffffffffu);
-                        if ((item >> 32) == 0 && p.g.row[c].len > p.chunk && ld_volatile(p.found + c) != (int32_t)tag)
+                        if ((item >> 32) == 1 && ld_volatile(p.found + c) != (int32_t)tag)
                             nt = atomicExch(&p.st_inval[c], p.epoch) != p.epoch;
                     }
                     int at = warp_append(nt, &p.ctr->list_count[0]);
                     if (nt) p.inval[at] = c;
                 }
                 if (!grid_sync(p.bar, 8)) return;
-                if (leader) p.ctr->list_count[2] = 0;
-                for (int i = wid; i < cnt; i += W) {
-                    const unsigned long long item = p.q[cur % 3][i];
+                for (int i = wid; i < nrest; i += W) {
+                    const unsigned long long item = p.q[rest % 3][i];
                     const int32_t c = (int32_t)(item & 0xffffffffu);
+                    if (ld_volatile(p.found + c) == (int32_t)tag || ld_volatile(p.st_inval + c) != p.epoch) continue;
                     const Row r = p.g.row[c];
-                    if (r.len <= p.chunk || ld_volatile(p.found + c) == (int32_t)tag ||
-                        ld_volatile(p.st_inval + c) != p.epoch)
-                        continue;
-                    const int lc = ld_level(p.level + c);
-                    const long long c0 = ((long long)(item >> 32) << p.chunk_log2);
-                    const int clen = (int)min((long long)p.chunk, (long long)r.len - c0);
+                    const int lc = ld_fixed(p.level + c);
+                    const int chunk = (int)(item >> 32);
+                    const long long c0 = chunk == 1 ? 0 : ((long long)chunk << p.chunk_log2);   // chunk 1 with chunk 0
+                    const int clen = (int)(min((long long)r.len, (long long)(chunk + 1) << p.chunk_log2) - c0);
                     const int32_t* rw = p.g.pool + r.start + c0;
-                    for (int b0 = 0; b0 < clen; b0 += WARP) {
-                        int k = b0 + (int)lane_id();
-                        bool ch = false;
-                        int32_t w = 0;
-                        if (k < clen) {
-                            w = rw[k];
-                            ch = ld_level(p.level + w) == lc + 1 && ld_volatile(p.st_inval + w) != p.epoch;
-                        }
-                        push_vertex(p, ch, w, nxt, tag, true, false);
-                    }
-                    if (lane_id() == 0) bytes += 8LL * clen;
+                    push_children(p, rw, clen, lc, nxt, tag, bytes);
                 }
                 if (!grid_sync(p.bar, 9)) return;
             }

@@ -232,7 +232,7 @@ static __device__ int cc_search(const CcParams& p, int32_t u, int32_t v, int32_t
 
 __device__ __forceinline__ void cc_body(const CcParams& p) {
     const int W = gwarp_count(), wid = gwarp_id();
-    const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t tid = gthread_id();
     const int64_t T = (int64_t)gridDim.x * blockDim.x;
     const int64_t n = p.g.n;
     const bool leader = blockIdx.x == 0 && threadIdx.x == 0;

@@ -72,7 +72,7 @@ __device__ __forceinline__ void coloring_body(const ColParams& p) {
     __shared__ int s_bres;
     __shared__ int s_flag;
     const int W = gwarp_count(), wid = gwarp_id(), wl = threadIdx.x / WARP;
-    const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t tid = gthread_id();
     const int64_t T = (int64_t)gridDim.x * blockDim.x;
     const bool leader = blockIdx.x == 0 && threadIdx.x == 0;
     long long bytes = 0;

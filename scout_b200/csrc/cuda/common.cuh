@@ -213,8 +213,10 @@ __device__ __forceinline__ void phase_mark(unsigned long long* slot) {
     if (blockIdx.x == 0 && threadIdx.x == 0) *slot = globaltimer_ns();
 }
 
-// Global warp index / count for grid-stride warp loops.
-__device__ __forceinline__ int gwarp_id() { return (int)((blockIdx.x * blockDim.x + threadIdx.x) / WARP); }
+// Global warp index / count for grid-stride warp loops: neighbouring indices lie in different
+// blocks, so that a few items go to as many SMs. gthread_id numbers the threads the same way.
+__device__ __forceinline__ int gwarp_id() { return (int)(threadIdx.x / WARP * gridDim.x + blockIdx.x); }
+__device__ __forceinline__ int64_t gthread_id() { return (int64_t)gwarp_id() * WARP + lane_id(); }
 __device__ __forceinline__ int gwarp_count() { return (int)((gridDim.x * blockDim.x) / WARP); }
 
 }  // namespace scout

@@ -28,6 +28,7 @@ struct DevCounters {
     // repair
     int q_count[12];          // queue counters (BFS: three rotating ones per phase, queue i lies in buffer i % 3)
     int list_count[4];        // auxiliary list counters
+    int tick[4];              // work handed out in a round (BFS invalidation, rotating)
     int rounds;
     int changed;
     int affected;

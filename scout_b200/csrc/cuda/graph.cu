@@ -823,8 +823,7 @@ static __device__ __forceinline__ void merge_rows(int32_t* __restrict__ pool, co
     // rows of a warp's turn: up to 32, fewer while that leaves warps without any
     const int per = min(WARP, max(MERGE_ROWS, (nsm + gwarp_count() - 1) / gwarp_count()));
     const int items = nsl + (nsm + per - 1) / per;
-    // the first item of every warp, neighbouring ones on different SMs; the rest are handed out
-    int it = (int)(threadIdx.x / WARP * gridDim.x + blockIdx.x);
+    int it = gwarp_id();   // the first item of every warp; the rest are handed out
     while (it < items) {
         int nx = 0;
         if (lane_id() == 0) nx = gwarp_count() + atomicAdd(&ctr->merge_ticket, 1);
@@ -913,7 +912,7 @@ __device__ __forceinline__ int first_above(const T* a, int n, T x) {
 // false when a barrier failed. Ends before a barrier: the caller's next one publishes the order.
 static __device__ bool update_sort(const UpdateParams& p, int n, unsigned long long SENT, unsigned char* smem) {
     const int t = threadIdx.x, w = t / WARP, l = (int)lane_id();
-    const int G = (int)gridDim.x, wid = w * G + (int)blockIdx.x, W = G * UPDATE_WARPS;
+    const int G = (int)gridDim.x, wid = gwarp_id(), W = gwarp_count();
     const int tid = (int)blockIdx.x * UPDATE_THREADS + t, T = G * UPDATE_THREADS;
     unsigned long long* k = (unsigned long long*)smem;
     if (n <= UPDATE_PAIRS) {
@@ -1078,7 +1077,7 @@ __global__ void __launch_bounds__(UPDATE_THREADS, 1) k_update(UpdateParams p) {
     if (!grid_sync(p.bar, 63)) return;
     const int A = (int)(all >> 32);
     if (A > UPDATE_ROWS) row_plan<true>(p.rp, A, (int)blockIdx.x, G);
-    else row_plan<false>(p.rp, A, w * G + (int)blockIdx.x, G * UPDATE_WARPS);
+    else row_plan<false>(p.rp, A, gwarp_id(), gwarp_count());
     if (!grid_sync(p.bar, 64)) return;
     merge_rows(p.pool, p.keys, B, ctr, p.epos, p.E, p.rp.mrow, p.rp.slices, p.rp.slice_cap, ((ChunkEvents*)s_mem)[w]);
 }

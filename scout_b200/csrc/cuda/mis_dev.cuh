@@ -41,7 +41,7 @@ __device__ __forceinline__ void mis_candidate(const MisParams& p, bool pred, int
 
 __device__ __forceinline__ void mis_body(const MisParams& p) {
     const int W = gwarp_count(), wid = gwarp_id();
-    const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t tid = gthread_id();
     const int64_t T = (int64_t)gridDim.x * blockDim.x;
     const bool leader = blockIdx.x == 0 && threadIdx.x == 0;
     const int nh = ld_volatile(&p.ctr->n_half);
