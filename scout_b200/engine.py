@@ -68,6 +68,18 @@ def as_edges(e) -> np.ndarray:
     return a
 
 
+_PAGE_LOCKED = weakref.WeakValueDictionary()   # the live buffers of pinned_empty, by id
+
+
+def _page_locked(a) -> bool:
+    """Whether `a` lies in memory of pinned_empty / pinned_copy."""
+    while isinstance(a, np.ndarray):
+        a = a.base
+    if isinstance(a, memoryview):
+        a = a.obj
+    return a is not None and _PAGE_LOCKED.get(id(a)) is a
+
+
 def pinned_empty(shape, dtype=np.int32) -> np.ndarray:
     """An uninitialised array in page-locked host memory (scout_host_alloc): edit batches in
     such memory are copied to the device without the staging copy."""
@@ -78,6 +90,7 @@ def pinned_empty(shape, dtype=np.int32) -> np.ndarray:
     _check(LIB.scout_host_alloc(nbytes, C.byref(ptr)))
     buf = (C.c_uint8 * nbytes).from_address(ptr.value)
     weakref.finalize(buf, LIB.scout_host_free, ptr.value)
+    _PAGE_LOCKED[id(buf)] = buf
     return np.frombuffer(buf, dtype=dt, count=count).reshape(shape)
 
 
@@ -207,10 +220,10 @@ class Context:
 
     # ---- repair -----------------------------------------------------------------------
     def repair(self, problem, edges, ops=None, sched: Optional[dict] = None) -> dict:
-        # the batch hinted by the last prefetch(): its device copy is already on the way
-        pf = getattr(self, "_pf", None)
+        # the batch hinted before the previous repair(), which copied it to the device
+        pf, nxt = getattr(self, "_pf", None), getattr(self, "_pf_next", None)
         hinted = pf is not None and edges is pf and ops is None
-        self._pf = None
+        self._pf = self._pf_next = None
         e = as_edges(edges)
         st = ScoutBatchStats()
         sd = ScoutSched()
@@ -223,18 +236,18 @@ class Context:
             ops = np.ascontiguousarray(ops, dtype=np.uint8)
             op = ops.ctypes.data_as(C.POINTER(C.c_uint8))
         self._c(LIB.scout_repair(self._h, _prob(problem), _pedge(e), op, len(e), C.byref(sd), C.byref(st)))
+        self._pf = nxt
         return st.as_dict()
 
     def prefetch(self, next_edges) -> None:
         """Hint the edits of the batch after the next repair: that repair copies them to the
-        device while it runs (and, tiered store, gathers their cold rows into HBM), and a later
-        repair() given the same object uses the copy. A page-locked array (pinned_copy) is read
-        in place and must stay unchanged until then."""
+        device while it runs (and, tiered store, gathers their cold rows into HBM). A page-locked
+        array (pinned_copy) is read in place and must stay unchanged until its own repair(),
+        which, given the same object, uses the device copy instead of uploading it again; any
+        other array is copied here, may change, and is uploaded by its repair()."""
         e = as_edges(next_edges)
         self._c(LIB.scout_prefetch(self._h, _pedge(e), len(e)))
-        # a converted temporary was copied by the call; only the caller's own array, passed to
-        # repair() unchanged, is declared as the hinted batch
-        self._pf = next_edges if e is next_edges else None
+        self._pf_next = next_edges if e is next_edges and _page_locked(e) else None
 
     def repair_probe(self, problem, edges, ops=None, sched: Optional[dict] = None):
         """One batch, every repair variant timed from the same pre-repair state (results must

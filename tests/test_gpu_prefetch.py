@@ -74,3 +74,46 @@ def test_unused_and_mismatched_hints(rmat16):
         o1, a1 = t.graph()
         o2, a2 = ref.graph()
         assert np.array_equal(o1, o2) and np.array_equal(a1, a2)
+
+
+def test_only_page_locked_hints_are_used(rmat16):
+    """A page-locked hint's device copy serves its own repair (nothing is uploaded then); a
+    pageable hint may be overwritten before its repair, which uploads what it holds; a hint
+    with ops, another array of the same content, or a batch in between is uploaded as well."""
+    g, (off, adj) = rmat16
+    init = g.init_state("bfs", 0)
+    b = [stream(off, adj, sb.STREAM_PREFERENTIAL, 200000, 1, seed=500 + i)[0] for i in range(6)]
+    with sb.Context(0) as t, sb.Context(0) as ref:
+        for c in (t, ref):
+            c.load_csr(off, adj)
+            c.upload("bfs", init)
+            c.reserve_batches(200000)
+
+        def both(e, plain=None, **kw):
+            st = t.repair("bfs", e, **kw)
+            ref.repair("bfs", np.array(e if plain is None else plain), **kw)
+            assert np.array_equal(t.download("bfs"), ref.download("bfs"))
+            return st
+
+        p1 = sb.pinned_copy(b[1])
+        t.prefetch(p1)
+        up = both(b[0])["ms_h2d"]
+        assert both(p1)["ms_h2d"] < 0.5 * up          # the copy was there
+        t.prefetch(b[2])
+        both(b[0])
+        b[2][:] = b[3]                                # pageable: free to change
+        both(b[2])
+        p4 = sb.pinned_copy(b[4])
+        t.prefetch(p4)
+        both(b[5])
+        both(np.array(p4))                            # another array
+        t.prefetch(p4)
+        both(b[5])
+        both(b[3])                                    # a batch in between
+        both(p4)
+        t.prefetch(p4)
+        both(b[5])
+        both(p4, ops=np.zeros(len(p4), dtype=np.uint8))
+        o1, a1 = t.graph()
+        o2, a2 = ref.graph()
+        assert np.array_equal(o1, o2) and np.array_equal(a1, a2)
