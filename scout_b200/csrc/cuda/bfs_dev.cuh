@@ -414,7 +414,7 @@ static __device__ void bu_step(const BfsParams& p, int32_t* lv, int nxt, int d, 
 static __device__ bool full_bfs(const BfsParams& p, int mode, long long& bytes, int& rounds) {
     int32_t* lv = p.lv_new;
     const int64_t n = p.g.n;
-    const int64_t tid = gthread_id();
+    const int64_t tid = lthread_id();
     const int64_t T = (int64_t)gridDim.x * blockDim.x;
     const bool leader = blockIdx.x == 0 && threadIdx.x == 0;
     for (int64_t v = tid; v < n; v += T) lv[v] = -1;

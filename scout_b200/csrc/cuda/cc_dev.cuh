@@ -10,7 +10,9 @@ namespace scout {
 constexpr int CC_HCAP = 8192;     // shared hash-set slots per side
 constexpr int CC_FCAP = 4096;     // frontier capacity
 constexpr int CC_MAX_BOUND = 4000;
-constexpr int CC_BIG = 4096;      // rows longer than this are scanned by a whole block in P3
+constexpr int CC_BIG = 1024;      // rows longer than this are scanned by a whole block in P3
+constexpr int CC_ITEMS = 4;       // vertices per thread whose reads overlap in P3's passes
+constexpr int CC_GROUP = 8;       // half-edits a warp takes at a time in P1a
 constexpr size_t CC_SMEM = (size_t)(2 * CC_HCAP + 3 * CC_FCAP) * sizeof(int32_t);
 
 struct CcParams {
@@ -102,17 +104,19 @@ __device__ __forceinline__ int hs_insert(int32_t* hs, int32_t x) {
 
 // Bounded bidirectional search of one deletion (u, v) by the whole block.
 // Returns 0 connected, 1 split (side written to p.side), 2 inconclusive.
-static __device__ int cc_search(const CcParams& p, int32_t u, int32_t v, int32_t cls, long long& bytes, bool record) {
+static __device__ int cc_search(const CcParams& p, int32_t u, int32_t v, int32_t cls, long long& bytes, bool record,
+                                bool neighbours) {
     extern __shared__ int32_t sm[];
     int32_t* hs[2] = {sm, sm + CC_HCAP};
     int32_t* fr[2] = {sm + 2 * CC_HCAP, sm + 2 * CC_HCAP + CC_FCAP};
     int32_t* nf = sm + 2 * CC_HCAP + 2 * CC_FCAP;
     __shared__ int s_fn[2], s_nn, s_touched, s_met, s_over;
     const int t = threadIdx.x;
-    // common-neighbour check: both endpoints adjacent to some w (settles hub-hub deletions)
+    // common-neighbour check: both endpoints adjacent to some w (settles hub-hub deletions; the
+    // deletions' own pairs were checked before they were listed)
     if (t == 0) s_met = 0;
     __syncthreads();
-    {
+    if (neighbours) {
         Row ru = p.g.row[u], rv = p.g.row[v];
         if (rv.len < ru.len) { Row tmp = ru; ru = rv; rv = tmp; }
         const int32_t* a = p.g.pool + ru.start;
@@ -233,6 +237,7 @@ static __device__ int cc_search(const CcParams& p, int32_t u, int32_t v, int32_t
 __device__ __forceinline__ void cc_body(const CcParams& p) {
     const int W = gwarp_count(), wid = gwarp_id();
     const int64_t tid = gthread_id();
+    const int64_t ltid = lthread_id();   // for passes over all vertices
     const int64_t T = (int64_t)gridDim.x * blockDim.x;
     const int64_t n = p.g.n;
     const bool leader = blockIdx.x == 0 && threadIdx.x == 0;
@@ -264,7 +269,7 @@ __device__ __forceinline__ void cc_body(const CcParams& p) {
         const int nm = ld_volatile(&p.ctr->list_count[1]);
         if (leader) p.ctr->ins_eff = nm;   // every successful hook merged two classes
         if (nm > 0) {
-            for (int64_t b = tid - (tid & (WARP - 1)); b < n; b += T) {
+            for (int64_t b = ltid - (ltid & (WARP - 1)); b < n; b += T) {
                 int64_t v = b + lane_id();
                 bool ch = false;
                 if (v < n) {
@@ -283,9 +288,10 @@ __device__ __forceinline__ void cc_body(const CcParams& p) {
         phase_mark(&p.ctr->phase_ns[1]);
         // ---- P1a: one warp per deletion: a common neighbour settles it (most deletions in a
         // dense component, hub-hub ones included); the rest go to the hard list -------------
-        for (int64_t b = (int64_t)wid * WARP; b < nh; b += (int64_t)W * WARP) {
-            // 32 half-edits per warp iteration, then each candidate checked by the whole warp
-            int64_t k0 = b + lane_id();
+        for (int64_t b = (int64_t)wid * CC_GROUP; b < nh; b += (int64_t)W * CC_GROUP) {
+            // CC_GROUP half-edits per warp and turn (few, so that the checks spread over all warps),
+            // then each candidate checked by the whole warp
+            int64_t k0 = lane_id() < CC_GROUP ? b + lane_id() : nh;
             bool cand = false;
             int32_t x = 0, y = 0;
             if (k0 < nh) {
@@ -335,28 +341,43 @@ __device__ __forceinline__ void cc_body(const CcParams& p) {
         // ---- P1b: one block per remaining deletion: the bounded bidirectional search ---------
         const int nhard = min(ld_volatile(&p.ctr->list_count[0]), p.hard_cap);
         if (leader) p.ctr->noop = ld_volatile(&p.ctr->searches) - nhard;   // settled by a common neighbour
+        // The listed deletions whose class is not dirty (few, when there are many) are listed again;
+        // a listed deletion's class is fixed since P0. (hard_cap is four times the most deletions.)
+        int32_t* open_list = p.hard + p.hard_cap / 2;
+        for (int64_t b = tid - (tid & (WARP - 1)); b < nhard; b += T) {
+            const int64_t i = b + lane_id();
+            bool open = false;
+            int32_t k = 0;
+            if (i < nhard) {
+                k = p.hard[i];
+                const int32_t cls = ld_volatile(p.label + (int32_t)(p.hkeys[k] >> (p.B + 1)));
+                p.hcnt[cls] = 0;
+                open = ld_volatile(p.dirty + cls) != p.epoch;
+            }
+            const int at = warp_append(open, &p.ctr->tick[0]);
+            if (open) open_list[at] = k;
+        }
+        if (!grid_sync(p.bar, 49)) return;
+        const int nopen = ld_volatile(&p.ctr->tick[0]);
         while (true) {
             if (threadIdx.x == 0) {
                 int j = atomicAdd(&p.ctr->list_count[3], 1);
-                if (j < nhard) {
-                    // the class of a listed deletion is fixed since P0; a dirty one is not searched
-                    unsigned long long key = p.hkeys[p.hard[j]];
-                    int32_t cls = ld_volatile(p.label + (int32_t)(key >> (p.B + 1)));
-                    p.hcnt[cls] = 0;
-                    if (ld_volatile(p.dirty + cls) == p.epoch) j = -1;
+                if (j < nopen) {
+                    const int32_t cls = ld_volatile(p.label + (int32_t)(p.hkeys[ld_volatile(open_list + j)] >> (p.B + 1)));
+                    if (ld_volatile(p.dirty + cls) == p.epoch) j = -1;   // dirty meanwhile
                 }
                 s_task = j;
             }
             __syncthreads();
             const int j = s_task;
             __syncthreads();
-            if (j >= nhard) break;
+            if (j >= nopen) break;
             if (j < 0) continue;
-            unsigned long long key = p.hkeys[p.hard[j]];
-            int32_t x = (int32_t)(key >> (p.B + 1));
-            int32_t y = (int32_t)(key & ((1ull << p.B) - 1));
-            int32_t cls = ld_volatile(p.label + x);
-            int res = cc_search(p, x, y, cls, bytes, true);
+            const unsigned long long key = p.hkeys[ld_volatile(open_list + j)];
+            const int32_t x = (int32_t)(key >> (p.B + 1));
+            const int32_t y = (int32_t)(key & ((1ull << p.B) - 1));
+            const int32_t cls = ld_volatile(p.label + x);
+            int res = cc_search(p, x, y, cls, bytes, true, false);
             if (threadIdx.x == 0 && res == 2 && atomicExch(p.dirty + cls, p.epoch) != p.epoch)
                 atomicAdd(&p.ctr->recomputes, 1);
             __syncthreads();
@@ -386,7 +407,7 @@ __device__ __forceinline__ void cc_body(const CcParams& p) {
             if (ld_volatile(p.cnt + cls) < 2 || ld_volatile(p.dirty + cls) == p.epoch) continue;
             int32_t w = (int32_t)p.rec[3 * i + 2], f = ld_volatile(p.firstw + cls);
             if (w == f || f < 0) continue;
-            int res = cc_search(p, w, f, cls, bytes, false);
+            int res = cc_search(p, w, f, cls, bytes, false, true);
             if (threadIdx.x == 0 && res != 0 && atomicExch(p.dirty + cls, p.epoch) != p.epoch)
                 atomicAdd(&p.ctr->recomputes, 1);
             __syncthreads();
@@ -400,7 +421,10 @@ __device__ __forceinline__ void cc_body(const CcParams& p) {
             if (ld_volatile(p.dirty + cls) == p.epoch) continue;
             if (lane_id() == 0) {
                 atomicAdd(&p.ctr->splits, 1);
-                if (mn == cls) p.remf[cls] = p.epoch;
+                if (mn == cls) {
+                    p.remf[cls] = p.epoch;
+                    atomicAdd((unsigned long long*)&p.ctr->aux64[2], 1ull);   // classes without their minimum
+                }
             }
             for (int b0 = 0; b0 < size; b0 += WARP) {
                 int j = b0 + (int)lane_id();
@@ -415,27 +439,29 @@ __device__ __forceinline__ void cc_body(const CcParams& p) {
             }
         }
         if (!grid_sync(p.bar, 33)) return;
-        // remainder of a class whose minimum left with the split side: its own minimum
-        for (int64_t v = tid; v < n; v += T) {
-            int32_t l = p.label[v];
-            if (ld_volatile(p.remf + l) == p.epoch && ld_volatile(p.st_side + v) != p.epoch &&
-                ld_volatile(p.dirty + l) != p.epoch)
-                atomicMin(p.newmin + l, (int32_t)v);
-        }
-        if (tid == 0) bytes += 12LL * n;
-        if (!grid_sync(p.bar, 34)) return;
-        for (int64_t b = tid - (tid & (WARP - 1)); b < n; b += T) {
-            int64_t v = b + lane_id();
-            bool ch = false;
-            if (v < n) {
+        if (ld_volatile(&p.ctr->aux64[2])) {
+            // remainder of a class whose minimum left with the split side: its own minimum
+            for (int64_t v = ltid; v < n; v += T) {
                 int32_t l = p.label[v];
                 if (ld_volatile(p.remf + l) == p.epoch && ld_volatile(p.st_side + v) != p.epoch &&
-                    ld_volatile(p.dirty + l) != p.epoch) {
-                    int32_t m = ld_volatile(p.newmin + l);
-                    if (m != l) { p.label[v] = m; ch = true; }
-                }
+                    ld_volatile(p.dirty + l) != p.epoch)
+                    atomicMin(p.newmin + l, (int32_t)v);
             }
-            cc_touch(p, ch, (int32_t)v);
+            if (tid == 0) bytes += 12LL * n;
+            if (!grid_sync(p.bar, 34)) return;
+            for (int64_t b = ltid - (ltid & (WARP - 1)); b < n; b += T) {
+                int64_t v = b + lane_id();
+                bool ch = false;
+                if (v < n) {
+                    int32_t l = p.label[v];
+                    if (ld_volatile(p.remf + l) == p.epoch && ld_volatile(p.st_side + v) != p.epoch &&
+                        ld_volatile(p.dirty + l) != p.epoch) {
+                        int32_t m = ld_volatile(p.newmin + l);
+                        if (m != l) { p.label[v] = m; ch = true; }
+                    }
+                }
+                cc_touch(p, ch, (int32_t)v);
+            }
         }
         if (!grid_sync(p.bar, 35)) return;
         // restore per-class scratch of split classes
@@ -454,33 +480,100 @@ __device__ __forceinline__ void cc_body(const CcParams& p) {
     if (!full && ld_volatile(&p.ctr->recomputes) == 0) {
         goto done;
     }
-    for (int64_t v = tid; v < n; v += T) {
-        bool d = full || ld_volatile(p.dirty + p.label[v]) == p.epoch;
-        p.vp[v] = d ? (int32_t)v : -1;
-    }
-    if (!grid_sync(p.bar, 36)) return;
     {
-        // Afforest (Sutton, Ben-Nun, Barak, IPDPS 2018): link every dirty vertex to its first
-        // two neighbours, compress, estimate the dominant root by sampling, then only vertices
-        // outside that root scan the rest of their rows (an edge between the dominant tree
-        // and another vertex is linked from the other vertex's row). An edge leaving a dirty
-        // class means the uploaded labels did not describe the components of the graph: it is
-        // flagged (SCOUT_E_STATE) instead of followed.
+        // Every vertex of a dirty class starts at its first neighbour if that has a lower id (rows are
+        // sorted, so it is the lowest; no cycle can arise and no one else writes the entry, so no
+        // atomics), else at itself. Then Afforest (Sutton, Ben-Nun, Barak, IPDPS 2018): compress,
+        // link the first two neighbours that are not joined yet, compress, estimate the dominant
+        // root by sampling, then only vertices outside that root scan the rest of their rows
+        // (an edge between the dominant tree and another vertex is linked from the other
+        // vertex's row). An edge leaving a dirty class means the uploaded labels did not describe
+        // the components of the graph: it is flagged (SCOUT_E_STATE) instead of followed.
+        // What bounds it: chains of random reads, so a thread's CC_ITEMS vertices read side by
+        // side, and after a compress most neighbours prove joined by one comparison. Recompute of
+        // 2 M vertices (32 M edges): 295 us with both neighbours linked by unions and
+        // volatile reads, 110 us so.
         constexpr int AF_FIRST = 2;
-        for (int r = 0; r < AF_FIRST; r++) {
-            for (int64_t v = tid; v < n; v += T) {
-                if (ld_volatile(p.vp + v) < 0) continue;
-                Row rr = p.g.row[v];
-                if (r < rr.len) {
-                    int32_t w = p.g.pool[rr.start + r];
-                    if (ld_volatile(p.vp + w) < 0) atomicExch(&p.ctr->pad, 1);
-                    else uf_union(p.vp, (int32_t)v, w);
-                }
+        for (int64_t b = ltid; b < n; b += CC_ITEMS * T) {
+            int32_t lab[CC_ITEMS], w[CC_ITEMS];
+            Row r[CC_ITEMS];
+            bool d[CC_ITEMS];
+#pragma unroll
+            for (int u = 0; u < CC_ITEMS; u++) {
+                const int64_t v = b + u * T;
+                lab[u] = v < n && !full ? p.label[v] : 0;
+                r[u] = v < n ? p.g.row[v] : Row{0, 0, 0};
             }
-            if (!grid_sync(p.bar, 42 + r)) return;
+#pragma unroll
+            for (int u = 0; u < CC_ITEMS; u++) {
+                d[u] = b + u * T < n && (full || p.dirty[lab[u]] == p.epoch);
+                w[u] = d[u] && r[u].len > 0 ? p.g.pool[r[u].start] : -1;
+            }
+#pragma unroll
+            for (int u = 0; u < CC_ITEMS; u++) {
+                const int64_t v = b + u * T;
+                if (v >= n) continue;
+                bool in = true;
+                if (!full && w[u] >= 0) {   // the neighbour's class must be dirty as well
+                    const int32_t lw = p.label[w[u]];
+                    in = lw == lab[u] || p.dirty[lw] == p.epoch;
+                    if (!in) atomicExch(&p.ctr->pad, 1);
+                }
+                p.vp[v] = !d[u] ? -1 : w[u] >= 0 && w[u] < v && in ? w[u] : (int32_t)v;
+            }
         }
-        for (int64_t v = tid; v < n; v += T)
-            if (ld_volatile(p.vp + v) >= 0) p.vp[v] = uf_find(p.vp, (int32_t)v);
+        if (!grid_sync(p.bar, 36)) return;
+        // Every vertex of a dirty class points at its root. No root moves meanwhile, and a parent
+        // that was read before it moved up is still an ancestor, so the reads may come from L1
+        // (all chains end at a few roots, one L2 line each).
+        auto compress = [&]() {
+            for (int64_t b = ltid; b < n; b += CC_ITEMS * T) {
+                int32_t q[CC_ITEMS], up[CC_ITEMS];
+#pragma unroll
+                for (int u = 0; u < CC_ITEMS; u++) q[u] = b + u * T < n ? p.vp[b + u * T] : -1;
+                for (bool more = true; more;) {
+                    more = false;
+#pragma unroll
+                    for (int u = 0; u < CC_ITEMS; u++) up[u] = q[u] >= 0 ? p.vp[q[u]] : -1;
+#pragma unroll
+                    for (int u = 0; u < CC_ITEMS; u++) {
+                        more |= up[u] != q[u];
+                        q[u] = up[u];
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < CC_ITEMS; u++)
+                    if (q[u] >= 0) p.vp[b + u * T] = q[u];
+            }
+        };
+        compress();
+        if (!grid_sync(p.bar, 42)) return;
+        for (int64_t b = ltid; b < n; b += CC_ITEMS * T) {
+            int32_t pv[CC_ITEMS], w0[CC_ITEMS], w1[CC_ITEMS], q0[CC_ITEMS], q1[CC_ITEMS];
+#pragma unroll
+            for (int u = 0; u < CC_ITEMS; u++) {
+                const int64_t v = b + u * T;
+                pv[u] = v < n ? p.vp[v] : -1;   // (an ancestor is enough)
+                const Row r = pv[u] >= 0 ? p.g.row[v] : Row{0, 0, 0};
+                w0[u] = r.len > 0 ? p.g.pool[r.start] : -1;
+                w1[u] = r.len > 1 ? p.g.pool[r.start + 1] : -1;
+                if (w0[u] < v) w0[u] = -1;   // joined by the start (or flagged there)
+            }
+#pragma unroll
+            for (int u = 0; u < CC_ITEMS; u++) {
+                q0[u] = w0[u] >= 0 ? p.vp[w0[u]] : pv[u];
+                q1[u] = w1[u] >= 0 ? p.vp[w1[u]] : pv[u];
+            }
+#pragma unroll
+            for (int u = 0; u < CC_ITEMS; u++) {
+                if (pv[u] < 0) continue;
+                if (q0[u] < 0 || q1[u] < 0) atomicExch(&p.ctr->pad, 1);
+                if (q0[u] >= 0 && q0[u] != pv[u]) uf_union(p.vp, pv[u], q0[u]);
+                if (q1[u] >= 0 && q1[u] != pv[u]) uf_union(p.vp, pv[u], q1[u]);
+            }
+        }
+        if (!grid_sync(p.bar, 43)) return;
+        compress();
         if (tid == 0) bytes += 24LL * n;
         if (!grid_sync(p.bar, 44)) return;
         if (blockIdx.x == 0) {   // mode of the roots of up to 1024 sampled dirty vertices
@@ -493,11 +586,12 @@ __device__ __forceinline__ void cc_body(const CcParams& p) {
             for (int i = threadIdx.x; i < 4096; i += (int)blockDim.x) {
                 int64_t v = (int64_t)(((unsigned long long)i * 2654435761ull) % (unsigned long long)n);
                 int32_t r = ld_volatile(p.vp + v);
-                if (r < 0) continue;
+                const unsigned same = __match_any_sync(__activemask(), r);   // one add per root and warp
+                if (r < 0 || (int)lane_id() != __ffs(same) - 1) continue;
                 unsigned h = ((unsigned)r * 2654435761u) & 2047u;
                 for (int pr = 0; pr < 2048; pr++) {
                     int32_t prev = atomicCAS(&s_key[h], -1, r);
-                    if (prev == -1 || prev == r) { atomicAdd(&s_cnt[h], 1); break; }
+                    if (prev == -1 || prev == r) { atomicAdd(&s_cnt[h], __popc(same)); break; }
                     h = (h + 1) & 2047u;
                 }
             }
@@ -510,10 +604,9 @@ __device__ __forceinline__ void cc_body(const CcParams& p) {
         }
         if (!grid_sync(p.bar, 45)) return;
         const int32_t gr = (int32_t)ld_volatile(&p.ctr->aux64[1]);
-        // compact lists of the vertices outside the dominant root (short rows / long rows)
-        if (leader) { p.ctr->q_count[1] = 0; p.ctr->q_count[2] = 0; }
-        if (!grid_sync(p.bar, 46)) return;
-        for (int64_t b = tid - (tid & (WARP - 1)); b < n; b += T) {
+        // compact lists of the vertices outside the dominant root (short rows / long rows; their
+        // counters are zero since the batch began)
+        for (int64_t b = ltid - (ltid & (WARP - 1)); b < n; b += T) {
             int64_t v = b + lane_id();
             bool sm_ = false, bg = false;
             if (v < n) {
@@ -535,12 +628,20 @@ __device__ __forceinline__ void cc_body(const CcParams& p) {
             const int32_t v = p.merged[i];
             Row r = p.g.row[v];
             const int32_t* rw = p.g.pool + r.start;
-            for (int b0 = AF_FIRST; b0 < r.len; b0 += WARP) {
-                int k = b0 + (int)lane_id();
-                if (k < r.len) {
-                    int32_t w = rw[k];
-                    if (ld_volatile(p.vp + w) < 0) atomicExch(&p.ctr->pad, 1);
-                    else uf_union(p.vp, v, w);
+            const int32_t pv = ld_volatile(p.vp + v);
+            for (int b0 = AF_FIRST; b0 < r.len; b0 += CC_ITEMS * WARP) {
+                int32_t w[CC_ITEMS], q[CC_ITEMS];
+#pragma unroll
+                for (int u = 0; u < CC_ITEMS; u++) {
+                    const int k = b0 + u * WARP + (int)lane_id();
+                    w[u] = k < r.len ? rw[k] : -1;
+                }
+#pragma unroll
+                for (int u = 0; u < CC_ITEMS; u++) q[u] = w[u] >= 0 ? ld_volatile(p.vp + w[u]) : pv;
+#pragma unroll
+                for (int u = 0; u < CC_ITEMS; u++) {
+                    if (q[u] < 0) atomicExch(&p.ctr->pad, 1);
+                    else if (q[u] != pv) uf_union(p.vp, pv, q[u]);
                 }
             }
             if (lane_id() == 0) bytes += 8LL * r.len;
@@ -549,23 +650,42 @@ __device__ __forceinline__ void cc_body(const CcParams& p) {
             const int32_t v = p.side[i];
             Row r = p.g.row[v];
             const int32_t* rw = p.g.pool + r.start;
+            const int32_t pv = ld_volatile(p.vp + v);
             for (long long k = AF_FIRST + threadIdx.x; k < r.len; k += blockDim.x) {
-                int32_t w = rw[k];
-                if (ld_volatile(p.vp + w) < 0) atomicExch(&p.ctr->pad, 1);
-                else uf_union(p.vp, v, w);
+                const int32_t q = ld_volatile(p.vp + rw[k]);
+                if (q < 0) atomicExch(&p.ctr->pad, 1);
+                else if (q != pv) uf_union(p.vp, pv, q);
             }
             if (threadIdx.x == 0) bytes += 8LL * r.len;
         }
     }
     if (!grid_sync(p.bar, 37)) return;
-    for (int64_t b = tid - (tid & (WARP - 1)); b < n; b += T) {
-        int64_t v = b + lane_id();
-        bool ch = false;
-        if (v < n && ld_volatile(p.vp + v) >= 0) {
-            int32_t root = uf_find(p.vp, (int32_t)v);
-            if (p.label[v] != root) { p.label[v] = root; ch = true; }
+    // the labels: every root is the minimum of its class (no union runs any more)
+    for (int64_t b = ltid - (ltid & (WARP - 1)); b < n; b += CC_ITEMS * T) {
+        int32_t q[CC_ITEMS], up[CC_ITEMS], lab[CC_ITEMS];
+#pragma unroll
+        for (int u = 0; u < CC_ITEMS; u++) {
+            const int64_t v = b + u * T + lane_id();
+            q[u] = v < n ? p.vp[v] : -1;
+            lab[u] = v < n ? p.label[v] : -1;
         }
-        cc_touch(p, ch, (int32_t)v);
+        for (bool more = true; more;) {
+            more = false;
+#pragma unroll
+            for (int u = 0; u < CC_ITEMS; u++) up[u] = q[u] >= 0 ? p.vp[q[u]] : -1;
+#pragma unroll
+            for (int u = 0; u < CC_ITEMS; u++) {
+                more |= up[u] != q[u];
+                q[u] = up[u];
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < CC_ITEMS; u++) {
+            const int64_t v = b + u * T + lane_id();
+            const bool ch = q[u] >= 0 && lab[u] != q[u];
+            if (ch) p.label[v] = q[u];
+            cc_touch(p, ch, (int32_t)v);
+        }
     }
     if (tid == 0) bytes += 16LL * n;
 done:

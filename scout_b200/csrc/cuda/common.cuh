@@ -214,9 +214,12 @@ __device__ __forceinline__ void phase_mark(unsigned long long* slot) {
 }
 
 // Global warp index / count for grid-stride warp loops: neighbouring indices lie in different
-// blocks, so that a few items go to as many SMs. gthread_id numbers the threads the same way.
+// blocks, so that a few items go to as many SMs. gthread_id numbers the threads the same way;
+// lthread_id numbers a block's threads together, for passes over whole arrays (what they list
+// comes out in stretches of consecutive ids, which the host's commit loop walks faster).
 __device__ __forceinline__ int gwarp_id() { return (int)(threadIdx.x / WARP * gridDim.x + blockIdx.x); }
 __device__ __forceinline__ int64_t gthread_id() { return (int64_t)gwarp_id() * WARP + lane_id(); }
+__device__ __forceinline__ int64_t lthread_id() { return blockIdx.x * (int64_t)blockDim.x + threadIdx.x; }
 __device__ __forceinline__ int gwarp_count() { return (int)((gridDim.x * blockDim.x) / WARP); }
 
 }  // namespace scout
