@@ -18,8 +18,9 @@ struct DevCounters {
     int n_del;          // edits classified as deletions
     int n_half;         // applied half-edits (2 per applied edit)
     int n_aff;          // vertices whose row changed
-    int n_small, n_large;     // rows of the short-row merge / long rows compacted in place
-    int n_slices, n_long;     // merge slices / rows they belong to
+    int n_one, n_short;       // short rows with one half-edit / with several
+    int n_slices, n_rest;     // merge slices / rows that are not of the first kind
+    int n_long;               // long rows compacted in place (tiered store)
     int plan_ticket, merge_ticket;   // tiles of the plan, items of the merge handed out so far
     long long new_elems;      // elements written to the pool this batch (HBM part when split)
     long long new_elems_host; // tiered store, split batch: elements written to the host pool
@@ -60,7 +61,7 @@ struct DevCounters {
 // What a batch zeroes at its start and copies back at its end, in one piece: the counters, the
 // barriers of the update and of the repair, and the changed entries when they are few (then
 // the commit needs no launch and no copy of its own; not zeroed).
-constexpr int COMMIT_PAIRS = 1024;
+constexpr int COMMIT_PAIRS = 2048;
 struct DevBatch {
     DevCounters ctr;
     scout::GridBar bar[2];
@@ -162,7 +163,8 @@ struct scout_ctx {
     int32_t* d_seg_b = nullptr;     // their segments' begins in the half-edits (2m + 1)
     int32_t* d_seg_d = nullptr;     // their segments' first deletions (2m)
     int32_t* d_longs = nullptr;     // long affected rows compacted in place (2m)
-    scout::MergeRow* d_mrow = nullptr;   // merge records: short rows from the front, others from the back (2m)
+    int32_t* d_shorts = nullptr;    // short affected rows of several half-edits (2m)
+    scout::MergeRow* d_mrow = nullptr;   // merge records: short rows of one half-edit from the front, others from the back (2m)
     int64_t* d_slices = nullptr;  int64_t cap_slices = 0;   // merge items (row << 32 | slice)
     void* d_update = nullptr;       // scratch of the one-launch update
     int64_t* d_coff = nullptr;      // compaction offsets (n + 1)

@@ -417,8 +417,9 @@ struct RowPlan {
     const int32_t* seg_b;
     const int32_t* seg_d;
     const int32_t* E;
-    MergeRow* mrow;        // short rows from the front, the others from the back
+    MergeRow* mrow;        // short rows of one half-edit from the front, the others from the back
     int64_t mcap;
+    int32_t* shorts;       // records of the other short rows
     int64_t* slices;       // (record << 32 | slice)
     int64_t slice_cap;
     int32_t* longs;        // records of long rows compacted in place
@@ -473,7 +474,7 @@ __global__ void __launch_bounds__(ROW_THREADS) k_row_sizes(RowPlan p) {
 template <bool BLOCK>
 __device__ __forceinline__ void row_plan(const RowPlan& p, int A, int group, int groups) {
     const int ROWS = BLOCK ? (int)blockDim.x : WARP;
-    __shared__ long long s_base[6];
+    __shared__ long long s_base[7];
     const int t = BLOCK ? (int)threadIdx.x : (int)lane_id();
     long long nnz_delta = 0, bytes = 0;
     for (int a0 = group * ROWS; a0 < A; a0 += groups * ROWS) {
@@ -482,7 +483,7 @@ __device__ __forceinline__ void row_plan(const RowPlan& p, int A, int group, int
         Row r{0, 0, 0};
         int32_t u = 0;
         int b = 0, d = 0, e = 0, nl = 0, ns = 0;
-        bool ip = false, cold = false, sm = false, lip = false;
+        bool ip = false, cold = false, one = false, sm = false, lip = false;
         if (ok) {
             u = p.aff[a];
             b = p.seg_b[a];
@@ -493,15 +494,16 @@ __device__ __forceinline__ void row_plan(const RowPlan& p, int A, int group, int
             ip = in_place_row(d - b, r.len, p.long_in_place);
             cold = p.split && !in_hbm(r, p.hbm_cap);
             lip = ip && r.len > IN_PLACE_LEN;
-            sm = r.len <= SMALL_LEN && e - b <= WARP;
-            ns = sm || lip ? 0 : ip ? 1 : max(1, (r.len + SLICE - 1) / SLICE);
+            one = r.len <= SMALL_LEN && e - b == 1;
+            sm = !one && r.len <= SMALL_LEN && e - b <= WARP;
+            ns = one || sm || lip ? 0 : ip ? 1 : max(1, (r.len + SLICE - 1) / SLICE);
             nnz_delta += nl - r.len;
             bytes += 4LL * ((long long)r.len + nl) + 8LL * (e - b) + 16;
         }
         const long long need = ok && !ip ? (long long)r.len + (d - b) : 0;
-        // counts packed: slices 30 bits, short rows, other rows, long rows in place 11 bits each
-        long long th, tc = 0, tn, t0, oh = cold ? 0 : need, oc = 0;
-        long long on = (long long)ns | ((long long)(ok && sm) << 30) | ((long long)(ok && !sm) << 41) | ((long long)lip << 52);
+        // counts packed: slices 30 bits, rows of one half-edit, other rows, short ones 11 bits each
+        long long th, tc = 0, tn, tl = 0, oh = cold ? 0 : need, oc = 0, ol = lip;
+        long long on = (long long)ns | ((long long)(ok && one) << 30) | ((long long)(ok && !one) << 41) | ((long long)sm << 52);
         auto scan2 = [](long long& x, long long& y, long long* tx, long long* ty) {
             if (BLOCK) {
                 block_scan2(x, y, tx, ty);
@@ -514,11 +516,10 @@ __device__ __forceinline__ void row_plan(const RowPlan& p, int A, int group, int
             }
         };
         scan2(oh, on, &th, &tn);
-        if (p.split) {
-            long long zero = 0;
+        if (p.long_in_place) {   // tiered store: the second destination, the long rows in place
             oc = cold ? need : 0;
             if (BLOCK) __syncthreads();   // the first scan's sums are read
-            scan2(oc, zero, &tc, &t0);
+            scan2(oc, ol, &tc, &tl);
         }
         // one thread per counter: the atomics' latencies overlap
         long long base = 0;
@@ -527,25 +528,27 @@ __device__ __forceinline__ void row_plan(const RowPlan& p, int A, int group, int
             if (x)
                 base = (long long)atomicAdd((unsigned long long*)(t ? &p.ctr->new_elems_host : &p.ctr->new_elems),
                                             (unsigned long long)x);
-        } else if (t < 6) {
-            int* to = t == 2 ? &p.ctr->n_slices : t == 3 ? &p.ctr->n_small : t == 4 ? &p.ctr->n_long : &p.ctr->n_large;
-            const int x = t == 2 ? (int)(tn & ((1ll << 30) - 1)) : (int)(tn >> (30 + 11 * (t - 3))) & 2047;
+        } else if (t < 7) {
+            int* to = t == 2 ? &p.ctr->n_slices : t == 3 ? &p.ctr->n_one : t == 4 ? &p.ctr->n_rest
+                      : t == 5 ? &p.ctr->n_short : &p.ctr->n_long;
+            const int x = t == 6 ? (int)tl : t == 2 ? (int)(tn & ((1ll << 30) - 1)) : (int)(tn >> (30 + 11 * (t - 3))) & 2047;
             if (x) base = atomicAdd(to, x);
         }
-        long long bs[6];
+        long long bs[7];
         if (BLOCK) {
-            if (t < 6) s_base[t] = base;
+            if (t < 7) s_base[t] = base;
             __syncthreads();
         }
 #pragma unroll
-        for (int j = 0; j < 6; j++) bs[j] = BLOCK ? s_base[j] : __shfl_sync(0xffffffffu, base, j);
+        for (int j = 0; j < 7; j++) bs[j] = BLOCK ? s_base[j] : __shfl_sync(0xffffffffu, base, j);
         if (ok) {
             long long dst = r.start;
             if (!ip) dst = cold ? p.base_host + bs[1] + oc : p.base_hbm + bs[0] + oh;
-            const long long at = sm ? bs[3] + ((on >> 30) & 2047) : p.mcap - 1 - (bs[4] + ((on >> 41) & 2047));
+            const long long at = one ? bs[3] + ((on >> 30) & 2047) : p.mcap - 1 - (bs[4] + ((on >> 41) & 2047));
             p.mrow[at] = MergeRow{r.start, dst, r.len, b, d, e};
             p.row[u] = ip ? Row{r.start, nl, r.cap} : Row{dst, nl, r.len + (d - b)};
-            if (lip) p.longs[bs[5] + ((on >> 52) & 2047)] = (int32_t)at;
+            if (sm) p.shorts[bs[5] + ((on >> 52) & 2047)] = (int32_t)at;
+            if (lip) p.longs[bs[6] + ol] = (int32_t)at;
             const long long s0 = bs[2] + (on & ((1ll << 30) - 1));
             if (s0 + ns > p.slice_cap) { if (ns) atomicExch(&p.ctr->overflow, 1); }
             else for (int s = 0; s < ns; s++) p.slices[s0 + s] = (at << 32) | s;
@@ -574,12 +577,14 @@ __global__ void __launch_bounds__(ROW_THREADS) k_row_plan(RowPlan p) {
 // row's sorted edit list the shift is constant, so the merge compares no values: a warp enters
 // the events of 1,024 old entries into bitmaps, a lane per event, and copies the entries 32 at a
 // time, each finding its shift by counting bits.
-//
-// What bounds it: for long rows HBM traffic (old rows read, new rows written) at 32 warps per SM
-// with up to 16 loads in flight per lane; for short ones the instructions per row. 10^6
-// preferential edits at scale 22 (0.92 GB of rows): 360 us, 10^4 edits there (0.25 GB): 64 us;
-// 680 and 122 us for the three kernels before it and the scan they waited on, which searched
-// the insertions for every surviving entry.
+// Rows go three ways: short ones of one half-edit (most rows of a batch) by eight lanes each, other
+// rows of at most 32 half-edits with a lane per event, the rest slice by slice with their
+// events entered chunk by chunk.
+// What bounds it: on large graphs reads of rows scattered over the pool (10^6 preferential edits
+// at scale 22, 0.92 GB of rows: 328 us; 10^4 there, 0.25 GB: 58 us), on smaller ones the
+// instructions per event (500,000 edits at scale 20: 120 us, 186 with every event of a slice
+// searched on its own). The three kernels before it and the scan they waited on, which searched
+// the insertions for every surviving entry, took 680 and 122 us at scale 22.
 constexpr int MERGE_THREADS = 256;
 constexpr int MERGE_WARPS = MERGE_THREADS / WARP;
 constexpr int MERGE_U = 8;                 // 32-entry groups of a slice in flight
@@ -728,17 +733,84 @@ static __device__ __forceinline__ void merge_slice(int32_t* __restrict__ pool, c
         for (int k = ii + l; k < r.d; k += WARP) N[r.len + (k - r.b) - gone] = key_v(keys[k], B);
 }
 
+// A whole row of at most 32 half-edits: a lane holds each event, no chunk is prepared.
+static __device__ __forceinline__ void merge_mid(int32_t* __restrict__ pool, const unsigned long long* __restrict__ keys,
+                                                 int B, const uint32_t* __restrict__ epos, const MergeRow& r) {
+    constexpr int STEP = MERGE_U * WARP;
+    const int l = (int)lane_id(), len = r.len;
+    const unsigned lt = (1u << l) - 1, le = lt | (1u << l);
+    const int32_t* O = pool + r.start + l;
+    int32_t* N = pool + r.dst;
+    int32_t x[MERGE_U];
+#pragma unroll
+    for (int u = 0; u < MERGE_U; u++) x[u] = u * WARP + l < len ? O[u * WARP] : 0;
+    const uint32_t ev = r.b + l < r.e ? epos[r.b + l] : 0u;
+    const int pos = (int)(ev >> 1);
+    const bool ins = r.b + l < r.d, del = (ev & 1u) != 0;
+    const int32_t y = ins ? key_v(keys[r.b + l], B) : 0;
+    int shift = 0, gone = 0;
+    for (int b0 = 0; b0 < len; b0 += STEP) {
+        int32_t nx[MERGE_U];
+        if (b0 + 2 * STEP <= len) {
+#pragma unroll
+            for (int u = 0; u < MERGE_U; u++) nx[u] = O[b0 + STEP + u * WARP];
+        } else {
+#pragma unroll
+            for (int u = 0; u < MERGE_U; u++) nx[u] = b0 + STEP + u * WARP + l < len ? O[b0 + STEP + u * WARP] : 0;
+        }
+        __syncwarp();   // a row compacted where it lies: these loads precede the stores below
+        int32_t* M = N + b0 + l;
+        if (!__any_sync(0xffffffffu, (ins || del) && (unsigned)(pos - b0) < STEP)) {
+            if (b0 + STEP <= len) {
+#pragma unroll
+                for (int u = 0; u < MERGE_U; u++) M[u * WARP + shift] = x[u];
+            } else {
+#pragma unroll
+                for (int u = 0; u < MERGE_U; u++)
+                    if (b0 + u * WARP + l < len) M[u * WARP + shift] = x[u];
+            }
+        } else {
+#pragma unroll
+            for (int u = 0; u < MERGE_U; u++) {
+                const int at = pos - b0 - u * WARP;
+                const bool here = (unsigned)at < WARP;
+                const unsigned bit = 1u << (at & 31);
+                const unsigned dm = __reduce_or_sync(0xffffffffu, del && here ? bit : 0u);
+                const bool in = ins && here && pos < len;
+                const unsigned mi = __ballot_sync(0xffffffffu, in);
+                int to = shift - __popc(dm & lt);
+                if (mi) {
+                    const unsigned im = __reduce_or_sync(0xffffffffu, in ? bit : 0u);
+                    if (__popc(im) == __popc(mi)) {
+                        to += __popc(im & le);
+                    } else {
+                        for (unsigned q = mi; q; q &= q - 1) to += __shfl_sync(0xffffffffu, at, __ffs(q) - 1) <= l;
+                    }
+                    if (in) N[pos + l - gone - __popc(dm & (bit - 1))] = y;
+                }
+                if (b0 + u * WARP + l < len && !((dm >> l) & 1u)) M[u * WARP + to] = x[u];
+                shift += __popc(mi) - __popc(dm);
+                gone += __popc(dm);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < MERGE_U; u++) x[u] = nx[u];
+    }
+    if (ins && pos == len) N[len + l - gone] = y;   // past the last entry
+}
+
 // Short rows (at most SMALL_LEN entries and 32 half-edits): all events of a row fit one warp.
 static __device__ __forceinline__ void merge_short(int32_t* __restrict__ pool, const unsigned long long* __restrict__ keys,
                                                    int B, const uint32_t* __restrict__ epos,
-                                                   const MergeRow* __restrict__ mrow, int i0, int cnt) {
+                                                   const MergeRow* __restrict__ mrow,
+                                                   const int32_t* __restrict__ shorts, int i0, int cnt) {
     const int l = (int)lane_id();
     const unsigned lt = (1u << l) - 1, le = lt | (1u << l);
     MergeRow r{0, 0, 0, 0, 0, 0};
-    if (l < cnt) r = mrow[i0 + l];
+    if (l < cnt) r = mrow[shorts[i0 + l]];
     for (int j0 = 0; j0 < cnt; j0 += MERGE_ROWS) {
         long long st[MERGE_ROWS], ds[MERGE_ROWS];
-        int len[MERGE_ROWS], pos[MERGE_ROWS], ne[MERGE_ROWS];
+        int len[MERGE_ROWS], pos[MERGE_ROWS];
         int32_t x0[MERGE_ROWS], x1[MERGE_ROWS], y[MERGE_ROWS];
         bool ins[MERGE_ROWS], del[MERGE_ROWS];
 #pragma unroll
@@ -750,9 +822,9 @@ static __device__ __forceinline__ void merge_short(int32_t* __restrict__ pool, c
             len[u] = __shfl_sync(0xffffffffu, r.len, j);
             const int b = __shfl_sync(0xffffffffu, r.b, j);
             int p = __shfl_sync(0xffffffffu, r.d, j) - b;
-            ne[u] = __shfl_sync(0xffffffffu, r.e, j) - b;
-            if (!have) { len[u] = 0; p = 0; ne[u] = 0; }
-            const uint32_t e = l < ne[u] ? epos[b + l] : 0u;
+            int ne = __shfl_sync(0xffffffffu, r.e, j) - b;
+            if (!have) { len[u] = 0; p = 0; ne = 0; }
+            const uint32_t e = l < ne ? epos[b + l] : 0u;
             pos[u] = (int)(e >> 1);
             del[u] = (e & 1u) != 0;   // matched deletions only
             ins[u] = l < p;
@@ -766,21 +838,6 @@ static __device__ __forceinline__ void merge_short(int32_t* __restrict__ pool, c
             int32_t* N = pool + ds[u];
             const int32_t* O = pool + st[u];
             int32_t x = x0[u], xn = x1[u];
-            if (ne[u] <= 1) {   // one half-edit (most rows) or none left here
-                const int at = __shfl_sync(0xffffffffu, pos[u], 0);
-                const bool in = __shfl_sync(0xffffffffu, (int)ins[u], 0) != 0;
-                const bool cut = __shfl_sync(0xffffffffu, (int)del[u], 0) != 0;
-                for (int e = l; e - l < len[u]; e += WARP) {
-                    const int32_t xnn = e + 2 * WARP < len[u] ? O[e + 2 * WARP] : 0;
-                    __syncwarp();
-                    const int to = e + (in && e >= at) - (cut && e > at);
-                    if (e < len[u] && !(cut && e == at)) N[to] = x;
-                    x = xn;
-                    xn = xnn;
-                }
-                if (l == 0 && in) N[at] = y[u];
-                continue;
-            }
             int shift = 0, gone = 0;   // insertions minus cancelled entries, and cancelled entries, before the group
             for (int e0 = 0; e0 < len[u]; e0 += WARP) {
                 int32_t xnn = 0;
@@ -814,31 +871,79 @@ static __device__ __forceinline__ void merge_short(int32_t* __restrict__ pool, c
     }
 }
 
+// Short rows of one half-edit (most of a batch's rows): eight lanes each, four rows at a time, 32
+// entries of each in flight. Every entry past the event moves by one place.
+static __device__ __forceinline__ void merge_one(int32_t* __restrict__ pool, const unsigned long long* __restrict__ keys,
+                                                 int B, const uint32_t* __restrict__ epos,
+                                                 const MergeRow* __restrict__ mrow, int i0, int cnt) {
+    const int l = (int)lane_id(), q = l & 7;
+    MergeRow r{0, 0, 0, 0, 0, 0};
+    auto load_row = [&](int j) { return j < cnt ? mrow[i0 + j] : MergeRow{0, 0, 0, 0, 0, 0}; };
+    MergeRow nr = load_row(l >> 3);
+    for (int j = l >> 3; j - (l >> 3) < cnt; j += 4) {
+        r = nr;
+        nr = load_row(j + 4);
+        const bool ok = j < cnt;
+        const int32_t* O = pool + r.start;
+        int32_t* N = pool + r.dst;
+        const uint32_t ev = ok ? epos[r.b] : 0u;
+        const bool in = r.d > r.b, cut = (ev & 1u) != 0;   // an insertion, a matched deletion, or neither
+        const int32_t y = in ? key_v(keys[r.b], B) : 0;
+        const int at = (int)(ev >> 1);
+        for (int b0 = 0; __any_sync(0xffffffffu, b0 < r.len); b0 += 32) {
+            int32_t x[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) x[u] = b0 + 8 * u + q < r.len ? O[b0 + 8 * u + q] : 0;
+            __syncwarp();   // rows compacted where they lie: these loads precede the stores
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const int e = b0 + 8 * u + q;
+                if (e < r.len && !(cut && e == at)) N[e + (in && e >= at) - (cut && e > at)] = x[u];
+            }
+        }
+        if (in && q == 0) N[at] = y;
+    }
+}
+
 // The batch's rows, by every warp of the grid; `ev`: the warp's chunk events.
+struct MergeList {
+    const MergeRow* mrow;
+    const int64_t* slices;
+    int64_t slice_cap;
+    const int32_t* shorts;
+};
 static __device__ __forceinline__ void merge_rows(int32_t* __restrict__ pool, const unsigned long long* __restrict__ keys,
                                                   int B, DevCounters* __restrict__ ctr, const uint32_t* __restrict__ epos,
-                                                  const int32_t* __restrict__ E, const MergeRow* __restrict__ mrow,
-                                                  const int64_t* __restrict__ slices, int64_t slice_cap, ChunkEvents& ev) {
-    const int over = ld_volatile(&ctr->overflow), sl = ld_volatile(&ctr->n_slices), nsm = ld_volatile(&ctr->n_small);
+                                                  const int32_t* __restrict__ E, const MergeList& m, ChunkEvents& ev) {
+    const int over = ld_volatile(&ctr->overflow), sl = ld_volatile(&ctr->n_slices), none = ld_volatile(&ctr->n_one),
+              nsh = ld_volatile(&ctr->n_short);
     if (over) return;   // the slice list did not fit (the host reports it)
-    const int nsl = (int)min((int64_t)sl, slice_cap);
-    // rows of a warp's turn: up to 32, fewer while that leaves warps without any
-    const int per = min(WARP, max(MERGE_ROWS, (nsm + gwarp_count() - 1) / gwarp_count()));
-    const int items = nsl + (nsm + per - 1) / per;
+    const int nsl = (int)min((int64_t)sl, m.slice_cap);
+    // short rows of a warp's turn: up to 32, fewer while that leaves warps without any
+    const int W = gwarp_count();
+    const int per_s = min(WARP, max(MERGE_ROWS, (nsh + W - 1) / W)), per_o = min(WARP, max(MERGE_ROWS, (none + W - 1) / W));
+    const int it_s = nsl + (nsh + per_s - 1) / per_s, items = it_s + (none + per_o - 1) / per_o;
     int it = gwarp_id();   // the first item of every warp; the rest are handed out
     while (it < items) {
         int nx = 0;
-        if (lane_id() == 0) nx = gwarp_count() + atomicAdd(&ctr->merge_ticket, 1);
+        if (lane_id() == 0) nx = W + atomicAdd(&ctr->merge_ticket, 1);
         if (it < nsl) {
-            const int64_t item = slices[it];
-            const MergeRow r = mrow[item >> 32];
+            const int64_t item = m.slices[it];
+            const MergeRow r = m.mrow[item >> 32];
             const int s = (int)(item & 0xffffffffLL);
             const bool whole = r.dst == r.start;   // compacted where it lies: one warp, front to back
-            const int s0 = whole ? 0 : s * SLICE;
-            merge_slice(pool, keys, B, epos, E, r, s0, whole ? r.len : min(r.len, s0 + SLICE), ev);
+            if (r.e - r.b <= WARP && (whole || r.len <= SLICE)) {
+                merge_mid(pool, keys, B, epos, r);
+            } else {
+                const int s0 = whole ? 0 : s * SLICE;
+                merge_slice(pool, keys, B, epos, E, r, s0, whole ? r.len : min(r.len, s0 + SLICE), ev);
+            }
+        } else if (it < it_s) {
+            const int i0 = (it - nsl) * per_s;
+            merge_short(pool, keys, B, epos, m.mrow, m.shorts, i0, min(per_s, nsh - i0));
         } else {
-            const int i0 = (it - nsl) * per;
-            merge_short(pool, keys, B, epos, mrow, i0, min(per, nsm - i0));
+            const int i0 = (it - it_s) * per_o;
+            merge_one(pool, keys, B, epos, m.mrow, i0, min(per_o, none - i0));
         }
         it = __shfl_sync(0xffffffffu, nx, 0);
     }
@@ -846,10 +951,9 @@ static __device__ __forceinline__ void merge_rows(int32_t* __restrict__ pool, co
 
 __global__ void __launch_bounds__(MERGE_THREADS, 4) k_merge(
         int32_t* __restrict__ pool, const unsigned long long* __restrict__ keys, int B, DevCounters* __restrict__ ctr,
-        const uint32_t* __restrict__ epos, const int32_t* __restrict__ E, const MergeRow* __restrict__ mrow,
-        const int64_t* __restrict__ slices, int64_t slice_cap) {
+        const uint32_t* __restrict__ epos, const int32_t* __restrict__ E, MergeList m) {
     __shared__ ChunkEvents s_ev[MERGE_WARPS];
-    merge_rows(pool, keys, B, ctr, epos, E, mrow, slices, slice_cap, s_ev[threadIdx.x / WARP]);
+    merge_rows(pool, keys, B, ctr, epos, E, m, s_ev[threadIdx.x / WARP]);
 }
 
 // ---- up to UPDATE_MAX edits: the whole update in one launch ------------------------------------
@@ -1081,7 +1185,8 @@ __global__ void __launch_bounds__(UPDATE_THREADS, 1) k_update(UpdateParams p) {
     if (A > UPDATE_ROWS) row_plan<true>(p.rp, A, (int)blockIdx.x, G);
     else row_plan<false>(p.rp, A, gwarp_id(), gwarp_count());
     if (!grid_sync(p.bar, 64)) return;
-    merge_rows(p.pool, p.keys, B, ctr, p.epos, p.E, p.rp.mrow, p.rp.slices, p.rp.slice_cap, ((ChunkEvents*)s_mem)[w]);
+    merge_rows(p.pool, p.keys, B, ctr, p.epos, p.E, MergeList{p.rp.mrow, p.rp.slices, p.rp.slice_cap, p.rp.shorts},
+               ((ChunkEvents*)s_mem)[w]);
 }
 
 // Long rows that only lose entries, compacted in place: one block per row streams it front to
@@ -1103,7 +1208,7 @@ __global__ void __launch_bounds__(LIP_THREADS) k_merge_long_inplace(int32_t* __r
     __shared__ int s_next;
     const int t = threadIdx.x, w = t / WARP;
     const unsigned lt = (1u << lane_id()) - 1;
-    const int nl = ctr->n_large;
+    const int nl = ctr->n_long;
     for (int li = blockIdx.x; li < nl; li += gridDim.x) {
         const MergeRow r = mrow[longs[li]];
         int32_t* O = pool + r.start;
@@ -1379,7 +1484,7 @@ int ws_ensure(scout_ctx* c, int64_t m) {
     size_t sz[] = {
         (size_t)M * sizeof(scout_edge), (size_t)M, (size_t)M,
         (size_t)H * 8, (size_t)H * 8, (size_t)(H + 1) * 8,
-        (size_t)H * 4, (size_t)(H + 1) * 4, (size_t)H * 4, (size_t)H * 4, (size_t)H * sizeof(MergeRow)};
+        (size_t)H * 4, (size_t)(H + 1) * 4, (size_t)H * 4, (size_t)H * 4, (size_t)H * 4, (size_t)H * sizeof(MergeRow)};
     size_t total = 0;
     for (size_t s : sz) total += align256(s);
     if (c->ws) dev_free(c, c->ws, (size_t)c->ws_bytes);
@@ -1400,7 +1505,8 @@ int ws_ensure(scout_ctx* c, int64_t m) {
     c->d_seg_b = (int32_t*)take(sz[7]);
     c->d_seg_d = (int32_t*)take(sz[8]);
     c->d_longs = (int32_t*)take(sz[9]);
-    c->d_mrow = (MergeRow*)take(sz[10]);
+    c->d_shorts = (int32_t*)take(sz[10]);
+    c->d_mrow = (MergeRow*)take(sz[11]);
     c->d_hkeys = c->d_keys;
     return SCOUT_OK;
 }
@@ -1804,6 +1910,7 @@ int graph_update(scout_ctx* c, const scout_edge* edits, const uint8_t* ops, int6
     rp.slices = c->d_slices;
     rp.slice_cap = c->cap_slices;
     rp.longs = c->d_longs;
+    rp.shorts = c->d_shorts;
     rp.long_in_place = c->tiered;
     rp.hbm_cap = c->pool_cap;
     rp.split = c->tiered;   // rows whose old version lives in HBM are rewritten into HBM, host rows into the host pool
@@ -1912,7 +2019,8 @@ int graph_update(scout_ctx* c, const scout_edge* edits, const uint8_t* ops, int6
         k_row_plan<<<nbr, ROW_THREADS, 0, c->s_main>>>(rp);
         SCOUT_LAUNCH(c, "k_row_plan");
         k_merge<<<(unsigned)std::min<int64_t>(4 * c->sm_count, (Amax + c->nnz / SLICE) / MERGE_WARPS + 1), MERGE_THREADS, 0,
-                  c->s_main>>>(c->pool, sorted, B, c->d_ctr, epos, E, c->d_mrow, c->d_slices, c->cap_slices);
+                  c->s_main>>>(c->pool, sorted, B, c->d_ctr, epos, E,
+                               MergeList{c->d_mrow, c->d_slices, c->cap_slices, c->d_shorts});
         SCOUT_LAUNCH(c, "k_merge");
         c->nlaunch += 2;
     }
