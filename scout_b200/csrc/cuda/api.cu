@@ -345,7 +345,7 @@ static int apply_tuning(scout_ctx* c, const scout_sched& sd) {
 }
 
 static int batch_prologue(scout_ctx* c, int problem, const scout_edge* edits, const uint8_t* ops, int64_t m,
-                          scout_batch_stats* st) {
+                          scout_batch_stats* st, UpdateParams* later = nullptr) {
     if (!c->sealed) return c->fail(SCOUT_E_STATE, "graph not sealed");
     int32_t** slot = state_slot(c, problem);
     if (!slot) return c->fail(SCOUT_E_INVALID, "unknown problem");
@@ -360,7 +360,7 @@ static int batch_prologue(scout_ctx* c, int problem, const scout_edge* edits, co
     SCOUT_RC(lists_ensure(c));
     c->epoch++;
     SCOUT_CU(c, cudaEventRecord(c->ev_t[0], c->s_main));
-    SCOUT_RC(graph_update(c, edits, ops, m, st));
+    SCOUT_RC(graph_update(c, edits, ops, m, st, later));
     SCOUT_CU(c, cudaEventRecord(c->ev_t[1], c->s_main));
     return SCOUT_OK;
 }
@@ -402,9 +402,9 @@ __global__ void k_count_diff(const int32_t* __restrict__ a, const int32_t* __res
     if ((threadIdx.x & 31) == 0 && d) atomicAdd(cnt, d);
 }
 
-// One round of several union stores of distinct problems (ne <= 4, one device): every batch is
-// merged on its store's stream, then ONE cooperative launch runs all the repairs (union.cu),
-// then each store's counters are read into its stats (ms_repair: the shared launch). The
+// One round of several union stores of distinct problems (ne <= 4, one device): the batches are
+// merged (in one launch where the repairs run side by side, else each on its store's stream), then
+// ONE cooperative launch runs all the repairs (union.cu), then each store's counters are read into its stats (ms_repair: the shared launch). The
 // repairs run their plain variants; the learned scheduler decides per launch and is not used.
 int union_run(scout_ctx* const* cs, const int* problems, const scout_edge* const* edits, const uint8_t* const* ops,
               const int64_t* counts, int ne, const scout_sched* sched, scout_batch_stats* stats) {
@@ -421,16 +421,22 @@ int union_run(scout_ctx* const* cs, const int* problems, const scout_edge* const
     scout_sched sds[4];
     int variants[4];
     int64_t launch0[4];
+    UpdateRound round;
+    int later = 0;
+    const bool side = union_side(cs, counts, ne);
     for (int i = 0; i < ne; i++) {
         std::memset(&sds[i], 0, sizeof(scout_sched));
         if (sched) sds[i] = *sched;
         sds[i].policy = SCOUT_SCHED_PLAIN;
         SCOUT_RC(apply_tuning(cs[i], sds[i]));
         launch0[i] = cs[i]->nlaunch;
-        SCOUT_RC(batch_prologue(cs[i], problems[i], edits[i], ops ? ops[i] : nullptr, counts[i], &stats[i]));
+        round.p[later].m = 0;
+        SCOUT_RC(batch_prologue(cs[i], problems[i], edits[i], ops ? ops[i] : nullptr, counts[i], &stats[i],
+                                side ? &round.p[later] : nullptr));
+        later += round.p[later].m > 0;
         variants[i] = plain_variant(problems[i], sds[i]);
     }
-    SCOUT_RC(union_launch(cs, problems, sds, variants, ne));
+    SCOUT_RC(union_launch(cs, problems, sds, variants, ne, round, later, side));
     for (int i = 0; i < ne; i++) {
         scout_ctx* c = cs[i];
         SCOUT_CU(c, cudaEventRecord(c->ev_t[2], c->s_main));

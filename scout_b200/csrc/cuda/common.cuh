@@ -177,7 +177,7 @@ __device__ __forceinline__ bool grid_sync(GridBar* b, int tag = 0) {
     __shared__ int s_ok;
     __syncthreads();
     if (threadIdx.x == 0) {
-        const unsigned nb = gridDim.x * gridDim.y * gridDim.z;
+        const unsigned nb = gridDim.x;   // (rows of a two-dimensional grid have barriers of their own)
         const unsigned old = atom_add_release_gpu(&b->count, 1u);
         const unsigned target = (old / nb + 1) * nb;
         uint64_t t0 = 0;

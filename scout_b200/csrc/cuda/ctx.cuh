@@ -291,7 +291,54 @@ int graph_reserve_batch(scout_ctx* c, int64_t m);
 int cc_ensure(scout_ctx* c);
 int coloring_ensure(scout_ctx* c);
 // graph.cu
-int graph_update(scout_ctx* c, const scout_edge* edits, const uint8_t* ops, int64_t m, scout_batch_stats* st);
+// A merge's row plan (k_row_plan) and a store's update in one launch (k_update)
+struct RowPlan {
+    Row* row;
+    DevCounters* ctr;
+    const int32_t* aff;
+    const int32_t* seg_b;
+    const int32_t* seg_d;
+    const int32_t* E;
+    MergeRow* mrow;        // short rows of one half-edit from the front, the others from the back
+    int64_t mcap;
+    int32_t* shorts;       // records of the other short rows
+    int64_t* slices;       // (record << 32 | slice)
+    int64_t slice_cap;
+    int32_t* longs;        // records of long rows compacted in place
+    bool long_in_place;
+    bool split;            // rows whose old version is not in HBM go to the second destination
+    long long hbm_cap;     // in HBM: 0 <= start < hbm_cap
+    long long base_hbm, base_host;
+};
+
+struct UpdateParams {
+    DGraph g;
+    int32_t* pool;
+    const scout_edge* e;
+    const uint8_t* ops;
+    int m, B;
+    unsigned long long* raw;    // half-edits as classified (2m)
+    unsigned long long* tmp;    // half-edits by bucket (may share E's memory, written later)
+    unsigned long long* keys;   // sorted
+    uint8_t* eflag;
+    uint32_t* epos;             // may share `raw`'s memory: written after the sort
+    unsigned long long* split;  // UPDATE_SPLIT
+    int* bucket;                // UPDATE_SPLIT + 1 counts
+    unsigned long long* cnt;    // heads << 32 | matches per block
+    int rows;                   // 0: stop after the plan (tiered store: the host decides where rows go)
+    RowPlan rp;                 // its aff, seg_b, seg_d and E are written here
+    int32_t *aff, *seg_b, *seg_d, *E;
+    GridBar* bar;
+};
+
+constexpr int SIDE_MAX = 4;
+struct UpdateRound { UpdateParams p[SIDE_MAX]; };
+// With `later`, an update of one launch is left to the caller: its parameters in *later, whose m is
+// unchanged if the update has been launched (or the batch is empty).
+int graph_update(scout_ctx* c, const scout_edge* edits, const uint8_t* ops, int64_t m, scout_batch_stats* st,
+                 UpdateParams* later = nullptr);
+// k stores' updates in one launch on c's stream, side by side: each on 1/k of the SMs
+int update_side(scout_ctx* c, const UpdateRound& r, int k);
 int graph_ensure_scratch(scout_ctx* c);
 int graph_compact(scout_ctx* c, int64_t min_free, bool nnz_exact = false);
 int ws_ensure(scout_ctx* c, int64_t m);
@@ -338,7 +385,9 @@ int bar_clear(scout_ctx* c, cudaStream_t s);
 int prefetch_launch(scout_ctx* c, long long base);
 // union.cu: one cooperative launch of the repairs of ne union stores of distinct problems whose
 // batches are merged (queued); api.cu: the whole round (merges, launch, counters, stats)
-int union_launch(scout_ctx* const* cs, const int* problems, const scout_sched* sds, const int* variants, int ne);
+int union_launch(scout_ctx* const* cs, const int* problems, const scout_sched* sds, const int* variants, int ne,
+                 const UpdateRound& round, int later, bool side);
+bool union_side(scout_ctx* const* cs, const int64_t* counts, int ne);
 int union_run(scout_ctx* const* cs, const int* problems, const scout_edge* const* edits, const uint8_t* const* ops,
               const int64_t* counts, int ne, const scout_sched* sched, scout_batch_stats* stats);
 // graph.cu: host copy into page-locked staging, over the host threads for large copies

@@ -410,25 +410,6 @@ __global__ void __launch_bounds__(PLAN_THREADS) k_plan(const Row* __restrict__ r
 // does not matter).
 constexpr int ROW_THREADS = 256;
 
-struct RowPlan {
-    Row* row;
-    DevCounters* ctr;
-    const int32_t* aff;
-    const int32_t* seg_b;
-    const int32_t* seg_d;
-    const int32_t* E;
-    MergeRow* mrow;        // short rows of one half-edit from the front, the others from the back
-    int64_t mcap;
-    int32_t* shorts;       // records of the other short rows
-    int64_t* slices;       // (record << 32 | slice)
-    int64_t slice_cap;
-    int32_t* longs;        // records of long rows compacted in place
-    bool long_in_place;
-    bool split;            // rows whose old version is not in HBM go to the second destination
-    long long hbm_cap;     // in HBM: 0 <= start < hbm_cap
-    long long base_hbm, base_host;
-};
-
 // Exclusive scans of two values over the block (at most 32 warps) at once, and their totals.
 __device__ __forceinline__ void block_scan2(long long& x, long long& y, long long* tx, long long* ty) {
     __shared__ long long ws[2][WARP + 1];
@@ -983,26 +964,6 @@ constexpr int UPDATE_ROWS = 16384;   // more affected rows are planned by blocks
 // device scratch: splitters, bucket counts, the blocks' plan counts
 constexpr int64_t UPDATE_SCRATCH = UPDATE_SPLIT * 8 + (UPDATE_SPLIT + 64) * 4 + 1024 * 8;
 
-struct UpdateParams {
-    DGraph g;
-    int32_t* pool;
-    const scout_edge* e;
-    const uint8_t* ops;
-    int m, B;
-    unsigned long long* raw;    // half-edits as classified (2m)
-    unsigned long long* tmp;    // half-edits by bucket (may share E's memory, written later)
-    unsigned long long* keys;   // sorted
-    uint8_t* eflag;
-    uint32_t* epos;             // may share `raw`'s memory: written after the sort
-    unsigned long long* split;  // UPDATE_SPLIT
-    int* bucket;                // UPDATE_SPLIT + 1 counts
-    unsigned long long* cnt;    // heads << 32 | matches per block
-    int rows;                   // 0: stop after the plan (tiered store: the host decides where rows go)
-    RowPlan rp;                 // its aff, seg_b, seg_d and E are written here
-    int32_t *aff, *seg_b, *seg_d, *E;
-    GridBar* bar;
-};
-
 // First index of the ascending a[0, n) whose value is above x (n <= 2^13).
 template <typename T>
 __device__ __forceinline__ int first_above(const T* a, int n, T x) {
@@ -1017,7 +978,7 @@ __device__ __forceinline__ int first_above(const T* a, int n, T x) {
 // The half-edits p.raw[0, n) in ascending order into p.keys, all blocks; `smem`: 32 KB. Returns
 // false when a barrier failed. Ends before a barrier: the caller's next one publishes the order.
 static __device__ bool update_sort(const UpdateParams& p, int n, unsigned long long SENT, unsigned char* smem) {
-    const int t = threadIdx.x, w = t / WARP, l = (int)lane_id();
+    const int t = threadIdx.x, l = (int)lane_id();
     const int G = (int)gridDim.x, wid = gwarp_id(), W = gwarp_count();
     const int tid = (int)blockIdx.x * UPDATE_THREADS + t, T = G * UPDATE_THREADS;
     unsigned long long* k = (unsigned long long*)smem;
@@ -1102,7 +1063,7 @@ static __device__ bool update_sort(const UpdateParams& p, int n, unsigned long l
     return true;
 }
 
-__global__ void __launch_bounds__(UPDATE_THREADS, 1) k_update(UpdateParams p) {
+static __device__ __forceinline__ void update_body(const UpdateParams& p) {
     __shared__ __align__(16) unsigned char s_mem[UPDATE_PAIRS * 8];   // the sort's, later the warps' chunk events
     static_assert(sizeof(s_mem) >= UPDATE_WARPS * sizeof(ChunkEvents) && sizeof(s_mem) >= UPDATE_SPLIT * 8, "fits");
     const int t = threadIdx.x, w = t / WARP, l = (int)lane_id();
@@ -1187,6 +1148,22 @@ __global__ void __launch_bounds__(UPDATE_THREADS, 1) k_update(UpdateParams p) {
     if (!grid_sync(p.bar, 64)) return;
     merge_rows(p.pool, p.keys, B, ctr, p.epos, p.E, MergeList{p.rp.mrow, p.rp.slices, p.rp.slice_cap, p.rp.shorts},
                ((ChunkEvents*)s_mem)[w]);
+}
+
+__global__ void __launch_bounds__(UPDATE_THREADS, 1) k_update(UpdateParams p) { update_body(p); }
+
+// Several stores' updates side by side: grid row y runs the y-th (at most 2 keys per thread of its
+// blocks: the callers' limit is far below).
+__global__ void __launch_bounds__(UPDATE_THREADS, 1) k_update_side(const __grid_constant__ UpdateRound r) {
+    update_body(r.p[blockIdx.y]);
+}
+
+int update_side(scout_ctx* c, const UpdateRound& r, int k) {
+    void* args[] = {(void*)&r};
+    SCOUT_CU(c, cudaLaunchCooperativeKernel((const void*)k_update_side, dim3((unsigned)(c->sm_count / k), (unsigned)k),
+                                            dim3(UPDATE_THREADS), args, 0, c->s_main));
+    c->nlaunch += 1;
+    return SCOUT_OK;
 }
 
 // Long rows that only lose entries, compacted in place: one block per row streams it front to
@@ -1870,7 +1847,8 @@ static int upload_edits(scout_ctx* c, const scout_edge* edits, const uint8_t* op
     return SCOUT_OK;
 }
 
-int graph_update(scout_ctx* c, const scout_edge* edits, const uint8_t* ops, int64_t m, scout_batch_stats* st) {
+int graph_update(scout_ctx* c, const scout_edge* edits, const uint8_t* ops, int64_t m, scout_batch_stats* st,
+                 UpdateParams* later) {
     const int64_t n = c->n;
     const int B = key_bits_for(n);
     c->key_bits = B;
@@ -1919,7 +1897,8 @@ int graph_update(scout_ctx* c, const scout_edge* edits, const uint8_t* ops, int6
     c->batch_dest = c->tiered ? 2 : 0;
     unsigned long long* sorted = c->d_keys;
     uint32_t* epos = (uint32_t*)c->d_keys_alt;
-    const bool one = m <= UPDATE_MAX && H <= 2 * (int64_t)c->sm_count * UPDATE_THREADS;
+    const int64_t sms = later ? c->sm_count / SIDE_MAX : c->sm_count;
+    const bool one = m <= UPDATE_MAX && H <= 2 * sms * UPDATE_THREADS;
     if (one) {
         SCOUT_RC(update_ensure(c));
         UpdateParams up;
@@ -1944,8 +1923,12 @@ int graph_update(scout_ctx* c, const scout_edge* edits, const uint8_t* ops, int6
         up.seg_d = c->d_seg_d;
         up.E = E;
         up.bar = &c->d_batch->bar[0];
-        void* args[] = {&up};
-        SCOUT_RC(coop_launch_own(c, (const void*)k_update, UPDATE_THREADS, args, 0));
+        if (later && !c->tiered) {   // the caller launches it (update_side)
+            *later = up;
+        } else {
+            void* args[] = {&up};
+            SCOUT_RC(coop_launch_own(c, (const void*)k_update, UPDATE_THREADS, args, 0));
+        }
     } else {
         k_classify<<<blocks_for(m, 256), 256, 0, c->s_main>>>(g, d_src, ops ? c->d_ops : nullptr, m, B, c->d_keys,
                                                              c->d_eflag, c->d_ctr, 1);
