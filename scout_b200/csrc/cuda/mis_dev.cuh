@@ -24,6 +24,8 @@ struct MisParams {
     GridBar* bar;
 };
 
+constexpr int MIS_ITEMS = 4;   // candidates a warp decides at a time, half-edits a thread reads at a time
+
 __device__ __forceinline__ void mis_touch(const MisParams& p, bool pred, int32_t v) {
     bool nt = false;
     if (pred) nt = atomicExch(&p.st_touch[v], p.epoch) != p.epoch;
@@ -50,23 +52,32 @@ __device__ __forceinline__ void mis_body(const MisParams& p) {
 
     if (update_failed(p.bar)) return;
     // ---- 1: conflicts of inserted edges, evaluated on the pre-batch set ----------------
-    for (int64_t b = tid - (tid & (WARP - 1)); b < nh; b += T) {
-        int64_t k = b + lane_id();
-        bool drop = false;
-        int32_t r = 0;
-        if (k < nh) {
-            unsigned long long key = p.hkeys[k];
-            int op = (int)((key >> p.B) & 1ull);
-            int32_t x = (int32_t)(key >> (p.B + 1));
-            int32_t y = (int32_t)(key & ((1ull << p.B) - 1));
-            if (op == 0 && x < y && ld_volatile(p.mis + x) && ld_volatile(p.mis + y)) {
-                r = y;
-                drop = atomicExch(&p.st_done[y], p.epoch) != p.epoch;
+    for (int64_t b = tid - (tid & (WARP - 1)); b < nh; b += MIS_ITEMS * T) {
+        int32_t x[MIS_ITEMS], y[MIS_ITEMS];
+        bool mx[MIS_ITEMS], my[MIS_ITEMS];
+#pragma unroll
+        for (int u = 0; u < MIS_ITEMS; u++) {
+            const int64_t k = b + u * T + lane_id();
+            const unsigned long long key = k < nh ? p.hkeys[k] : ~0ull;
+            x[u] = (int32_t)(key >> (p.B + 1));
+            y[u] = (int32_t)(key & ((1ull << p.B) - 1));
+            if (k >= nh || ((key >> p.B) & 1ull) || x[u] >= y[u]) x[u] = -1;   // insertions, once each
+        }
+#pragma unroll
+        for (int u = 0; u < MIS_ITEMS; u++) {
+            mx[u] = x[u] >= 0 && ld_volatile(p.mis + x[u]) != 0;
+            my[u] = x[u] >= 0 && ld_volatile(p.mis + y[u]) != 0;
+        }
+#pragma unroll
+        for (int u = 0; u < MIS_ITEMS; u++) {
+            bool drop = false;
+            if (mx[u] && my[u]) {
+                drop = atomicExch(&p.st_done[y[u]], p.epoch) != p.epoch;
                 atomicAdd(&p.ctr->conflicts, 1);
             }
+            const int at = warp_append(drop, &p.ctr->list_count[2]);
+            if (drop) p.removed[at] = y[u];
         }
-        int at = warp_append(drop, &p.ctr->list_count[2]);
-        if (drop) p.removed[at] = r;
     }
     if (!grid_sync(p.bar, 20)) return;
     // ---- 2: drop them; candidates = dropped vertices, their neighbours, deletion endpoints ---
@@ -90,16 +101,24 @@ __device__ __forceinline__ void mis_body(const MisParams& p) {
         }
         if (lane_id() == 0) bytes += 4LL * rr.len + 16;
     }
-    for (int64_t b = tid - (tid & (WARP - 1)); b < nh; b += T) {
-        int64_t k = b + lane_id();
-        bool del = false;
-        int32_t x = 0;
-        if (k < nh) {
-            unsigned long long key = p.hkeys[k];
-            del = ((key >> p.B) & 1ull) == 1ull;
-            x = (int32_t)(key >> (p.B + 1));
+    for (int64_t b = tid - (tid & (WARP - 1)); b < nh; b += MIS_ITEMS * T) {
+        int32_t x[MIS_ITEMS];
+        bool first[MIS_ITEMS];
+#pragma unroll
+        for (int u = 0; u < MIS_ITEMS; u++) {
+            const int64_t k = b + u * T + lane_id();
+            const unsigned long long key = k < nh ? p.hkeys[k] >> p.B : 0ull;
+            // (sorted: a vertex's deletions are consecutive, the first one speaks for them)
+            const bool del = (key & 1ull) && (k == 0 || (p.hkeys[k - 1] >> p.B) != key);
+            x[u] = del ? (int32_t)(key >> 1) : -1;
         }
-        mis_candidate(p, del, x);
+#pragma unroll
+        for (int u = 0; u < MIS_ITEMS; u++) first[u] = x[u] >= 0 && atomicExch(&p.st_cand[x[u]], p.epoch) != p.epoch;
+#pragma unroll
+        for (int u = 0; u < MIS_ITEMS; u++) {
+            const int at = warp_append(first[u], &p.ctr->list_count[0]);
+            if (first[u]) p.list[0][at] = x[u];
+        }
     }
     if (!grid_sync(p.bar, 22)) return;
     if (leader) p.ctr->affected = ld_volatile(&p.ctr->list_count[0]);
@@ -116,45 +135,72 @@ __device__ __forceinline__ void mis_body(const MisParams& p) {
         // neighbour read once is either undecided or decided with its final membership (a
         // separate flag read after the set entry could pair a new flag with a stale entry).
         const int32_t DONE_IN = p.epoch + 0x40000000, DONE_OUT = p.epoch + 0x20000000;
-        for (int i = wid; i < cnt; i += W) {
-            int32_t c = p.list[cur][i];
-            Row r = p.g.row[c];
-            const int32_t* rw = p.g.pool + r.start;
-            const bool was_in = ld_volatile(p.mis + c) != 0;
-            bool member_nb = false, lower_undecided = false;
-            if (!was_in) {
-                for (int b0 = 0; b0 < r.len && !member_nb; b0 += WARP) {
-                    int k = b0 + (int)lane_id();
-                    bool m = false, l = false;
-                    if (k < r.len) {
-                        int32_t w = rw[k];
-                        const int32_t sd = ld_volatile(p.st_done + w);
-                        if (sd == DONE_IN) {
-                            m = true;
-                        } else if (sd != DONE_OUT) {
-                            m = ld_volatile(p.mis + w) != 0;
-                            l = w < c && ld_volatile(p.st_cand + w) == p.epoch;
+        // A set entry is one read per neighbour and settles most candidates: an entry of 1 is final
+        // here. Only if a row shows none are the decision words and candidate marks read. A warp
+        // reads the last 32 entries of up to MIS_ITEMS candidates side by side, longer rows then one
+        // by one towards the front. What bounds it: chains of dependent reads, 22 candidates per warp
+        // one after the other (three reads per neighbour) when 300,007 edits on 10^6 vertices leave
+        // 104,000 of them: that repair took 165 us, so 95 (108 with eight at a time).
+        const int per = min(MIS_ITEMS, max(1, (cnt + W - 1) / W));
+        for (int i0 = wid * per; i0 < cnt; i0 += W * per) {
+            int32_t cv[MIS_ITEMS], w[MIS_ITEMS];
+            Row r[MIS_ITEMS];
+            bool in[MIS_ITEMS], m[MIS_ITEMS];
+#pragma unroll
+            for (int u = 0; u < MIS_ITEMS; u++) cv[u] = u < per && i0 + u < cnt ? p.list[cur][i0 + u] : -1;
+#pragma unroll
+            for (int u = 0; u < MIS_ITEMS; u++) {
+                r[u] = cv[u] >= 0 ? p.g.row[cv[u]] : Row{0, 0, 0};
+                in[u] = cv[u] >= 0 && ld_volatile(p.mis + cv[u]) != 0;
+            }
+#pragma unroll
+            for (int u = 0; u < MIS_ITEMS; u++) {
+                const int k = r[u].len - 1 - (int)lane_id();
+                w[u] = !in[u] && k >= 0 ? p.g.pool[r[u].start + k] : -1;
+            }
+#pragma unroll
+            for (int u = 0; u < MIS_ITEMS; u++) m[u] = w[u] >= 0 && ld_volatile(p.mis + w[u]) != 0;
+#pragma unroll
+            for (int u = 0; u < MIS_ITEMS; u++) {
+                if (cv[u] < 0) continue;   // uniform per warp
+                const int32_t c = cv[u];
+                const bool was_in = in[u];
+                bool member_nb = __any_sync(0xffffffffu, m[u]), lower_undecided = false;
+                if (w[u] >= 0) bytes += 8;
+                if (!was_in && !member_nb) {
+                    int32_t x = w[u];
+                    for (int k = r[u].len - 1 - (int)lane_id();;) {
+                        bool mm = false, l = false;
+                        if (x >= 0) {
+                            const int32_t sd = ld_volatile(p.st_done + x);
+                            mm = sd == DONE_IN;
+                            l = !mm && sd != DONE_OUT && x < c && ld_volatile(p.st_cand + x) == p.epoch;
                         }
+                        member_nb = __any_sync(0xffffffffu, mm);
+                        lower_undecided = lower_undecided || __any_sync(0xffffffffu, l);
+                        k -= WARP;
+                        if (member_nb || k + (int)lane_id() < 0) break;
+                        x = k >= 0 ? p.g.pool[r[u].start + k] : -1;
+                        member_nb = __any_sync(0xffffffffu, x >= 0 && ld_volatile(p.mis + x) != 0);
+                        if (x >= 0) bytes += 8;
+                        if (member_nb) break;
                     }
-                    member_nb = __any_sync(0xffffffffu, m);
-                    lower_undecided = lower_undecided || __any_sync(0xffffffffu, l);
-                    if (k < r.len) bytes += 8;
                 }
-            }
-            const bool joined = !was_in && !member_nb && !lower_undecided;
-            if (lane_id() == 0) {
-                if (was_in) {
-                    p.st_done[c] = DONE_IN;    // kept
-                } else if (member_nb) {
-                    p.st_done[c] = DONE_OUT;
-                } else if (joined) {
-                    p.mis[c] = 1;
-                    p.st_done[c] = DONE_IN;
-                } else {
-                    p.list[nxt][atomicAdd(&p.ctr->list_count[nxt], 1)] = c;   // wait
+                const bool joined = !was_in && !member_nb && !lower_undecided;
+                if (lane_id() == 0) {
+                    if (was_in) {
+                        p.st_done[c] = DONE_IN;    // kept
+                    } else if (member_nb) {
+                        p.st_done[c] = DONE_OUT;
+                    } else if (joined) {
+                        p.mis[c] = 1;
+                        p.st_done[c] = DONE_IN;
+                    } else {
+                        p.list[nxt][atomicAdd(&p.ctr->list_count[nxt], 1)] = c;   // wait
+                    }
                 }
+                mis_touch(p, lane_id() == 0 && joined, c);
             }
-            mis_touch(p, lane_id() == 0 && joined, c);
         }
         rounds++;
         if (!grid_sync(p.bar, 24)) return;

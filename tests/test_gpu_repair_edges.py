@@ -2,14 +2,17 @@
 the parent in the first, a middle or the last one, or in none; changed entries around the number
 that comes back with the counters; component recomputes whose joining edge is the last entry
 of a row around the block-wide length; classes split with and without their minimum. Levels and
-labels equal the oracle's after every batch."""
+labels equal the oracle's after every batch. MIS candidates whose only member neighbour is the first
+entry of a row around one to many 32-entry groups, next to neighbours decided in the same round,
+and batches with several candidates per warp."""
 import numpy as np
 import pytest
 
 import scout_b200 as sb
 from oracle import oracle as orc
 from test_gpu_bfs import _run
-from test_gpu_problems import _cc
+from gpu_util import stream
+from test_gpu_problems import _cc, _mis
 
 pytestmark = pytest.mark.gpu
 
@@ -96,3 +99,26 @@ def test_cc_splits_of_many_classes(mode):
     cuts = [e[rng.choice(len(e), size=s, replace=False)] for s in (1, 50, 400, 3000)]
     batches = [b.astype(np.int32) for c in cuts for b in (c, c)]   # cut, then joined again
     _cc(off, adj, batches, sched={"mode": mode}, check_ref=False)
+
+
+def test_mis_candidates_of_long_rows():
+    lens = (1, 2, 30, 31, 32, 33, 62, 63, 64, 65, 95, 96, 97, 1000, 3000)
+    k, m = len(lens), 4000                  # ids: 0 | own members | m neighbours (held out by 0) | the hubs
+    rng = np.random.default_rng(7)
+    own, e, hub = 1 + np.arange(k), 1 + k + np.arange(m), 1 + k + m + np.arange(k)
+    ed = [(0, int(v)) for v in e]
+    for i, d in enumerate(lens):
+        ed += [(int(own[i]), int(hub[i]))] + [(int(hub[i]), int(v)) for v in rng.choice(e, size=d, replace=False)]
+    off, adj = _csr(1 + 2 * k + m, ed)
+    first = np.array([[h, adj[off[h] + 1]] for h in hub])     # a neighbour held out: candidates stay out
+    last = np.array([[h, adj[off[h + 1] - 1]] for h in hub[1:]])
+    mine = np.stack([hub, own], axis=1)
+    free = np.stack([np.zeros(200, int), e[-200:]], axis=1)   # neighbours of lower id, undecided as well
+    batches = [first, mine, mine, np.concatenate([last, free]), np.concatenate([mine, last]), free,
+               np.concatenate([mine, free])]
+    _mis(off, adj, [b.astype(np.int32) for b in batches])
+
+
+def test_mis_many_candidates_per_warp():
+    off, adj = sb.gen_rmat(16, 8, seed=12).arrays()
+    _mis(off, adj, stream(off, adj, sb.STREAM_LOWDEG, 80000, 1, seed=5, insert_ratio=0.2, lowdeg_frac=0.5))
