@@ -4,7 +4,8 @@ that comes back with the counters; component recomputes whose joining edge is th
 of a row around the block-wide length; classes split with and without their minimum. Levels and
 labels equal the oracle's after every batch. MIS candidates whose only member neighbour is the first
 entry of a row around one to many 32-entry groups, next to neighbours decided in the same round,
-and batches with several candidates per warp."""
+and batches with several candidates per warp. Colouring rounds of few and of many vertices with rows
+around the lengths that go to a whole block."""
 import numpy as np
 import pytest
 
@@ -12,7 +13,7 @@ import scout_b200 as sb
 from oracle import oracle as orc
 from test_gpu_bfs import _run
 from gpu_util import stream
-from test_gpu_problems import _cc, _mis
+from test_gpu_problems import _cc, _coloring, _mis
 
 pytestmark = pytest.mark.gpu
 
@@ -122,3 +123,16 @@ def test_mis_candidates_of_long_rows():
 def test_mis_many_candidates_per_warp():
     off, adj = sb.gen_rmat(16, 8, seed=12).arrays()
     _mis(off, adj, stream(off, adj, sb.STREAM_LOWDEG, 80000, 1, seed=5, insert_ratio=0.2, lowdeg_frac=0.5))
+
+
+@pytest.mark.parametrize("lens", [(0, 1, 31, 32, 33, 127, 128, 129, 1023, 1025, 4095, 4096, 4097, 5000), (126, 127, 128, 4096) * 75])
+def test_coloring_rounds_of_long_rows(lens):
+    k, m = len(lens), 6000                  # ids: m spokes | k hubs | k hubs with the same neighbours
+    rng = np.random.default_rng(13)
+    spokes = [rng.choice(m, size=d, replace=False) for d in lens]
+    ed = [(i, i + 1) for i in range(0, m - 1, 3)]
+    for i in range(k):
+        ed += [(int(v), m + i) for v in spokes[i]] + [(int(v), m + k + i) for v in spokes[i]]
+    off, adj = _csr(m + 2 * k, ed)
+    twins = np.stack([m + np.arange(k), m + k + np.arange(k)], axis=1).astype(np.int32)   # of one colour
+    _coloring(off, adj, orc.gt_greedy_color(off, adj), [twins, twins, twins[::2]])
