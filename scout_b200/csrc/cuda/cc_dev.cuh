@@ -492,10 +492,12 @@ __device__ __forceinline__ void cc_body(const CcParams& p) {
         // What bounds it: chains of random reads, so a thread's CC_ITEMS vertices read side by
         // side, and after a compress most neighbours prove joined by one comparison. Recompute of
         // 2 M vertices (32 M edges): 295 us with both neighbours linked by unions and
-        // volatile reads, 110 us so.
+        // volatile reads, 100 us so. The first two entries are read once, by the start, and kept for
+        // the link (cold rows of the tiered store lie across the host link: 100,000-edit batches at
+        // scale 21, repair of 6.2 ms with a second read, 4.6 so).
         constexpr int AF_FIRST = 2;
         for (int64_t b = ltid; b < n; b += CC_ITEMS * T) {
-            int32_t lab[CC_ITEMS], w[CC_ITEMS];
+            int32_t lab[CC_ITEMS], w[CC_ITEMS], w1[CC_ITEMS];
             Row r[CC_ITEMS];
             bool d[CC_ITEMS];
 #pragma unroll
@@ -508,6 +510,7 @@ __device__ __forceinline__ void cc_body(const CcParams& p) {
             for (int u = 0; u < CC_ITEMS; u++) {
                 d[u] = b + u * T < n && (full || p.dirty[lab[u]] == p.epoch);
                 w[u] = d[u] && r[u].len > 0 ? p.g.pool[r[u].start] : -1;
+                w1[u] = d[u] && r[u].len > 1 ? p.g.pool[r[u].start + 1] : -1;
             }
 #pragma unroll
             for (int u = 0; u < CC_ITEMS; u++) {
@@ -520,6 +523,8 @@ __device__ __forceinline__ void cc_body(const CcParams& p) {
                     if (!in) atomicExch(&p.ctr->pad, 1);
                 }
                 p.vp[v] = !d[u] ? -1 : w[u] >= 0 && w[u] < v && in ? w[u] : (int32_t)v;
+                p.merged[v] = w[u] < v ? -1 : w[u];   // left to link
+                p.side[v] = w1[u];
             }
         }
         if (!grid_sync(p.bar, 36)) return;
@@ -554,10 +559,8 @@ __device__ __forceinline__ void cc_body(const CcParams& p) {
             for (int u = 0; u < CC_ITEMS; u++) {
                 const int64_t v = b + u * T;
                 pv[u] = v < n ? p.vp[v] : -1;   // (an ancestor is enough)
-                const Row r = pv[u] >= 0 ? p.g.row[v] : Row{0, 0, 0};
-                w0[u] = r.len > 0 ? p.g.pool[r.start] : -1;
-                w1[u] = r.len > 1 ? p.g.pool[r.start + 1] : -1;
-                if (w0[u] < v) w0[u] = -1;   // joined by the start (or flagged there)
+                w0[u] = pv[u] >= 0 ? p.merged[v] : -1;   // not if joined by the start (or flagged there)
+                w1[u] = pv[u] >= 0 ? p.side[v] : -1;
             }
 #pragma unroll
             for (int u = 0; u < CC_ITEMS; u++) {
