@@ -474,7 +474,7 @@ def scout_arm(a, dist):
                      "frac": achieved / peak, "peak_kind": peak_kind, "traffic": profiled_traffic(f"k_{kp}", a.scale),
                      "algorithmic_bytes_per_launch": b / max(nl, 1), "ms_per_launch": ms / max(nl, 1),
                      "launches": nl},
-        "roofline_merge": {"kernels": "k_classify .. k_merge_slices (batch merge pipeline)",
+        "roofline_merge": {"kernels": "k_update, or k_classify .. k_merge (batch merge)",
                            "achieved": bytes_upd / (ms_upd / 1e3) / 1e9 if ms_upd else 0.0,
                            "frac": (bytes_upd / (ms_upd / 1e3) / 1e9) / peak if ms_upd else 0.0,
                            "ms": ms_upd, "bytes": bytes_upd},
