@@ -370,9 +370,12 @@ int commit_gather(scout_ctx* c, int problem, const int32_t** pairs, int64_t* cou
 // repair, whose hash sets take half an SM's shared memory, runs 1,024 threads per SM instead of
 // one 256-thread block (recompute of 2 M vertices: 544 -> 339 us; 50,000-edit batch at scale 20:
 // 1,187 -> 1,016 us with its merge). The blocks_per_sm knob takes fewer 256-thread quarters.
+// Four quarters hold all of an SM's registers; while the tiered store gathers the next batch's rows
+// a repair takes three, so that the gather's blocks run beside it and not after it.
 constexpr int REPAIR_THREADS = 1024;
 inline int repair_threads(const scout_ctx* c) {
-    return c->tune_blocks_per_sm > 0 ? 256 * c->tune_blocks_per_sm : REPAIR_THREADS;
+    if (c->tune_blocks_per_sm > 0) return 256 * c->tune_blocks_per_sm;
+    return c->tiered && c->gather_active ? REPAIR_THREADS - 256 : REPAIR_THREADS;
 }
 // persistent launch helpers: a launch that waits on d_bar (cleared when it was used before), one
 // on a barrier of its own
