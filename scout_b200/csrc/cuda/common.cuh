@@ -8,6 +8,7 @@
 //   Counters   small device block of per-batch counters (copied back once per batch).
 #pragma once
 
+#include <cstddef>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -146,26 +147,35 @@ __device__ __forceinline__ bool dg_adjacent_wide(const DGraph& g, int32_t u, int
 // so the last block's own arrival releases the others (no reset and no second counter to bump).
 // Every block passes the same sequence of barriers, so a block arriving at barrier k sees
 // old in [(k - 1) * blocks, k * blocks). The host zeroes the block before each launch.
+// `count` and `err` are the halves of ONE 64-bit word, and a launch touches it by 64-bit
+// operations only: an arrival and the poll that sees it order memory between blocks because
+// both are strong operations on the same eight bytes (a 32-bit arrival under a 64-bit poll would
+// overlap it in part and order nothing).
 // ---------------------------------------------------------------------------------------
 struct __align__(16) GridBar {
-    unsigned int count;
-    int err;            // 0 ok, 1 barrier timeout, 2 capacity overflow inside a kernel; beside
-                        // `count`, so that a waiting block reads both in one 8-byte load
+    unsigned int count; // low half of the barrier's word
+    int err;            // its high half: 0 ok, bit 0 barrier timeout, bit 1 capacity overflow inside a kernel
     int where;          // tag of the barrier that timed out
     unsigned int pad;
 };
+static_assert(offsetof(GridBar, count) == 0 && offsetof(GridBar, err) == 4, "one word, count below err");
 
 constexpr uint64_t GRID_WAIT_LIMIT_NS = 4000000000ull;   // 4 s
 
-__device__ __forceinline__ unsigned long long ld_acquire_gpu64(const void* p) {
+__device__ __forceinline__ unsigned long long ld_acquire_gpu(const unsigned long long* p) {
     unsigned long long v;
     asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
     return v;
 }
-__device__ __forceinline__ unsigned atom_add_release_gpu(unsigned* p, unsigned x) {
-    unsigned old;
-    asm volatile("atom.add.release.gpu.global.u32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(x) : "memory");
+__device__ __forceinline__ unsigned long long atom_add_release_gpu(unsigned long long* p, unsigned long long x) {
+    unsigned long long old;
+    asm volatile("atom.add.release.gpu.global.u64 %0, [%1], %2;" : "=l"(old) : "l"(p), "l"(x) : "memory");
     return old;
+}
+
+// The first error of a launch (true for the thread that set it): every wait ends on it.
+__device__ __forceinline__ bool grid_error(GridBar* b, unsigned code) {
+    return (atomicOr((unsigned long long*)b, (unsigned long long)code << 32) >> 32) == 0;
 }
 
 // What bounds it: the latency of one arrival (a release atomic) and of the poll that sees the
@@ -177,20 +187,21 @@ __device__ __forceinline__ bool grid_sync(GridBar* b, int tag = 0) {
     __shared__ int s_ok;
     __syncthreads();
     if (threadIdx.x == 0) {
+        unsigned long long* word = (unsigned long long*)b;
         const unsigned nb = gridDim.x;   // (rows of a two-dimensional grid have barriers of their own)
-        const unsigned old = atom_add_release_gpu(&b->count, 1u);
+        const unsigned old = (unsigned)atom_add_release_gpu(word, 1ull);
         const unsigned target = (old / nb + 1) * nb;
         uint64_t t0 = 0;
         unsigned long long w;
         for (unsigned it = 1;; it++) {
-            w = ld_acquire_gpu64(b);
+            w = ld_acquire_gpu(word);
             if ((int)((unsigned)w - target) >= 0 || (w >> 32) != 0) break;
             if ((it & 63u) == 0) {
                 const uint64_t t = globaltimer_ns();
                 if (t0 == 0) {
                     t0 = t;
                 } else if (t - t0 > GRID_WAIT_LIMIT_NS) {
-                    if (atomicCAS(&b->err, 0, 1) == 0) b->where = tag;
+                    if (grid_error(b, 1)) b->where = tag;
                     w |= 1ull << 32;
                     break;
                 }
@@ -206,7 +217,6 @@ __device__ __forceinline__ bool grid_sync(GridBar* b, int tag = 0) {
 // repair (given its own) does not start on a store whose update gave up.
 __device__ __forceinline__ bool update_failed(const GridBar* repair_bar) { return ld_volatile(&(repair_bar - 1)->err) != 0; }
 
-__device__ __forceinline__ void grid_fail(GridBar* b, int code) { atomicCAS(&b->err, 0, code); }
 
 // Phase timestamp written by one thread right after a grid barrier (profiling aid).
 __device__ __forceinline__ void phase_mark(unsigned long long* slot) {

@@ -1534,7 +1534,7 @@ int counters_fetch(scout_ctx* c) {
     SCOUT_CU(c, cudaMemcpyAsync(c->h_batch, c->d_batch, sizeof(DevBatch), cudaMemcpyDeviceToHost, c->s_main));
     SCOUT_CU(c, cudaStreamSynchronize(c->s_main));
     for (const GridBar& b : c->h_batch->bar)
-        if (b.err == 1)
+        if (b.err & 1)
             return c->fail(SCOUT_E_TIMEOUT, "a device grid barrier timed out (tag " + std::to_string(b.where) + ")");
     if (c->h_ctr->pad)
         return c->fail(SCOUT_E_STATE, "the component labels do not describe the components of the graph "
