@@ -236,15 +236,18 @@ class Context:
             ops = np.ascontiguousarray(ops, dtype=np.uint8)
             op = ops.ctypes.data_as(C.POINTER(C.c_uint8))
         self._c(LIB.scout_repair(self._h, _prob(problem), _pedge(e), op, len(e), C.byref(sd), C.byref(st)))
-        self._pf = nxt
+        # a hint ends with its batch: once that has been repaired its memory may be refilled
+        self._pf = None if nxt is None or np.may_share_memory(e, nxt) else nxt
         return st.as_dict()
 
     def prefetch(self, next_edges) -> None:
         """Hint the edits of the batch after the next repair: that repair copies them to the
         device while it runs (and, tiered store, gathers their cold rows into HBM). A page-locked
         array (pinned_copy) is read in place and must stay unchanged until its own repair(),
-        which, given the same object, uses the device copy instead of uploading it again; any
-        other array is copied here, may change, and is uploaded by its repair()."""
+        which, given the same object right after the repair that made the copy, uses it instead of
+        uploading the edits again (a hint for the very batch that is repaired next is dropped by
+        that repair: the memory may then be refilled); any other array is copied here, may change,
+        and is uploaded by its repair()."""
         e = as_edges(next_edges)
         self._c(LIB.scout_prefetch(self._h, _pedge(e), len(e)))
         self._pf_next = next_edges if e is next_edges and _page_locked(e) else None
