@@ -129,9 +129,8 @@ __global__ void k_fill_i32(int32_t* __restrict__ a, int64_t n, int32_t x) {
 }
 
 // (id, value) pairs of the touched list for the commit.
-__global__ void k_commit_gather(const int32_t* __restrict__ list, const DevCounters* __restrict__ ctr,
-                                const int32_t* __restrict__ val, int32_t* __restrict__ out) {
-    const int cnt = ctr->changed;
+__global__ void k_commit_gather(const int32_t* __restrict__ list, int cnt, const int32_t* __restrict__ val,
+                                int32_t* __restrict__ out) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += gridDim.x * blockDim.x) {
         int32_t v = list[i];
         out[2 * i] = v;
@@ -380,7 +379,7 @@ int commit_gather(scout_ctx* c, int problem, const int32_t** pairs, int64_t* cou
     } else if (cnt > 0) {
         cudaSetDevice(c->device);
         SCOUT_RC(pin_grow(c, &c->h_pin_commit, &c->cap_pin_commit, cnt * 8));
-        k_commit_gather<<<blocks_for(cnt, 256), 256, 0, c->s_main>>>(c->d_list[0], c->d_ctr, *slot, c->d_commit);
+        k_commit_gather<<<blocks_for(cnt, 256), 256, 0, c->s_main>>>(c->d_list[0], (int)cnt, *slot, c->d_commit);
         SCOUT_LAUNCH(c, "k_commit_gather");
         c->nlaunch += 1;
         SCOUT_CU(c, cudaMemcpyAsync(c->h_pin_commit, c->d_commit, (size_t)cnt * 8, cudaMemcpyDeviceToHost, c->s_main));

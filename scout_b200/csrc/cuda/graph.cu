@@ -148,7 +148,7 @@ __global__ void k_classify(DGraph g, const scout_edge* __restrict__ e, const uin
         unsigned mi = __ballot_sync(__activemask(), valid && ins);
         unsigned md = __ballot_sync(__activemask(), valid && !ins);
         unsigned ma = __ballot_sync(__activemask(), valid && applied);
-        if (lane_id() == (unsigned)(__ffs(__activemask()) - 1)) {
+        if (ctr && lane_id() == (unsigned)(__ffs(__activemask()) - 1)) {
             if (mi) atomicAdd(&ctr->n_ins, __popc(mi));
             if (md) atomicAdd(&ctr->n_del, __popc(md));
             if (ma) atomicAdd(&ctr->n_half, 2 * __popc(ma));
@@ -1527,6 +1527,7 @@ int batch_begin(scout_ctx* c) {
     SCOUT_CU(c, cudaMemsetAsync(c->d_batch, 0, offsetof(DevBatch, pairs), c->s_main));
     c->bar_used = false;
     c->pairs_ready = false;
+    c->last_changed = 0;   // counted again when the batch has run; until then there is nothing to commit
     return SCOUT_OK;
 }
 
@@ -2378,11 +2379,12 @@ int scout_classify(scout_ctx* c, const scout_edge* e, int64_t m, uint8_t* out) {
     if (m == 0) return SCOUT_OK;
     cudaSetDevice(c->device);
     SCOUT_RC(ws_ensure(c, m));
-    SCOUT_RC(batch_begin(c));
+    // (no batch begins: the last repair's counters and changed entries stay, for its commit)
+    SCOUT_RC(gather_finish(c, nullptr, nullptr, nullptr));
     SCOUT_RC(pin_grow(c, &c->h_pin_edits, &c->cap_pin_edits, m * (int64_t)sizeof(scout_edge) + m));
     std::memcpy(c->h_pin_edits, e, (size_t)m * sizeof(scout_edge));
     SCOUT_CU(c, cudaMemcpyAsync(c->d_edits, c->h_pin_edits, (size_t)m * sizeof(scout_edge), cudaMemcpyHostToDevice, c->s_main));
-    k_classify<<<blocks_for(m, 256), 256, 0, c->s_main>>>(dgraph(c), c->d_edits, nullptr, m, 1, nullptr, c->d_eflag, c->d_ctr, 0);
+    k_classify<<<blocks_for(m, 256), 256, 0, c->s_main>>>(dgraph(c), c->d_edits, nullptr, m, 1, nullptr, c->d_eflag, nullptr, 0);
     SCOUT_LAUNCH(c, "k_classify");
     uint8_t* pf = (uint8_t*)c->h_pin_edits + m * sizeof(scout_edge);
     SCOUT_CU(c, cudaMemcpyAsync(pf, c->d_eflag, (size_t)m, cudaMemcpyDeviceToHost, c->s_main));
