@@ -220,8 +220,9 @@ int scout_repair_cc(scout_ctx* ctx, const scout_edge* edits, const uint8_t* ops,
  * copy instead of uploading its edits. On a tiered store the same call also gathers the rows
  * of these edits' endpoints that are still in host memory into free HBM, so the hinted batch's
  * merge and repair find them in HBM (its stats report the gather). A page-locked `next` is
- * read in place by that copy and must stay unchanged until the repair that uses it; other
- * buffers are copied here and are free on return. The fetch of batch K+1 overlapping the
+ * read in place by that copy: it must stay unchanged until the repair that uses it and
+ * allocated until the next scout_prefetch call has returned (or the context is destroyed), used
+ * or not; other buffers are copied here and are free on return. The fetch of batch K+1 overlapping the
  * repair of batch K replaces the reference's per-round host fetch (scout_bfs.cu:199-229) and
  * MIS's K+1 || K channels (scout_mis.cu:855-912). A hint that is not used only costs the copy. */
 int scout_prefetch(scout_ctx* ctx, const scout_edge* next, int64_t m);

@@ -203,9 +203,10 @@ extern "C" int scout_prefetch(scout_ctx* c, const scout_edge* next, int64_t m) {
     c->pf_pending = false;
     c->pf_m = 0;
     // the copy stream may still read the previous hint's edits (from the staging buffer
-    // overwritten below) or gather its rows; a copy already made stays usable
+    // overwritten below, or where the caller may now drop them), whether or not a repair used
+    // the copy, or gather its rows; a copy already made stays usable
     if (c->gather_active) SCOUT_CU(c, cudaEventSynchronize(c->ev_gather1));
-    if (c->pf_ready) SCOUT_CU(c, cudaEventSynchronize(c->ev_pf));
+    SCOUT_CU(c, cudaEventSynchronize(c->ev_pf));
     if (m == 0) return SCOUT_OK;
     cudaPointerAttributes at;
     const bool pinned = cudaPointerGetAttributes(&at, next) == cudaSuccess && at.type == cudaMemoryTypeHost;

@@ -129,6 +129,7 @@ class Context:
     def close(self) -> None:
         if self._h and self._own:
             LIB.scout_ctx_destroy(self._h)
+            self._pf = self._pf_next = self._pf_keep = None
         self._h = None
 
     def __enter__(self):
@@ -242,14 +243,18 @@ class Context:
 
     def prefetch(self, next_edges) -> None:
         """Hint the edits of the batch after the next repair: that repair copies them to the
-        device while it runs (and, tiered store, gathers their cold rows into HBM). A page-locked
-        array (pinned_copy) is read in place and must stay unchanged until its own repair(),
-        which, given the same object right after the repair that made the copy, uses it instead of
-        uploading the edits again (a hint for the very batch that is repaired next is dropped by
-        that repair: the memory may then be refilled); any other array is copied here, may change,
-        and is uploaded by its repair()."""
+        device while it runs (and, tiered store, gathers their cold rows into HBM). An array in
+        page-locked memory, wherever that came from, is read in place: it is kept alive here and
+        must stay unchanged until its own repair(). That repair, given the same array of
+        pinned_empty / pinned_copy right after the repair that made the copy, uses the copy instead
+        of uploading the edits again, and uploads any other (a hint for the very batch that is
+        repaired next is dropped by that repair: the memory may then be refilled). A pageable array
+        is copied here, may change, and is uploaded by its repair()."""
         e = as_edges(next_edges)
         self._c(LIB.scout_prefetch(self._h, _pedge(e), len(e)))
+        # the library has let go of the previous hint's memory and may read this one's until the
+        # next hint, or the context's end, whatever the repairs in between do
+        self._pf_keep = e
         self._pf_next = next_edges if e is next_edges and _page_locked(e) else None
 
     def repair_probe(self, problem, edges, ops=None, sched: Optional[dict] = None):
@@ -358,7 +363,7 @@ class MultiEngine:
     def close(self) -> None:
         if self._h:
             LIB.scout_multi_destroy(self._h)
-            self._h = None
+            self._h = self._ctx = None
 
     def __enter__(self):
         return self
@@ -377,8 +382,11 @@ class MultiEngine:
 
     @property
     def context(self) -> "Context":
-        """The underlying device context (not owned): scheduler install, graph info."""
-        return Context._borrow(LIB.scout_multi_context(self._h))
+        """The underlying device context (not owned): scheduler install, graph info. One object for
+        the engine's life: it keeps what was hinted through it."""
+        if getattr(self, "_ctx", None) is None:
+            self._ctx = Context._borrow(LIB.scout_multi_context(self._h))
+        return self._ctx
 
     def add_stream(self, off, adj, init, source: int = 0) -> int:
         off = _i64(off)

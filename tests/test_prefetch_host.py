@@ -61,3 +61,49 @@ def test_a_hint_ends_with_its_batch(ctx, alias):
     b[:] = _edges(4)
     c.repair("bfs", b)
     assert lib.declared == [0, 0]
+
+
+@pytest.mark.parametrize("page_locked", [True, False])
+@pytest.mark.parametrize("between", ["nothing", "repair", "refused repair", "its own repair"])
+def test_the_hinted_array_outlives_the_copy(ctx, monkeypatch, page_locked, between):
+    """Whether memory is page-locked the library decides by itself (an array of another library may
+    be), and it may read such memory until the next hint: the array lives until then, however it
+    was allocated, used or not, and also where the repair in between was refused."""
+    c, lib = ctx
+    monkeypatch.setattr(engine, "_page_locked", lambda a: page_locked)
+    b = _edges(5)
+    c.prefetch(b)
+    ref = weakref.ref(b)
+    if between == "its own repair":
+        c.repair("bfs", _edges(6))
+        c.repair("bfs", b)
+    del b
+    if between == "repair":
+        c.repair("bfs", _edges(6))
+    if between == "refused repair":
+        lib.fail = -1
+        with pytest.raises(engine.ScoutError):
+            c.repair("bfs", _edges(6))
+    gc.collect()
+    assert ref() is not None
+    c.prefetch(_edges(7))
+    gc.collect()
+    assert (ref() is None) or between in ("repair",) and page_locked   # (declared for the repair to come)
+
+
+def test_a_converted_array_lives_as_long(ctx, monkeypatch):
+    """as_edges may hand the library another object than the caller's."""
+    c, lib = ctx
+    kept = []
+    monkeypatch.setattr(lib, "scout_prefetch", lambda h, e, m: kept.append(C.addressof(e.contents)) or 0, raising=False)
+    b = _edges(8).astype(np.int64)
+    c.prefetch(b)
+    assert c._pf_keep.ctypes.data == kept[0]
+
+
+def test_an_engine_has_one_context(monkeypatch):
+    """A hint through MultiEngine.context is kept by the engine, not by a passing view."""
+    monkeypatch.setattr(engine, "LIB", type("L", (), {"scout_multi_context": staticmethod(lambda h: 7)})())
+    e = engine.MultiEngine.__new__(engine.MultiEngine)
+    e._h = None
+    assert e.context is e.context
