@@ -5,7 +5,7 @@
 // (tools/greedy_color.cpp:37-52), BFS levels (tools/bfs_ground_truth.cu:39-151) and min-id
 // component labels (tools/excc_src/excc_v1.cu:520-531). scout_seed computes the same solutions
 // on the GPU: BFS and CC by the engine's own full traversal and recompute, the two greedy
-// rules by one persistent kernel of rounds. A vertex decides once every lower-id neighbour has
+// rules by persistent kernels of rounds. A vertex decides once every lower-id neighbour has
 // decided (rows are sorted, so those neighbours are a prefix of its row):
 //   MIS       in iff no lower-id neighbour is in
 //   colouring the smallest colour no lower-id neighbour has
@@ -14,8 +14,17 @@
 // The number of rounds is the longest chain of vertices each waiting on a lower-id neighbour
 // (about 900 on an R-MAT graph of 500,000 vertices, edge factor 16).
 //
-// What bounds it: the latency of a round (a few hundred open vertices decide in each), so a
-// round only touches vertices that can move. An open vertex waits on ONE undecided neighbour,
+// A greedy MIS decides an open vertex as soon as any lower neighbour joins, so its chains are short
+// (6 to 13 rounds on R-MAT graphs of 2,000 to 2 M vertices and on random graphs): k_seed_rounds
+// looks at every open vertex again in each of up to SEED_ROUNDS rounds. Waiting in lists, below,
+// hears of a joined neighbour only when the one waited for decides: 35 to 233 rounds there, and
+// 1.7 to 2.3 times the time (whole call, R-MAT of edge factor 16, by rounds and by lists: 8,000
+// vertices 249 and 424 us; 100,000: 447 and 917; 2 M: 2,180 and 4,950). What is still open after
+// SEED_ROUNDS rounds lies on long chains (a path or a grid numbered in order), and the lists finish
+// it, being the faster there (grid of 700 x 700: 9.2 ms by lists, 17.4 by rounds, 9.7 by both).
+//
+// The lists (k_seed_greedy; colourings from the start). What bounds it: the latency of a round (a
+// few hundred open vertices decide in each), so a round only touches vertices that can move. An open vertex waits on ONE undecided neighbour,
 // the highest-id one (it tends to decide last, so few waits follow one another), in that
 // neighbour's list of waiters; a vertex that decides closes its list and queues the waiters for
 // the next round. The list of w holds at most as many waiters as w has higher-id neighbours; a
@@ -34,6 +43,7 @@ namespace scout {
 
 constexpr int SEED_THREADS = 1024;
 constexpr int32_t UNDECIDED = -1;
+constexpr int SEED_ROUNDS = 32;             // MIS rounds before the lists take over
 constexpr int SEED_BIG = 1024;              // longer prefixes are scanned by a whole block
 constexpr int SEED_WORDS = 32;              // bitmap window: 1024 colours
 constexpr int SEED_CLOSED = 0x40000000;     // a closed waiter list's count
@@ -53,17 +63,72 @@ struct SeedParams {
     GridBar* bar;
 };
 
-// Per vertex: the row prefix of neighbours below it, the slots its waiter list gets.
+// Rounds of the MIS rule over all open vertices, one thread each, until none is open or SEED_ROUNDS
+// are done. ctr->affected: the vertices left open.
+__global__ void __launch_bounds__(SEED_THREADS, 1) k_seed_rounds(SeedParams p) {
+    const int64_t n = p.g.n;
+    const int64_t tid = lthread_id();
+    const int64_t T = (int64_t)gridDim.x * blockDim.x;
+    const bool leader = blockIdx.x == 0 && threadIdx.x == 0;
+    for (int64_t v = tid; v < n; v += T) p.out[v] = UNDECIDED;
+    if (!grid_sync(p.bar, 50)) return;
+    int cur = 2, rounds = 0, cnt = (int)n;
+    long long bytes = 0;
+    while (cnt > 0 && rounds < SEED_ROUNDS) {
+        const int nxt = (cur + 1) % 3, zer = (cur + 2) % 3;
+        const int32_t* wl = p.wl[rounds & 1];
+        int32_t* wn = p.wl[(rounds & 1) ^ 1];
+        if (leader) p.ctr->list_count[zer] = 0;
+        for (int64_t b = tid - (tid & (WARP - 1)); b < cnt; b += T) {
+            const int64_t i = b + lane_id();
+            bool open = false;
+            int32_t v = 0;
+            if (i < cnt) {
+                v = rounds ? wl[i] : (int32_t)i;   // every vertex in the first round
+                const Row r = p.g.row[v];
+                const int32_t* row = p.g.pool + r.start;
+                const int k = (int)lower_bound_i32(row, r.len, v);
+                bytes += 16 + 4LL * k * 2;
+                bool any_in = false, all_done = true;
+                for (int j = 0; j < k && !any_in; j++) {
+                    const int32_t s = ld_volatile(p.out + row[j]);
+                    any_in = s == 1;
+                    all_done &= s != UNDECIDED;
+                }
+                if (any_in) p.out[v] = 0;
+                else if (all_done) p.out[v] = 1;
+                else open = true;
+            }
+            const int at = warp_append(open, &p.ctr->list_count[nxt]);
+            if (open) wn[at] = v;
+        }
+        rounds++;
+        if (!grid_sync(p.bar, 51)) return;
+        cur = nxt;
+        cnt = ld_volatile(&p.ctr->list_count[cur]);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) bytes += __shfl_xor_sync(0xffffffffu, bytes, o);
+    if (lane_id() == 0) atomicAdd((unsigned long long*)&p.ctr->hbm_bytes, (unsigned long long)bytes);
+    if (leader) {
+        p.ctr->rounds = rounds;
+        p.ctr->affected = cnt;
+    }
+}
+
+// Per vertex: the row prefix of neighbours below it, the slots its waiter list gets. `fresh`: no vertex
+// is decided yet; else the decided ones keep their value and their list is closed.
 __global__ void k_seed_prep(DGraph g, int32_t* __restrict__ out, int32_t* __restrict__ pre, int32_t* __restrict__ open,
-                            int32_t* __restrict__ nwait, int64_t* __restrict__ slots) {
+                            int32_t* __restrict__ nwait, int64_t* __restrict__ slots, bool fresh) {
     for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < g.n; v += (int64_t)gridDim.x * blockDim.x) {
         const Row r = g.row[v];
         const int32_t* row = g.pool + r.start;
         const int k = (int)lower_bound_i32(row, r.len, (int32_t)v);
+        const bool decided = !fresh && out[v] != UNDECIDED;
         pre[v] = k;
         open[v] = k;
-        nwait[v] = 0;
-        out[v] = UNDECIDED;
+        nwait[v] = decided ? SEED_CLOSED : 0;
+        if (fresh) out[v] = UNDECIDED;
         slots[v] = r.len - k;   // a loop's own entry only adds a slot
     }
 }
@@ -200,7 +265,7 @@ __global__ void __launch_bounds__(SEED_THREADS, 1) k_seed_greedy(SeedParams p) {
         const int64_t v = b + lane_id();
         bool again = false;
         int cnt = 0;
-        if (v < n) {
+        if (v < n && ld_volatile(p.nwait + v) < SEED_CLOSED) {   // (closed: decided by the rounds before)
             const int k = p.pre[v];
             bytes += 24;
             if (k == 0) {
@@ -333,7 +398,41 @@ __global__ void __launch_bounds__(SEED_THREADS, 1) k_seed_greedy(SeedParams p) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) bytes += __shfl_xor_sync(0xffffffffu, bytes, o);
     if (lane_id() == 0) atomicAdd((unsigned long long*)&p.ctr->hbm_bytes, (unsigned long long)bytes);
-    if (leader) p.ctr->rounds = rounds;
+    if (leader) p.ctr->rounds += rounds;
+}
+
+// The lists' scratch and kernel, and the counters. `fresh`: no vertex is decided yet.
+static int seed_lists(scout_ctx* c, SeedParams p, bool fresh) {
+    const int64_t n = c->n;
+    if (!c->d_coff) SCOUT_RC(dev_alloc(c, (void**)&c->d_coff, (size_t)(n + 1) * sizeof(int64_t), "compaction offsets"));
+    p.pre = (int32_t*)c->d_qbuf[0];    // the work queues are free outside a repair (qcap >= n items)
+    p.open = (int32_t*)c->d_qbuf[1];
+    p.nwait = (int32_t*)c->d_qbuf[2];
+    p.off = c->d_coff;
+    k_seed_prep<<<blocks_for(n, 256), 256, 0, c->s_main>>>(p.g, p.out, p.pre, p.open, p.nwait, c->d_coff, fresh);
+    SCOUT_LAUNCH(c, "k_seed_prep");
+    SCOUT_RC(scan_i64(c, c->d_coff, n, c->d_coff + n));
+    // the waiter lists hold at most nnz slots in all: the compaction spare's memory (its contents
+    // are dead between compactions), or an allocation of its own if the budget has room
+    const int64_t slots = std::max<int64_t>(c->nnz, 1);
+    int32_t* own = nullptr;
+    if (c->spare && c->spare_cap >= slots) {
+        p.waiters = c->spare;
+    } else {
+        const std::string before = c->err;
+        if (dev_alloc(c, (void**)&own, (size_t)slots * 4, "waiter lists") != SCOUT_OK) { own = nullptr; c->err = before; }
+        p.waiters = own;
+    }
+    void* args[] = {&p};
+    int rc = SCOUT_OK;
+    if (p.waiters && cudaMemsetAsync(p.waiters, 0xff, (size_t)slots * 4, c->s_main) != cudaSuccess)
+        rc = cuda_fail(c, cudaGetLastError(), "seed");
+    if (rc == SCOUT_OK) rc = coop_launch(c, (const void*)k_seed_greedy, SEED_THREADS, args, 0);
+    c->nlaunch += 1;
+    if (rc == SCOUT_OK && cudaEventRecord(c->ev_t[2], c->s_main) != cudaSuccess) rc = cuda_fail(c, cudaGetLastError(), "seed");
+    if (rc == SCOUT_OK) rc = counters_fetch(c);
+    if (own) dev_free(c, own, (size_t)slots * 4);
+    return rc;
 }
 
 }  // namespace scout
@@ -368,44 +467,28 @@ int scout_seed(scout_ctx* c, int problem, int32_t source, scout_batch_stats* st)
     if (problem == SCOUT_CC) return scout_recompute_cc(c, st);
     SCOUT_RC(lists_ensure(c));
     SCOUT_RC(batch_begin(c));
-    const int64_t n = c->n;
-    if (!c->d_coff) SCOUT_RC(dev_alloc(c, (void**)&c->d_coff, (size_t)(n + 1) * sizeof(int64_t), "compaction offsets"));
     SeedParams p;
     p.g = dgraph(c);
     p.out = *slot;
     p.mode = problem == SCOUT_MIS ? 0 : 1;
     p.wl[0] = c->d_list[0];
     p.wl[1] = c->d_list[1];
-    p.pre = (int32_t*)c->d_qbuf[0];    // the work queues are free outside a repair (qcap >= n items)
-    p.open = (int32_t*)c->d_qbuf[1];
-    p.nwait = (int32_t*)c->d_qbuf[2];
-    p.off = c->d_coff;
     p.ctr = c->d_ctr;
     p.bar = c->d_bar;
+    p.pre = p.open = p.nwait = p.waiters = nullptr;
+    p.off = nullptr;
     c->last_problem = problem;
     SCOUT_CU(c, cudaEventRecord(c->ev_t[1], c->s_main));
-    k_seed_prep<<<blocks_for(n, 256), 256, 0, c->s_main>>>(p.g, p.out, p.pre, p.open, p.nwait, c->d_coff);
-    SCOUT_LAUNCH(c, "k_seed_prep");
-    SCOUT_RC(scan_i64(c, c->d_coff, n, c->d_coff + n));
-    // the waiter lists hold at most nnz slots in all: the compaction spare's memory (its contents
-    // are dead between compactions), or an allocation of its own if the budget has room
-    const int64_t slots = std::max<int64_t>(c->nnz, 1);
-    int32_t* own = nullptr;
-    if (c->spare && c->spare_cap >= slots) {
-        p.waiters = c->spare;
-    } else {
-        const std::string before = c->err;
-        if (dev_alloc(c, (void**)&own, (size_t)slots * 4, "waiter lists") != SCOUT_OK) { own = nullptr; c->err = before; }
-        p.waiters = own;
+    bool open = true;
+    if (p.mode == 0) {
+        void* args[] = {&p};
+        SCOUT_RC(coop_launch(c, (const void*)k_seed_rounds, SEED_THREADS, args, 0));
+        SCOUT_CU(c, cudaEventRecord(c->ev_t[2], c->s_main));
+        SCOUT_RC(counters_fetch(c));
+        open = c->h_ctr->affected > 0;
+        if (open) SCOUT_CU(c, cudaMemsetAsync(c->d_ctr->list_count, 0, sizeof(c->d_ctr->list_count), c->s_main));
     }
-    if (p.waiters) SCOUT_CU(c, cudaMemsetAsync(p.waiters, 0xff, (size_t)slots * 4, c->s_main));
-    void* args[] = {&p};
-    int rc = coop_launch(c, (const void*)k_seed_greedy, SEED_THREADS, args, 0);
-    c->nlaunch += 1;
-    if (rc == SCOUT_OK && cudaEventRecord(c->ev_t[2], c->s_main) != cudaSuccess) rc = cuda_fail(c, cudaGetLastError(), "seed");
-    if (rc == SCOUT_OK) rc = counters_fetch(c);
-    if (own) dev_free(c, own, (size_t)slots * 4);
-    SCOUT_RC(rc);
+    if (open) SCOUT_RC(seed_lists(c, p, problem != SCOUT_MIS));
     float ms = 0.f;
     cudaEventElapsedTime(&ms, c->ev_t[1], c->ev_t[2]);
     st->ms_repair = ms;
