@@ -292,6 +292,19 @@ static void advance_tails(scout_ctx* c, const DevCounters& h) {
     if (c->batch_dest == 2) c->host_tail += h.new_elems_host;
 }
 
+// The end of a batch: its counters, and the store's bookkeeping by them. The rows were merged
+// whether or not the repair then failed, so the tails and the entry count move in either case (the
+// next merge would overwrite those rows, and buffers sized by the count would be too small).
+static int batch_account(scout_ctx* c) {
+    const int rc = counters_fetch(c);
+    if (!c->fetched) return rc;
+    const DevCounters& h = *c->h_ctr;
+    advance_tails(c, h);
+    c->nnz += h.nnz_delta;
+    c->qtag += (uint32_t)h.rounds + 8;
+    return rc;
+}
+
 // Batch statistics from the counters of the last repair run (already fetched).
 static void fill_stats(scout_ctx* c, scout_batch_stats* st, int64_t launch0) {
     const DevCounters& h = *c->h_ctr;
@@ -436,17 +449,17 @@ int union_run(scout_ctx* const* cs, const int* problems, const scout_edge* const
         variants[i] = plain_variant(problems[i], sds[i]);
     }
     SCOUT_RC(union_launch(cs, problems, sds, variants, ne, round, later, side));
+    int first = SCOUT_OK;
     for (int i = 0; i < ne; i++) {
         scout_ctx* c = cs[i];
         SCOUT_CU(c, cudaEventRecord(c->ev_t[2], c->s_main));
-        SCOUT_RC(counters_fetch(c));
-        const DevCounters& h = *c->h_ctr;
-        advance_tails(c, h);
-        c->nnz += h.nnz_delta;
-        c->qtag += (uint32_t)h.rounds + 8;
+        const int rc = batch_account(c);   // every store's, before an error of one is returned
+        if (first == SCOUT_OK) first = rc;
+        if (rc != SCOUT_OK) continue;
         fill_stats(c, &stats[i], launch0[i]);
         stats[i].variant = variants[i];
     }
+    SCOUT_RC(first);
     const double ms = ev_ms(cs[0]->ev_t[4], cs[0]->ev_t[5]);
     const double total = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
     for (int i = 0; i < ne; i++) {
@@ -476,19 +489,27 @@ int scout_repair(scout_ctx* c, int problem, const scout_edge* edits, const uint8
     const int prc = batch_prologue(c, problem, edits, ops, m, st);
     c->pf_use = false;
     SCOUT_RC(prc);
-    // the hinted next batch: its edits' copy (and, tiered, its cold rows' gather) during this repair
-    SCOUT_RC(prefetch_launch(c, c->merge_tail));
     const int* mode_dev = nullptr;
     const int variant = plain_variant(problem, sd);
-    if (sd.policy == SCOUT_SCHED_LEARNED && sched_variants(problem) > 1)
-        SCOUT_RC(sched_decide(c, problem, m, true, &mode_dev));
-    SCOUT_RC(run_repair(c, problem, sd, variant, mode_dev, st));
-    SCOUT_CU(c, cudaEventRecord(c->ev_t[2], c->s_main));
-    SCOUT_RC(counters_fetch(c));
+    auto repair = [&]() -> int {
+        // the hinted next batch: its edits' copy (and, tiered, its cold rows' gather) during this repair
+        SCOUT_RC(prefetch_launch(c, c->merge_tail));
+        if (sd.policy == SCOUT_SCHED_LEARNED && sched_variants(problem) > 1)
+            SCOUT_RC(sched_decide(c, problem, m, true, &mode_dev));
+        SCOUT_RC(run_repair(c, problem, sd, variant, mode_dev, st));
+        SCOUT_CU(c, cudaEventRecord(c->ev_t[2], c->s_main));
+        return SCOUT_OK;
+    };
+    const int rrc = repair();
+    if (rrc != SCOUT_OK) {   // refused (no room for its scratch, say): the merge is queued all the same
+        const std::string why = c->err;
+        batch_account(c);
+        c->last_changed = 0;
+        c->err = why;
+        return rrc;
+    }
+    SCOUT_RC(batch_account(c));
     const DevCounters& h = *c->h_ctr;
-    advance_tails(c, h);
-    c->nnz += h.nnz_delta;
-    c->qtag += (uint32_t)h.rounds + 8;
     fill_stats(c, st, launch0);
     st->variant = mode_dev ? h.decision : variant;
     st->ms_repair = ev_ms(c->ev_t[1], c->ev_t[2]);
@@ -541,10 +562,11 @@ int scout_repair_probe(scout_ctx* c, int problem, const scout_edge* edits, const
         SCOUT_CU(c, cudaEventRecord(c->ev_t[4], c->s_main));
         SCOUT_RC(run_repair(c, problem, sd, v, nullptr, st));
         SCOUT_CU(c, cudaEventRecord(c->ev_t[5], c->s_main));
-        SCOUT_RC(counters_fetch(c));
+        // (the first variant's counters hold the merge's as well)
+        SCOUT_RC(i == 0 ? batch_account(c) : counters_fetch(c));
         variant_ms[v] = ev_ms(c->ev_t[4], c->ev_t[5]);
         best = std::min(best, variant_ms[v]);
-        c->qtag += (uint32_t)c->h_ctr->rounds + 8;
+        if (i > 0) c->qtag += (uint32_t)c->h_ctr->rounds + 8;
         if (i == 0) {
             SCOUT_CU(c, cudaMemcpyAsync(ref, state, (size_t)n * 4, cudaMemcpyDeviceToDevice, c->s_main));
         } else {
@@ -560,8 +582,6 @@ int scout_repair_probe(scout_ctx* c, int problem, const scout_edge* edits, const
     }
     for (int v = nv; v < 3; v++) variant_ms[v] = -1.0;
     const DevCounters& h = *c->h_ctr;
-    advance_tails(c, h);
-    c->nnz += h.nnz_delta;
     fill_stats(c, st, launch0);
     st->variant = 0;
     st->ms_repair = variant_ms[0];

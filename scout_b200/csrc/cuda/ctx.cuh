@@ -194,6 +194,7 @@ struct scout_ctx {
     DevCounters* h_ctr = nullptr;
     scout::GridBar* d_bar = nullptr; // the repair's barrier (d_batch->bar[1])
     bool bar_used = false;           // a kernel has used it since the batch began
+    bool fetched = false;            // the last counters_fetch read them (they may hold an error)
     bool pairs_ready = false;        // h_batch->pairs holds the last repair's changed entries
     int* d_flags = nullptr;          // staging / seal error flags (int[16])
 

@@ -1532,8 +1532,10 @@ int batch_begin(scout_ctx* c) {
 }
 
 int counters_fetch(scout_ctx* c) {
+    c->fetched = false;
     SCOUT_CU(c, cudaMemcpyAsync(c->h_batch, c->d_batch, sizeof(DevBatch), cudaMemcpyDeviceToHost, c->s_main));
     SCOUT_CU(c, cudaStreamSynchronize(c->s_main));
+    c->fetched = true;
     for (const GridBar& b : c->h_batch->bar)
         if (b.err & 1)
             return c->fail(SCOUT_E_TIMEOUT, "a device grid barrier timed out (tag " + std::to_string(b.where) + ")");
