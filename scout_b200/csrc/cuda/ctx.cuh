@@ -303,7 +303,7 @@ struct RowPlan {
     MergeRow* mrow;        // short rows of one half-edit from the front, the others from the back
     int64_t mcap;
     int32_t* shorts;       // records of the other short rows
-    int64_t* slices;       // (record << 32 | slice)
+    int64_t* slices;       // (record << 32 | slice, or an insertion item)
     int64_t slice_cap;
     int32_t* longs;        // records of long rows compacted in place
     bool long_in_place;

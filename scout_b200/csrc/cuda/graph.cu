@@ -39,6 +39,9 @@ namespace scout {
 constexpr int SLICE = 2048;          // old-row entries merged by one warp at a time
 constexpr int SMALL_LEN = 128;       // rows up to this length (and 32 half-edits) are short
 constexpr int IN_PLACE_LEN = 4096;   // longest deletion-only row compacted in place by one warp
+constexpr int HEAVY = 1024;          // rows of more half-edits: no warp walks them (merge_heavy), and as many
+                                     // insertions are a merge item of their own
+constexpr int64_t INS_ITEM = 1ll << 31;   // marks such an item in the slice list
 
 // A row whose half-edits are all deletions is rewritten in place: its survivors only move
 // towards the row start, it keeps its start and capacity, and it takes no pool space (one warp
@@ -463,7 +466,7 @@ __device__ __forceinline__ void row_plan(const RowPlan& p, int A, int group, int
         const bool ok = a < A;
         Row r{0, 0, 0};
         int32_t u = 0;
-        int b = 0, d = 0, e = 0, nl = 0, ns = 0;
+        int b = 0, d = 0, e = 0, nl = 0, ns = 0, ni = 0;   // ns old slices, ni insertion items
         bool ip = false, cold = false, one = false, sm = false, lip = false;
         if (ok) {
             u = p.aff[a];
@@ -478,13 +481,14 @@ __device__ __forceinline__ void row_plan(const RowPlan& p, int A, int group, int
             one = r.len <= SMALL_LEN && e - b == 1;
             sm = !one && r.len <= SMALL_LEN && e - b <= WARP;
             ns = one || sm || lip ? 0 : ip ? 1 : max(1, (r.len + SLICE - 1) / SLICE);
+            if (e - b > HEAVY) ni = (d - b + HEAVY - 1) / HEAVY;
             nnz_delta += nl - r.len;
             bytes += 4LL * ((long long)r.len + nl) + 8LL * (e - b) + 16;
         }
         const long long need = ok && !ip ? (long long)r.len + (d - b) : 0;
         // counts packed: slices 30 bits, rows of one half-edit, other rows, short ones 11 bits each
         long long th, tc = 0, tn, tl = 0, oh = cold ? 0 : need, oc = 0, ol = lip;
-        long long on = (long long)ns | ((long long)(ok && one) << 30) | ((long long)(ok && !one) << 41) | ((long long)sm << 52);
+        long long on = (long long)(ns + ni) | ((long long)(ok && one) << 30) | ((long long)(ok && !one) << 41) | ((long long)sm << 52);
         auto scan2 = [](long long& x, long long& y, long long* tx, long long* ty) {
             if (BLOCK) {
                 block_scan2(x, y, tx, ty);
@@ -531,8 +535,12 @@ __device__ __forceinline__ void row_plan(const RowPlan& p, int A, int group, int
             if (sm) p.shorts[bs[5] + ((on >> 52) & 2047)] = (int32_t)at;
             if (lip) p.longs[bs[6] + ol] = (int32_t)at;
             const long long s0 = bs[2] + (on & ((1ll << 30) - 1));
-            if (s0 + ns > p.slice_cap) { if (ns) atomicExch(&p.ctr->overflow, 1); }
-            else for (int s = 0; s < ns; s++) p.slices[s0 + s] = (at << 32) | s;
+            if (s0 + ns + ni > p.slice_cap) {
+                if (ns + ni) atomicExch(&p.ctr->overflow, 1);
+            } else {
+                for (int s = 0; s < ns; s++) p.slices[s0 + s] = (at << 32) | s;
+                for (int s = 0; s < ni; s++) p.slices[s0 + ns + s] = (at << 32) | INS_ITEM | s;
+            }
         }
         if (BLOCK) __syncthreads();   // the bases and sums are read before the next rows overwrite them
     }
@@ -712,6 +720,76 @@ static __device__ __forceinline__ void merge_slice(int32_t* __restrict__ pool, c
     }
     if (s1 == r.len)   // insertions past the last entry
         for (int k = ii + l; k < r.d; k += WARP) N[r.len + (k - r.b) - gone] = key_v(keys[k], B);
+}
+
+// First half-edit in [lo, hi) whose position is >= x, by one lane.
+__device__ __forceinline__ int lb_event(const uint32_t* __restrict__ epos, int lo, int hi, int x) {
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if ((int)(epos[mid] >> 1) < x) lo = mid + 1; else hi = mid;
+    }
+    return lo;
+}
+
+// Rows of more than HEAVY half-edits. Their events may all lie in one gap of a short row (a vertex
+// that gains its neighbours in one batch) or repeat one pair, so nothing walks them: insertions
+// are items of HEAVY of them, each placed by a lane (merge_insertions), and old entries [s0, s1)
+// find their own shift by searching the slice's events (merge_heavy). A warp that walked them took
+// a turn per 32 events, on one word of its chunk: update of 10^6 edits at one vertex of three
+// neighbours, on 2^20 vertices, 101.8 ms; so 0.46 (random pairs: 0.51). Up to HEAVY events the walk
+// is at most 32 turns, and reads far less than the two searches of every old entry.
+static __device__ __forceinline__ void merge_insertions(int32_t* __restrict__ pool,
+                                                        const unsigned long long* __restrict__ keys, int B,
+                                                        const uint32_t* __restrict__ epos, const int32_t* __restrict__ E,
+                                                        const MergeRow& r, int item) {
+    const int k0 = r.b + item * HEAVY, k1 = min(r.d, k0 + HEAVY);
+    int dlo = r.d, dhi = r.e;   // the deletions among these insertions' positions
+    if (r.d < r.e) {
+        dlo = warp_lb_event(epos, r.d, r.e, (int)(epos[k0] >> 1));
+        dhi = warp_lb_event(epos, dlo, r.e, (int)(epos[k1 - 1] >> 1));
+    }
+    const int before = r.d < r.e ? E[r.d] : 0;
+    for (int k = k0 + (int)lane_id(); k < k1; k += WARP) {
+        const int pos = (int)(epos[k] >> 1);
+        const int gone = r.d < r.e ? E[lb_event(epos, dlo, dhi, pos)] - before : 0;
+        pool[r.dst + pos + (k - r.b) - gone] = key_v(keys[k], B);
+    }
+}
+
+static __device__ __forceinline__ void merge_heavy(int32_t* __restrict__ pool, const uint32_t* __restrict__ epos,
+                                                   const int32_t* __restrict__ E, const MergeRow& r, int s0, int s1) {
+    constexpr int U = 4;
+    const int l = (int)lane_id();
+    const int ilo = warp_lb_event(epos, r.b, r.d, s0), ihi = warp_lb_event(epos, ilo, r.d, s1);
+    const int dlo = warp_lb_event(epos, r.d, r.e, s0), dhi = warp_lb_event(epos, dlo, r.e, s1);
+    const int before = r.d < r.e ? E[r.d] : 0;
+    for (int b0 = s0; b0 < s1; b0 += U * WARP) {
+        int32_t x[U];
+        int to[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int i = b0 + u * WARP + l;
+            x[u] = 0;
+            to[u] = -1;
+            if (i >= s1) continue;
+            x[u] = pool[r.start + i];
+            const int ins = lb_event(epos, ilo, ihi, i + 1) - r.b;   // insertions before it
+            int gone = 0;
+            bool keep = true;
+            if (r.d < r.e) {
+                const int j = lb_event(epos, dlo, dhi, i);
+                gone = E[j] - before;
+                // (deletions that cancel nothing may share its position)
+                keep = j == dhi || (int)(epos[j] >> 1) != i || E[lb_event(epos, j, dhi, i + 1)] - before == gone;
+            }
+            if (keep) to[u] = i + ins - gone;
+        }
+        __syncwarp();   // a row compacted where it lies: these loads precede the stores below
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            if (to[u] >= 0) pool[r.dst + to[u]] = x[u];
+        __syncwarp();   // ... and these stores the next loads
+    }
 }
 
 // A whole row of at most 32 half-edits: a lane holds each event, no chunk is prepared.
@@ -911,13 +989,16 @@ static __device__ __forceinline__ void merge_rows(int32_t* __restrict__ pool, co
         if (it < nsl) {
             const int64_t item = m.slices[it];
             const MergeRow r = m.mrow[item >> 32];
-            const int s = (int)(item & 0xffffffffLL);
+            const int s = (int)(item & (INS_ITEM - 1));
             const bool whole = r.dst == r.start;   // compacted where it lies: one warp, front to back
             if (r.e - r.b <= WARP && (whole || r.len <= SLICE)) {
                 merge_mid(pool, keys, B, epos, r);
+            } else if (item & INS_ITEM) {
+                merge_insertions(pool, keys, B, epos, E, r, s);
             } else {
-                const int s0 = whole ? 0 : s * SLICE;
-                merge_slice(pool, keys, B, epos, E, r, s0, whole ? r.len : min(r.len, s0 + SLICE), ev);
+                const int s0 = whole ? 0 : s * SLICE, s1 = whole ? r.len : min(r.len, s0 + SLICE);
+                if (r.e - r.b > HEAVY) merge_heavy(pool, epos, E, r, s0, s1);
+                else merge_slice(pool, keys, B, epos, E, r, s0, s1, ev);
             }
         } else if (it < it_s) {
             const int i0 = (it - nsl) * per_s;
@@ -1488,6 +1569,10 @@ int ws_ensure(scout_ctx* c, int64_t m) {
     return SCOUT_OK;
 }
 
+// Merge items of a batch of m edits: the long rows' ceil(len / SLICE) sum to at most nnz / SLICE +
+// Amax, the heavy rows' ceil(insertions / HEAVY) to at most twice their half-edits / HEAVY.
+static int64_t slices_for(int64_t nnz, int64_t m, int64_t Amax) { return nnz / SLICE + Amax + 4 * m / HEAVY + 1024; }
+
 static int update_ensure(scout_ctx* c) {   // scratch of the one-launch update
     if (c->d_update) return SCOUT_OK;
     return dev_alloc(c, &c->d_update, (size_t)UPDATE_SCRATCH, "update scratch");
@@ -1498,7 +1583,7 @@ int graph_reserve_batch(scout_ctx* c, int64_t m) {
     SCOUT_RC(ws_ensure(c, m));
     SCOUT_RC(update_ensure(c));
     const int64_t Amax = std::min<int64_t>(2 * m, c->n);
-    SCOUT_RC(dev_grow(c, &c->d_slices, &c->cap_slices, c->pool_cap / SLICE + Amax + 1024, "merge slices"));
+    SCOUT_RC(dev_grow(c, &c->d_slices, &c->cap_slices, slices_for(c->pool_cap, m, Amax), "merge slices"));
     SCOUT_RC(sort_reserve(c, std::max<int64_t>(2 * c->ws_m, c->n + 1)));
     if (!c->d_coff) SCOUT_RC(dev_alloc(c, (void**)&c->d_coff, (size_t)(c->n + 1) * sizeof(int64_t), "compaction offsets"));
     // the compaction target, when the budget leaves room for a second pool
@@ -1876,8 +1961,7 @@ int graph_update(scout_ctx* c, const scout_edge* edits, const uint8_t* ops, int6
     DGraph g = dgraph(c);
     const int64_t H = 2 * m;
     const int64_t Amax = std::min<int64_t>(H, n);
-    // merge slices: the long rows' ceil(len / SLICE) sum to at most nnz / SLICE + Amax
-    SCOUT_RC(dev_grow(c, &c->d_slices, &c->cap_slices, c->nnz / SLICE + Amax + 1024, "merge slices"));
+    SCOUT_RC(dev_grow(c, &c->d_slices, &c->cap_slices, slices_for(c->nnz, m, Amax), "merge slices"));
     int32_t* E = (int32_t*)c->d_mdp;
     RowPlan rp;
     rp.row = c->row;
