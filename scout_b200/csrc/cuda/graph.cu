@@ -259,10 +259,18 @@ __device__ __forceinline__ void plan_search(const Row* __restrict__ row, const i
             if (key_op(kk, B) == 0) {
                 if (here) pos += (int)upper_bound_i32(O[s] + pos, len[s] - pos, y);
             } else {
-                int rank = 0;   // copies of this deletion before it
+                int rank = 0;   // copies of this deletion before it: doubling steps back, then a search
                 if (pk == kk) {
-                    int j = k - 1;
-                    while (j > 0 && at(j - 1) == kk) j--;
+                    int j = k - 1, step = 1;   // j is a copy, lo2 lies before the first one (or at -1)
+                    while (j - step >= 0 && at(j - step) == kk) {
+                        j -= step;
+                        step <<= 1;
+                    }
+                    int lo2 = max(j - step, -1);
+                    while (j - lo2 > 1) {
+                        const int mid = (lo2 + j) >> 1;
+                        if (at(mid) == kk) j = mid; else lo2 = mid;
+                    }
                     rank = k - j;
                 }
                 matched = here && pos + rank < len[s] && O[s][pos + rank] == y;
