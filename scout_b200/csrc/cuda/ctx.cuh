@@ -324,7 +324,7 @@ struct UpdateParams {
     uint8_t* eflag;
     uint32_t* epos;             // may share `raw`'s memory: written after the sort
     unsigned long long* split;  // UPDATE_SPLIT
-    int* bucket;                // UPDATE_SPLIT + 1 counts
+    int* bucket;                // UPDATE_BUCKETS counts
     unsigned long long* cnt;    // heads << 32 | matches per block
     int rows;                   // 0: stop after the plan (tiered store: the host decides where rows go)
     RowPlan rp;                 // its aff, seg_b, seg_d and E are written here

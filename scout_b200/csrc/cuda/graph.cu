@@ -1033,9 +1033,14 @@ __global__ void __launch_bounds__(MERGE_THREADS, 4) k_merge(
 // rows' plan; the merge. The sort is one of two:
 //   up to UPDATE_PAIRS half-edits   every key's place is the number of smaller keys: a warp per
 //                                   key against all of them in shared memory
-//   more                            sample sort: 2,048 or 4,096 keys at regular places are ranked
-//                                   that way; they split the keys into buckets (10 to 64 keys on
-//                                   average), whose keys are ranked among themselves
+//   more                            sample sort: 2,048 or 4,096 keys are ranked that way and split
+//                                   the others into buckets (10 to 64 keys on average), whose keys
+//                                   are ranked among themselves. The sample takes one key of every
+//                                   stretch at a hashed place: an edit's two half-edits lie side by
+//                                   side, and an even stride would sample one orientation alone
+//                                   (pairs written low id first, or all of one vertex, then fall into
+//                                   few buckets). Keys equal to a splitter have a bucket of their
+//                                   own and are not ranked, so a pair that is repeated costs nothing.
 //
 // What bounds it: the latency of two searches in rows, the barriers (6 to 9 of them) and the
 // merge's traffic. Up to UPDATE_MAX edits it is faster than the launches it replaces (each about
@@ -1050,10 +1055,14 @@ constexpr int UPDATE_PAIRS = 4096;
 constexpr int UPDATE_SPLIT = 4096;   // splitters; half of them up to UPDATE_FEW half-edits
 constexpr int UPDATE_FEW = 65536;
 constexpr int UPDATE_ROWS = 16384;   // more affected rows are planned by blocks, fewer by warps
-// device scratch: splitters, bucket counts, the blocks' plan counts
-constexpr int64_t UPDATE_SCRATCH = UPDATE_SPLIT * 8 + (UPDATE_SPLIT + 64) * 4 + 1024 * 8;
+constexpr int UPDATE_BUCKETS = 2 * UPDATE_SPLIT + 1;   // between the splitters, and equal to each
+// device scratch: splitters, the blocks' plan counts, bucket counts
+constexpr int64_t UPDATE_SCRATCH = UPDATE_SPLIT * 8 + 1024 * 8 + (UPDATE_BUCKETS + 63) * 4;
 
-// First index of the ascending a[0, n) whose value is above x (n <= 2^13).
+constexpr int UPDATE_SMEM = (UPDATE_BUCKETS + 1) * 4 + 8;   // the buckets' first places and the end: 32 KB and 16 bytes
+static_assert(UPDATE_SMEM % 16 == 0, "aligned");
+
+// First index of the ascending a[0, n) whose value is above x.
 template <typename T>
 __device__ __forceinline__ int first_above(const T* a, int n, T x) {
     int lo = 0, hi = n;
@@ -1064,7 +1073,7 @@ __device__ __forceinline__ int first_above(const T* a, int n, T x) {
     return lo;
 }
 
-// The half-edits p.raw[0, n) in ascending order into p.keys, all blocks; `smem`: 32 KB. Returns
+// The half-edits p.raw[0, n) in ascending order into p.keys, all blocks; `smem`: UPDATE_SMEM. Returns
 // false when a barrier failed. Ends before a barrier: the caller's next one publishes the order.
 static __device__ bool update_sort(const UpdateParams& p, int n, unsigned long long SENT, unsigned char* smem) {
     const int t = threadIdx.x, l = (int)lane_id();
@@ -1086,7 +1095,8 @@ static __device__ bool update_sort(const UpdateParams& p, int n, unsigned long l
     }
     const int S = n <= UPDATE_FEW ? UPDATE_SPLIT / 2 : UPDATE_SPLIT;   // 2,048 or 4,096
     // the sample, ranked like that
-    for (int i = t; i < S; i += UPDATE_THREADS) k[i] = ld_volatile(p.raw + (long long)i * n / S);
+    for (int i = t; i < S; i += UPDATE_THREADS)
+        k[i] = ld_volatile(p.raw + (long long)i * n / S + (((unsigned)i * 2654435761u) >> 16) % (unsigned)(n / S));
     __syncthreads();
     for (int j = wid; j < S; j += W) {
         const unsigned long long x = k[j];
@@ -1105,31 +1115,47 @@ static __device__ bool update_sort(const UpdateParams& p, int n, unsigned long l
     for (int s = 0; s < 2; s++) {
         const int i = tid + s * T;
         if (i < n) key[s] = ld_volatile(p.raw + i);
+        // bucket 2 q: between splitters q - 1 and q; 2 q + 1: equal to splitter q (to the first of equals)
+        bool eq = false;
         if (key[s] != SENT) {
-            b[s] = first_above(k, S, key[s]);
-            at[s] = atomicAdd(p.bucket + b[s], 1);
+            int q = 0, hi = S;
+            while (q < hi) {
+                const int mid = (q + hi) >> 1;
+                if (k[mid] < key[s]) q = mid + 1; else hi = mid;
+            }
+            eq = q < S && k[q] == key[s];
+            b[s] = 2 * q + (eq ? 1 : 0);
         }
+        // equal keys of a warp take their places by one atomic (a pair may be repeated all batch long)
+        const unsigned em = __ballot_sync(0xffffffffu, eq);
+        const int first = em ? __ffs(em) - 1 : 0;
+        const int b1 = __shfl_sync(0xffffffffu, b[s], first);   // (every lane takes part)
+        const bool same = eq && b[s] == b1;
+        const unsigned sm = __ballot_sync(0xffffffffu, same);
+        if (key[s] != SENT && (!same || l == first)) at[s] = atomicAdd(p.bucket + b[s], same ? __popc(sm) : 1);
+        const int base = __shfl_sync(0xffffffffu, at[s], first);
+        if (same) at[s] = base + __popc(sm & ((1u << l) - 1));
     }
     if (!grid_sync(p.bar, 66)) return false;
     int* off = (int*)smem;   // the buckets' first places, and the end
     {
-        const int per = S / UPDATE_THREADS;   // 2 or 4 buckets per thread, and the last one
-        int c[4];
+        const int per = 2 * S / UPDATE_THREADS;   // 4 or 8 buckets per thread, and the last one
+        int c[8];
         long long x = 0, y = 0, tx, ty;
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
+        for (int q = 0; q < 8; q++) {
             c[q] = q < per ? ld_volatile(p.bucket + per * t + q) : 0;
             x += c[q];
         }
         block_scan2(x, y, &tx, &ty);   // its barriers are past the splitters' last reader
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
+        for (int q = 0; q < 8; q++) {
             if (q < per) off[per * t + q] = (int)x;
             x += c[q];
         }
         if (t == 0) {
-            off[S] = (int)tx;
-            off[S + 1] = (int)tx + ld_volatile(p.bucket + S);
+            off[2 * S] = (int)tx;
+            off[2 * S + 1] = (int)tx + ld_volatile(p.bucket + 2 * S);
         }
         __syncthreads();
     }
@@ -1137,10 +1163,14 @@ static __device__ bool update_sort(const UpdateParams& p, int n, unsigned long l
     for (int s = 0; s < 2; s++)
         if (key[s] != SENT) p.tmp[off[b[s]] + at[s]] = key[s];
     if (!grid_sync(p.bar, 67)) return false;
-    const int total = off[S + 1];
+    const int total = off[2 * S + 1];
     for (int i = tid; i < total; i += T) {
         const unsigned long long x = ld_volatile(p.tmp + i);
-        const int q = first_above(off, S + 2, i) - 1;   // the bucket of place i
+        const int q = first_above(off, 2 * S + 2, i) - 1;   // the bucket of place i
+        if (q & 1) {   // equal keys: in order as they lie
+            p.keys[i] = x;
+            continue;
+        }
         const int q0 = off[q], q1 = off[q + 1];
         int c = 0;
         for (int j = q0; j < q1; j++) {
@@ -1153,8 +1183,9 @@ static __device__ bool update_sort(const UpdateParams& p, int n, unsigned long l
 }
 
 static __device__ __forceinline__ void update_body(const UpdateParams& p) {
-    __shared__ __align__(16) unsigned char s_mem[UPDATE_PAIRS * 8];   // the sort's, later the warps' chunk events
-    static_assert(sizeof(s_mem) >= UPDATE_WARPS * sizeof(ChunkEvents) && sizeof(s_mem) >= UPDATE_SPLIT * 8, "fits");
+    __shared__ __align__(16) unsigned char s_mem[UPDATE_SMEM];   // the sort's, later the warps' chunk events
+    static_assert(sizeof(s_mem) >= UPDATE_WARPS * sizeof(ChunkEvents) && sizeof(s_mem) >= UPDATE_SPLIT * 8 &&
+                  sizeof(s_mem) >= UPDATE_PAIRS * 8, "fits");
     const int t = threadIdx.x, w = t / WARP, l = (int)lane_id();
     const int G = (int)gridDim.x, T = G * UPDATE_THREADS;
     const int B = p.B;
@@ -1162,7 +1193,7 @@ static __device__ __forceinline__ void update_body(const UpdateParams& p) {
     // classification; neighbouring edits on different SMs
     const unsigned long long SENT = (B + B + 1) >= 64 ? ~0ull : ((1ull << (B + B + 1)) - 1);
     if (blockIdx.x == 0)
-        for (int i = t; i <= UPDATE_SPLIT; i += UPDATE_THREADS) p.bucket[i] = 0;
+        for (int i = t; i < UPDATE_BUCKETS; i += UPDATE_THREADS) p.bucket[i] = 0;
     for (int i0 = t * G; i0 - l * G < p.m; i0 += T) {   // uniform per warp
         const int i = i0 + (int)blockIdx.x;
         int f = 0;
