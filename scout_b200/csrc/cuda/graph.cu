@@ -1294,10 +1294,12 @@ int update_side(scout_ctx* c, const UpdateRound& r, int k) {
 constexpr int LIP_THREADS = 256;
 constexpr int LIP_U = 4;
 constexpr int LIP_CHUNK = LIP_THREADS * LIP_U;
+constexpr int LIP_TURNS = 2 * LIP_U;   // a chunk's own deletions take LIP_U + 1 turns at most, the rest are copies
 
 __global__ void __launch_bounds__(LIP_THREADS) k_merge_long_inplace(int32_t* __restrict__ pool,
                                                                     const DevCounters* __restrict__ ctr,
                                                                     const uint32_t* __restrict__ epos,
+                                                                    const int32_t* __restrict__ E,
                                                                     const int32_t* __restrict__ longs,
                                                                     const MergeRow* __restrict__ mrow) {
     __shared__ int s_warp[LIP_U][LIP_THREADS / WARP];
@@ -1316,7 +1318,8 @@ __global__ void __launch_bounds__(LIP_THREADS) k_merge_long_inplace(int32_t* __r
             if (t < LIP_CHUNK / WARP) s_gone[t] = 0;
             if (t == 0) s_next = r.e;
             __syncthreads();
-            for (bool more = true; more;) {
+            bool more = true;
+            for (int turn = 0; more && turn < LIP_TURNS; turn++) {
                 const int i = k + t;
                 const uint32_t e = i < r.e ? epos[i] : 0u;
                 const bool in = i < r.e && (int)(e >> 1) < lim;
@@ -1324,6 +1327,15 @@ __global__ void __launch_bounds__(LIP_THREADS) k_merge_long_inplace(int32_t* __r
                 if (i < r.e && !in) atomicMin(&s_next, i);
                 more = __syncthreads_and(in) != 0;
                 if (more) k += LIP_THREADS;
+            }
+            if (more) {   // many copies of some pair: every entry searches the events that are left
+                const int end = lb_event(epos, k, r.e, lim);
+                for (int rel = t; rel < LIP_CHUNK && b + rel < r.len; rel += LIP_THREADS) {
+                    const int j = lb_event(epos, k, end, b + rel), j1 = lb_event(epos, j, end, b + rel + 1);
+                    if (E[j1] != E[j]) atomicOr(&s_gone[rel >> 5], 1u << (rel & 31));
+                }
+                if (t == 0) s_next = end;
+                __syncthreads();
             }
             k = s_next;
             int32_t x[LIP_U];
@@ -2135,7 +2147,7 @@ int graph_update(scout_ctx* c, const scout_edge* edits, const uint8_t* ops, int6
     }
     if (c->tiered) {
         k_merge_long_inplace<<<(unsigned)std::min<int64_t>(std::max<int64_t>(1, Amax), 8 * (int64_t)c->sm_count),
-                               LIP_THREADS, 0, c->s_main>>>(c->pool, c->d_ctr, epos, c->d_longs, c->d_mrow);
+                               LIP_THREADS, 0, c->s_main>>>(c->pool, c->d_ctr, epos, E, c->d_longs, c->d_mrow);
         SCOUT_LAUNCH(c, "k_merge_long_inplace");
         c->nlaunch += 1;
     }
