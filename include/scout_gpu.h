@@ -78,7 +78,8 @@ typedef struct scout_sched {
     int64_t search_limit;     /* CC: a class with more deletions left to search than this is
                                  recomputed instead (0 = 32; < 0 = always search)        */
     int32_t blocks_per_sm;    /* persistent repair kernels: 256-thread quarters of the one
-                                 block per SM (1..4; 0 = all four)                       */
+                                 block per SM (1..4; 0 = all four); at most three are used
+                                 while a tiered store's gather runs beside the repair    */
     int32_t chunk_log2;       /* BFS queue item = 2^chunk_log2 row entries (8..13; 0 = 8,
                                  the best measured on a B200)                            */
     int32_t prefetched;       /* 1: this call's edits (same count, no ops) are the batch given

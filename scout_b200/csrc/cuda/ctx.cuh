@@ -371,12 +371,18 @@ int commit_gather(scout_ctx* c, int problem, const int32_t** pairs, int64_t* cou
 // repair, whose hash sets take half an SM's shared memory, runs 1,024 threads per SM instead of
 // one 256-thread block (recompute of 2 M vertices: 544 -> 339 us; 50,000-edit batch at scale 20:
 // 1,187 -> 1,016 us with its merge). The blocks_per_sm knob takes fewer 256-thread quarters.
-// Four quarters hold all of an SM's registers; while the tiered store gathers the next batch's rows
-// a repair takes three, so that the gather's blocks run beside it and not after it.
+// While the tiered store gathers the next batch's rows, a repair takes at most three, whatever the
+// knob says, so that the gather's blocks run beside it: four quarters of 64 registers a thread (BFS,
+// colouring) hold all of an SM's, and of 56 (components, MIS) leave exactly a gather block's, which
+// then started beside the components repair in some runs and after it in others. BFS, 1,000-edit batches
+// on 300,000 vertices: the gather ends 70 us after the merge beside three quarters, 118 to 127 beside
+// four. The repairs lose nothing by it where the rows lie across the host link (20,000 edits at scale
+// 20, three and four quarters: components 1,406 and 1,408 us, MIS 185 and 189; BFS 300 and 215, within
+// a call of 3.3 ms that is no shorter for it).
 constexpr int REPAIR_THREADS = 1024;
 inline int repair_threads(const scout_ctx* c) {
-    if (c->tune_blocks_per_sm > 0) return 256 * c->tune_blocks_per_sm;
-    return c->tiered && c->gather_active ? REPAIR_THREADS - 256 : REPAIR_THREADS;
+    const int quarters = c->tune_blocks_per_sm > 0 ? c->tune_blocks_per_sm : 4;
+    return 256 * (c->tiered && c->gather_active && quarters > 3 ? 3 : quarters);
 }
 // persistent launch helpers: a launch that waits on d_bar (cleared when it was used before), one
 // on a barrier of its own

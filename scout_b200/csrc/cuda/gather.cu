@@ -139,7 +139,7 @@ int prefetch_launch(scout_ctx* c, long long base) {
         c->row, (int32_t)c->n, dst, m, (long long)c->pool_cap, c->gather_stamp, (int32_t)c->gather_tag, base, room,
         c->d_gather_list, c->d_gather_dst, (GatherCtr*)c->d_gctr);
     // one block per SM: the copy is bound by the host link, and the repair's persistent kernel
-    // (one 1,024-thread block per SM) must still fit beside it to run concurrently
+    // leaves the registers of one block (repair_threads), so that both run at the same time
     k_gather_copy<<<c->sm_count, GATHER_THREADS, 0, s>>>(c->row, c->pool, c->d_gather_list, c->d_gather_dst,
                                                          (GatherCtr*)c->d_gctr);
     SCOUT_LAUNCH(c, "gather");
