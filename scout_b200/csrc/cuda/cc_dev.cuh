@@ -13,6 +13,11 @@ constexpr int CC_MAX_BOUND = 4000;
 constexpr int CC_BIG = 1024;      // rows longer than this are scanned by a whole block in P3
 constexpr int CC_ITEMS = 4;       // vertices per thread whose reads overlap in P3's passes
 constexpr int CC_GROUP = 8;       // half-edits a warp takes at a time in P1a
+constexpr int CC_LINKS = 6;       // most rounds of links between two roots in P3
+constexpr int CC_FEW_FIRST = 8;   // up to n / 8 links in the first round, n / 64 in a later one: the rest
+constexpr int CC_FEW_LINKS = 64;  // from the rows (the first joins nearly all of R-MAT's few)
+constexpr int CC_Q_LINKS = 6;     // queue counters of those rounds
+constexpr int CC_Q_FAR = 3;       // three rotating ones of the compress passes
 constexpr size_t CC_SMEM = (size_t)(2 * CC_HCAP + 3 * CC_FCAP) * sizeof(int32_t);
 
 struct CcParams {
@@ -69,6 +74,40 @@ __device__ __forceinline__ int32_t uf_union(int32_t* uf, int32_t a, int32_t b) {
         int32_t hi = a > b ? a : b, lo = a > b ? b : a;
         if (atomicCAS(uf + hi, hi, lo) == hi) return hi;
     }
+}
+
+// A thread's vertices up to their roots, side by side, at most `hops` steps each; q[u]: the parent of
+// c[u] (-1: none), then the root, or how far it came (true is returned). No root moves meanwhile, and a
+// parent that was read before it moved up is still an ancestor, so the first reads may come from L1
+// (chains are short on most graphs and end at a few roots, one L2 line each). Past CC_HOPS a chain is
+// halved on the way for all that walk it, by reads and stores that others see.
+constexpr int CC_HOPS = 8;
+__device__ __forceinline__ bool cc_chase(int32_t* vp, int32_t (&c)[CC_ITEMS], int32_t (&q)[CC_ITEMS], int hops) {
+    for (int hop = 0;; hop++) {
+        bool more = false;
+        int32_t up[CC_ITEMS];
+#pragma unroll
+        for (int u = 0; u < CC_ITEMS; u++) up[u] = q[u] < 0 ? -1 : hop < CC_HOPS ? vp[q[u]] : ld_volatile(vp + q[u]);
+#pragma unroll
+        for (int u = 0; u < CC_ITEMS; u++) more |= up[u] != q[u];
+        if (!more || hop == hops) return more;
+#pragma unroll
+        for (int u = 0; u < CC_ITEMS; u++) {
+            if (up[u] == q[u]) continue;
+            if (hop >= CC_HOPS) *(volatile int32_t*)(vp + c[u]) = up[u];
+            c[u] = q[u];
+            q[u] = up[u];
+        }
+    }
+}
+
+// Two roots (or ancestors; q -1: none) of an edge's ends: the higher one's parent is at most the lower
+// one. The word is read first, as most offers at a root come too late. Returns 1 if they differed.
+__device__ __forceinline__ int cc_link(int32_t* vp, int32_t a, int32_t q) {
+    if (q < 0 || q == a) return 0;
+    const int32_t hi = max(a, q), lo = min(a, q);
+    if (ld_volatile(vp + hi) > lo) atomicMin(vp + hi, lo);
+    return 1;
 }
 
 __device__ __forceinline__ void cc_touch(const CcParams& p, bool pred, int32_t v) {
@@ -483,15 +522,23 @@ __device__ __forceinline__ void cc_body(const CcParams& p) {
     {
         // Every vertex of a dirty class starts at its first neighbour if that has a lower id (rows are
         // sorted, so it is the lowest; no cycle can arise and no one else writes the entry, so no
-        // atomics), else at itself. Then Afforest (Sutton, Ben-Nun, Barak, IPDPS 2018): compress,
-        // link the first two neighbours that are not joined yet, compress, estimate the dominant
-        // root by sampling, then only vertices outside that root scan the rest of their rows
-        // (an edge between the dominant tree and another vertex is linked from the other
-        // vertex's row). An edge leaving a dirty class means the uploaded labels did not describe
-        // the components of the graph: it is flagged (SCOUT_E_STATE) instead of followed.
+        // atomics), else at itself (the initialisation of Jaiganesh and Burtscher's ECL-CC, HPDC 2018).
+        // Then after Afforest (Sutton, Ben-Nun, Barak, IPDPS 2018): compress, link the first two
+        // neighbours that are not joined yet, compress, estimate the dominant root by sampling,
+        // then only vertices outside that root scan the rest of their rows (an edge between the
+        // dominant tree and another vertex is linked from the other vertex's row). An edge leaving a
+        // dirty class means the uploaded labels did not describe the components of the graph: it
+        // is flagged (SCOUT_E_STATE) instead of followed.
+        // The link is an atomic minimum on the higher of two roots (Shiloach and Vishkin's hooking): of
+        // several edges at one root the lowest neighbour wins and the others wait, so it is repeated
+        // while many edges joined different roots, and what is lost at the end is linked from the rows
+        // outside the dominant root, which are then scanned from their first entry. (Unions of the
+        // edges' ends, followed to the top, all meet at a few roots: recompute of a random graph of 10^6
+        // vertices and 3 M edges 893 us, 174 so; of a shuffled grid of 10^6, 685 and 184; with both
+        // neighbours linked from the vertices themselves 529 and 442.)
         // What bounds it: chains of random reads, so a thread's CC_ITEMS vertices read side by
         // side, and after a compress most neighbours prove joined by one comparison. Recompute of
-        // 2 M vertices (32 M edges): 295 us with both neighbours linked by unions and
+        // 2 M vertices (32 M edges, R-MAT): 295 us with both neighbours linked by unions and
         // volatile reads, 100 us so. The first two entries are read once, by the start, and kept for
         // the link (cold rows of the tiered store lie across the host link: 100,000-edit batches at
         // scale 21, repair of 6.2 ms with a second read, 4.6 so).
@@ -528,57 +575,67 @@ __device__ __forceinline__ void cc_body(const CcParams& p) {
             }
         }
         if (!grid_sync(p.bar, 36)) return;
-        // Every vertex of a dirty class points at its root. No root moves meanwhile, and a parent
-        // that was read before it moved up is still an ancestor, so the reads may come from L1
-        // (all chains end at a few roots, one L2 line each).
-        auto compress = [&]() {
-            for (int64_t b = ltid; b < n; b += CC_ITEMS * T) {
-                int32_t q[CC_ITEMS], up[CC_ITEMS];
-#pragma unroll
-                for (int u = 0; u < CC_ITEMS; u++) q[u] = b + u * T < n ? p.vp[b + u * T] : -1;
-                for (bool more = true; more;) {
-                    more = false;
-#pragma unroll
-                    for (int u = 0; u < CC_ITEMS; u++) up[u] = q[u] >= 0 ? p.vp[q[u]] : -1;
+        // Every vertex of a dirty class points at its root: passes of CC_HOPS steps each, between grid
+        // barriers, until none has farther to go (a chain's steps multiply: nine times as long a
+        // one per pass). One pass on most graphs; a path of 10^6 vertices numbered in order, one
+        // chain, seven (111 ms when every vertex walked its part of it in one).
+        int pass = 0;
+        auto compress = [&](int tag) {
+            while (true) {
+                int* far = &p.ctr->q_count[CC_Q_FAR];
+                if (leader) far[(pass + 1) % 3] = 0;
+                for (int64_t b = ltid; b < n; b += CC_ITEMS * T) {
+                    int32_t c[CC_ITEMS], q[CC_ITEMS], q0[CC_ITEMS];
 #pragma unroll
                     for (int u = 0; u < CC_ITEMS; u++) {
-                        more |= up[u] != q[u];
-                        q[u] = up[u];
+                        c[u] = (int32_t)(b + u * T);
+                        q[u] = q0[u] = b + u * T < n ? p.vp[b + u * T] : -1;
                     }
-                }
+                    if (cc_chase(p.vp, c, q, CC_HOPS)) far[pass % 3] = 1;
 #pragma unroll
-                for (int u = 0; u < CC_ITEMS; u++)
-                    if (q[u] >= 0) p.vp[b + u * T] = q[u];
+                    for (int u = 0; u < CC_ITEMS; u++)
+                        if (q[u] != q0[u]) p.vp[b + u * T] = q[u];
+                }
+                if (!grid_sync(p.bar, tag)) return false;
+                if (!ld_volatile(far + pass++ % 3)) return true;
             }
         };
-        compress();
-        if (!grid_sync(p.bar, 42)) return;
-        for (int64_t b = ltid; b < n; b += CC_ITEMS * T) {
-            int32_t pv[CC_ITEMS], w0[CC_ITEMS], w1[CC_ITEMS], q0[CC_ITEMS], q1[CC_ITEMS];
+        if (!compress(42)) return;
+        int lost = 0;   // edges that may not be linked
+        for (int r = 0; r < CC_LINKS; r++) {
+            int tries = 0;
+            for (int64_t b = ltid; b < n; b += CC_ITEMS * T) {
+                int32_t pv[CC_ITEMS], w0[CC_ITEMS], w1[CC_ITEMS], q0[CC_ITEMS], q1[CC_ITEMS];
 #pragma unroll
-            for (int u = 0; u < CC_ITEMS; u++) {
-                const int64_t v = b + u * T;
-                pv[u] = v < n ? p.vp[v] : -1;   // (an ancestor is enough)
-                w0[u] = pv[u] >= 0 ? p.merged[v] : -1;   // not if joined by the start (or flagged there)
-                w1[u] = pv[u] >= 0 ? p.side[v] : -1;
-            }
+                for (int u = 0; u < CC_ITEMS; u++) {
+                    const int64_t v = b + u * T;
+                    pv[u] = v < n ? p.vp[v] : -1;
+                    w0[u] = pv[u] >= 0 ? p.merged[v] : -1;   // not if joined by the start (or flagged there)
+                    w1[u] = pv[u] >= 0 ? p.side[v] : -1;
+                }
 #pragma unroll
-            for (int u = 0; u < CC_ITEMS; u++) {
-                q0[u] = w0[u] >= 0 ? p.vp[w0[u]] : pv[u];
-                q1[u] = w1[u] >= 0 ? p.vp[w1[u]] : pv[u];
-            }
+                for (int u = 0; u < CC_ITEMS; u++) {
+                    q0[u] = w0[u] >= 0 ? p.vp[w0[u]] : pv[u];
+                    q1[u] = w1[u] >= 0 ? p.vp[w1[u]] : pv[u];
+                }
 #pragma unroll
-            for (int u = 0; u < CC_ITEMS; u++) {
-                if (pv[u] < 0) continue;
-                if (q0[u] < 0 || q1[u] < 0) atomicExch(&p.ctr->pad, 1);
-                if (q0[u] >= 0 && q0[u] != pv[u]) uf_union(p.vp, pv[u], q0[u]);
-                if (q1[u] >= 0 && q1[u] != pv[u]) uf_union(p.vp, pv[u], q1[u]);
+                for (int u = 0; u < CC_ITEMS; u++) {
+                    if (pv[u] < 0) continue;
+                    if (q0[u] < 0 || q1[u] < 0) atomicExch(&p.ctr->pad, 1);
+                    tries += cc_link(p.vp, pv[u], q0[u]);
+                    tries += cc_link(p.vp, pv[u], q1[u]);
+                }
             }
+            __syncwarp();
+            tries = __reduce_add_sync(0xffffffffu, tries);
+            if (lane_id() == 0 && tries) atomicAdd(&p.ctr->q_count[CC_Q_LINKS + r], tries);
+            if (!grid_sync(p.bar, 43)) return;
+            if (!compress(44)) return;
+            if (tid == 0) bytes += 24LL * n;
+            lost = ld_volatile(&p.ctr->q_count[CC_Q_LINKS + r]);
+            if (lost <= n / (r == 0 ? CC_FEW_FIRST : CC_FEW_LINKS)) break;
         }
-        if (!grid_sync(p.bar, 43)) return;
-        compress();
-        if (tid == 0) bytes += 24LL * n;
-        if (!grid_sync(p.bar, 44)) return;
+        const int scan0 = lost ? 0 : AF_FIRST;
         if (blockIdx.x == 0) {   // mode of the roots of up to 1024 sampled dirty vertices
             __shared__ int32_t s_key[2048];
             __shared__ int s_cnt[2048];
@@ -615,8 +672,17 @@ __device__ __forceinline__ void cc_body(const CcParams& p) {
             if (v < n) {
                 int32_t pv = ld_volatile(p.vp + v);
                 if (pv >= 0 && pv != gr) {
-                    int len = p.g.row[v].len;
-                    if (len > AF_FIRST) { bg = len > CC_BIG; sm_ = !bg; }
+                    const Row r = p.g.row[v];
+                    if (r.len > AF_FIRST) {
+                        bg = r.len > CC_BIG;
+                        sm_ = !bg;
+                    } else {
+                        for (int k = scan0; k < r.len; k++) {   // a short row's own links, where some are lost
+                            const int32_t q = ld_volatile(p.vp + p.g.pool[r.start + k]);
+                            if (q < 0) atomicExch(&p.ctr->pad, 1);
+                            else if (q != pv) uf_union(p.vp, pv, q);
+                        }
+                    }
                 }
             }
             int a = warp_append(sm_, &p.ctr->q_count[1]);
@@ -632,7 +698,7 @@ __device__ __forceinline__ void cc_body(const CcParams& p) {
             Row r = p.g.row[v];
             const int32_t* rw = p.g.pool + r.start;
             const int32_t pv = ld_volatile(p.vp + v);
-            for (int b0 = AF_FIRST; b0 < r.len; b0 += CC_ITEMS * WARP) {
+            for (int b0 = scan0; b0 < r.len; b0 += CC_ITEMS * WARP) {
                 int32_t w[CC_ITEMS], q[CC_ITEMS];
 #pragma unroll
                 for (int u = 0; u < CC_ITEMS; u++) {
@@ -654,7 +720,7 @@ __device__ __forceinline__ void cc_body(const CcParams& p) {
             Row r = p.g.row[v];
             const int32_t* rw = p.g.pool + r.start;
             const int32_t pv = ld_volatile(p.vp + v);
-            for (long long k = AF_FIRST + threadIdx.x; k < r.len; k += blockDim.x) {
+            for (long long k = scan0 + threadIdx.x; k < r.len; k += blockDim.x) {
                 const int32_t q = ld_volatile(p.vp + rw[k]);
                 if (q < 0) atomicExch(&p.ctr->pad, 1);
                 else if (q != pv) uf_union(p.vp, pv, q);
@@ -665,23 +731,15 @@ __device__ __forceinline__ void cc_body(const CcParams& p) {
     if (!grid_sync(p.bar, 37)) return;
     // the labels: every root is the minimum of its class (no union runs any more)
     for (int64_t b = ltid - (ltid & (WARP - 1)); b < n; b += CC_ITEMS * T) {
-        int32_t q[CC_ITEMS], up[CC_ITEMS], lab[CC_ITEMS];
+        int32_t c[CC_ITEMS], q[CC_ITEMS], lab[CC_ITEMS];
 #pragma unroll
         for (int u = 0; u < CC_ITEMS; u++) {
             const int64_t v = b + u * T + lane_id();
+            c[u] = (int32_t)v;
             q[u] = v < n ? p.vp[v] : -1;
             lab[u] = v < n ? p.label[v] : -1;
         }
-        for (bool more = true; more;) {
-            more = false;
-#pragma unroll
-            for (int u = 0; u < CC_ITEMS; u++) up[u] = q[u] >= 0 ? p.vp[q[u]] : -1;
-#pragma unroll
-            for (int u = 0; u < CC_ITEMS; u++) {
-                more |= up[u] != q[u];
-                q[u] = up[u];
-            }
-        }
+        cc_chase(p.vp, c, q, INT32_MAX);
 #pragma unroll
         for (int u = 0; u < CC_ITEMS; u++) {
             const int64_t v = b + u * T + lane_id();
