@@ -14,20 +14,23 @@
 // The number of rounds is the longest chain of vertices each waiting on a lower-id neighbour
 // (about 900 on an R-MAT graph of 500,000 vertices, edge factor 16).
 //
-// A greedy MIS decides an open vertex as soon as any lower neighbour joins, so its chains are short
-// (6 to 13 rounds on R-MAT graphs of 2,000 to 2 M vertices and on random graphs): k_seed_rounds
-// looks at every open vertex again in each of up to SEED_ROUNDS rounds. Waiting in lists, below,
-// hears of a joined neighbour only when the one waited for decides: 35 to 233 rounds there, and
-// 1.7 to 2.3 times the time (whole call, R-MAT of edge factor 16, by rounds and by lists: 8,000
-// vertices 249 and 424 us; 100,000: 447 and 917; 2 M: 2,180 and 4,950). What is still open after
-// SEED_ROUNDS rounds lies on long chains (a path or a grid numbered in order), and the lists finish
-// it, being the faster there (grid of 700 x 700: 9.2 ms by lists, 17.4 by rounds, 9.7 by both).
+// Both rules begin with rounds that look at every open vertex (k_seed_rounds). That settles graphs of
+// short chains alone: a greedy MIS decides a vertex as soon as any lower neighbour joins (6 to 13
+// rounds on R-MAT graphs of 2,000 to 2 M vertices and on random graphs, where waiting in lists takes
+// 35 to 233, as a waiter hears of a joined neighbour only when the one it waits for decides), and so
+// are a colouring's chains on shuffled grids or with a few hubs. What is open after SEED_ROUNDS rounds
+// (a colouring: after SEED_FIRST, once a round leaves more than 7/8 open; its prefixes of more than
+// SEED_BIG entries at once) is finished by waiter lists. Whole calls, lists alone and so: MIS,
+// R-MAT of edge factor 16, 8,000 vertices 424 and 249 us, 100,000 917 and 447, 2 M 4,950 and 2,180;
+// grid of 700 x 700 numbered in order 9.2 and 9.7 ms (17.4 by rounds alone); colouring, the same grid
+// shuffled 637 and 181 us, 300,000 vertices on 60 hubs 1,383 and 227, R-MAT of 500,000 11.4 and
+// 11.1 ms.
 //
-// The lists (k_seed_greedy; colourings from the start). What bounds it: the latency of a round (a
-// few hundred open vertices decide in each), so a round only touches vertices that can move. An open vertex waits on ONE undecided neighbour,
-// the highest-id one (it tends to decide last, so few waits follow one another), in that
-// neighbour's list of waiters; a vertex that decides closes its list and queues the waiters for
-// the next round. The list of w holds at most as many waiters as w has higher-id neighbours; a
+// The lists (k_seed_greedy). What bounds it: the latency of a round (a few hundred open vertices
+// decide in each), so a round only touches vertices that can move. An open vertex waits on ONE
+// undecided neighbour, the highest-id one (it tends to decide last, so few waits follow one
+// another), in that neighbour's list of waiters; a vertex that decides closes its list and queues
+// the waiters for the next round. The list of w holds at most as many waiters as w has higher-id neighbours; a
 // vertex that finds it full (rows that are not symmetric, or no memory for the lists) is queued
 // again itself and simply looks again next round. One grid barrier per round.
 // Greedy colouring of 500,009 vertices (edge factor 16): 1,073 ms with every open vertex
@@ -44,6 +47,7 @@ namespace scout {
 constexpr int SEED_THREADS = 1024;
 constexpr int32_t UNDECIDED = -1;
 constexpr int SEED_ROUNDS = 32;             // MIS rounds before the lists take over
+constexpr int SEED_FIRST = 12;              // colouring rounds whatever they decide
 constexpr int SEED_BIG = 1024;              // longer prefixes are scanned by a whole block
 constexpr int SEED_WORDS = 32;              // bitmap window: 1024 colours
 constexpr int SEED_CLOSED = 0x40000000;     // a closed waiter list's count
@@ -63,8 +67,8 @@ struct SeedParams {
     GridBar* bar;
 };
 
-// Rounds of the MIS rule over all open vertices, one thread each, until none is open or SEED_ROUNDS
-// are done. ctr->affected: the vertices left open.
+// Rounds over all open vertices, one thread each, until none is open, SEED_ROUNDS are done or
+// (colouring) a round has left more than 7/8 of them open. ctr->affected: the vertices left open.
 __global__ void __launch_bounds__(SEED_THREADS, 1) k_seed_rounds(SeedParams p) {
     const int64_t n = p.g.n;
     const int64_t tid = lthread_id();
@@ -72,9 +76,9 @@ __global__ void __launch_bounds__(SEED_THREADS, 1) k_seed_rounds(SeedParams p) {
     const bool leader = blockIdx.x == 0 && threadIdx.x == 0;
     for (int64_t v = tid; v < n; v += T) p.out[v] = UNDECIDED;
     if (!grid_sync(p.bar, 50)) return;
-    int cur = 2, rounds = 0, cnt = (int)n;
+    int cur = 2, rounds = 0, cnt = (int)n, before = INT32_MAX;
     long long bytes = 0;
-    while (cnt > 0 && rounds < SEED_ROUNDS) {
+    while (cnt > 0 && rounds < SEED_ROUNDS && (p.mode == 0 || rounds < SEED_FIRST || cnt <= before - before / 8)) {
         const int nxt = (cur + 1) % 3, zer = (cur + 2) % 3;
         const int32_t* wl = p.wl[rounds & 1];
         int32_t* wn = p.wl[(rounds & 1) ^ 1];
@@ -90,14 +94,31 @@ __global__ void __launch_bounds__(SEED_THREADS, 1) k_seed_rounds(SeedParams p) {
                 const int k = (int)lower_bound_i32(row, r.len, v);
                 bytes += 16 + 4LL * k * 2;
                 bool any_in = false, all_done = true;
-                for (int j = 0; j < k && !any_in; j++) {
-                    const int32_t s = ld_volatile(p.out + row[j]);
-                    any_in = s == 1;
-                    all_done &= s != UNDECIDED;
+                if (p.mode == 0) {
+                    for (int j = 0; j < k && !any_in; j++) {
+                        const int32_t s = ld_volatile(p.out + row[j]);
+                        any_in = s == 1;
+                        all_done &= s != UNDECIDED;
+                    }
+                    open = !any_in && !all_done;
+                    if (!open) p.out[v] = any_in ? 0 : 1;
+                } else {
+                    if (k > SEED_BIG) all_done = false;   // left to the lists' blocks
+                    for (int j = 0; j < k && all_done; j++) all_done = ld_volatile(p.out + row[j]) != UNDECIDED;
+                    open = !all_done;
+                    if (!open) {
+                        int32_t colour = 0;
+                        for (int32_t base = 0;; base += 64) {   // smallest colour absent below
+                            unsigned long long used = 0;
+                            for (int j = 0; j < k; j++) {
+                                const int32_t c = ld_volatile(p.out + row[j]) - base;
+                                if (c >= 0 && c < 64) used |= 1ull << c;
+                            }
+                            if (~used) { colour = base + __ffsll((long long)~used) - 1; break; }
+                        }
+                        p.out[v] = colour;
+                    }
                 }
-                if (any_in) p.out[v] = 0;
-                else if (all_done) p.out[v] = 1;
-                else open = true;
             }
             const int at = warp_append(open, &p.ctr->list_count[nxt]);
             if (open) wn[at] = v;
@@ -105,6 +126,7 @@ __global__ void __launch_bounds__(SEED_THREADS, 1) k_seed_rounds(SeedParams p) {
         rounds++;
         if (!grid_sync(p.bar, 51)) return;
         cur = nxt;
+        before = cnt;
         cnt = ld_volatile(&p.ctr->list_count[cur]);
     }
 #pragma unroll
@@ -116,19 +138,17 @@ __global__ void __launch_bounds__(SEED_THREADS, 1) k_seed_rounds(SeedParams p) {
     }
 }
 
-// Per vertex: the row prefix of neighbours below it, the slots its waiter list gets. `fresh`: no vertex
-// is decided yet; else the decided ones keep their value and their list is closed.
-__global__ void k_seed_prep(DGraph g, int32_t* __restrict__ out, int32_t* __restrict__ pre, int32_t* __restrict__ open,
-                            int32_t* __restrict__ nwait, int64_t* __restrict__ slots, bool fresh) {
+// Per vertex: the row prefix of neighbours below it, the slots its waiter list gets. The list of a vertex
+// that the rounds have decided is closed.
+__global__ void k_seed_prep(DGraph g, const int32_t* __restrict__ out, int32_t* __restrict__ pre,
+                            int32_t* __restrict__ open, int32_t* __restrict__ nwait, int64_t* __restrict__ slots) {
     for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < g.n; v += (int64_t)gridDim.x * blockDim.x) {
         const Row r = g.row[v];
         const int32_t* row = g.pool + r.start;
         const int k = (int)lower_bound_i32(row, r.len, (int32_t)v);
-        const bool decided = !fresh && out[v] != UNDECIDED;
         pre[v] = k;
         open[v] = k;
-        nwait[v] = decided ? SEED_CLOSED : 0;
-        if (fresh) out[v] = UNDECIDED;
+        nwait[v] = out[v] != UNDECIDED ? SEED_CLOSED : 0;
         slots[v] = r.len - k;   // a loop's own entry only adds a slot
     }
 }
@@ -401,15 +421,15 @@ __global__ void __launch_bounds__(SEED_THREADS, 1) k_seed_greedy(SeedParams p) {
     if (leader) p.ctr->rounds += rounds;
 }
 
-// The lists' scratch and kernel, and the counters. `fresh`: no vertex is decided yet.
-static int seed_lists(scout_ctx* c, SeedParams p, bool fresh) {
+// The lists' scratch and kernel, and the counters.
+static int seed_lists(scout_ctx* c, SeedParams p) {
     const int64_t n = c->n;
     if (!c->d_coff) SCOUT_RC(dev_alloc(c, (void**)&c->d_coff, (size_t)(n + 1) * sizeof(int64_t), "compaction offsets"));
     p.pre = (int32_t*)c->d_qbuf[0];    // the work queues are free outside a repair (qcap >= n items)
     p.open = (int32_t*)c->d_qbuf[1];
     p.nwait = (int32_t*)c->d_qbuf[2];
     p.off = c->d_coff;
-    k_seed_prep<<<blocks_for(n, 256), 256, 0, c->s_main>>>(p.g, p.out, p.pre, p.open, p.nwait, c->d_coff, fresh);
+    k_seed_prep<<<blocks_for(n, 256), 256, 0, c->s_main>>>(p.g, p.out, p.pre, p.open, p.nwait, c->d_coff);
     SCOUT_LAUNCH(c, "k_seed_prep");
     SCOUT_RC(scan_i64(c, c->d_coff, n, c->d_coff + n));
     // the waiter lists hold at most nnz slots in all: the compaction spare's memory (its contents
@@ -479,16 +499,14 @@ int scout_seed(scout_ctx* c, int problem, int32_t source, scout_batch_stats* st)
     p.off = nullptr;
     c->last_problem = problem;
     SCOUT_CU(c, cudaEventRecord(c->ev_t[1], c->s_main));
-    bool open = true;
-    if (p.mode == 0) {
-        void* args[] = {&p};
-        SCOUT_RC(coop_launch(c, (const void*)k_seed_rounds, SEED_THREADS, args, 0));
-        SCOUT_CU(c, cudaEventRecord(c->ev_t[2], c->s_main));
-        SCOUT_RC(counters_fetch(c));
-        open = c->h_ctr->affected > 0;
-        if (open) SCOUT_CU(c, cudaMemsetAsync(c->d_ctr->list_count, 0, sizeof(c->d_ctr->list_count), c->s_main));
+    void* args[] = {&p};
+    SCOUT_RC(coop_launch(c, (const void*)k_seed_rounds, SEED_THREADS, args, 0));
+    SCOUT_CU(c, cudaEventRecord(c->ev_t[2], c->s_main));
+    SCOUT_RC(counters_fetch(c));
+    if (c->h_ctr->affected > 0) {
+        SCOUT_CU(c, cudaMemsetAsync(c->d_ctr->list_count, 0, sizeof(c->d_ctr->list_count), c->s_main));
+        SCOUT_RC(seed_lists(c, p));
     }
-    if (open) SCOUT_RC(seed_lists(c, p, problem != SCOUT_MIS));
     float ms = 0.f;
     cudaEventElapsedTime(&ms, c->ev_t[1], c->ev_t[2]);
     st->ms_repair = ms;
