@@ -580,8 +580,33 @@ __device__ __forceinline__ void bfs_body(const BfsParams& p) {
                 }
                 return d;
             };
+            // a candidate without a valid parent in its first chunk (the warp, all lanes)
+            auto invalidate = [&](int32_t c, const Row& r, int lc) {
+                if (r.len > p.chunk) {
+                    push_rest(p, c, (r.len + p.chunk - 1) >> p.chunk_log2, rest);
+                    return;
+                }
+                if (l == 0) {
+                    p.st_inval[c] = p.epoch;
+                    int at = atomicAdd(&p.ctr->list_count[0], 1);
+                    p.inval[at] = c;
+                }
+                __syncwarp();
+                push_children(p, p.g.pool + r.start, r.len, lc, nxt, tag, bytes);
+                if (l == 0) bytes += 24;
+            };
+            // No more candidates than warps: a cascade that is bound by the latency of its rounds, one
+            // candidate per warp and its whole chunk at once (eight entries first, and turns handed
+            // out, made the rounds of a narrow cascade a fifth longer).
+            if (per == 1 && wid < cnt) {
+                const int32_t c = (int32_t)p.q[cur % 3][wid];
+                const Cand d = load_cand(c);
+                if (c != p.source && d.lc > 0 && d.si != p.epoch &&
+                    !parent_among(p, p.g.pool + d.r.start, min(p.chunk, d.r.len), d.lc, bytes))
+                    invalidate(c, d.r, d.lc);
+            }
             // the first two turns of every warp are fixed, the rest handed out (rows take unequal time)
-            long long i = (long long)wid * per, i_n = i + (long long)W * per;
+            long long i = per == 1 ? cnt : (long long)wid * per, i_n = i + (long long)W * per;
             int32_t it_n = load_item(i);
             Cand cd_n = load_cand(it_n);
             int32_t it_nn = load_item(i_n);
@@ -664,19 +689,8 @@ __device__ __forceinline__ void bfs_body(const BfsParams& p) {
                     Row r;
                     r.start = __shfl_sync(0xffffffffu, cd.r.start, u);
                     r.len = __shfl_sync(0xffffffffu, cd.r.len, u);
-                    const int lc = __shfl_sync(0xffffffffu, cd.lc, u);
-                    if (r.len > p.chunk) {
-                        push_rest(p, c, (r.len + p.chunk - 1) >> p.chunk_log2, rest);
-                        continue;
-                    }
-                    if (lane_id() == 0) {
-                        p.st_inval[c] = p.epoch;
-                        int at = atomicAdd(&p.ctr->list_count[0], 1);
-                        p.inval[at] = c;
-                    }
-                    __syncwarp();
-                    push_children(p, p.g.pool + r.start, r.len, lc, nxt, tag, bytes);
-                    if (lane_id() == 0) bytes += 24;
+                    r.cap = 0;
+                    invalidate(c, r, __shfl_sync(0xffffffffu, cd.lc, u));
                 }
             }
             if (!grid_sync(p.bar, 3)) return;
