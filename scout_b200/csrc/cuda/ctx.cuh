@@ -300,6 +300,7 @@ struct RowPlan {
     const int32_t* seg_b;
     const int32_t* seg_d;
     const int32_t* E;
+    const uint32_t* epos;
     MergeRow* mrow;        // short rows of one half-edit from the front, the others from the back
     int64_t mcap;
     int32_t* shorts;       // records of the other short rows

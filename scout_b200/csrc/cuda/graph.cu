@@ -39,9 +39,10 @@ namespace scout {
 constexpr int SLICE = 2048;          // old-row entries merged by one warp at a time
 constexpr int SMALL_LEN = 128;       // rows up to this length (and 32 half-edits) are short
 constexpr int IN_PLACE_LEN = 4096;   // longest deletion-only row compacted in place by one warp
-constexpr int HEAVY = 1024;          // rows of more half-edits: no warp walks them (merge_heavy), and as many
-                                     // insertions are a merge item of their own
-constexpr int64_t INS_ITEM = 1ll << 31;   // marks such an item in the slice list
+constexpr int HEAVY = 1024;          // half-edits from which a row may be heavy (heavy_row), and the insertions
+                                     // of one merge item of such a row
+constexpr int64_t INS_ITEM = 1ll << 31;     // in the slice list: such an item,
+constexpr int64_t HEAVY_ITEM = 1ll << 30;   // a slice of a heavy row
 
 // A row whose half-edits are all deletions is rewritten in place: its survivors only move
 // towards the row start, it keeps its start and capacity, and it takes no pool space (one warp
@@ -461,6 +462,19 @@ __global__ void __launch_bounds__(ROW_THREADS) k_row_sizes(RowPlan p) {
     if (lane_id() == 0 && nc) atomicAdd((unsigned long long*)&p.ctr->new_elems_host, (unsigned long long)nc);
 }
 
+// Rows whose events crowd: more than twice as many as old entries, or HEAVY in a row (of insertions, or
+// of deletions) within HEAVY / 2 entries. A warp walks a slice's events 32 at a time, which is the
+// faster where they are spread (64 streams of small graphs under batches of up to a quarter of
+// their entries: updates of all their batches 11.8 ms, 13.2 when every row of more than HEAVY half-edits
+// was searched).
+__device__ __forceinline__ bool heavy_row(const uint32_t* epos, int len, int b, int d, int e) {
+    if (e - b <= HEAVY) return false;
+    bool crowd = (long long)(e - b) > 2LL * len;
+    for (int k = b; !crowd && k + HEAVY < d; k += HEAVY) crowd = (epos[k + HEAVY] >> 1) - (epos[k] >> 1) < HEAVY / 2;
+    for (int k = d; !crowd && k + HEAVY < e; k += HEAVY) crowd = (epos[k + HEAVY] >> 1) - (epos[k] >> 1) < HEAVY / 2;
+    return crowd;
+}
+
 // BLOCK: rows are taken a block's threads at a time, with one set of atomics on the counters;
 // else 32 at a time by a warp, with no barrier (few rows, nothing to save on atomics).
 template <bool BLOCK>
@@ -475,7 +489,7 @@ __device__ __forceinline__ void row_plan(const RowPlan& p, int A, int group, int
         Row r{0, 0, 0};
         int32_t u = 0;
         int b = 0, d = 0, e = 0, nl = 0, ns = 0, ni = 0;   // ns old slices, ni insertion items
-        bool ip = false, cold = false, one = false, sm = false, lip = false;
+        bool ip = false, cold = false, one = false, sm = false, lip = false, heavy = false;
         if (ok) {
             u = p.aff[a];
             b = p.seg_b[a];
@@ -489,7 +503,8 @@ __device__ __forceinline__ void row_plan(const RowPlan& p, int A, int group, int
             one = r.len <= SMALL_LEN && e - b == 1;
             sm = !one && r.len <= SMALL_LEN && e - b <= WARP;
             ns = one || sm || lip ? 0 : ip ? 1 : max(1, (r.len + SLICE - 1) / SLICE);
-            if (e - b > HEAVY) ni = (d - b + HEAVY - 1) / HEAVY;
+            heavy = ns > 0 && heavy_row(p.epos, r.len, b, d, e);
+            if (heavy) ni = (d - b + HEAVY - 1) / HEAVY;
             nnz_delta += nl - r.len;
             bytes += 4LL * ((long long)r.len + nl) + 8LL * (e - b) + 16;
         }
@@ -546,7 +561,7 @@ __device__ __forceinline__ void row_plan(const RowPlan& p, int A, int group, int
             if (s0 + ns + ni > p.slice_cap) {
                 if (ns + ni) atomicExch(&p.ctr->overflow, 1);
             } else {
-                for (int s = 0; s < ns; s++) p.slices[s0 + s] = (at << 32) | s;
+                for (int s = 0; s < ns; s++) p.slices[s0 + s] = (at << 32) | (heavy ? HEAVY_ITEM : 0) | s;
                 for (int s = 0; s < ni; s++) p.slices[s0 + ns + s] = (at << 32) | INS_ITEM | s;
             }
         }
@@ -739,13 +754,12 @@ __device__ __forceinline__ int lb_event(const uint32_t* __restrict__ epos, int l
     return lo;
 }
 
-// Rows of more than HEAVY half-edits. Their events may all lie in one gap of a short row (a vertex
-// that gains its neighbours in one batch) or repeat one pair, so nothing walks them: insertions
-// are items of HEAVY of them, each placed by a lane (merge_insertions), and old entries [s0, s1)
-// find their own shift by searching the slice's events (merge_heavy). A warp that walked them took
-// a turn per 32 events, on one word of its chunk: update of 10^6 edits at one vertex of three
-// neighbours, on 2^20 vertices, 101.8 ms; so 0.46 (random pairs: 0.51). Up to HEAVY events the walk
-// is at most 32 turns, and reads far less than the two searches of every old entry.
+// Heavy rows. Their events may all lie in one gap of a short row (a vertex that gains its neighbours in
+// one batch) or repeat one pair, so nothing walks them: insertions are items of HEAVY of them, each
+// placed by a lane (merge_insertions), and old entries [s0, s1) find their own shift by searching the
+// slice's events (merge_heavy). A warp that walked them took a turn per 32 events, on one word of its
+// chunk: update of 10^6 edits at one vertex of three neighbours, on 2^20 vertices, 101.8 ms; so 0.46
+// (random pairs: 0.51).
 static __device__ __forceinline__ void merge_insertions(int32_t* __restrict__ pool,
                                                         const unsigned long long* __restrict__ keys, int B,
                                                         const uint32_t* __restrict__ epos, const int32_t* __restrict__ E,
@@ -997,7 +1011,7 @@ static __device__ __forceinline__ void merge_rows(int32_t* __restrict__ pool, co
         if (it < nsl) {
             const int64_t item = m.slices[it];
             const MergeRow r = m.mrow[item >> 32];
-            const int s = (int)(item & (INS_ITEM - 1));
+            const int s = (int)(item & (HEAVY_ITEM - 1));
             const bool whole = r.dst == r.start;   // compacted where it lies: one warp, front to back
             if (r.e - r.b <= WARP && (whole || r.len <= SLICE)) {
                 merge_mid(pool, keys, B, epos, r);
@@ -1005,7 +1019,7 @@ static __device__ __forceinline__ void merge_rows(int32_t* __restrict__ pool, co
                 merge_insertions(pool, keys, B, epos, E, r, s);
             } else {
                 const int s0 = whole ? 0 : s * SLICE, s1 = whole ? r.len : min(r.len, s0 + SLICE);
-                if (r.e - r.b > HEAVY) merge_heavy(pool, epos, E, r, s0, s1);
+                if (item & HEAVY_ITEM) merge_heavy(pool, epos, E, r, s0, s1);
                 else merge_slice(pool, keys, B, epos, E, r, s0, s1, ev);
             }
         } else if (it < it_s) {
@@ -1140,13 +1154,12 @@ static __device__ bool update_sort(const UpdateParams& p, int n, unsigned long l
     int* off = (int*)smem;   // the buckets' first places, and the end
     {
         const int per = 2 * S / UPDATE_THREADS;   // 4 or 8 buckets per thread, and the last one
-        int c[8];
+        const int4* mine = (const int4*)(p.bucket + per * t);   // (from L2: other blocks counted them)
+        const int4 ca = __ldcg(mine), cb = per == 8 ? __ldcg(mine + 1) : make_int4(0, 0, 0, 0);
+        const int c[8] = {ca.x, ca.y, ca.z, ca.w, cb.x, cb.y, cb.z, cb.w};
         long long x = 0, y = 0, tx, ty;
 #pragma unroll
-        for (int q = 0; q < 8; q++) {
-            c[q] = q < per ? ld_volatile(p.bucket + per * t + q) : 0;
-            x += c[q];
-        }
+        for (int q = 0; q < 8; q++) x += c[q];
         block_scan2(x, y, &tx, &ty);   // its barriers are past the splitters' last reader
 #pragma unroll
         for (int q = 0; q < 8; q++) {
@@ -1192,8 +1205,8 @@ static __device__ __forceinline__ void update_body(const UpdateParams& p) {
     DevCounters* ctr = p.rp.ctr;
     // classification; neighbouring edits on different SMs
     const unsigned long long SENT = (B + B + 1) >= 64 ? ~0ull : ((1ull << (B + B + 1)) - 1);
-    if (blockIdx.x == 0)
-        for (int i = t; i < UPDATE_BUCKETS; i += UPDATE_THREADS) p.bucket[i] = 0;
+    if (2 * p.m > UPDATE_PAIRS)
+        for (int i = (int)blockIdx.x * UPDATE_THREADS + t; i < UPDATE_BUCKETS; i += T) p.bucket[i] = 0;
     for (int i0 = t * G; i0 - l * G < p.m; i0 += T) {   // uniform per warp
         const int i = i0 + (int)blockIdx.x;
         int f = 0;
@@ -2035,6 +2048,7 @@ int graph_update(scout_ctx* c, const scout_edge* edits, const uint8_t* ops, int6
     c->batch_dest = c->tiered ? 2 : 0;
     unsigned long long* sorted = c->d_keys;
     uint32_t* epos = (uint32_t*)c->d_keys_alt;
+    rp.epos = epos;
     const int64_t sms = later ? c->sm_count / SIDE_MAX : c->sm_count;
     const bool one = m <= UPDATE_MAX && H <= 2 * sms * UPDATE_THREADS;
     if (one) {
@@ -2074,6 +2088,7 @@ int graph_update(scout_ctx* c, const scout_edge* edits, const uint8_t* ops, int6
         c->nlaunch += 1;
         SCOUT_RC(sort_keys(c, c->d_keys, c->d_keys_alt, 2 * m, 2 * B + 1, &sorted));
         epos = (uint32_t*)(sorted == c->d_keys ? c->d_keys_alt : c->d_keys);   // the free ping-pong half
+        rp.epos = epos;
         const int64_t tiles = (H + PLAN_TILE - 1) / PLAN_TILE;
         SCOUT_RC(dev_grow(c, &c->d_scan_tmp, &c->cap_scan, std::max<int64_t>(64, 1 + 3 * tiles), "scan look-back"));
         k_plan<<<(unsigned)tiles, PLAN_THREADS, 0, c->s_main>>>(c->row, c->pool, sorted, B, c->d_ctr, c->d_aff, c->d_seg_b,
