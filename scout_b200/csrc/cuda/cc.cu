@@ -16,8 +16,8 @@
 //   P2  split sides take their minimum id as label; when a side holds the class minimum, the
 //       remainder gets its own minimum. With several splits in a class the remainder must be
 //       shown connected first (endpoint searches); otherwise the class is marked dirty
-//   P3  dirty classes are recomputed exactly (Afforest-style: link the first two neighbours,
-//       compress, sample the dominant root, union the rest of the rows of the others)
+//   P3  dirty classes are recomputed exactly (start at the lowest neighbour, compress, hook the
+//       first two neighbours' roots, sample the dominant root, union the rows of the others)
 // A full recompute (scout_recompute_cc) is P3 with every class dirty. One cooperative launch,
 // phases separated by the bounded grid barrier.
 #include "ctx.cuh"

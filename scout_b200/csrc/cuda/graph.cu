@@ -24,7 +24,8 @@
 //                     the list of short rows or of slices of longer ones
 //   k_merge           the new rows: survivors and insertions of short rows (a few rows per warp)
 //                     and of slices of SLICE old entries (a warp each, so a hub row is spread
-//                     over many warps), positions taken from the sorted edit events
+//                     over many warps), positions taken from the sorted edit events; rows whose
+//                     events crowd have their insertions placed by items of their own
 //   k_merge_long_inplace  tiered store: rows longer than IN_PLACE_LEN that only lose entries
 #include "ctx.cuh"
 
@@ -2102,7 +2103,7 @@ int graph_update(scout_ctx* c, const scout_edge* edits, const uint8_t* ops, int6
     if (c->tiered) {
         // the exact growth, before anything is written. HBM part too large: compact (evicting
         // short rows to the host pool); larger than three quarters of the HBM pool: the whole
-        // batch goes to the host pool. Host pool full: compacted in place on the host.
+        // batch goes to the host pool. Host pool full: compacted (host_compact, by the device).
         long long grow[2] = {0, 0};   // HBM, host
         auto read_grow = [&](bool again) -> int {
             if (again) SCOUT_CU(c, cudaMemsetAsync(&c->d_ctr->new_elems, 0, 16, c->s_main));
