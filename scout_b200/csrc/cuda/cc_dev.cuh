@@ -437,15 +437,25 @@ __device__ __forceinline__ void cc_body(const CcParams& p) {
         }
         if (!grid_sync(p.bar, 40)) return;
         while (true) {
-            if (threadIdx.x == 0) s_task = atomicAdd(&p.ctr->q_count[0], 1);
+            // One thread decides for the block: another block may mark the class dirty meanwhile, and
+            // threads that read the mark on both sides of that would part ways before a barrier.
+            if (threadIdx.x == 0) {
+                int i = atomicAdd(&p.ctr->q_count[0], 1);
+                if (i < nrec) {
+                    const int32_t cls = (int32_t)(p.rec[3 * i] >> 32), f = ld_volatile(p.firstw + cls);
+                    if (ld_volatile(p.cnt + cls) < 2 || ld_volatile(p.dirty + cls) == p.epoch || f < 0 ||
+                        (int32_t)p.rec[3 * i + 2] == f)
+                        i = -1;
+                }
+                s_task = i;
+            }
             __syncthreads();
             const int i = s_task;
             __syncthreads();
             if (i >= nrec) break;
-            int32_t cls = (int32_t)(p.rec[3 * i] >> 32);
-            if (ld_volatile(p.cnt + cls) < 2 || ld_volatile(p.dirty + cls) == p.epoch) continue;
-            int32_t w = (int32_t)p.rec[3 * i + 2], f = ld_volatile(p.firstw + cls);
-            if (w == f || f < 0) continue;
+            if (i < 0) continue;
+            const int32_t cls = (int32_t)(p.rec[3 * i] >> 32);
+            const int32_t w = (int32_t)p.rec[3 * i + 2], f = ld_volatile(p.firstw + cls);
             int res = cc_search(p, w, f, cls, bytes, false, true);
             if (threadIdx.x == 0 && res != 0 && atomicExch(p.dirty + cls, p.epoch) != p.epoch)
                 atomicAdd(&p.ctr->recomputes, 1);
