@@ -23,8 +23,8 @@
 // SEED_BIG entries at once) is finished by waiter lists. Whole calls, lists alone and so: MIS,
 // R-MAT of edge factor 16, 8,000 vertices 424 and 249 us, 100,000 917 and 447, 2 M 4,950 and 2,180;
 // grid of 700 x 700 numbered in order 9.2 and 9.7 ms (17.4 by rounds alone); colouring, the same grid
-// shuffled 637 and 181 us, 300,000 vertices on 60 hubs 1,383 and 227, R-MAT of 500,000 11.4 and
-// 11.1 ms.
+// shuffled 644 and 187 us, 300,000 vertices on 60 hubs 1,850 and 286, R-MAT of 500,000 11.1 and
+// 11.2 ms.
 //
 // The lists (k_seed_greedy). What bounds it: the latency of a round (a few hundred open vertices
 // decide in each), so a round only touches vertices that can move. An open vertex waits on ONE
@@ -47,7 +47,8 @@ namespace scout {
 constexpr int SEED_THREADS = 1024;
 constexpr int32_t UNDECIDED = -1;
 constexpr int SEED_ROUNDS = 32;             // MIS rounds before the lists take over
-constexpr int SEED_FIRST = 12;              // colouring rounds whatever they decide
+constexpr int SEED_FIRST = 7;               // colouring rounds whatever they decide
+constexpr int SEED_ASK = 16384;             // vertices from which a colouring's rounds are waited for
 constexpr int SEED_BIG = 1024;              // longer prefixes are scanned by a whole block
 constexpr int SEED_WORDS = 32;              // bitmap window: 1024 colours
 constexpr int SEED_CLOSED = 0x40000000;     // a closed waiter list's count
@@ -501,9 +502,16 @@ int scout_seed(scout_ctx* c, int problem, int32_t source, scout_batch_stats* st)
     SCOUT_CU(c, cudaEventRecord(c->ev_t[1], c->s_main));
     void* args[] = {&p};
     SCOUT_RC(coop_launch(c, (const void*)k_seed_rounds, SEED_THREADS, args, 0));
-    SCOUT_CU(c, cudaEventRecord(c->ev_t[2], c->s_main));
-    SCOUT_RC(counters_fetch(c));
-    if (c->h_ctr->affected > 0) {
+    // Whether vertices are open is read back before the lists are prepared, a wait of 20 us; on a small
+    // graph the lists of a colouring, which nearly always needs them, follow without it (with
+    // nothing open they take about as long there).
+    bool lists = true;
+    if (p.mode == 0 || c->n >= SEED_ASK) {
+        SCOUT_CU(c, cudaEventRecord(c->ev_t[2], c->s_main));
+        SCOUT_RC(counters_fetch(c));
+        lists = c->h_ctr->affected > 0;
+    }
+    if (lists) {
         SCOUT_CU(c, cudaMemsetAsync(c->d_ctr->list_count, 0, sizeof(c->d_ctr->list_count), c->s_main));
         SCOUT_RC(seed_lists(c, p));
     }
