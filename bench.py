@@ -471,7 +471,7 @@ def scout_arm(a, dist):
         "e2e": {"value": edits_all / e2e_s if e2e_s else None, "unit": "edge-updates/s",
                 "h2d_bytes_per_step": int(h2d / max(n_steps, 1)), "d2h_bytes_per_step": int(d2h / max(n_steps, 1))},
         "roofline": {"bound": "hbm", "kernel": f"k_{kp}", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                     "frac": achieved / peak, "peak_kind": peak_kind, "traffic": profiled_traffic(f"k_{kp}", a.scale),
+                     "frac": achieved / peak, "peak_kind": peak_kind, "traffic": profiled_traffic(f"k_{kp}/148x1024", a.scale),
                      "algorithmic_bytes_per_launch": b / max(nl, 1), "ms_per_launch": ms / max(nl, 1),
                      "launches": nl},
         "roofline_merge": {"kernels": "k_update, or k_classify .. k_merge (batch merge)",
